@@ -20,6 +20,7 @@
 #include "elementwise.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_tc2.cuh"
+#include "gemm_pair.cuh"
 #include "int8.cuh"
 #include "sampling.cuh"
 #include "matmul.cuh"
@@ -632,7 +633,7 @@ struct SplitHandoff {
 // C = A[M,K] (row stride lda) . Wt[N,K]^T on the tensor cores; x3 selects 3 x TF32.
 static int32_t launch_gemm_tc(wgpt_device *dev, bool x3, const float *A, size_t lda, const float *Wt, int M, int K,
                               int N, const Epilogue &epi, LnAfter *ln = nullptr, bool b_static = true,
-                              const float *Wt_lo = nullptr, SplitHandoff *handoff = nullptr, bool b_exact = false) {
+                              SplitHandoff *handoff = nullptr, bool b_exact = false) {
   REQUIRE(aligned16(A) && aligned16(Wt) && (lda % 4) == 0 && (K % 4) == 0, WGPT_ERR_ALIGN,
           "tensor-core GEMM operands must be 16-byte aligned with row strides that are multiples of 16 bytes");
   CUtensorMap ma, mb;
@@ -676,50 +677,42 @@ static int32_t launch_gemm_tc(wgpt_device *dev, bool x3, const float *A, size_t 
   const CUtensorMap &m_first = exchanged ? mb : ma, &m_second = exchanged ? ma : mb;
   const int km = exchanged ? N : M, kn = exchanged ? M : N;
   const int static_op = b_static ? (exchanged ? 2 : 1) : 0;
-  // Compute-bound 3xTF32 products read the weight's precomputed low part (x - tf32(x), same layout) by TMA
-  // instead of deriving it in shared memory; skinny products are HBM-bound on the weights and keep deriving it.
-  const bool lo_tma = x3 && Wt_lo != nullptr && !exchanged && b_static;
-  CUtensorMap mlo = mb;
-  if (lo_tma) TRY(make_tile_map(&mlo, Wt_lo, (uint64_t)N, (uint64_t)K, (uint64_t)K));
-  // Large 3xTF32 products without split-K and without a precomputed low part of the weight (the per-operator
-  // entry points) run on the CTA-pair kernel (256 x 256 tile per two SMs) when its tiles fill the pairs evenly
-  // enough. Measured back to back: 8192x768x2304 226-232 against 171-182 TFLOP/s; with 96 tiles on 74 pairs it is
-  // no faster than the 128 x 128 tiles, in plain TF32 it is slower (302 against 330-360), and inside the model's
-  // prefill the one-CTA kernel with the low part fetched by TMA measured the same or better (10.9 against 11.1 ms),
-  // so the model path keeps that. WGPT_PAIR_GEMM=0 turns the pair kernel off, 2 uses it wherever it fits.
+  // Large 3xTF32 products without split-K (the per-operator entry points) run on the CTA-pair kernel (256 x 256 tile
+  // per two SMs) when its tiles fill the pairs evenly enough. Measured back to back: 8192x768x2304 226-232 against
+  // 171-182 TFLOP/s; with 96 tiles on 74 pairs it is no faster than the 128 x 128 tiles, in plain TF32 it is slower
+  // (302 against 330-360). WGPT_PAIR_GEMM=0 turns the pair kernel off, 2 uses it wherever it fits.
   static const int pair_mode = [] { const char *ev = getenv("WGPT_PAIR_GEMM"); return ev ? atoi(ev) : 1; }();
   const int work2 = ((M + 255) / 256) * ((N + TC2_BN - 1) / TC2_BN);
   int pairs = dev->sm_count / 2;
   const int rounds2 = (work2 + pairs - 1) / pairs;
   const bool pair_fits = work2 * 5 >= rounds2 * pairs * 4;  // at least 80 % of the pair slots do useful work
-  if (pair_mode > 0 && ((x3 && !lo_tma) || pair_mode == 2) && split_out == nullptr && !exchanged && M >= 512 &&
+  if (pair_mode > 0 && (x3 || pair_mode == 2) && split_out == nullptr && !exchanged && M >= 512 &&
       N >= 256 && pair_fits) {
     if (pairs > work2) pairs = work2;
     dim3 grid2(2 * pairs);
     if (x3) {
       auto kern = gemm_tc2_kernel<true>;
       CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcPlan<true>::kSmemBytes));
-      LAUNCH_PDL(dev, kern, grid2, TcPlan<true>::kThreads, TcPlan<true>::kSmemBytes, ma, mb, mlo, M, K, N, epi,
-                 dev->d_err, lo_tma ? 1 : 0);
+      LAUNCH_PDL(dev, kern, grid2, TcPlan<true>::kThreads, TcPlan<true>::kSmemBytes, ma, mb, M, K, N, epi,
+                 dev->d_err);
     } else {
       auto kern = gemm_tc2_kernel<false>;
       CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcPlan<false>::kSmemBytes));
-      LAUNCH_PDL(dev, kern, grid2, TcPlan<false>::kThreads, TcPlan<false>::kSmemBytes, ma, mb, mlo, M, K, N, epi,
-                 dev->d_err, 0);
+      LAUNCH_PDL(dev, kern, grid2, TcPlan<false>::kThreads, TcPlan<false>::kSmemBytes, ma, mb, M, K, N, epi,
+                 dev->d_err);
     }
     return WGPT_OK;
   }
   if (x3) {
     auto kern = gemm_tc_kernel<true>;
     CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcPlan<true>::kSmemBytes));
-    LAUNCH_PDL(dev, kern, grid, TcPlan<true>::kThreads, TcPlan<true>::kSmemBytes, m_first, m_second, mlo, km, K, kn,
-               epi, dev->d_err, kb_per_split, splits, split_out, static_op, exchanged ? 1 : 0,
-               lo_tma ? 1 : (b_exact && !exchanged ? 2 : 0));
+    LAUNCH_PDL(dev, kern, grid, TcPlan<true>::kThreads, TcPlan<true>::kSmemBytes, m_first, m_second, km, K, kn, epi,
+               dev->d_err, kb_per_split, splits, split_out, static_op, exchanged ? 1 : 0, b_exact && !exchanged ? 1 : 0);
   } else {
     auto kern = gemm_tc_kernel<false>;
     CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcPlan<false>::kSmemBytes));
-    LAUNCH_PDL(dev, kern, grid, TcPlan<false>::kThreads, TcPlan<false>::kSmemBytes, m_first, m_second, mlo, km, K, kn,
-               epi, dev->d_err, kb_per_split, splits, split_out, static_op, exchanged ? 1 : 0, 0);
+    LAUNCH_PDL(dev, kern, grid, TcPlan<false>::kThreads, TcPlan<false>::kSmemBytes, m_first, m_second, km, K, kn, epi,
+               dev->d_err, kb_per_split, splits, split_out, static_op, exchanged ? 1 : 0, 0);
   }
   if (split_out != nullptr && handoff != nullptr && exchanged) {
     handoff->part = split_out;
@@ -742,16 +735,72 @@ static int32_t launch_gemm_tc(wgpt_device *dev, bool x3, const float *A, size_t 
 
 // Matrix product for more than 8 rows against a weight stored [N,K]: tensor cores or CUDA cores per dev->precision.
 static int32_t launch_gemm_nk(wgpt_device *dev, const float *A, size_t lda, const float *Wt, int M, int K, int N,
-                              const Epilogue &epi, LnAfter *ln = nullptr, const float *Wt_lo = nullptr,
-                              SplitHandoff *handoff = nullptr) {
+                              const Epilogue &epi, LnAfter *ln = nullptr, SplitHandoff *handoff = nullptr) {
   if (dev->precision == WGPT_PRECISION_FP32) return launch_gemm_simt(dev, true, A, lda, Wt, M, K, N, epi);
-  return launch_gemm_tc(dev, dev->precision == WGPT_PRECISION_TF32X3, A, lda, Wt, M, K, N, epi, ln, true, Wt_lo,
-                        handoff);
+  return launch_gemm_tc(dev, dev->precision == WGPT_PRECISION_TF32X3, A, lda, Wt, M, K, N, epi, ln, true, handoff);
 }
 
+// Rows of up to 2048 values stay in registers (V float4 per lane, see layernorm_kernel).
 static int32_t launch_layernorm(wgpt_device *dev, const float *in, size_t ld_in, const float *gamma, const float *beta,
-                                float *out, size_t ld_out, int rows, int N) {
-  LAUNCH_PDL(dev, layernorm_kernel, (rows + 3) / 4, 128, 0, in, ld_in, gamma, beta, out, ld_out, rows, N);
+                                float *out, size_t ld_out, int rows, int N, __half *planes = nullptr, size_t plane = 0,
+                                float scale = 1.f) {
+  const int grid = (rows + 3) / 4;
+#define LN_CASE(V) \
+  LAUNCH_PDL(dev, layernorm_kernel<V>, grid, 128, 0, in, ld_in, gamma, beta, out, ld_out, rows, N, planes, plane, scale)
+  if (N <= 128 * 3) LN_CASE(3);
+  else if (N <= 128 * 6) LN_CASE(6);
+  else if (N <= 128 * 13) LN_CASE(13);
+  else if (N <= 128 * 16) LN_CASE(16);
+  else LN_CASE(0);
+#undef LN_CASE
+  return WGPT_OK;
+}
+
+// ---- products of pair operands (pair.cuh) ----
+// Tensor map of both planes of a pair matrix [2][rows][K]: boxes of {64 halves, box_rows, 2}, 128-byte swizzle, zero
+// fill outside. K % 8 == 0 (16-byte row and plane strides).
+static int32_t make_pair_map(CUtensorMap *map, const __half *planes, uint64_t rows, uint64_t K, int box_rows) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  REQUIRE(fn != nullptr, WGPT_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t dims[3] = {K, rows, 2};
+  cuuint64_t strides[2] = {K * 2, rows * K * 2};
+  cuuint32_t box[3] = {(cuuint32_t)GP_BK, (cuuint32_t)box_rows, 2};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half *>(planes), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  REQUIRE(r == CUDA_SUCCESS, WGPT_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+  return WGPT_OK;
+}
+
+// Tile width of gemm_pair_kernel: the multiple of 32 whose rounds over the pairs cost least, a tile costing
+// max(tensor pipe, shared memory) cycles per k-block (gemm_pair.cuh).
+static int pair_tile_columns(const wgpt_device *dev, int M, int N) {
+  const int pairs = dev->sm_count / 2, m_tiles = (M + 255) / 256;
+  int best = 256;
+  long long best_cost = -1;
+  for (int bn = 256; bn >= 64; bn -= 32) {
+    const long long rounds = ((long long)m_tiles * ((N + bn - 1) / bn) + pairs - 1) / pairs;
+    const long long cost = rounds * (6 * bn > 640 + 5 * bn / 2 ? 6 * bn : 640 + 5 * bn / 2);
+    if (best_cost < 0 || cost < best_cost) { best = bn; best_cost = cost; }
+  }
+  return best;
+}
+
+// C = A . Wt^T from pair planes A [2][M][K] and W [2][N][K]; the exponents are in epi.colscale / epi.rowscale.
+static int32_t launch_gemm_pair(wgpt_device *dev, const __half *A, const __half *W, int M, int K, int N,
+                                const Epilogue &epi, bool b_exact = false) {
+  REQUIRE(aligned16(A) && aligned16(W) && K % 8 == 0, WGPT_ERR_ALIGN, "pair operands need 16-byte aligned rows");
+  const int bn = pair_tile_columns(dev, M, N);
+  CUtensorMap ma, mb;
+  TRY(make_pair_map(&ma, A, (uint64_t)M, (uint64_t)K, GP_BM));
+  TRY(make_pair_map(&mb, W, (uint64_t)N, (uint64_t)K, bn / 2));
+  const int work = ((M + 255) / 256) * ((N + bn - 1) / bn);
+  int pairs = dev->sm_count / 2;
+  if (pairs > work) pairs = work;
+  CK(cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM_BYTES));
+  LAUNCH_PDL(dev, gemm_pair_kernel, 2 * pairs, GP_THREADS, GP_SMEM_BYTES, ma, mb, M, K, N, bn, b_exact ? 1 : 0, epi,
+             dev->d_err);
   return WGPT_OK;
 }
 
@@ -838,21 +887,26 @@ static int32_t launch_attn_prefill_t(wgpt_device *dev, const float *q, int ldq, 
   return WGPT_OK;
 }
 
+static bool attn_prefill_uses_mma(const wgpt_device *dev, int hs, int n_tok) {
+  static const bool mma64 = [] { const char *ev = getenv("WGPT_ATTN_PREFILL_MMA"); return !(ev && ev[0] == '0'); }();
+  return hs == 64 && mma64 && dev->precision != WGPT_PRECISION_FP32 && n_tok >= 16;
+}
+
+// planes: the output as a pair (only where attn_prefill_uses_mma; the other kernels write FP32 to out).
 static int32_t launch_attn_prefill(wgpt_device *dev, int hs, const float *q, int ldq, const float *kc, const float *vc,
                                    int ldkv, size_t kv_seq_stride, float *out, int ldo, int n_tok, int n_seq, int H,
-                                   const int *pos, float scale) {
+                                   const int *pos, float scale, __half *planes = nullptr, size_t plane = 0,
+                                   float pair_scale = 1.f) {
   static const bool tiled64 = [] { const char *ev = getenv("WGPT_ATTN_PREFILL64"); return !(ev && ev[0] == '0'); }();
-  static const bool mma64 = [] { const char *ev = getenv("WGPT_ATTN_PREFILL_MMA"); return !(ev && ev[0] == '0'); }();
-  if (hs == 64 && mma64 && dev->precision != WGPT_PRECISION_FP32 && n_tok >= 16 && (ldq % 4) == 0 && (ldkv % 4) == 0 &&
-      (ldo % 2) == 0) {
+  if (attn_prefill_uses_mma(dev, hs, n_tok) && (ldq % 4) == 0 && (ldkv % 4) == 0 && (ldo % 2) == 0) {
     // products in TF32 / 3xTF32: the warp-level tensor-core kernel; FP32 mode keeps the CUDA-core kernels below
     dim3 grid((n_tok + 63) / 64, H, n_seq);
     if (dev->precision == WGPT_PRECISION_TF32X3)
       LAUNCH(dev, attn_prefill64_mma_kernel<true>, grid, 128, 0, q, ldq, kc, vc, ldkv, kv_seq_stride, out, ldo, n_tok, pos,
-             scale);
+             scale, planes, plane, pair_scale);
     else
       LAUNCH(dev, attn_prefill64_mma_kernel<false>, grid, 128, 0, q, ldq, kc, vc, ldkv, kv_seq_stride, out, ldo, n_tok,
-             pos, scale);
+             pos, scale, planes, plane, pair_scale);
     return WGPT_OK;
   }
   if (hs == 64 && tiled64 && n_tok >= 16 && (ldq % 4) == 0 && (ldkv % 4) == 0 && (ldo % 4) == 0) {
@@ -1136,7 +1190,7 @@ WGPT_EXPORT int32_t wgpt_int8_matmul(wgpt_device *dev, int32_t M, int32_t K, int
       // the expanded weight was written by the kernel just before: no reads of it ahead of the dependency wait
       // the expanded codes are integers: exact in TF32, no low part
       return launch_gemm_tc(dev, dev->precision == WGPT_PRECISION_TF32X3, A, (size_t)K, wt, M, K, N, e, nullptr, false,
-                            nullptr, nullptr, true);
+                            nullptr, true);
     }
     dim3 grid((N + 63) / 64, (M + 63) / 64);
     LAUNCH(dev, int8_gemm_simt_kernel, grid, 256, 0, A, Bq, M, K, N, e);
@@ -1260,16 +1314,25 @@ WGPT_EXPORT int32_t wgpt_int8_matmul_w(wgpt_device *dev, int32_t M, const wgpt_i
     Epilogue e = plain_epi(out, N, nullptr);
     e.colscale = w->scale;
     return launch_gemm_tc(dev, dev->precision == WGPT_PRECISION_TF32X3, A, (size_t)K, wt, M, K, N, e, nullptr, false,
-                          nullptr, nullptr, true);
+                          nullptr, true);
   }
   return wgpt_int8_matmul(dev, M, K, N, A, w->words, w->scale, out);
 }
 
 // ------------------------------------------------------------------------------------------ model
+// A weight [N,K] as pair planes [2][N][K]; cs[n] = descale of its row n times the descale of the product's input.
+struct PairWeight {
+  __half *p = nullptr;
+  float *cs = nullptr;
+};
+
 struct LayerWeights {
   float *ln1_g, *ln1_b, *wqkv_t, *bqkv, *wo_t, *bo, *ln2_g, *ln2_b, *wfc_t, *bfc, *wpr_t, *bpr;
-  // low parts of the four matrices for 3xTF32 (w - tf32(w), same [N,K] layout), filled by wgpt_model_finalize
-  float *wqkv_lo = nullptr, *wo_lo = nullptr, *wfc_lo = nullptr, *wpr_lo = nullptr;
+  // the four matrices as pairs of half-precision planes, filled by wgpt_model_finalize when the model takes them, and
+  // the powers of two that their input rows (both LayerNorm outputs, attention output, GELU output) are scaled by
+  PairWeight wqkv_p, wo_p, wfc_p, wpr_p;
+  float s_h1 = 1.f, s_o = 1.f, s_h2 = 1.f, s_f = 1.f;
+  float s_qk = 1.f;  // the attention's queries and keys
   // single-sequence fused decode (decode_fused.cuh): per-(head, cluster rank) blocks of the attention weights and
   // the MLP down-projection in the [K,N] orientation, filled by wgpt_model_finalize when the plan applies
   float *attn_blk = nullptr, *wpr_kn = nullptr;
@@ -1298,6 +1361,9 @@ struct wgpt_model {
   bool finalized;
   std::vector<void *> allocs;
   FusedPlan fused;
+  bool pair_ok = false;  // products of many rows run on half-precision pairs in 3xTF32 mode (pair_prepare)
+  PairWeight wte_p;
+  float s_hf = 1.f;
 };
 
 static int32_t model_alloc(wgpt_model *m, float **p, size_t floats) {
@@ -1568,24 +1634,111 @@ static int32_t fused_plan(wgpt_model *m) {
   return WGPT_OK;
 }
 
+// Lays the matrices out as pairs and derives the scale of each product's input. The inputs need no run-time maxima: a
+// LayerNorm's z has a 2-norm of at most sqrt(E), so its output y = gamma z + beta is bounded element by element, every
+// product of it by (max|gamma| sqrt(E) + |beta|_2) |w_n|_2 + |b_n| (Cauchy-Schwarz), the attention output by its values
+// (a convex combination) and gelu(x) by |x|. A bound is typically 2^3..2^5 above what occurs, against the 2^16 that the
+// format keeps below FP32's own rounding (pair.cuh); a model whose bounds are more than 2^13 above the typical magnitude
+// (or not finite) stays on 3xTF32, as does one whose n_embd is not a multiple of 8 (TMA strides).
+static int32_t pair_prepare(wgpt_model *m) {
+  wgpt_device *dev = m->dev;
+  const int E = m->p.n_embd, F = 4 * E, V = m->p.vocab_size;
+  m->pair_ok = false;
+  if (E % 8 != 0) return WGPT_OK;
+  const double loosest = 8192.0;
+  std::vector<float> norm, cs, g(E), b(E), bias;
+  TRY(scratch_reserve(dev, (size_t)(V > F ? V : F) * 4));
+  float *d_norm = static_cast<float *>(dev->scratch);
+  auto split = [&](PairWeight &w, const float *src, int N, int K) -> int32_t {  // planes, row descales and row norms
+    if (w.p == nullptr) {
+      float *p = nullptr;
+      TRY(model_alloc(m, &p, (size_t)N * K));
+      w.p = reinterpret_cast<__half *>(p);
+      TRY(model_alloc(m, &w.cs, N));
+    }
+    LAUNCH_PDL(dev, pair_rows_kernel, (N + 7) / 8, 256, 0, src, (size_t)K, N, K, w.p, w.cs, d_norm);
+    norm.resize(N);
+    cs.resize(N);
+    CK(cudaMemcpyAsync(norm.data(), d_norm, (size_t)N * 4, cudaMemcpyDeviceToHost, dev->stream));
+    CK(cudaMemcpyAsync(cs.data(), w.cs, (size_t)N * 4, cudaMemcpyDeviceToHost, dev->stream));
+    CK(cudaStreamSynchronize(dev->stream));
+    return WGPT_OK;
+  };
+  auto rescale = [&](PairWeight &w, float in_scale) -> int32_t {  // the input's descale joins the row descales
+    for (float &c : cs) c /= in_scale;
+    CK(cudaMemcpyAsync(w.cs, cs.data(), cs.size() * 4, cudaMemcpyHostToDevice, dev->stream));
+    CK(cudaStreamSynchronize(dev->stream));
+    return WGPT_OK;
+  };
+  bool ok = true;
+  double in_bound = 0, in_norm = 0, in_rms = 0;  // of the LayerNorm output at hand: largest element, 2-norm, typical element
+  auto layernorm_bound = [&](const float *gamma, const float *beta) -> int32_t {
+    CK(cudaMemcpyAsync(g.data(), gamma, (size_t)E * 4, cudaMemcpyDeviceToHost, dev->stream));
+    CK(cudaMemcpyAsync(b.data(), beta, (size_t)E * 4, cudaMemcpyDeviceToHost, dev->stream));
+    CK(cudaStreamSynchronize(dev->stream));
+    double gmax = 0, b2 = 0, sq = 0;
+    in_bound = 0;
+    for (int i = 0; i < E; i++) {
+      const double ga = std::fabs((double)g[i]), ba = std::fabs((double)b[i]);
+      in_bound = std::fmax(in_bound, 1.01 * (ga * std::sqrt((double)E) + ba));
+      gmax = std::fmax(gmax, ga);
+      b2 += ba * ba;
+      sq += ga * ga + ba * ba;
+    }
+    in_norm = gmax * std::sqrt((double)E) + std::sqrt(b2);
+    in_rms = std::sqrt(sq / E);
+    ok = ok && std::isfinite(sq) && in_bound <= loosest * in_rms;
+    return WGPT_OK;
+  };
+  // bound of outputs [n0, n1) of the product whose row norms are in `norm` (loose when far above their typical size)
+  auto output_bound = [&](const float *d_bias, int n0, int n1) -> float {
+    bias.resize(n1);
+    if (cudaMemcpyAsync(bias.data(), d_bias, (size_t)n1 * 4, cudaMemcpyDeviceToHost, dev->stream) != cudaSuccess ||
+        cudaStreamSynchronize(dev->stream) != cudaSuccess) {
+      ok = false;
+      return 1.f;
+    }
+    double top = 0, sq = 0;
+    for (int n = n0; n < n1; n++) {
+      const double bn = std::fabs((double)bias[n]), wn = norm[n];
+      if (!std::isfinite(bn) || !std::isfinite(wn)) ok = false;
+      top = std::fmax(top, 1.01 * (in_norm * wn + bn));
+      sq += in_rms * wn * in_rms * wn + bn * bn;
+    }
+    if (top > loosest * std::sqrt(sq / (n1 - n0))) ok = false;
+    return (float)top;
+  };
+  for (auto &L : m->layers) {
+    TRY(layernorm_bound(L.ln1_g, L.ln1_b));
+    L.s_h1 = pair_scale_for((float)in_bound);
+    TRY(split(L.wqkv_p, L.wqkv_t, 3 * E, E));
+    L.s_qk = pair_scale_for(output_bound(L.bqkv, 0, 2 * E));
+    L.s_o = pair_scale_for(output_bound(L.bqkv, 2 * E, 3 * E));
+    TRY(rescale(L.wqkv_p, L.s_h1));
+    TRY(split(L.wo_p, L.wo_t, E, E));
+    TRY(rescale(L.wo_p, L.s_o));
+    TRY(layernorm_bound(L.ln2_g, L.ln2_b));
+    L.s_h2 = pair_scale_for((float)in_bound);
+    TRY(split(L.wfc_p, L.wfc_t, F, E));
+    L.s_f = pair_scale_for(output_bound(L.bfc, 0, F));
+    TRY(rescale(L.wfc_p, L.s_h2));
+    TRY(split(L.wpr_p, L.wpr_t, E, F));
+    TRY(rescale(L.wpr_p, L.s_f));
+  }
+  TRY(layernorm_bound(m->lnf_g, m->lnf_b));
+  m->s_hf = pair_scale_for((float)in_bound);
+  TRY(split(m->wte_p, m->wte, V, E));
+  TRY(rescale(m->wte_p, m->s_hf));
+  m->pair_ok = ok;
+  return WGPT_OK;
+}
+
 WGPT_EXPORT int32_t wgpt_model_finalize(wgpt_model *m) {
   REQUIRE(m != nullptr, WGPT_ERR_ARG, "model handle is null");
   for (size_t i = 0; i < m->have.size(); i++)
     REQUIRE(m->have[i], WGPT_ERR_STATE, "tensor slot %zu was never set (4 + 12*layer + index)", i);
   TRY(use(m->dev));
-  {
-    const size_t E = m->p.n_embd, F = 4 * E;
-    for (auto &L : m->layers) {
-      struct { const float *src; float **dst; size_t n; } jobs[4] = {
-          {L.wqkv_t, &L.wqkv_lo, 3 * E * E}, {L.wo_t, &L.wo_lo, E * E}, {L.wfc_t, &L.wfc_lo, F * E}, {L.wpr_t, &L.wpr_lo, E * F}};
-      for (auto &j : jobs) {
-        if (*j.dst == nullptr) TRY(model_alloc(m, j.dst, j.n));
-        size_t n4 = j.n / 4;
-        LAUNCH(m->dev, tf32_lo_kernel, grid_for(n4, 256, m->dev->sm_count), 256, 0,
-               reinterpret_cast<const float4 *>(j.src), reinterpret_cast<float4 *>(*j.dst), n4);
-      }
-    }
-  }
+  TRY(pair_prepare(m));
   TRY(fused_plan(m));
   if (m->fused.ok) {
     const int E = m->p.n_embd, F = 4 * E, H = m->p.n_head;
@@ -1816,6 +1969,62 @@ static int32_t forward_blocks_fused(wgpt_session *s, const uint32_t *ids) {
   return WGPT_OK;
 }
 
+// The transformer blocks of a pass of many rows on pairs (pair.cuh): both LayerNorms, the attention and the MLP
+// up-projection write the pair form that the product after them reads. s->h, s->o and s->f hold planes here (the same
+// bytes as the FP32 rows).
+constexpr int kPairMinRows = 300;
+static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
+  wgpt_model *m = s->m;
+  wgpt_device *dev = m->dev;
+  const wgpt_params &p = m->p;
+  const int E = p.n_embd, F = 4 * E, H = p.n_head, hs = m->hs, M = s->n_seq * n_tok;
+  const size_t kv_layer = (size_t)s->n_seq * p.n_ctx * E, plane_e = (size_t)M * E, plane_f = (size_t)M * F;
+  __half *h = reinterpret_cast<__half *>(s->h), *o = reinterpret_cast<__half *>(s->o), *f = reinterpret_cast<__half *>(s->f);
+  const bool o_pair = n_tok > 1 && attn_prefill_uses_mma(dev, hs, n_tok);
+  for (int l = 0; l < p.n_layer; l++) {
+    const LayerWeights &L = m->layers[l];
+    float *kc = s->kc + (size_t)l * kv_layer, *vc = s->vc + (size_t)l * kv_layer;
+    TRY(launch_layernorm(dev, s->x, (size_t)E, L.ln1_g, L.ln1_b, nullptr, (size_t)E, M, E, h, plane_e, L.s_h1));
+    Epilogue e = plain_epi(s->q, E, L.bqkv);
+    e.colscale = L.wqkv_p.cs;
+    e.kc = kc; e.vc = vc; e.E = E; e.n_tok = n_tok; e.n_ctx = p.n_ctx; e.pos = s->d_pos;
+    TRY(launch_gemm_pair(dev, h, L.wqkv_p.p, M, E, 3 * E, e));
+    if (n_tok == 1) {
+      TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, s->n_seq, H, s->n_split, s->d_pos,
+                             m->scale, s->attn_part));
+      if (s->n_split > 1) {
+        AttnPartials ap;
+        ap.part = s->attn_part; ap.n_split = s->n_split; ap.H = H; ap.hs = hs;
+        LAUNCH_PDL(dev, attn_merge_kernel, dim3((E / 4 + 127) / 128, M), 128, 0, ap, s->o, E);
+      }
+    } else {
+      TRY(launch_attn_prefill(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, n_tok, s->n_seq, H, s->d_pos,
+                              m->scale, o_pair ? o : nullptr, plane_e, L.s_o));
+    }
+    const __half *o_in = o;
+    if (!o_pair) {  // an attention kernel that writes FP32 rows
+      LAUNCH_PDL(dev, pair_convert_kernel, grid_for(plane_e / 4, 256, dev->sm_count), 256, 0, (const float *)s->o,
+                 plane_e, L.s_o, h);
+      o_in = h;
+    }
+    e = plain_epi(s->x, E, L.bo);
+    e.colscale = L.wo_p.cs;
+    e.residual = s->x;
+    TRY(launch_gemm_pair(dev, o_in, L.wo_p.p, M, E, E, e));
+    TRY(launch_layernorm(dev, s->x, (size_t)E, L.ln2_g, L.ln2_b, nullptr, (size_t)E, M, E, h, plane_e, L.s_h2));
+    e = plain_epi(nullptr, F, L.bfc);
+    e.colscale = L.wfc_p.cs;
+    e.act = 1;
+    e.pair = f; e.pair_plane = plane_f; e.pair_scale = L.s_f;
+    TRY(launch_gemm_pair(dev, h, L.wfc_p.p, M, E, F, e));
+    e = plain_epi(s->x, E, L.bpr);
+    e.colscale = L.wpr_p.cs;
+    e.residual = s->x;
+    TRY(launch_gemm_pair(dev, f, L.wpr_p.p, M, F, E, e));
+  }
+  return WGPT_OK;
+}
+
 // With pick, the greedy choice of every sequence is also made (next_ids, out_ids) and the position advanced.
 static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pick = false) {
   wgpt_model *m = s->m;
@@ -1832,8 +2041,7 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
   // s->h already holds the LayerNorm of s->x that the next product wants (left there by the split-K second
   // stage of the product that wrote s->x)
   bool h_ready = false;
-  auto mm = [&](const float *a, const float *gamma, const float *beta, const float *Wt, const float *Wt_lo, int K,
-                int N, const Epilogue &e, const float *next_gamma = nullptr, const float *next_beta = nullptr,
+  auto mm = [&](const float *a, const float *gamma, const float *beta, const float *Wt, int K, int N, const Epilogue &e, const float *next_gamma = nullptr, const float *next_beta = nullptr,
                 SplitHandoff *handoff = nullptr) -> int32_t {
     // a: [M,K] contiguous. Small M: weight-streaming GEMV with the LayerNorm fused in; otherwise a LayerNorm pass
     // into s->h (separate, or riding on the previous product's second stage) and a tiled GEMM. next_gamma/beta:
@@ -1858,13 +2066,15 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
     LnAfter ln = {next_gamma, next_beta, s->h, false};
     // the product must not read s->h itself while its second stage rewrites it
     bool can_fuse = next_gamma != nullptr && src != s->h;
-    TRY(launch_gemm_nk(dev, src, (size_t)K, Wt, M, K, N, e, can_fuse ? &ln : nullptr, Wt_lo, handoff));
+    TRY(launch_gemm_nk(dev, src, (size_t)K, Wt, M, K, N, e, can_fuse ? &ln : nullptr, handoff));
     h_ready = ln.done;
     return WGPT_OK;
   };
 
+  const bool pair = m->pair_ok && dev->precision == WGPT_PRECISION_TF32X3 && M > kPairMinRows;
   if (fused) TRY(forward_blocks_fused(s, ids));
-  for (int l = 0; l < (fused ? 0 : p.n_layer); l++) {
+  if (pair) TRY(forward_blocks_pair(s, n_tok));
+  for (int l = 0; l < (fused || pair ? 0 : p.n_layer); l++) {
     const LayerWeights &L = m->layers[l];
     float *kc = s->kc + (size_t)l * kv_layer, *vc = s->vc + (size_t)l * kv_layer;
     SplitHandoff qkv_slices;
@@ -1873,7 +2083,7 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
       e.kc = kc; e.vc = vc; e.E = E; e.n_tok = n_tok; e.n_ctx = p.n_ctx; e.pos = s->d_pos;
       // one query per sequence and one position slice: the attention CTAs can add the product's slices themselves
       const bool consumer_sums = n_tok == 1 && s->n_split == 1 && 3 * hs <= 256;
-      TRY(mm(s->x, L.ln1_g, L.ln1_b, L.wqkv_t, L.wqkv_lo, E, 3 * E, e, nullptr, nullptr,
+      TRY(mm(s->x, L.ln1_g, L.ln1_b, L.wqkv_t, E, 3 * E, e, nullptr, nullptr,
              consumer_sums ? &qkv_slices : nullptr));
     }
     if (n_tok == 1 && qkv_slices.taken) {
@@ -1898,16 +2108,16 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
         } else {
           dim3 mg((E / 4 + 127) / 128, M);
           LAUNCH_PDL(dev, attn_merge_kernel, mg, 128, 0, ap, s->o, E);
-          TRY(mm(s->o, nullptr, nullptr, L.wo_t, L.wo_lo, E, E, e, L.ln2_g, L.ln2_b));
+          TRY(mm(s->o, nullptr, nullptr, L.wo_t, E, E, e, L.ln2_g, L.ln2_b));
         }
       } else {
-        TRY(mm(s->o, nullptr, nullptr, L.wo_t, L.wo_lo, E, E, e, L.ln2_g, L.ln2_b));
+        TRY(mm(s->o, nullptr, nullptr, L.wo_t, E, E, e, L.ln2_g, L.ln2_b));
       }
     }
     {  // LN2 + MLP up-projection + GELU
       Epilogue e = plain_epi(s->f, F, L.bfc);
       e.act = 1;
-      TRY(mm(s->x, L.ln2_g, L.ln2_b, L.wfc_t, L.wfc_lo, E, F, e));
+      TRY(mm(s->x, L.ln2_g, L.ln2_b, L.wfc_t, E, F, e));
     }
     {  // MLP down-projection + residual
       Epilogue e = plain_epi(s->x, E, L.bpr);
@@ -1916,7 +2126,7 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
       // the next consumer of s->x: the following block's ln_1, or ln_f when every row is a newest row
       const float *ng = last ? (n_tok == 1 ? m->lnf_g : nullptr) : m->layers[l + 1].ln1_g;
       const float *nb = last ? (n_tok == 1 ? m->lnf_b : nullptr) : m->layers[l + 1].ln1_b;
-      TRY(mm(s->f, nullptr, nullptr, L.wpr_t, L.wpr_lo, F, E, e, ng, nb));
+      TRY(mm(s->f, nullptr, nullptr, L.wpr_t, F, E, e, ng, nb));
     }
   }
   // ln_f + tied de-embedding on the newest row of each sequence only (the reference normalises all rows and

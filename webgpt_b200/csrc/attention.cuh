@@ -466,7 +466,8 @@ template <bool X3>
 __global__ void __launch_bounds__(128)
 attn_prefill64_mma_kernel(const float *__restrict__ q, int ldq, const float *__restrict__ kc,
                           const float *__restrict__ vc, int ldkv, size_t kv_seq_stride, float *__restrict__ out,
-                          int ldo, int n_tok, const int *__restrict__ pos, float scale) {
+                          int ldo, int n_tok, const int *__restrict__ pos, float scale, __half *__restrict__ planes,
+                          size_t plane, float pair_scale) {
   constexpr int HS = 64, T = 64, KLD = kAttnMmaKLd, VLD = kAttnMmaVLd;
   __shared__ __align__(16) float Ks[T * KLD];
   __shared__ __align__(16) float Vs[T * VLD];
@@ -598,14 +599,24 @@ attn_prefill64_mma_kernel(const float *__restrict__ q, int ldq, const float *__r
   l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
   const float i0 = 1.f / l0, i1 = 1.f / l1;
+  // planes != nullptr: the output goes out as a pair of half-precision planes (pair.cuh), rows of ldo values
+  auto put = [&](int r, int d, float x, float y) {
+    const size_t at = ((size_t)seq * n_tok + t0 + r) * ldo + h * HS + d;
+    if (planes == nullptr) {
+      *reinterpret_cast<float2 *>(out + at) = make_float2(x, y);
+    } else {
+      x *= pair_scale;
+      y *= pair_scale;
+      const __half2 a = __floats2half2_rn(x, y);
+      const float2 f = __half22float2(a);
+      *reinterpret_cast<__half2 *>(planes + at) = a;
+      *reinterpret_cast<__half2 *>(planes + plane + at) = __floats2half2_rn(x - f.x, y - f.y);
+    }
+  };
 #pragma unroll
   for (int j = 0; j < 8; j++) {
-    if (r0 < nq)
-      *reinterpret_cast<float2 *>(out + ((size_t)seq * n_tok + t0 + r0) * ldo + h * HS + 8 * j + 2 * t) =
-          make_float2(o[j][0] * i0, o[j][1] * i0);
-    if (r1 < nq)
-      *reinterpret_cast<float2 *>(out + ((size_t)seq * n_tok + t0 + r1) * ldo + h * HS + 8 * j + 2 * t) =
-          make_float2(o[j][2] * i1, o[j][3] * i1);
+    if (r0 < nq) put(r0, 8 * j + 2 * t, o[j][0] * i0, o[j][1] * i0);
+    if (r1 < nq) put(r1, 8 * j + 2 * t, o[j][2] * i1, o[j][3] * i1);
   }
 }
 

@@ -1,5 +1,6 @@
 // Shared device helpers for the sm_100a kernels.
 #pragma once
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -24,6 +25,13 @@ struct Epilogue {
   int E, n_tok, n_ctx;
   const int *pos;  // device position counter; a kernel that stores many elements reads it once into pos_base
   int pos_base;    // used when pos == nullptr
+  // Operands stored as pairs of half-precision values (pair.cuh). rowscale: [M] or nullptr, multiplies the raw product
+  // beside colscale. pair != nullptr: the finished value goes out as a pair (scaled by the power of two pair_scale)
+  // into the planes pair and pair + pair_plane, rows of ld values, instead of to out.
+  const float *rowscale;
+  __half *pair;
+  size_t pair_plane;
+  float pair_scale;
 };
 
 __device__ __forceinline__ float gelu_f(float x) {

@@ -2,6 +2,7 @@
 // arg-max, transposition. All are 128-bit vectorised where the shape allows.
 #pragma once
 #include "common.cuh"
+#include "pair.cuh"
 
 namespace wgpt {
 
@@ -29,36 +30,73 @@ __global__ void gelu_kernel(const float4 *__restrict__ in, float4 *__restrict__ 
 // LayerNorm, one warp per row (normStats + norm, instructions.js:451-550):
 // mean = sum/N, var = sum((x-mean)^2)/N, y = gamma*((x-mean)/sqrt(var+1e-5))+beta.
 // Row r of the input starts at in + r*ld_in (lets the caller normalise only the last row of each sequence).
-__global__ void layernorm_kernel(const float *__restrict__ in, size_t ld_in, const float *__restrict__ gamma,
-                                 const float *__restrict__ beta, float *__restrict__ out, size_t ld_out, int rows,
-                                 int N) {
+// V > 0: the row stays in registers, V float4 per lane (N <= 128 V), so it is read once and all its loads are in
+// flight together; V = 0 reads it three times (any N). planes != nullptr: the result goes out as a pair of
+// half-precision planes scaled by the power of two `scale` (pair.cuh), contiguous rows, plane stride `plane`.
+template <int V>
+__global__ void __launch_bounds__(128)
+layernorm_kernel(const float *__restrict__ in, size_t ld_in, const float *__restrict__ gamma,
+                 const float *__restrict__ beta, float *__restrict__ out, size_t ld_out, int rows, int N,
+                 __half *__restrict__ planes, size_t plane, float scale) {
   int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   int lane = threadIdx.x & 31;
   pdl_launch_dependents();
   pdl_wait();  // the rows come from the previous kernel (read through L2, see common.cuh)
   if (row >= rows) return;
   const float4 *x = reinterpret_cast<const float4 *>(in + (size_t)row * ld_in);
-  int n4 = N >> 2;
+  const int n4 = N >> 2;
+  constexpr int R = V > 0 ? V : 1;
+  float4 v[R];
   float s = 0.f;
-  for (int i = lane; i < n4; i += 32) {
-    float4 v = __ldcg(x + i);
-    s += (v.x + v.y) + (v.z + v.w);
+  if (V > 0) {
+#pragma unroll
+    for (int j = 0; j < R; j++) v[j] = lane + 32 * j < n4 ? __ldcg(x + lane + 32 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < R; j++) s += (v[j].x + v[j].y) + (v[j].z + v[j].w);
+  } else {
+    for (int i = lane; i < n4; i += 32) {
+      const float4 t = __ldcg(x + i);
+      s += (t.x + t.y) + (t.z + t.w);
+    }
   }
-  float mean = warp_sum(s) / (float)N;
+  const float mean = warp_sum(s) / (float)N;
   float q = 0.f;
-  for (int i = lane; i < n4; i += 32) {
-    float4 v = __ldcg(x + i);
-    float a = v.x - mean, b = v.y - mean, c = v.z - mean, d = v.w - mean;
-    q += (a * a + b * b) + (c * c + d * d);
+  if (V > 0) {
+#pragma unroll
+    for (int j = 0; j < R; j++)
+      if (lane + 32 * j < n4) {
+        const float a = v[j].x - mean, b = v[j].y - mean, c = v[j].z - mean, d = v[j].w - mean;
+        q += (a * a + b * b) + (c * c + d * d);
+      }
+  } else {
+    for (int i = lane; i < n4; i += 32) {
+      const float4 t = __ldcg(x + i);
+      const float a = t.x - mean, b = t.y - mean, c = t.z - mean, d = t.w - mean;
+      q += (a * a + b * b) + (c * c + d * d);
+    }
   }
-  float sd = sqrtf(warp_sum(q) / (float)N + 1e-5f);
+  const float sd = sqrtf(warp_sum(q) / (float)N + 1e-5f);
   const float4 *g4 = reinterpret_cast<const float4 *>(gamma);
   const float4 *b4 = reinterpret_cast<const float4 *>(beta);
-  float4 *o = reinterpret_cast<float4 *>(out + (size_t)row * ld_out);
-  for (int i = lane; i < n4; i += 32) {
-    float4 v = __ldcg(x + i), g = g4[i], b = b4[i];
-    o[i] = make_float4(g.x * ((v.x - mean) / sd) + b.x, g.y * ((v.y - mean) / sd) + b.y,
-                       g.z * ((v.z - mean) / sd) + b.z, g.w * ((v.w - mean) / sd) + b.w);
+  auto put = [&](int i, float4 t) {
+    const float4 g = __ldg(g4 + i), b = __ldg(b4 + i);
+    const float4 y = make_float4(g.x * ((t.x - mean) / sd) + b.x, g.y * ((t.y - mean) / sd) + b.y,
+                                 g.z * ((t.z - mean) / sd) + b.z, g.w * ((t.w - mean) / sd) + b.w);
+    if (planes != nullptr) {
+      uint2 p0, p1;
+      pair_split4(scale4(y, scale), p0, p1);
+      reinterpret_cast<uint2 *>(planes + (size_t)row * N)[i] = p0;
+      reinterpret_cast<uint2 *>(planes + plane + (size_t)row * N)[i] = p1;
+    } else {
+      reinterpret_cast<float4 *>(out + (size_t)row * ld_out)[i] = y;
+    }
+  };
+  if (V > 0) {
+#pragma unroll
+    for (int j = 0; j < R; j++)
+      if (lane + 32 * j < n4) put(lane + 32 * j, v[j]);
+  } else {
+    for (int i = lane; i < n4; i += 32) put(i, __ldcg(x + i));
   }
 }
 
@@ -169,21 +207,6 @@ __global__ void argmax_kernel(const float *__restrict__ logits, int V, uint32_t 
         *done_counter = 0u;
       }
     }
-  }
-}
-
-// lo = w - tf32(w): what a TF32 tensor-core product drops from each weight (it reads the top 19 bits of an FP32
-// operand), kept as a second matrix so that the 3xTF32 GEMM can fetch it by TMA. Load time only.
-__global__ void tf32_lo_kernel(const float4 *__restrict__ w, float4 *__restrict__ lo, size_t n4) {
-  size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (; i < n4; i += stride) {
-    float4 x = w[i], l;
-    l.x = x.x - __uint_as_float(__float_as_uint(x.x) & 0xFFFFE000u);
-    l.y = x.y - __uint_as_float(__float_as_uint(x.y) & 0xFFFFE000u);
-    l.z = x.z - __uint_as_float(__float_as_uint(x.z) & 0xFFFFE000u);
-    l.w = x.w - __uint_as_float(__float_as_uint(x.w) & 0xFFFFE000u);
-    lo[i] = l;
   }
 }
 

@@ -1,0 +1,274 @@
+// C[M,N] = A[M,K] . Wt[N,K]^T (+ epilogue) for operands stored as pairs of half-precision planes (pair.cuh), many rows.
+//
+// Two CTAs of a cluster (two SMs) share one 256 x BN output tile through tcgen05 cta_group::2 (kind::f16, FP32
+// accumulation). Per 64-deep k-block each CTA fetches its 128 rows of both planes of A (32 KB) and its BN/2 rows of both
+// planes of Wt (one 3-D TMA box each, 128-byte swizzle), and the leader issues twelve MMAs: four 16-deep steps of
+// h0 g0, h0 g1, h1 g0. Nothing passes through registers on the way in: both planes come ready from the producer of the
+// matrix, so the only signals are TMA -> MMA -> TMA, and both CTAs' copies are counted on the leader's barrier.
+//
+// What bounds it: the tensor pipe, 6 BN cycles per k-block and pair; shared memory (operand reads of the MMAs, 4 KB + 16
+// BN bytes each, plus the copies coming in) needs 640 + 2.5 BN cycles at 128 bytes a cycle, so a tile of fewer than
+// about 180 columns is bound by shared memory instead. BN is a run-time multiple of 32 chosen by the host so that
+// rounds x max(6 BN, 640 + 2.5 BN) is smallest (pair_tile_columns in api.cu): products of a few tiles per pair would
+// otherwise leave a nearly empty last round (8192 x 768: 96 tiles of 256 columns on 74 pairs take two rounds, 128 of
+// 192 columns take two shorter ones). 8192 x 8192 x 8192 runs at 470 TFLOP/s = 1410 issued, the rate a plain
+// half-precision product sustains under the power cap.
+//
+// Accumulation: the tensor core truncates each time it adds to its FP32 accumulator, always towards zero, so the error
+// grows with the number of MMAs that one accumulator takes (12 per k-block here, 24 in the 3xTF32 kernel). It holds
+// at most GP_CHUNK k-blocks; for a longer K the epilogue warps add the chunks into registers, rounding to nearest
+// (128 values per thread). The two accumulators alternate by chunk, so this costs the MMAs nothing, and a tile's epilogue
+// overlaps the next tile's MMAs; with short chunks it did not: chunks of 2 / 4 / 6 k-blocks took 109 / 91 / 79 us for
+// 8192 x 2304 x 768 (3xTF32: 135 us), because the MMAs may run ahead of the epilogue by two chunks only.
+//
+// Roles: warp 0 TMA producer, warp 1 MMA issuer (leader CTA only), warps 2-9 epilogue, two per quarter of the
+// accumulator lanes. Every wait is bounded; on expiry the CTA sets *err = 3, drains and exits.
+#pragma once
+#include "gemm_tc2.cuh"
+#include "pair.cuh"
+
+namespace wgpt {
+
+constexpr int GP_BM = 128, GP_BK = 64;             // rows of A per CTA; 64 halves = one 128-byte swizzle row
+constexpr int GP_MAX_STAGES = 4;
+constexpr int GP_CHUNK = 25;                       // most k-blocks accumulated in tensor memory before a sum in registers
+constexpr int GP_A_BYTES = 2 * GP_BM * GP_BK * 2;  // both planes
+constexpr int GP_RING_BYTES = 3 * 2 * GP_A_BYTES;  // stages of A, then Wt: three of a 256-column tile
+constexpr int GP_EPI_WARPS = 8;
+constexpr int GP_THREADS = 32 * (2 + GP_EPI_WARPS);
+constexpr int GP_PAD = 32 * 33;
+constexpr size_t GP_SMEM_BYTES = 1024 + (size_t)GP_RING_BYTES + 256;
+
+// One box of both planes of a pair matrix: {64 halves, box rows, 2 planes}.
+__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+          smem_addr(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(0), "r"(smem_addr(bar))
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void *dst, const CUtensorMap *map, int x, int y, uint32_t bar_addr) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_addr(dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(0), "r"(bar_addr)
+      : "memory");
+}
+// Low word of umma_desc_sw128 (start address) and its constant high word. One thread issues every MMA of an SM, so what
+// it computes per instruction is on the critical path of the narrow tiles: with the descriptors' low words as sums of a
+// per-stage base and a constant there is one addition per operand.
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr) { return (saddr & 0x3FFFFu) >> 4; }
+constexpr uint32_t kUmmaDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ void umma2_f16(uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi)
+      : "memory");
+}
+// 32 lanes x 16 consecutive 32-bit columns (see tmem_ld_32x32).
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, float (&v)[16]) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
+}
+// Instruction descriptor of kind::f16: FP32 accumulate, half A and B, both K-major.
+__host__ __device__ constexpr uint32_t f16_idesc(int m, int n) {
+  return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+}
+
+// gridDim.x = 2 x pairs, cluster (2,1,1). Pair p walks the 256 x bn tiles p, p + pairs, ... (row tile fastest).
+// map_a: box of 128 rows; map_b: box of bn/2 rows. bn % 32 == 0, bn <= 256.
+// b_exact: the weight's second plane is zero (integers of at most 11 bits); the product with it is not issued.
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int K,
+                 int N, int bn, int b_exact, Epilogue epi, int *err) {
+  // narrower tiles leave room for a fourth stage (a copy takes about 3000 cycles to arrive under load)
+  const int stage_bytes = GP_A_BYTES + bn * (GP_BK * 2);
+  const int S = 4 * stage_bytes <= GP_RING_BYTES ? 4 : 3;
+  extern __shared__ uint8_t gp_smem_raw[];
+  uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(gp_smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t *bars = reinterpret_cast<uint64_t *>(tiles + GP_RING_BYTES);
+  uint64_t *full = bars, *empty = bars + GP_MAX_STAGES, *acc_full = bars + 2 * GP_MAX_STAGES;
+  uint64_t *acc_empty = acc_full + 2;  // the leader's: an arrival of every epilogue warp of both CTAs
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+  __shared__ float epi_pad[GP_EPI_WARPS * GP_PAD];
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_ctarank();
+  const bool leader = rank == 0;
+  const int total_kb = (K + GP_BK - 1) / GP_BK;
+  const int m_tiles = (M + 255) / 256, n_tiles = (N + bn - 1) / bn;
+  const int n_work = m_tiles * n_tiles;
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < S; i++) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < 2; i++) {
+      mbar_init(&acc_full[i], 1);
+      mbar_init(&acc_empty[i], 2 * GP_EPI_WARPS);
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_async_smem();
+  }
+  if (warp == 1) tmem_alloc2(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // both CTAs' barriers exist before anything is signalled across the pair
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  pdl_launch_dependents();
+  pdl_wait();  // A (activations) comes from the previous kernel
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const uint32_t stage_tx = 2u * (uint32_t)stage_bytes;  // both CTAs
+      int s = 0, phase = 0;  // ring position and the parity of the round through the ring
+      for (int w = pair; w < n_work && !*abort_flag; w += pairs) {
+        const int nt = w / m_tiles, mt = w - nt * m_tiles;
+        const int m0 = mt * 256 + (int)rank * GP_BM, nb0 = nt * bn + (int)rank * (bn >> 1);
+        for (int kb = 0; kb < total_kb; kb++) {
+          uint8_t *st = tiles + (size_t)s * stage_bytes;
+          if (*abort_flag || !mbar_wait(&empty[s], phase ^ 1, TC_POLLS)) { *abort_flag = 1; break; }
+          const uint32_t lead_full = peer_smem_addr(&full[s], 0);
+          if (leader) mbar_expect_tx(&full[s], stage_tx);
+          tma_load_3d_pair(st, &map_a, kb * GP_BK, m0, lead_full);
+          tma_load_3d_pair(st + GP_A_BYTES, &map_b, kb * GP_BK, nb0, lead_full);
+          if (++s == S) { s = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && leader) {
+      const uint32_t idesc = f16_idesc(256, bn);
+      const uint32_t b_plane = ((uint32_t)(bn >> 1) * (GP_BK * 2)) >> 4, desc0 = umma_desc_lo(smem_addr(tiles));
+      int s = 0, phase = 0, i = 0;  // i: chunks issued by this CTA; accumulator = i & 1, its use count = i >> 1
+      for (int w = pair; w < n_work && !*abort_flag; w += pairs) {
+        for (int kb0 = 0; kb0 < total_kb; kb0 += GP_CHUNK, i++) {
+          const int buf = i & 1, use = i >> 1;
+          if (*abort_flag || !mbar_wait(&acc_empty[buf], (use & 1) ^ 1, TC_POLLS << 4)) { *abort_flag = 1; break; }
+          tc_fence_after();
+          const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * 256);
+          const int kb1 = min(kb0 + GP_CHUNK, total_kb);
+          for (int kb = kb0; kb < kb1; kb++) {
+            if (*abort_flag || !mbar_wait(&full[s], phase, TC_POLLS)) { *abort_flag = 1; break; }
+            tc_fence_after();
+            const uint32_t a0 = desc0 + (uint32_t)s * ((uint32_t)stage_bytes >> 4), a1 = a0 + (GP_A_BYTES >> 5);
+            const uint32_t b0 = a0 + (GP_A_BYTES >> 4), b1 = b0 + b_plane;
+#pragma unroll
+            for (int k = 0; k < GP_BK / 16; k++) {
+              umma2_f16(tmem_acc, a0 + 2 * k, b0 + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+              if (!b_exact) umma2_f16(tmem_acc, a0 + 2 * k, b1 + 2 * k, idesc, 1u);
+              umma2_f16(tmem_acc, a1 + 2 * k, b0 + 2 * k, idesc, 1u);
+            }
+            umma2_commit(smem_addr(&empty[s]));  // both CTAs may refill the stage once these MMAs have read it
+            umma2_commit(peer_smem_addr(&empty[s], 1));
+            if (++s == S) { s = 0; phase ^= 1; }
+          }
+          umma2_commit(smem_addr(&acc_full[buf]));  // (also reached after an abort)
+          umma2_commit(peer_smem_addr(&acc_full[buf], 1));
+        }
+      }
+    }
+  } else {
+    const int quad = warp & 3, half = (warp - 2) >> 2;  // two warps share a quarter of the lanes, alternate chunks
+    float *pad = epi_pad + (warp - 2) * GP_PAD;
+    const int sub_r = lane >> 3, col4 = (lane & 7) * 4;
+    Epilogue e = epi;
+    if (e.kc != nullptr && e.pos != nullptr) {  // one read of the position counter instead of one per store
+      e.pos_base = __ldcg(e.pos);
+      e.pos = nullptr;
+    }
+    const int chunks = bn >> 5;
+    const bool vec_ok = ((N | e.ld) & 3) == 0;
+    int i = 0;
+    for (int w = pair; w < n_work; w += pairs) {
+      const int nt = w / m_tiles, mt = w - nt * m_tiles;
+      const int row0 = mt * 256 + (int)rank * GP_BM + quad * 32, n0 = nt * bn;
+      float acc[4][32];  // this warp's 32-column chunks half, half + 2, ... of the tile
+#pragma unroll
+      for (int c = 0; c < 4; c++)
+#pragma unroll
+        for (int j = 0; j < 32; j++) acc[c][j] = 0.f;
+      bool ok = true;
+      for (int kb0 = 0; kb0 < total_kb; kb0 += GP_CHUNK, i++) {
+        const int buf = i & 1, use = i >> 1;
+        ok = mbar_wait(&acc_full[buf], use & 1, TC_POLLS << 4) && !*abort_flag;
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * 256) + ((uint32_t)(quad * 32) << 16);
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+          if (half + 2 * c < chunks) {
+#pragma unroll
+            for (int p = 0; p < 2; p++) {  // 16 at a time: 32 more registers would spill
+              float v[16];
+              tmem_ld_32x16(tmem_acc + (uint32_t)((half + 2 * c) * 32 + 16 * p), v);
+#pragma unroll
+              for (int j = 0; j < 16; j++) acc[c][16 * p + j] += v[j];
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(peer_smem_addr(&acc_empty[buf], 0));
+      }
+      if (!ok) { *abort_flag = 1; break; }
+      if (row0 >= M) continue;
+#pragma unroll 1
+      for (int c = 0; c < 4; c++) {  // one copy of the epilogue code (see pair_epi_block); only the stores to pad are per chunk
+        const int nb = n0 + (half + 2 * c) * 32;
+        if (half + 2 * c >= chunks || nb >= N) continue;  // same for the whole warp
+#pragma unroll
+        for (int cc = 0; cc < 4; cc++)
+          if (cc == c) {
+#pragma unroll
+            for (int j = 0; j < 32; j++) pad[lane * 33 + j] = acc[cc][j];
+          }
+        __syncwarp();
+        const int n = nb + col4;
+        if (vec_ok) {
+          if (n < N) pair_epi_block(e, pad, row0, sub_r, col4, n, M);
+        } else {
+#pragma unroll 1
+          for (int it = 0; it < 8; it++) {
+            const int r = it * 4 + sub_r, m = row0 + r;
+            if (m >= M) break;
+#pragma unroll 1
+            for (int k = 0; k < 4; k++)
+              if (n + k < N) pair_epi1(e, pad[r * 33 + col4 + k], m, n + k);
+          }
+        }
+        __syncwarp();
+      }
+    }
+    tc_fence_before();
+  }
+
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag) atomicExch(err, 3);
+  cluster_sync_all();  // neither CTA leaves (or frees tensor memory) while the other may still signal it
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc2(tmem_base, 512);
+  }
+}
+
+}  // namespace wgpt

@@ -144,9 +144,9 @@ __device__ __forceinline__ TcWork tc_work(int w, int m_tiles, int n_tiles, int k
 // Two accumulators in tensor memory alternate, so the epilogue of one tile overlaps the main loop of the next.
 template <bool X3>
 __global__ void __launch_bounds__(TcPlan<X3>::kThreads, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-               const __grid_constant__ CUtensorMap map_b_lo, int M, int K, int N, Epilogue epi, int *err,
-               int kb_per_split, int splits, float *split_out, int static_op, int transposed, int b_lo_tma) {
+gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int K,
+               int N, Epilogue epi, int *err, int kb_per_split, int splits, float *split_out, int static_op,
+               int transposed, int exact_b) {
   using Plan = TcPlan<X3>;
   constexpr int S = Plan::kStages;
   extern __shared__ uint8_t tc_smem_raw[];
@@ -163,18 +163,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int total_kb = (K + TC_BK - 1) / TC_BK;
   const int m_tiles = (M + TC_BM - 1) / TC_BM, n_tiles = (N + TC_BN - 1) / TC_BN;
   const int n_work = m_tiles * n_tiles * splits;
-  // 3xTF32 with the weight operand's low part precomputed in HBM (map_b_lo): TMA brings it into the stage's B-lo
-  // slot and the split warps only treat the A tile. Requires B to be the static operand or no early loads.
-  // b_lo_tma == 2: the weight operand is exact in TF32 (small integers, the int8 codes): it has no low part, so its
+  // exact_b: the weight operand is exact in TF32 (small integers, the int8 codes): it has no low part, so its
   // tile is not split and the a_hi x b_lo product is not issued (two MMAs per k-step instead of three).
-  const bool lo_tma = X3 && b_lo_tma == 1;
-  const bool b_exact = X3 && b_lo_tma == 2;
+  const bool b_exact = X3 && exact_b != 0;
   // Exchanged operands: the second operand's live rows are the few activation rows, so the instruction is issued
   // only as wide as they need (a multiple of 16 columns) and only that part of the tile is split into hi and lo.
   const int n_mma = transposed ? min(TC_BN, (N + 15) & ~15) : TC_BN;
   const uint32_t idesc = (TC_IDESC & ~(0x3Fu << 17)) | ((uint32_t)(n_mma >> 3) << 17);
   // ... and the tensor map of that operand has a box of n_mma rows: bytes one stage receives
-  const uint32_t stage_tx = (uint32_t)TC_TILE_BYTES + (uint32_t)n_mma * (TC_BK * 4) + (lo_tma ? (uint32_t)TC_TILE_BYTES : 0u);
+  const uint32_t stage_tx = (uint32_t)TC_TILE_BYTES + (uint32_t)n_mma * (TC_BK * 4);
 #ifdef WGPT_TRACE
   __shared__ unsigned int tc_trace_base;  // the roles below are different threads: they share thread 0's record
   {
@@ -219,10 +216,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     for (int kb = 0; kb < pre; kb++) {
       uint8_t *st = tiles + (size_t)kb * Plan::kStageBytes;
       mbar_expect_tx(&full[kb], stage_tx);
-      if (static_op == 1) {
+      if (static_op == 1)
         tma_load_2d(st + TC_TILE_BYTES, &map_b, (t.kb0 + kb) * TC_BK, t.n0, &full[kb]);
-        if (lo_tma) tma_load_2d(st + 3 * TC_TILE_BYTES, &map_b_lo, (t.kb0 + kb) * TC_BK, t.n0, &full[kb]);
-      } else
+      else
         tma_load_2d(st, &map_a, (t.kb0 + kb) * TC_BK, t.m0, &full[kb]);
     }
   }
@@ -249,7 +245,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           mbar_expect_tx(&full[s], stage_tx);
           tma_load_2d(st, &map_a, (t.kb0 + kb) * TC_BK, t.m0, &full[s]);
           tma_load_2d(st + TC_TILE_BYTES, &map_b, (t.kb0 + kb) * TC_BK, t.n0, &full[s]);
-          if (lo_tma) tma_load_2d(st + 3 * TC_TILE_BYTES, &map_b_lo, (t.kb0 + kb) * TC_BK, t.n0, &full[s]);
         }
         if (w == blockIdx.x) TC_TRACE(3);
       }
@@ -406,9 +401,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int tix = threadIdx.x - 6 * 32;  // 0..127
     int kc = 0;
     // 2 KiB pieces (16 tile rows) to split: the whole first tile, and of the second tile nothing when its low part
-    // came by TMA or is zero, otherwise the rows the instruction reads.
+    // is zero, otherwise the rows the instruction reads.
     constexpr int kTilePieces = TC_TILE_BYTES / (16 * 128);
-    const int q_end = kTilePieces + ((lo_tma || b_exact) ? 0 : n_mma / 16);
+    const int q_end = kTilePieces + (b_exact ? 0 : n_mma / 16);
     for (int w = blockIdx.x; w < n_work && !*abort_flag; w += gridDim.x) {
       const TcWork t = tc_work(w, m_tiles, n_tiles, kb_per_split, total_kb);
       for (int kb = 0; kb < t.num_kb; kb++, kc++) {

@@ -73,9 +73,8 @@ __device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *m
 // gridDim.x = 2 x pairs, cluster (2,1,1). Pair p walks the 256 x 256 tiles p, p + pairs, ... (row tile fastest).
 template <bool X3>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TcPlan<X3>::kThreads, 1)
-gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                const __grid_constant__ CUtensorMap map_b_lo, int M, int K, int N, Epilogue epi, int *err,
-                int b_lo_tma) {
+gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int K,
+                int N, Epilogue epi, int *err) {
   using Plan = TcPlan<X3>;
   constexpr int S = Plan::kStages;
   extern __shared__ uint8_t tc_smem_raw[];
@@ -94,7 +93,6 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   const int m_tiles = (M + 255) / 256, n_tiles = (N + TC2_BN - 1) / TC2_BN;
   const int n_work = m_tiles * n_tiles;
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-  const bool lo_tma = X3 && b_lo_tma != 0;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < S; i++) {
@@ -142,10 +140,9 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             tma_load_2d_pair(st + TC_TILE_BYTES, &map_b, kb * TC_BK, nb0, lead_full);
             continue;
           }
-          mbar_expect_tx(&full[s], (lo_tma ? 3 : 2) * TC_TILE_BYTES);
+          mbar_expect_tx(&full[s], 2 * TC_TILE_BYTES);
           tma_load_2d(st, &map_a, kb * TC_BK, m0, &full[s]);
           tma_load_2d(st + TC_TILE_BYTES, &map_b, kb * TC_BK, nb0, &full[s]);
-          if (lo_tma) tma_load_2d(st + 3 * TC_TILE_BYTES, &map_b_lo, kb * TC_BK, nb0, &full[s]);
         }
       }
     }
@@ -279,7 +276,6 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         const uint32_t lo = hi + 2 * TC_TILE_BYTES;
 #pragma unroll 8
         for (int q = 0; q < (2 * TC_TILE_BYTES) / (16 * 128); q++) {
-          if (lo_tma && q == TC_TILE_BYTES / (16 * 128)) break;  // the Wt tile's low part came by TMA
           float4 x = lds128(hi + (uint32_t)q * 2048u), l;
           l.x = x.x - __uint_as_float(__float_as_uint(x.x) & 0xFFFFE000u);
           l.y = x.y - __uint_as_float(__float_as_uint(x.y) & 0xFFFFE000u);
