@@ -14,12 +14,13 @@
 // 192 columns take two shorter ones). 8192 x 8192 x 8192 runs at 470 TFLOP/s = 1410 issued, the rate a plain
 // half-precision product sustains under the power cap.
 //
-// Accumulation: the tensor core truncates each time it adds to its FP32 accumulator, always towards zero, so the error
-// grows with the number of MMAs that one accumulator takes (12 per k-block here, 24 in the 3xTF32 kernel). It holds
-// at most GP_CHUNK k-blocks; for a longer K the epilogue warps add the chunks into registers, rounding to nearest
-// (128 values per thread). The two accumulators alternate by chunk, so this costs the MMAs nothing, and a tile's epilogue
-// overlaps the next tile's MMAs; with short chunks it did not: chunks of 2 / 4 / 6 k-blocks took 109 / 91 / 79 us for
-// 8192 x 2304 x 768 (3xTF32: 135 us), because the MMAs may run ahead of the epilogue by two chunks only.
+// Accumulation: one FP32 accumulator in tensor memory over the whole of K. The tensor core truncates each time it adds to
+// it, always towards zero, so the error grows with the number of MMAs: 12 per 64 of K here, 24 in the 3xTF32 kernel
+// (GPT-2 XL logits of a 1024-token window, against FP32 mode: 2.3e-5 in 2-norm, 4.7e-5 in 3xTF32). Two accumulators
+// alternate by tile, so a tile's epilogue (18 000 cycles for 128 x 256 FP32 values, most of it waiting for stores that
+// L2 takes at about 2.2 TB/s when every SM stores at once) runs beside the next tile's MMAs. Summing shorter pieces
+// of K into registers instead leaves the MMAs no room to run ahead: pieces of 128 / 256 / 384 took 109 / 91 / 79 us for
+// 8192 x 2304 x 768 (3xTF32: 135 us).
 //
 // Roles: warp 0 TMA producer, warp 1 MMA issuer (leader CTA only), warps 2-9 epilogue, two per quarter of the
 // accumulator lanes. Every wait is bounded; on expiry the CTA sets *err = 3, drains and exits.
@@ -31,7 +32,6 @@ namespace wgpt {
 
 constexpr int GP_BM = 128, GP_BK = 64;             // rows of A per CTA; 64 halves = one 128-byte swizzle row
 constexpr int GP_MAX_STAGES = 4;
-constexpr int GP_CHUNK = 25;                       // most k-blocks accumulated in tensor memory before a sum in registers
 constexpr int GP_A_BYTES = 2 * GP_BM * GP_BK * 2;  // both planes
 constexpr int GP_RING_BYTES = 3 * 2 * GP_A_BYTES;  // stages of A, then Wt: three of a 256-column tile
 constexpr int GP_EPI_WARPS = 8;
@@ -68,20 +68,6 @@ __device__ __forceinline__ void umma2_f16(uint32_t tmem_d, uint32_t alo, uint32_
       "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
       "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi)
       : "memory");
-}
-// 32 lanes x 16 consecutive 32-bit columns (see tmem_ld_32x32).
-__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int j = 0; j < 16; j++) v[j] = __uint_as_float(r[j]);
 }
 // Instruction descriptor of kind::f16: FP32 accumulate, half A and B, both K-major.
 __host__ __device__ constexpr uint32_t f16_idesc(int m, int n) {
@@ -159,32 +145,29 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (lane == 0 && leader) {
       const uint32_t idesc = f16_idesc(256, bn);
       const uint32_t b_plane = ((uint32_t)(bn >> 1) * (GP_BK * 2)) >> 4, desc0 = umma_desc_lo(smem_addr(tiles));
-      int s = 0, phase = 0, i = 0;  // i: chunks issued by this CTA; accumulator = i & 1, its use count = i >> 1
-      for (int w = pair; w < n_work && !*abort_flag; w += pairs) {
-        for (int kb0 = 0; kb0 < total_kb; kb0 += GP_CHUNK, i++) {
-          const int buf = i & 1, use = i >> 1;
-          if (*abort_flag || !mbar_wait(&acc_empty[buf], (use & 1) ^ 1, TC_POLLS << 4)) { *abort_flag = 1; break; }
+      int s = 0, phase = 0, i = 0;  // i: tiles of this pair so far; accumulator = i & 1, its use count = i >> 1
+      for (int w = pair; w < n_work && !*abort_flag; w += pairs, i++) {
+        const int buf = i & 1, use = i >> 1;
+        if (!mbar_wait(&acc_empty[buf], (use & 1) ^ 1, TC_POLLS << 4)) { *abort_flag = 1; break; }
+        tc_fence_after();
+        const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * 256);
+        for (int kb = 0; kb < total_kb; kb++) {
+          if (*abort_flag || !mbar_wait(&full[s], phase, TC_POLLS)) { *abort_flag = 1; break; }
           tc_fence_after();
-          const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * 256);
-          const int kb1 = min(kb0 + GP_CHUNK, total_kb);
-          for (int kb = kb0; kb < kb1; kb++) {
-            if (*abort_flag || !mbar_wait(&full[s], phase, TC_POLLS)) { *abort_flag = 1; break; }
-            tc_fence_after();
-            const uint32_t a0 = desc0 + (uint32_t)s * ((uint32_t)stage_bytes >> 4), a1 = a0 + (GP_A_BYTES >> 5);
-            const uint32_t b0 = a0 + (GP_A_BYTES >> 4), b1 = b0 + b_plane;
+          const uint32_t a0 = desc0 + (uint32_t)s * ((uint32_t)stage_bytes >> 4), a1 = a0 + (GP_A_BYTES >> 5);
+          const uint32_t b0 = a0 + (GP_A_BYTES >> 4), b1 = b0 + b_plane;
 #pragma unroll
-            for (int k = 0; k < GP_BK / 16; k++) {
-              umma2_f16(tmem_acc, a0 + 2 * k, b0 + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
-              if (!b_exact) umma2_f16(tmem_acc, a0 + 2 * k, b1 + 2 * k, idesc, 1u);
-              umma2_f16(tmem_acc, a1 + 2 * k, b0 + 2 * k, idesc, 1u);
-            }
-            umma2_commit(smem_addr(&empty[s]));  // both CTAs may refill the stage once these MMAs have read it
-            umma2_commit(peer_smem_addr(&empty[s], 1));
-            if (++s == S) { s = 0; phase ^= 1; }
+          for (int k = 0; k < GP_BK / 16; k++) {
+            umma2_f16(tmem_acc, a0 + 2 * k, b0 + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            if (!b_exact) umma2_f16(tmem_acc, a0 + 2 * k, b1 + 2 * k, idesc, 1u);
+            umma2_f16(tmem_acc, a1 + 2 * k, b0 + 2 * k, idesc, 1u);
           }
-          umma2_commit(smem_addr(&acc_full[buf]));  // (also reached after an abort)
-          umma2_commit(peer_smem_addr(&acc_full[buf], 1));
+          umma2_commit(smem_addr(&empty[s]));  // both CTAs may refill the stage once these MMAs have read it
+          umma2_commit(peer_smem_addr(&empty[s], 1));
+          if (++s == S) { s = 0; phase ^= 1; }
         }
+        umma2_commit(smem_addr(&acc_full[buf]));  // (also reached after an abort)
+        umma2_commit(peer_smem_addr(&acc_full[buf], 1));
       }
     }
   } else {
@@ -199,51 +182,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     const int chunks = bn >> 5;
     const bool vec_ok = ((N | e.ld) & 3) == 0;
     int i = 0;
-    for (int w = pair; w < n_work; w += pairs) {
+    for (int w = pair; w < n_work; w += pairs, i++) {
       const int nt = w / m_tiles, mt = w - nt * m_tiles;
       const int row0 = mt * 256 + (int)rank * GP_BM + quad * 32, n0 = nt * bn;
-      float acc[4][32];  // this warp's 32-column chunks half, half + 2, ... of the tile
-#pragma unroll
-      for (int c = 0; c < 4; c++)
-#pragma unroll
-        for (int j = 0; j < 32; j++) acc[c][j] = 0.f;
-      bool ok = true;
-      for (int kb0 = 0; kb0 < total_kb; kb0 += GP_CHUNK, i++) {
-        const int buf = i & 1, use = i >> 1;
-        ok = mbar_wait(&acc_full[buf], use & 1, TC_POLLS << 4) && !*abort_flag;
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * 256) + ((uint32_t)(quad * 32) << 16);
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-          if (half + 2 * c < chunks) {
-#pragma unroll
-            for (int p = 0; p < 2; p++) {  // 16 at a time: 32 more registers would spill
-              float v[16];
-              tmem_ld_32x16(tmem_acc + (uint32_t)((half + 2 * c) * 32 + 16 * p), v);
-#pragma unroll
-              for (int j = 0; j < 16; j++) acc[c][16 * p + j] += v[j];
-            }
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(peer_smem_addr(&acc_empty[buf], 0));
-      }
-      if (!ok) { *abort_flag = 1; break; }
-      if (row0 >= M) continue;
+      const int buf = i & 1, use = i >> 1;
+      if (!mbar_wait(&acc_full[buf], use & 1, TC_POLLS << 4) || *abort_flag) { *abort_flag = 1; break; }
+      tc_fence_after();
+      const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * 256) + ((uint32_t)(quad * 32) << 16);
 #pragma unroll 1
-      for (int c = 0; c < 4; c++) {  // one copy of the epilogue code (see pair_epi_block); only the stores to pad are per chunk
-        const int nb = n0 + (half + 2 * c) * 32;
-        if (half + 2 * c >= chunks || nb >= N) continue;  // same for the whole warp
+      for (int c = half; c < chunks; c += 2) {
+        const int nb = n0 + c * 32, n = nb + col4;
+        if (row0 >= M || nb >= N) break;  // same for the whole warp; nothing to read from here on
+        float v[32];
+        tmem_ld_32x32(tmem_acc + (uint32_t)(c * 32), v);
 #pragma unroll
-        for (int cc = 0; cc < 4; cc++)
-          if (cc == c) {
-#pragma unroll
-            for (int j = 0; j < 32; j++) pad[lane * 33 + j] = acc[cc][j];
-          }
+        for (int j = 0; j < 32; j++) pad[lane * 33 + j] = v[j];
         __syncwarp();
-        const int n = nb + col4;
         if (vec_ok) {
           if (n < N) pair_epi_block(e, pad, row0, sub_r, col4, n, M);
         } else {
@@ -258,6 +212,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
         __syncwarp();
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(peer_smem_addr(&acc_empty[buf], 0));
     }
     tc_fence_before();
   }
