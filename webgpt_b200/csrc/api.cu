@@ -21,6 +21,7 @@
 #include "gemm_tc.cuh"
 #include "gemm_tc2.cuh"
 #include "gemm_pair.cuh"
+#include "gemm_split.cuh"
 #include "int8.cuh"
 #include "sampling.cuh"
 #include "matmul.cuh"
@@ -99,6 +100,32 @@ struct wgpt_device {
 template <typename... KArgs, typename... Args>
 static cudaError_t launch_ex(bool pdl, int cluster_z, cudaStream_t stream, void (*kernel)(KArgs...), dim3 grid,
                              dim3 block, size_t smem, Args... args);
+// The same with clusters of cluster_x CTAs along x.
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_ex_x(bool pdl, int cluster_x, cudaStream_t stream, void (*kernel)(KArgs...), dim3 grid,
+                               dim3 block, size_t smem, const Args &...args) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (pdl) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    n++;
+  }
+  attr[n].id = cudaLaunchAttributeClusterDimension;
+  attr[n].val.clusterDim.x = (unsigned)cluster_x;
+  attr[n].val.clusterDim.y = 1;
+  attr[n].val.clusterDim.z = 1;
+  n++;
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
 
 // Launch with thread-block clusters of cluster_x CTAs along x (and programmatic dependent launch if pdl).
 template <typename P>
@@ -859,6 +886,59 @@ static int32_t gemm_kn_via_transpose(wgpt_device *dev, const float *A, size_t ld
   return launch_gemm_tc(dev, dev->precision == WGPT_PRECISION_TF32X3, A, lda, wt, M, K, N, epi, nullptr, false);
 }
 
+// Launch shape of gemm_split_kernel.
+struct SplitShape {
+  int row_tiles, rn, S, stages;
+};
+// One row tile of RN rows (kNorm / decode): the K slices that leave one CTA per SM, and of the slice counts with the same
+// longest slice the smallest.
+static SplitShape split_shape_decode(const wgpt_device *dev, int M, int K, int N) {
+  SplitShape sh;
+  sh.row_tiles = 1;
+  sh.rn = (M + 15) & ~15;
+  const int ft = (N + 127) / 128, kb = (K + GP_BK - 1) / GP_BK;
+  int most = dev->sm_count / ft;
+  if (most > 8) most = 8;
+  if (most > kb) most = kb;
+  if (most < 1) most = 1;
+  sh.S = most;
+  while (sh.S > 1 && (kb + sh.S - 2) / (sh.S - 1) == (kb + most - 1) / most) sh.S--;
+  const int stage_bytes = GS_W_BYTES + sh.rn * (GP_BK * 4);
+  const int need = (kb + sh.S - 1) / sh.S, room = (int)((size_t(200) << 10) / stage_bytes);
+  sh.stages = need < room ? need : room;
+  if (sh.stages > GS_MAX_STAGES) sh.stages = GS_MAX_STAGES;
+  return sh;
+}
+
+// X: pair planes [2][M][K], or nullptr with the LayerNorm input described in a (kNorm, M <= 64).
+static int32_t launch_gemm_split(wgpt_device *dev, const SplitShape &sh, const __half *X, const __half *W, int M, int K,
+                                 int N, const Epilogue &epi, SplitArgs a) {
+  a.M = M; a.K = K; a.N = N;
+  a.rn = sh.rn; a.f_tiles = (N + 127) / 128; a.stages = sh.stages;
+  a.epi = epi;
+  a.err = dev->d_err;
+  CUtensorMap mw, mx;
+  TRY(make_pair_map(&mw, W, (uint64_t)N, (uint64_t)K, 128));
+  mx = mw;
+  if (X != nullptr) TRY(make_pair_map(&mx, X, (uint64_t)M, (uint64_t)K, sh.rn));
+  const size_t smem = 1024 + (size_t)sh.stages * (GS_W_BYTES + sh.rn * (GP_BK * 4));
+  const dim3 grid(sh.row_tiles * a.f_tiles * sh.S);
+#define SPLIT_CASE(RNV)                                                                                              \
+  do {                                                                                                               \
+    CK(cudaFuncSetAttribute(gemm_split_kernel<RNV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));        \
+    CK(launch_ex_x(dev->pdl, sh.S, dev->stream, gemm_split_kernel<RNV>, grid, dim3(GS_THREADS), smem, mw, mx, a));   \
+  } while (0)
+  if (X != nullptr) SPLIT_CASE(0);
+  else if (sh.rn == 16) SPLIT_CASE(16);
+  else if (sh.rn == 32) SPLIT_CASE(32);
+  else if (sh.rn == 48) SPLIT_CASE(48);
+  else if (sh.rn == 64) SPLIT_CASE(64);
+  else return fail(WGPT_ERR_SHAPE, "no normalising product for row tiles of %d", sh.rn);
+#undef SPLIT_CASE
+  dev->launches++;
+  return WGPT_OK;
+}
+
 // The reference-layout matmul used by the per-operator API: W is [K,N].
 static int32_t matmul_kn(wgpt_device *dev, int M, int K, int N, const float *in, const float *W, const Epilogue &epi) {
   if (M <= 8) {
@@ -927,14 +1007,30 @@ static int32_t launch_attn_prefill(wgpt_device *dev, int hs, const float *q, int
 
 static int32_t launch_attn_decode(wgpt_device *dev, int hs, const float *q, int ldq, const float *kc, const float *vc,
                                   int ldkv, size_t kv_seq_stride, float *out, int ldo, int n_seq, int H, int n_split,
-                                  const int *pos, float scale, float *part, const QkvPartials *qp = nullptr) {
+                                  const int *pos, float scale, float *part, const QkvPartials *qp = nullptr,
+                                  bool merge_here = false, __half *planes = nullptr, size_t plane = 0,
+                                  float pair_scale = 1.f) {
   dim3 grid(H, n_seq, n_split);
+  if (merge_here) {  // the slices of a (sequence, head) merge inside their cluster; the output may be a pair
+#define CASE_M(HSV)                                                                                                  \
+  case HSV:                                                                                                          \
+    CK(launch_ex(dev->pdl, n_split, dev->stream, (attn_decode_kernel<HSV>), grid, dim3(256), 0, q, ldq, kc, vc, ldkv, \
+                 kv_seq_stride, out, ldo, pos, scale, part, QkvPartials(), n_split > 1 ? 1 : 0, planes, plane,       \
+                 pair_scale));                                                                                       \
+    dev->launches++;                                                                                                 \
+    return WGPT_OK;
+    switch (hs) {
+      CASE_M(4) CASE_M(8) CASE_M(16) CASE_M(32) CASE_M(64) CASE_M(128)
+    }
+#undef CASE_M
+    return fail(WGPT_ERR_UNSUPPORTED, "head_size %d: supported sizes are 4, 8, 16, 32, 64, 128", hs);
+  }
   if (qp != nullptr) {  // the attention CTAs are the QKV product's second stage (one position slice, 3*hs <= 256)
     switch (hs) {
 #define CASE_Q(HSV)                                                                                                  \
   case HSV:                                                                                                          \
     LAUNCH_PDL(dev, (attn_decode_kernel<HSV, true>), grid, 256, 0, q, ldq, kc, vc, ldkv, kv_seq_stride, out, ldo, pos, \
-               scale, part, *qp);                                                                                    \
+               scale, part, *qp, 0, (__half *)nullptr, (size_t)0, 1.f);                                               \
     return WGPT_OK;
       CASE_Q(4) CASE_Q(8) CASE_Q(16) CASE_Q(32) CASE_Q(64)
 #undef CASE_Q
@@ -944,7 +1040,7 @@ static int32_t launch_attn_decode(wgpt_device *dev, int hs, const float *q, int 
 #define CASE(HSV)                                                                                                   \
   case HSV:                                                                                                         \
     LAUNCH_PDL(dev, attn_decode_kernel<HSV>, grid, 256, 0, q, ldq, kc, vc, ldkv, kv_seq_stride, out, ldo, pos, scale, \
-               part, QkvPartials());                                                                                \
+               part, QkvPartials(), 0, (__half *)nullptr, (size_t)0, 1.f);                                          \
     return WGPT_OK;
   switch (hs) {
     CASE(4) CASE(8) CASE(16) CASE(32) CASE(64) CASE(128)
@@ -1090,7 +1186,7 @@ WGPT_EXPORT int32_t wgpt_embed(wgpt_device *dev, const uint32_t *idx, int32_t se
   REQUIRE(n_embd >= 4 && n_embd % 4 == 0, WGPT_ERR_SHAPE, "n_embd must be divisible by 4.");
   REQUIRE(aligned16(wte) && aligned16(wpe) && aligned16(out), WGPT_ERR_ALIGN, "buffers must be 16-byte aligned");
   LAUNCH_PDL(dev, embed_kernel, seq_length, 128, 0, idx, wte, wpe, out, seq_length, seq_length, n_embd, vocab_size,
-             (const int *)nullptr, dev->d_err);
+             (const int *)nullptr, dev->d_err, (float2 *)nullptr);
   // While a pass list is being recorded nothing runs yet: an id out of range then surfaces at the next
   // wgpt_device_check after a replay.
   if (dev->capturing) return WGPT_OK;
@@ -1769,6 +1865,7 @@ struct wgpt_session {
   int n_split;        // position slices of the decode attention (attn_split_for), fixed while a step graph lives
   bool split_forced;  // set by WGPT_ATTN_SPLIT
   float *x, *h, *q, *o, *f, *logits;
+  float2 *stats = nullptr;  // [rows][n_embd / 128] (mean, squared deviations) of the residual stream's tiles
   float *kc, *vc;  // [n_layer][n_seq][n_ctx][E]
   float *fx_a = nullptr, *fx_b = nullptr;     // fused decode: residual stream entering the attention / MLP kernel
   float *fpart_a = nullptr, *fpart_b = nullptr;  // fused decode: partial results [n_head][E] and [mlp CTAs][E]
@@ -1796,6 +1893,8 @@ static void drop_step_graph(wgpt_session *s);
 
 static void session_free_act(wgpt_session *s) {
   cudaFree(s->x); cudaFree(s->h); cudaFree(s->q); cudaFree(s->o); cudaFree(s->f); cudaFree(s->ids);
+  cudaFree(s->stats);
+  s->stats = nullptr;
   s->x = s->h = s->q = s->o = s->f = nullptr;
   s->ids = nullptr;
 }
@@ -1810,6 +1909,7 @@ static int32_t session_reserve(wgpt_session *s, int n_tok) {
   size_t M = (size_t)s->n_seq * n_tok, E = s->m->p.n_embd;
   CK(cudaMalloc(&s->x, M * E * 4)); CK(cudaMalloc(&s->h, M * E * 4)); CK(cudaMalloc(&s->q, M * E * 4));
   CK(cudaMalloc(&s->o, M * E * 4)); CK(cudaMalloc(&s->f, M * 4 * E * 4)); CK(cudaMalloc(&s->ids, M * 4));
+  CK(cudaMalloc(&s->stats, M * ((E + 127) / 128) * sizeof(float2)));
   s->cap_tok = n_tok;
   return WGPT_OK;
 }
@@ -2025,6 +2125,51 @@ static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
   return WGPT_OK;
 }
 
+// The transformer blocks of a decode step of up to 64 sequences as five kernels per block (gemm_split.cuh): both LayerNorms
+// ride on the products that consume them, the attention finishes its own output, and every product is complete in one
+// launch.
+static int32_t forward_blocks_split(wgpt_session *s) {
+  wgpt_model *m = s->m;
+  wgpt_device *dev = m->dev;
+  const wgpt_params &p = m->p;
+  const int E = p.n_embd, F = 4 * E, H = p.n_head, hs = m->hs, M = s->n_seq, xt = (E + 127) / 128;
+  const size_t kv_layer = (size_t)s->n_seq * p.n_ctx * E, plane_e = (size_t)M * E, plane_f = (size_t)M * F;
+  __half *o = reinterpret_cast<__half *>(s->o), *f = reinterpret_cast<__half *>(s->f);
+  const SplitShape sh_qkv = split_shape_decode(dev, M, E, 3 * E), sh_o = split_shape_decode(dev, M, E, E),
+                   sh_fc = split_shape_decode(dev, M, E, F), sh_pr = split_shape_decode(dev, M, F, E);
+  SplitArgs norm, plain;
+  memset(&norm, 0, sizeof norm);
+  memset(&plain, 0, sizeof plain);
+  norm.x = s->x; norm.x_stats = s->stats; norm.x_tiles = xt;
+  plain.stats = s->stats;
+  for (int l = 0; l < p.n_layer; l++) {
+    const LayerWeights &L = m->layers[l];
+    float *kc = s->kc + (size_t)l * kv_layer, *vc = s->vc + (size_t)l * kv_layer;
+    Epilogue e = plain_epi(s->q, E, L.bqkv);
+    e.colscale = L.wqkv_p.cs;
+    e.kc = kc; e.vc = vc; e.E = E; e.n_tok = 1; e.n_ctx = p.n_ctx; e.pos = s->d_pos;
+    norm.gamma = L.ln1_g; norm.beta = L.ln1_b; norm.x_scale = L.s_h1;
+    TRY(launch_gemm_split(dev, sh_qkv, nullptr, L.wqkv_p.p, M, E, 3 * E, e, norm));
+    TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, nullptr, E, M, H, s->n_split, s->d_pos, m->scale,
+                           nullptr, nullptr, true, o, plane_e, L.s_o));
+    e = plain_epi(s->x, E, L.bo);
+    e.colscale = L.wo_p.cs;
+    e.residual = s->x;
+    TRY(launch_gemm_split(dev, sh_o, o, L.wo_p.p, M, E, E, e, plain));
+    e = plain_epi(nullptr, F, L.bfc);
+    e.colscale = L.wfc_p.cs;
+    e.act = 1;
+    e.pair = f; e.pair_plane = plane_f; e.pair_scale = L.s_f;
+    norm.gamma = L.ln2_g; norm.beta = L.ln2_b; norm.x_scale = L.s_h2;
+    TRY(launch_gemm_split(dev, sh_fc, nullptr, L.wfc_p.p, M, E, F, e, norm));
+    e = plain_epi(s->x, E, L.bpr);
+    e.colscale = L.wpr_p.cs;
+    e.residual = s->x;
+    TRY(launch_gemm_split(dev, sh_pr, f, L.wpr_p.p, M, F, E, e, plain));
+  }
+  return WGPT_OK;
+}
+
 // With pick, the greedy choice of every sequence is also made (next_ids, out_ids) and the position advanced.
 static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pick = false) {
   wgpt_model *m = s->m;
@@ -2034,9 +2179,11 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
   const size_t kv_layer = (size_t)s->n_seq * p.n_ctx * E;
 
   const bool fused = n_tok == 1 && s->n_seq == 1 && m->fused.ok && s->fx_a != nullptr;
+  const bool pair_mode = m->pair_ok && dev->precision == WGPT_PRECISION_TF32X3;
+  const bool split = pair_mode && n_tok == 1 && M > 8 && M <= 64 && (E + 127) / 128 <= GS_MAX_TILES;
   if (!fused)
     LAUNCH_PDL(dev, embed_kernel, M, 128, 0, ids, m->wte, m->wpe, s->x, M, n_tok, E, p.vocab_size,
-               (const int *)s->d_pos, dev->d_err);
+               (const int *)s->d_pos, dev->d_err, split ? s->stats : nullptr);
 
   // s->h already holds the LayerNorm of s->x that the next product wants (left there by the split-K second
   // stage of the product that wrote s->x)
@@ -2071,10 +2218,11 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
     return WGPT_OK;
   };
 
-  const bool pair = m->pair_ok && dev->precision == WGPT_PRECISION_TF32X3 && M > kPairMinRows;
+  const bool pair = pair_mode && M > kPairMinRows;
   if (fused) TRY(forward_blocks_fused(s, ids));
   if (pair) TRY(forward_blocks_pair(s, n_tok));
-  for (int l = 0; l < (fused || pair ? 0 : p.n_layer); l++) {
+  if (split) TRY(forward_blocks_split(s));
+  for (int l = 0; l < (fused || pair || split ? 0 : p.n_layer); l++) {
     const LayerWeights &L = m->layers[l];
     float *kc = s->kc + (size_t)l * kv_layer, *vc = s->vc + (size_t)l * kv_layer;
     SplitHandoff qkv_slices;
@@ -2155,6 +2303,17 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
     TRY(launch_gemv_nk(dev, s->n_seq, x_last, ld_last, m->lnf_g, m->lnf_b, m->wte, E, p.vocab_size, e, gp));
     if (pick && s->sample_k > 0) return pick_and_advance(s, n_tok);
     if (pick) s->len += n_tok;
+    return WGPT_OK;
+  }
+  if (pair_mode) {
+    // pairs: the 256-row tile of the two-CTA kernel is mostly padding here, but 256 weight rows per 1536 tensor-core
+    // cycles and pair are what HBM delivers anyway
+    __half *h = reinterpret_cast<__half *>(s->h);
+    const size_t plane = (size_t)s->n_seq * E;
+    TRY(launch_layernorm(dev, x_last, ld_last, m->lnf_g, m->lnf_b, nullptr, (size_t)E, s->n_seq, E, h, plane, m->s_hf));
+    e.colscale = m->wte_p.cs;
+    TRY(launch_gemm_pair(dev, h, m->wte_p.p, s->n_seq, E, p.vocab_size, e));
+    if (pick) TRY(pick_and_advance(s, n_tok));
     return WGPT_OK;
   }
   if (!h_ready) TRY(launch_layernorm(dev, x_last, ld_last, m->lnf_g, m->lnf_b, s->h, (size_t)E, s->n_seq, E));

@@ -29,11 +29,24 @@ struct QkvPartials {
   int splits, n_rows, E;
 };
 
+// One output value, as FP32 or (planes != nullptr) as a pair (pair.cuh).
+__device__ __forceinline__ void attn_put(float *out, __half *planes, size_t plane, float pair_scale, size_t at, float v) {
+  if (planes == nullptr) {
+    out[at] = v;
+  } else {
+    v *= pair_scale;
+    const __half h0 = __float2half_rn(v);
+    planes[at] = h0;
+    planes[plane + at] = __float2half_rn(v - __half2float(h0));
+  }
+}
+
 template <int HS, bool FROM_QKV_PART = false>
 __global__ void __launch_bounds__(256)
 attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict__ kc, const float *__restrict__ vc,
                    int ldkv, size_t kv_seq_stride, float *__restrict__ out, int ldo, const int *__restrict__ pos,
-                   float scale, float *__restrict__ part, QkvPartials qp = QkvPartials()) {
+                   float scale, float *__restrict__ part, QkvPartials qp = QkvPartials(), int merge_here = 0,
+                   __half *__restrict__ planes = nullptr, size_t plane = 0, float pair_scale = 1.f) {
   constexpr int LPP = HS / 4;      // lanes per position (one float4 each)
   constexpr int G = 32 / LPP;      // positions per warp iteration
   constexpr int NW = 8;
@@ -44,6 +57,7 @@ attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict
   const float *vb = vc + (size_t)seq * kv_seq_stride * ldkv + h * HS;
   TRACE_BEGIN(3);
   trace(3, 0);
+  if (merge_here) cluster_arrive();  // pairs with the wait ahead of the first remote store
   pdl_launch_dependents();
   {
     const int Ls = __ldcg(pos) + 1;
@@ -134,6 +148,7 @@ attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict
     if (lig == 0) { sm_m[warp] = m; sm_l[warp] = l; }
   }
   __syncthreads();
+  float keep_a = 0.f, keep_m = -INFINITY, keep_l = 0.f;
   if (tid < HS) {
     float mm = sm_m[0];
 #pragma unroll
@@ -146,11 +161,38 @@ attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict
       a += sm_acc[w][tid] * c;
     }
     if (n_split == 1) {
-      out[(size_t)seq * ldo + h * HS + tid] = a / ll;
+      attn_put(out, planes, plane, pair_scale, (size_t)seq * ldo + h * HS + tid, a / ll);
+    } else if (merge_here) {
+      keep_a = a;
+      keep_m = mm;
+      keep_l = ll;
     } else {
       float *my = part + ((size_t)(seq * H + h) * n_split + split) * (HS + 4);
       my[tid] = a;
       if (tid == 0) { my[HS] = mm; my[HS + 1] = ll; }
+    }
+  }
+  if (merge_here && n_split > 1) {
+    // The slices of a (sequence, head) are a cluster along z: every CTA hands its record to the first one, which merges
+    // them in slice order and finishes the output, so no consumer has to (and no merge pass stands before it).
+    __shared__ float mrg[8][HS + 2];
+    cluster_wait();
+    if (tid < HS) {
+      dsmem_st(dsmem_addr(&mrg[split][tid], 0), keep_a);
+      if (tid == 0) { dsmem_st(dsmem_addr(&mrg[split][HS], 0), keep_m); dsmem_st(dsmem_addr(&mrg[split][HS + 1], 0), keep_l); }
+    }
+    cluster_arrive();
+    cluster_wait();
+    if (split == 0 && tid < HS) {
+      float mm = mrg[0][HS];
+      for (int r = 1; r < n_split; r++) mm = fmaxf(mm, mrg[r][HS]);
+      float ll = 0.f, a = 0.f;
+      for (int r = 0; r < n_split; r++) {
+        const float c = (mrg[r][HS] == -INFINITY) ? 0.f : expf(mrg[r][HS] - mm);
+        ll += mrg[r][HS + 1] * c;
+        a += mrg[r][tid] * c;
+      }
+      attn_put(out, planes, plane, pair_scale, (size_t)seq * ldo + h * HS + tid, a / ll);
     }
   }
   trace(3, 4);

@@ -209,6 +209,29 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   return r;
 }
 
+// Cluster barrier (hardware; threads that have exited count as arrived). release/acquire order the
+// st.shared::cluster stores before it against the reads after it.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Address of this CTA's shared-memory location p in CTA `cta` of the cluster.
+__device__ __forceinline__ uint32_t dsmem_addr(const void *p, uint32_t cta) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(cta));
+  return r;
+}
+__device__ __forceinline__ void dsmem_st(uint32_t addr, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void dsmem_st4(uint32_t addr, float4 v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+               : "memory");
+}
+__device__ __forceinline__ float4 dsmem_ld4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -221,6 +244,15 @@ __device__ __forceinline__ float warp_max(float v) {
 }
 
 __device__ __forceinline__ float dot4(float4 a, float4 b) { return a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w; }
+
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
+
+// The (mean, sum of squared deviations) of the `cnt` live columns of a 128-column tile whose four values a lane holds.
+__device__ __forceinline__ float2 tile_row_stats(float4 v, bool live, int cnt) {
+  const float s = warp_sum(live ? (v.x + v.y) + (v.z + v.w) : 0.f), m = s / (float)cnt;
+  const float a = v.x - m, b = v.y - m, c = v.z - m, d = v.w - m;
+  return make_float2(m, warp_sum(live ? (a * a + b * b) + (c * c + d * d) : 0.f));
+}
 
 // LayerNorm of one row of E floats (normStats + norm, instructions.js:451-550) by a whole CTA of NT threads:
 // thread t < E/4 holds elements 4t..4t+3 in v. Two block-wide sums (mean, then the squared deviations from it),

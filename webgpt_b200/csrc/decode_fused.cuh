@@ -27,28 +27,9 @@
 
 namespace wgpt {
 
-// Cluster barrier (hardware; threads that have exited count as arrived). release/acquire order the
-// st.shared::cluster stores before it against the reads after it.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// Address of this CTA's shared-memory location p in CTA `cta` of the cluster.
-__device__ __forceinline__ uint32_t dsmem_addr(const void *p, uint32_t cta) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(cta));
-  return r;
-}
-__device__ __forceinline__ void dsmem_st(uint32_t addr, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ void dsmem_st4(uint32_t addr, float4 v) {
-  asm volatile("st.shared::cluster.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
-               : "memory");
-}
 // Orders this thread's earlier generic-proxy accesses to shared memory before later asynchronous-proxy (bulk
 // copy) writes to it.
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-
-__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
 // Sums over the rows of a row-major float4 matrix the previous kernel wrote (partial results, one row per
 // producer). Two things decide what this costs. A round trip to L2 for lines another SM has just written takes

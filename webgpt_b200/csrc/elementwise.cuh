@@ -120,7 +120,7 @@ __global__ void softmax_kernel(const float *__restrict__ in, float *__restrict__
 // Row m = seq*n_tok + t reads wte[idx[m]] and wpe[*pos + t]. An id >= vocab sets *err and leaves zeros.
 __global__ void embed_kernel(const uint32_t *__restrict__ idx, const float *__restrict__ wte,
                              const float *__restrict__ wpe, float *__restrict__ out, int rows, int n_tok, int E,
-                             int vocab, const int *__restrict__ pos, int *err) {
+                             int vocab, const int *__restrict__ pos, int *err, float2 *__restrict__ stats) {
   int m = blockIdx.x;
   if (m >= rows) return;
   TRACE_BEGIN(4);
@@ -134,13 +134,28 @@ __global__ void embed_kernel(const uint32_t *__restrict__ idx, const float *__re
   if (id >= (uint32_t)vocab) {
     if (threadIdx.x == 0) atomicExch(err, 1);
     for (int i = threadIdx.x; i < E / 4; i += blockDim.x) o[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (stats != nullptr)
+      for (int i = threadIdx.x; i < (E + 127) / 128; i += blockDim.x) stats[(size_t)m * ((E + 127) / 128) + i] = make_float2(0.f, 0.f);
     return;
   }
   const float4 *a = reinterpret_cast<const float4 *>(wte + (size_t)id * E);
   const float4 *b = reinterpret_cast<const float4 *>(wpe + (size_t)p * E);
-  for (int i = threadIdx.x; i < E / 4; i += blockDim.x) {
-    float4 x = a[i], y = b[i];
-    o[i] = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+  // 32 float4 are one 128-column tile: a warp's pass over the row covers one, whose (mean, squared deviations) go out
+  // with it when the first block normalises from tile statistics (gemm_split.cuh)
+  const int tiles = (E + 127) / 128;
+  for (int t = threadIdx.x >> 5; t < tiles; t += blockDim.x >> 5) {
+    const int i = 32 * t + (threadIdx.x & 31);
+    const bool live = i < E / 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (live) {
+      const float4 x = a[i], y = b[i];
+      v = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+      o[i] = v;
+    }
+    if (stats != nullptr) {
+      const float2 st = tile_row_stats(v, live, min(128, E - 128 * t));
+      if ((threadIdx.x & 31) == 0) stats[(size_t)m * tiles + t] = st;
+    }
   }
 }
 

@@ -1,0 +1,312 @@
+// C[M,N] = X[M,K] . Wt[N,K]^T (+ epilogue) on pairs (pair.cuh) for few to some hundred rows: batched decode and short
+// prefills, where a 256-row tile would be mostly padding and the product is a stream of weights.
+//
+// A CTA owns 128 output features (the 128 lanes of the accumulator: tcgen05.mma with the weight tile as A), a tile of RN
+// activation rows (the instruction's N) and a slice of K. The S CTAs of a cluster share one output tile, each taking a
+// slice of K, and add their partial tiles through distributed shared memory, so the product is finished in one launch:
+// the kernel it replaces (gemm_tc_kernel, operands exchanged) left split-K slices in HBM for a second kernel, and eight
+// dependent launches per transformer block at 5-8 us each were what a 64-row decode pass took its time for.
+//
+//   weights   : both planes of a {64 of K, 128 rows} tile per TMA box (32 KB) into a ring, requested before the
+//               dependency wait (they are written by no kernel);
+//   activations: MODE kPlanes - both planes by TMA;
+//               MODE kNorm   - FP32 rows, normalised on the way in (LayerNorm, instructions.js:451-550) by six warps:
+//               their producer left (mean, sum of squared deviations) of every row and 128-column tile, which are
+//               merged here, so that neither a LayerNorm pass nor a grid-wide exchange stands between two products;
+//   reduction : every CTA puts its [RN][128] partial tile into its own shared memory (the ring's, by then read), the
+//               cluster synchronises once, and CTA r finishes rows r RN/S ..: it reads the S partial rows in rank order
+//               (results do not depend on timing), applies scale, bias, GELU / residual, and stores 512 contiguous
+//               bytes per row. stats != nullptr: also this tile's (mean, squared deviations) of each finished row.
+//
+// Accumulation in tensor memory is over one slice of K (at most 12 MMAs per 64 of it), the slices are added in FP32
+// rounding to nearest.
+// Every wait is bounded; on expiry the CTA sets *err = 3 and carries on through its cluster barriers (the result is void).
+#pragma once
+#include "gemm_pair.cuh"
+
+namespace wgpt {
+
+constexpr int GS_THREADS = 256;        // warp 0 TMA, warp 1 MMA, warps 2-7 staging, warps 4-7 accumulator read-back
+constexpr int GS_STAGERS = 192;
+constexpr int GS_MAX_STAGES = 6;
+constexpr int GS_W_BYTES = GP_A_BYTES;  // both planes of a 128 x 64 weight tile
+constexpr int GS_MAX_TILES = 64;        // feature tiles whose row statistics a consumer merges (K <= 8192)
+
+struct SplitArgs {
+  int M, K, N;
+  int rn;              // activation rows per CTA: a multiple of 16, at most 128 (kPlanes) / RN (kNorm)
+  int f_tiles;         // ceil(N / 128)
+  int stages;          // ring stages (<= GS_MAX_STAGES); stages * stage_bytes >= rn * 512
+  Epilogue epi;
+  float2 *stats;       // [M][f_tiles] or nullptr
+  // kNorm
+  const float *x;      // [M][K] FP32
+  const float2 *x_stats;  // [M][x_tiles]: mean and sum of squared deviations of columns 128 t ..
+  int x_tiles;
+  const float *gamma, *beta;
+  float x_scale;
+  int *err;
+};
+
+__device__ __forceinline__ void umma1_f16(uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t idesc,
+                                          uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "mov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi)
+      : "memory");
+}
+__device__ __forceinline__ void sts64(uint32_t saddr, uint2 v) {
+  asm volatile("st.shared.v2.u32 [%0], {%1,%2};" ::"r"(saddr), "r"(v.x), "r"(v.y) : "memory");
+}
+
+// Mean and 1/sqrt(var + eps) of a row of K values from the (mean, sum of squared deviations) of its 128-column tiles.
+__device__ __forceinline__ float2 merge_row_stats(const float2 *__restrict__ st, int tiles, int K) {
+  float m = 0.f, q = 0.f;
+  float2 v[GS_MAX_TILES > 16 ? 16 : GS_MAX_TILES];
+  if (tiles <= 16) {  // all in flight together
+#pragma unroll
+    for (int t = 0; t < 16; t++) v[t] = t < tiles ? __ldcg(st + t) : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < 16; t++) m += t < tiles ? v[t].x * (float)min(128, K - 128 * t) : 0.f;
+    m /= (float)K;
+#pragma unroll
+    for (int t = 0; t < 16; t++)
+      if (t < tiles) q += v[t].y + (float)min(128, K - 128 * t) * (v[t].x - m) * (v[t].x - m);
+  } else {
+    for (int t = 0; t < tiles; t++) m += __ldcg(st + t).x * (float)min(128, K - 128 * t);
+    m /= (float)K;
+    for (int t = 0; t < tiles; t++) {
+      const float2 a = __ldcg(st + t);
+      q += a.y + (float)min(128, K - 128 * t) * (a.x - m) * (a.x - m);
+    }
+  }
+  return make_float2(m, 1.0f / sqrtf(q / (float)K + 1e-5f));
+}
+
+// grid.x = row tiles x feature tiles x S, cluster (S, 1, 1). map_w: box of 128 rows; map_x (RN == 0): box of rn rows.
+// RN == 0: activations as planes by TMA, rn at run time. RN > 0: normalised on the way in, rn == RN.
+template <int RN>
+__global__ void __launch_bounds__(GS_THREADS, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+                  const __grid_constant__ SplitArgs p) {
+  extern __shared__ uint8_t gs_smem_raw[];
+  uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(gs_smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ uint64_t full_w[GS_MAX_STAGES], full_x[GS_MAX_STAGES], empty[GS_MAX_STAGES], acc_full;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_word;
+  __shared__ float2 row_norm[RN > 0 ? RN : 1];
+  volatile int *abort_flag = &abort_word;
+  float *part = reinterpret_cast<float *>(tiles);  // [rn][128], over the ring once its last tile has been read
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rn = RN > 0 ? RN : p.rn;
+  uint32_t S;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(S));
+  const int rank = (int)cluster_ctarank();
+  const int tile = blockIdx.x / S, ft = tile % p.f_tiles, row0 = (tile / p.f_tiles) * rn, f0 = ft * 128;
+  const int total_kb = (p.K + GP_BK - 1) / GP_BK;
+  const int kb0 = (int)((long long)total_kb * rank / S), nkb = (int)((long long)total_kb * (rank + 1) / S) - kb0;
+  const int stages = p.stages, stage_bytes = GS_W_BYTES + rn * (GP_BK * 4);
+  const uint32_t tmem_cols = rn <= 32 ? 32u : (rn <= 64 ? 64u : 128u);
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < stages; i++) {
+      mbar_init(&full_w[i], 1);
+      mbar_init(&full_x[i], RN > 0 ? GS_STAGERS / 32 : 1);
+      mbar_init(&empty[i], 1);
+    }
+    mbar_init(&acc_full, 1);
+    abort_word = 0;
+    fence_async_smem();
+    const int pre = min(stages, nkb);
+    for (int j = 0; j < pre; j++) {  // weights: ahead of the dependency wait
+      mbar_expect_tx(&full_w[j], GS_W_BYTES);
+      tma_load_3d(tiles + (size_t)j * stage_bytes, &map_w, (kb0 + j) * GP_BK, f0, &full_w[j]);
+    }
+  }
+  if (warp == 1) tmem_alloc(&tmem_slot, tmem_cols);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_acc = tmem_slot;
+  Epilogue e = p.epi;
+  // this lane's four columns of the tile: their constants ahead of the wait too
+  const int n = f0 + lane * 4;
+  const bool n_live = n < p.N;
+  float4 cs = make_float4(1.f, 1.f, 1.f, 1.f), bs = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (n_live && e.colscale != nullptr) cs = __ldg(reinterpret_cast<const float4 *>(e.colscale + n));
+  if (n_live && e.bias != nullptr) bs = __ldg(reinterpret_cast<const float4 *>(e.bias + n));
+  pdl_launch_dependents();
+  pdl_wait();  // the activations come from the previous kernel
+  if (e.kc != nullptr && e.pos != nullptr) {
+    e.pos_base = __ldcg(e.pos);
+    e.pos = nullptr;
+  }
+  const int r_beg = rn * rank / (int)S, r_end = rn * (rank + 1) / (int)S;
+  float4 res_first = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (e.residual != nullptr && n_live && r_beg + warp < r_end && row0 + r_beg + warp < p.M)
+    res_first = __ldcg(reinterpret_cast<const float4 *>(e.residual + (size_t)(row0 + r_beg + warp) * e.ld + n));
+
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int j = 0; j < nkb; j++) {
+        const int s = j % stages, use = j / stages;
+        uint8_t *st = tiles + (size_t)s * stage_bytes;
+        if (j >= stages) {
+          if (*abort_flag || !mbar_wait(&empty[s], (use & 1) ^ 1, TC_POLLS)) { *abort_flag = 1; break; }
+          mbar_expect_tx(&full_w[s], GS_W_BYTES);
+          tma_load_3d(st, &map_w, (kb0 + j) * GP_BK, f0, &full_w[s]);
+        }
+        if (RN == 0) {
+          mbar_expect_tx(&full_x[s], (uint32_t)rn * (GP_BK * 4));
+          tma_load_3d(st + GS_W_BYTES, &map_x, (kb0 + j) * GP_BK, row0, &full_x[s]);
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = f16_idesc(128, rn), desc0 = umma_desc_lo(smem_addr(tiles));
+      const uint32_t x_plane = ((uint32_t)rn * (GP_BK * 2)) >> 4;
+      for (int j = 0; j < nkb; j++) {
+        const int s = j % stages, use = j / stages;
+        if (*abort_flag || !mbar_wait(&full_w[s], use & 1, TC_POLLS) || !mbar_wait(&full_x[s], use & 1, TC_POLLS)) {
+          *abort_flag = 1;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t w0 = desc0 + (uint32_t)s * ((uint32_t)stage_bytes >> 4), w1 = w0 + (GS_W_BYTES >> 5);
+        const uint32_t x0 = w0 + (GS_W_BYTES >> 4), x1 = x0 + x_plane;
+#pragma unroll
+        for (int k = 0; k < GP_BK / 16; k++) {
+          umma1_f16(tmem_acc, w0 + 2 * k, x0 + 2 * k, idesc, (j > 0 || k > 0) ? 1u : 0u);
+          umma1_f16(tmem_acc, w0 + 2 * k, x1 + 2 * k, idesc, 1u);
+          umma1_f16(tmem_acc, w1 + 2 * k, x0 + 2 * k, idesc, 1u);
+        }
+        umma_commit(&empty[s]);
+      }
+      umma_commit(&acc_full);  // (also reached after an abort)
+    }
+    __syncwarp();
+  } else if (RN > 0) {
+    // ---------------- activations: 16 lanes per row (one float4 each), 12 rows per step ----------------
+    constexpr int ITERS = RN > 0 ? (RN + 11) / 12 : 1, G = 12 / ITERS;  // G k-blocks of loads in flight together
+    const int t = threadIdx.x - 64, k4 = t & 15, mrow = t >> 4;
+    const int rows = min(RN, p.M - row0);
+    for (int j0 = 0; j0 < nkb; j0 += G) {
+      float4 v[G][ITERS], gm[G], bt[G];
+#pragma unroll
+      for (int g = 0; g < G; g++) {
+        const int col = (kb0 + j0 + g) * GP_BK + 4 * k4;
+        const bool in = j0 + g < nkb && col < p.K;
+        gm[g] = in ? __ldg(reinterpret_cast<const float4 *>(p.gamma + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        bt[g] = in ? __ldg(reinterpret_cast<const float4 *>(p.beta + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < ITERS; i++) {
+          const int m = mrow + 12 * i;
+          v[g][i] = in && m < rows ? __ldcg(reinterpret_cast<const float4 *>(p.x + (size_t)(row0 + m) * p.K + col))
+                                   : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      }
+      if (j0 == 0) {
+        if (t < rows) row_norm[t] = merge_row_stats(p.x_stats + (size_t)(row0 + t) * p.x_tiles, p.x_tiles, p.K);
+        asm volatile("bar.sync 1, %0;" ::"n"(GS_STAGERS) : "memory");
+      }
+#pragma unroll
+      for (int g = 0; g < G; g++) {
+        const int j = j0 + g;
+        if (j >= nkb) break;
+        const int s = j % stages, use = j / stages;
+        if (j >= stages && (*abort_flag || !mbar_wait(&empty[s], (use & 1) ^ 1, TC_POLLS))) { *abort_flag = 1; break; }
+        const uint32_t xt = smem_addr(tiles + (size_t)s * stage_bytes) + GS_W_BYTES;
+        const float4 ga = scale4(gm[g], p.x_scale), be = scale4(bt[g], p.x_scale);
+#pragma unroll
+        for (int i = 0; i < ITERS; i++) {
+          const int m = mrow + 12 * i;
+          if (m < rows) {  // other columns of the accumulator are never read
+            const float2 mr = row_norm[m];
+            const float4 a = v[g][i];
+            uint2 h0, h1;
+            pair_split4(make_float4(ga.x * ((a.x - mr.x) * mr.y) + be.x, ga.y * ((a.y - mr.x) * mr.y) + be.y,
+                                    ga.z * ((a.z - mr.x) * mr.y) + be.z, ga.w * ((a.w - mr.x) * mr.y) + be.w), h0, h1);
+            // 128-byte swizzle: 16-byte chunk c of row m sits at chunk c ^ (m % 8)
+            const uint32_t at = xt + (uint32_t)m * 128u + ((uint32_t)((k4 >> 1) ^ (m & 7)) << 4) + (uint32_t)(k4 & 1) * 8u;
+            sts64(at, h0);
+            sts64(at + (uint32_t)RN * 128u, h1);
+          }
+        }
+        fence_async_smem();  // visible to the tensor core's reads
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&full_x[s]);
+      }
+    }
+  }
+  if (warp >= 4) {  // accumulator -> this CTA's partial tile; lane = feature, one shared-memory row per activation row
+    if (!mbar_wait(&acc_full, 0, TC_POLLS << 2)) *abort_flag = 1;
+    tc_fence_after();
+    const int quad = warp & 3;
+#pragma unroll 1
+    for (int c = 0; c < rn; c += 32) {
+      float v[32];
+      tmem_ld_32x32(tmem_acc + ((uint32_t)(quad * 32) << 16) + (uint32_t)c, v);
+#pragma unroll
+      for (int j = 0; j < 32; j++)
+        if (c + j < rn) part[(c + j) * 128 + quad * 32 + lane] = v[j];
+    }
+    tc_fence_before();
+  }
+  if (S > 1) {
+    cluster_arrive();
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
+  if (threadIdx.x == 0 && *abort_flag) atomicExch(p.err, 3);
+
+  const int cnt = min(128, p.N - f0);
+  const uint32_t pbase = smem_addr(part) + (uint32_t)lane * 16u;
+  for (int r = r_beg + warp; r < r_end; r += GS_THREADS / 32) {
+    const int m = row0 + r;
+    if (m >= p.M) break;
+    float4 res = res_first;
+    if (r != r_beg + warp && e.residual != nullptr && n_live)
+      res = __ldcg(reinterpret_cast<const float4 *>(e.residual + (size_t)m * e.ld + n));
+    float4 q[8];
+    const uint32_t at = pbase + (uint32_t)r * 512u;
+#pragma unroll
+    for (int s = 0; s < 8; s++)
+      if (s < (int)S) {
+        uint32_t ra;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(at), "r"(s));
+        q[s] = dsmem_ld4(ra);
+      }
+    float4 v = q[0];
+#pragma unroll
+    for (int s = 1; s < 8; s++)
+      if (s < (int)S) v = add4(v, q[s]);
+    if (n_live) {
+      v = pair_epi_value4(e, v, cs, bs, res, m);
+      pair_epi_store4(e, v, m, n);
+    }
+    if (p.stats != nullptr) {
+      const float2 st = tile_row_stats(v, n_live, cnt);
+      if (lane == 0) p.stats[(size_t)m * p.f_tiles + ft] = st;
+    }
+  }
+  if (S > 1) {  // no CTA leaves while another may still read its partial tile (nothing is published by this barrier)
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_acc, tmem_cols);
+  }
+}
+
+}  // namespace wgpt

@@ -40,13 +40,15 @@ __device__ __forceinline__ void pair_split4(float4 v, uint2 &p0, uint2 &p1) {
 }
 __device__ __forceinline__ float4 scale4(float4 v, float s) { return make_float4(v.x * s, v.y * s, v.z * s, v.w * s); }
 
-// Epilogue of the kernels that multiply pairs: four raw sums of row m, columns n..n+3, with the column's constants and
-// the residual already in registers.
-__device__ __forceinline__ void pair_epi4(const Epilogue &e, float4 v, float4 cs, float4 bs, float4 res, int m, int n) {
+// Epilogue of the kernels that multiply pairs: four raw sums of row m, columns n..n+3, with the columns' constants and
+// the residual already in registers -> the finished values, and their store.
+__device__ __forceinline__ float4 pair_epi_value4(const Epilogue &e, float4 v, float4 cs, float4 bs, float4 res, int m) {
   if (e.rowscale != nullptr) v = scale4(v, __ldg(e.rowscale + m));
   v = make_float4(v.x * cs.x + bs.x, v.y * cs.y + bs.y, v.z * cs.z + bs.z, v.w * cs.w + bs.w);
   if (e.act == 1) v = make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
-  v = make_float4(v.x + res.x, v.y + res.y, v.z + res.z, v.w + res.w);
+  return make_float4(v.x + res.x, v.y + res.y, v.z + res.z, v.w + res.w);
+}
+__device__ __forceinline__ void pair_epi_store4(const Epilogue &e, float4 v, int m, int n) {
   if (e.pair != nullptr) {
     uint2 p0, p1;
     pair_split4(scale4(v, e.pair_scale), p0, p1);
@@ -93,7 +95,7 @@ __device__ __forceinline__ void pair_epi_block(const Epilogue &e, const float *p
       if (m >= M) break;
       const float *src = pad + r * 33 + col4;
       const float4 res = e.residual != nullptr ? __ldcg(reinterpret_cast<const float4 *>(e.residual + (size_t)m * e.ld + n)) : zero4;
-      pair_epi4(e, make_float4(src[0], src[1], src[2], src[3]), cs, bs, res, m, n);
+      pair_epi_store4(e, pair_epi_value4(e, make_float4(src[0], src[1], src[2], src[3]), cs, bs, res, m), m, n);
     }
   }
 }
