@@ -85,6 +85,7 @@ struct wgpt_device {
   int gemv_stream_max_rows;  // most rows the register-streaming GEMV takes for a layer product (WGPT_GEMV_MAX_ROWS)
   unsigned int *d_work;  // two counters of gemv_loop_kernel (left zero by every launch)
   bool loop_gemv;     // products against matrices larger than L2 through gemv_loop_kernel (WGPT_LOOP_GEMV=0: off)
+  int max_clusters[9];  // clusters of S CTAs of gemm_split_kernel resident at once with one CTA per SM
   bool fused_decode;  // single-sequence decode with two kernels per block (WGPT_FUSED_DECODE=0 turns it off)
 };
 
@@ -268,6 +269,24 @@ WGPT_EXPORT int32_t wgpt_device_create(int32_t ordinal, wgpt_device **out) {
   if (e != cudaSuccess) {
     delete dev;
     return fail(WGPT_ERR_CUDA, "device setup: %s", cudaGetErrorString(e));
+  }
+  for (int S = 1; S <= 8; S++) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof cfg);
+    cfg.gridDim = dim3(S * dev->sm_count);
+    cfg.blockDim = dim3(GS_THREADS);
+    cfg.dynamicSmemBytes = size_t(200) << 10;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)S;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    dev->max_clusters[S] = 0;
+    if (cudaFuncSetAttribute(gemm_split_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) ==
+        cudaSuccess)
+      cudaOccupancyMaxActiveClusters(&dev->max_clusters[S], gemm_split_kernel<0>, &cfg);
   }
   *out = dev;
   return WGPT_OK;
@@ -890,19 +909,16 @@ static int32_t gemm_kn_via_transpose(wgpt_device *dev, const float *A, size_t ld
 struct SplitShape {
   int row_tiles, rn, S, stages;
 };
-// One row tile of RN rows (kNorm / decode): the K slices that leave one CTA per SM, and of the slice counts with the same
-// longest slice the smallest.
+// One row tile of RN rows (kNorm / decode): the smallest number of K slices with the shortest longest slice, among those
+// whose clusters are all resident at once with one CTA per SM (a second round would double the product's time).
 static SplitShape split_shape_decode(const wgpt_device *dev, int M, int K, int N) {
   SplitShape sh;
   sh.row_tiles = 1;
   sh.rn = (M + 15) & ~15;
   const int ft = (N + 127) / 128, kb = (K + GP_BK - 1) / GP_BK;
-  int most = dev->sm_count / ft;
-  if (most > 8) most = 8;
-  if (most > kb) most = kb;
-  if (most < 1) most = 1;
-  sh.S = most;
-  while (sh.S > 1 && (kb + sh.S - 2) / (sh.S - 1) == (kb + most - 1) / most) sh.S--;
+  sh.S = 1;
+  for (int S = 2; S <= 8 && S <= kb; S++)
+    if (ft <= dev->max_clusters[S] && (kb + S - 1) / S < (kb + sh.S - 1) / sh.S) sh.S = S;
   const int stage_bytes = GS_W_BYTES + sh.rn * (GP_BK * 4);
   const int need = (kb + sh.S - 1) / sh.S, room = (int)((size_t(200) << 10) / stage_bytes);
   sh.stages = need < room ? need : room;
@@ -921,7 +937,9 @@ static int32_t launch_gemm_split(wgpt_device *dev, const SplitShape &sh, const _
   TRY(make_pair_map(&mw, W, (uint64_t)N, (uint64_t)K, 128));
   mx = mw;
   if (X != nullptr) TRY(make_pair_map(&mx, X, (uint64_t)M, (uint64_t)K, sh.rn));
-  const size_t smem = 1024 + (size_t)sh.stages * (GS_W_BYTES + sh.rn * (GP_BK * 4));
+  const int kb = (K + GP_BK - 1) / GP_BK;
+  const size_t smem = 1024 + (size_t)sh.stages * (GS_W_BYTES + sh.rn * (GP_BK * 4)) +
+                      (X == nullptr ? (size_t)((kb + sh.S - 1) / sh.S) * GP_BK * 8 + (size_t)sh.rn * a.x_tiles * 8 : 0);
   const dim3 grid(sh.row_tiles * a.f_tiles * sh.S);
 #define SPLIT_CASE(RNV)                                                                                              \
   do {                                                                                                               \
@@ -2180,7 +2198,7 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
 
   const bool fused = n_tok == 1 && s->n_seq == 1 && m->fused.ok && s->fx_a != nullptr;
   const bool pair_mode = m->pair_ok && dev->precision == WGPT_PRECISION_TF32X3;
-  const bool split = pair_mode && n_tok == 1 && M > 8 && M <= 64 && (E + 127) / 128 <= GS_MAX_TILES;
+  const bool split = pair_mode && n_tok == 1 && M > 8 && M <= 64;
   if (!fused)
     LAUNCH_PDL(dev, embed_kernel, M, 128, 0, ids, m->wte, m->wpe, s->x, M, n_tok, E, p.vocab_size,
                (const int *)s->d_pos, dev->d_err, split ? s->stats : nullptr);

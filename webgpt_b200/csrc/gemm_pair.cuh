@@ -54,19 +54,28 @@ __device__ __forceinline__ void tma_load_3d_pair(void *dst, const CUtensorMap *m
       "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(0), "r"(bar_addr)
       : "memory");
 }
-// Low word of umma_desc_sw128 (start address) and its constant high word. One thread issues every MMA of an SM, so what
-// it computes per instruction is on the critical path of the narrow tiles: with the descriptors' low words as sums of a
-// per-stage base and a constant there is one addition per operand.
+// Low word of umma_desc_sw128 (start address) and its constant high word. One lane issues every MMA of an SM, so what an
+// instruction costs to issue bounds the narrow tiles: the descriptors' low words are sums of a per-stage base and a
+// constant, and the loop around them is run by the whole warp, the lane being elected inside the instruction. Issued
+// from a branch that one lane had taken, an MMA took about 98 cycles whatever its size (operands have to be moved to
+// the uniform registers it reads, one by one); a decode product of 128 x 16 x 832 took 8.4 us, elected 5.5.
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t saddr) { return (saddr & 0x3FFFFu) >> 4; }
 constexpr uint32_t kUmmaDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ void umma2_f16(uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t idesc,
                                           uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t"
       "mov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
+      "setp.ne.b32 p, %4, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
       "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi)
+      : "memory");
+}
+// umma2_commit by one elected lane of a converged warp.
+__device__ __forceinline__ void umma2_commit_elect(uint32_t cluster_addr) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(cluster_addr)
       : "memory");
 }
 // Instruction descriptor of kind::f16: FP32 accumulate, half A and B, both K-major.
@@ -92,7 +101,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
   __shared__ float epi_pad[GP_EPI_WARPS * GP_PAD];
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int total_kb = (K + GP_BK - 1) / GP_BK;
@@ -142,17 +151,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && leader) {
+    if (leader) {
       const uint32_t idesc = f16_idesc(256, bn);
       const uint32_t b_plane = ((uint32_t)(bn >> 1) * (GP_BK * 2)) >> 4, desc0 = umma_desc_lo(smem_addr(tiles));
       int s = 0, phase = 0, i = 0;  // i: tiles of this pair so far; accumulator = i & 1, its use count = i >> 1
-      for (int w = pair; w < n_work && !*abort_flag; w += pairs, i++) {
+      for (int w = pair; w < n_work; w += pairs, i++) {
         const int buf = i & 1, use = i >> 1;
-        if (!mbar_wait(&acc_empty[buf], (use & 1) ^ 1, TC_POLLS << 4)) { *abort_flag = 1; break; }
+        if (!mbar_wait(&acc_empty[buf], (use & 1) ^ 1, TC_POLLS << 4)) *abort_flag = 1;
+        if (__any_sync(0xffffffffu, *abort_flag)) break;
         tc_fence_after();
         const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * 256);
         for (int kb = 0; kb < total_kb; kb++) {
-          if (*abort_flag || !mbar_wait(&full[s], phase, TC_POLLS)) { *abort_flag = 1; break; }
+          if (!mbar_wait(&full[s], phase, TC_POLLS)) *abort_flag = 1;
+          if (__any_sync(0xffffffffu, *abort_flag)) break;
           tc_fence_after();
           const uint32_t a0 = desc0 + (uint32_t)s * ((uint32_t)stage_bytes >> 4), a1 = a0 + (GP_A_BYTES >> 5);
           const uint32_t b0 = a0 + (GP_A_BYTES >> 4), b1 = b0 + b_plane;
@@ -162,12 +173,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             if (!b_exact) umma2_f16(tmem_acc, a0 + 2 * k, b1 + 2 * k, idesc, 1u);
             umma2_f16(tmem_acc, a1 + 2 * k, b0 + 2 * k, idesc, 1u);
           }
-          umma2_commit(smem_addr(&empty[s]));  // both CTAs may refill the stage once these MMAs have read it
-          umma2_commit(peer_smem_addr(&empty[s], 1));
+          umma2_commit_elect(smem_addr(&empty[s]));  // both CTAs may refill the stage once these MMAs have read it
+          umma2_commit_elect(peer_smem_addr(&empty[s], 1));
           if (++s == S) { s = 0; phase ^= 1; }
         }
-        umma2_commit(smem_addr(&acc_full[buf]));  // (also reached after an abort)
-        umma2_commit(peer_smem_addr(&acc_full[buf], 1));
+        umma2_commit_elect(smem_addr(&acc_full[buf]));  // (also reached after an abort)
+        umma2_commit_elect(peer_smem_addr(&acc_full[buf], 1));
       }
     }
   } else {

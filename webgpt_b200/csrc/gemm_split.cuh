@@ -18,8 +18,10 @@
 //               (results do not depend on timing), applies scale, bias, GELU / residual, and stores 512 contiguous
 //               bytes per row. stats != nullptr: also this tile's (mean, squared deviations) of each finished row.
 //
-// Accumulation in tensor memory is over one slice of K (at most 12 MMAs per 64 of it), the slices are added in FP32
-// rounding to nearest.
+// The activations' two planes lie one behind the other, so one MMA multiplies the weights' first plane with both (2 RN
+// columns: the main products and the first correction side by side) and a second one adds the other correction to the
+// latter: two instructions per 16 of K instead of three, and the large and the small sums have accumulators of their own.
+// The slices of K are added in FP32, rounding to nearest.
 // Every wait is bounded; on expiry the CTA sets *err = 3 and carries on through its cluster barriers (the result is void).
 #pragma once
 #include "gemm_pair.cuh"
@@ -30,7 +32,6 @@ constexpr int GS_THREADS = 256;        // warp 0 TMA, warp 1 MMA, warps 2-7 stag
 constexpr int GS_STAGERS = 192;
 constexpr int GS_MAX_STAGES = 6;
 constexpr int GS_W_BYTES = GP_A_BYTES;  // both planes of a 128 x 64 weight tile
-constexpr int GS_MAX_TILES = 64;        // feature tiles whose row statistics a consumer merges (K <= 8192)
 
 struct SplitArgs {
   int M, K, N;
@@ -51,11 +52,31 @@ struct SplitArgs {
 __device__ __forceinline__ void umma1_f16(uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t idesc,
                                           uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+      "{\n\t.reg .pred p, e;\n\t.reg .b64 da, db;\n\t"
       "mov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
+      "setp.ne.b32 p, %4, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %3, p;\n\t}" ::"r"(tmem_d),
       "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "r"(kUmmaDescHi)
+      : "memory");
+}
+// Twice 32 lanes x 16 consecutive 32-bit columns, both loads in flight together.
+__device__ __forceinline__ void tmem_ld_2x16(uint32_t t0, uint32_t t1, float (&v)[16], float (&w)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
+      : "=&f"(v[0]), "=&f"(v[1]), "=&f"(v[2]), "=&f"(v[3]), "=&f"(v[4]), "=&f"(v[5]), "=&f"(v[6]), "=&f"(v[7]), "=&f"(v[8]), "=&f"(v[9]), "=&f"(v[10]), "=&f"(v[11]), "=&f"(v[12]), "=&f"(v[13]), "=&f"(v[14]), "=&f"(v[15]),
+        "=&f"(w[0]), "=&f"(w[1]), "=&f"(w[2]), "=&f"(w[3]), "=&f"(w[4]), "=&f"(w[5]), "=&f"(w[6]), "=&f"(w[7]), "=&f"(w[8]), "=&f"(w[9]), "=&f"(w[10]), "=&f"(w[11]), "=&f"(w[12]), "=&f"(w[13]), "=&f"(w[14]), "=&f"(w[15])
+      : "r"(t0), "r"(t1)
+      : "memory");
+}
+// umma_commit by one elected lane of a converged warp.
+__device__ __forceinline__ void umma_commit_elect(uint64_t *bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_addr(bar))
       : "memory");
 }
 __device__ __forceinline__ void sts64(uint32_t saddr, uint2 v) {
@@ -63,33 +84,20 @@ __device__ __forceinline__ void sts64(uint32_t saddr, uint2 v) {
 }
 
 // Mean and 1/sqrt(var + eps) of a row of K values from the (mean, sum of squared deviations) of its 128-column tiles.
-__device__ __forceinline__ float2 merge_row_stats(const float2 *__restrict__ st, int tiles, int K) {
+__device__ __forceinline__ float2 merge_row_stats(const float2 *st, int tiles, int K) {
   float m = 0.f, q = 0.f;
-  float2 v[GS_MAX_TILES > 16 ? 16 : GS_MAX_TILES];
-  if (tiles <= 16) {  // all in flight together
-#pragma unroll
-    for (int t = 0; t < 16; t++) v[t] = t < tiles ? __ldcg(st + t) : make_float2(0.f, 0.f);
-#pragma unroll
-    for (int t = 0; t < 16; t++) m += t < tiles ? v[t].x * (float)min(128, K - 128 * t) : 0.f;
-    m /= (float)K;
-#pragma unroll
-    for (int t = 0; t < 16; t++)
-      if (t < tiles) q += v[t].y + (float)min(128, K - 128 * t) * (v[t].x - m) * (v[t].x - m);
-  } else {
-    for (int t = 0; t < tiles; t++) m += __ldcg(st + t).x * (float)min(128, K - 128 * t);
-    m /= (float)K;
-    for (int t = 0; t < tiles; t++) {
-      const float2 a = __ldcg(st + t);
-      q += a.y + (float)min(128, K - 128 * t) * (a.x - m) * (a.x - m);
-    }
-  }
+#pragma unroll 4
+  for (int t = 0; t < tiles; t++) m += st[t].x * (float)min(128, K - 128 * t);
+  m /= (float)K;
+#pragma unroll 4
+  for (int t = 0; t < tiles; t++) q += st[t].y + (float)min(128, K - 128 * t) * (st[t].x - m) * (st[t].x - m);
   return make_float2(m, 1.0f / sqrtf(q / (float)K + 1e-5f));
 }
 
 // grid.x = row tiles x feature tiles x S, cluster (S, 1, 1). map_w: box of 128 rows; map_x (RN == 0): box of rn rows.
 // RN == 0: activations as planes by TMA, rn at run time. RN > 0: normalised on the way in, rn == RN.
 template <int RN>
-__global__ void __launch_bounds__(GS_THREADS, 1)
+__global__ void __launch_bounds__(GS_THREADS, 2)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                   const __grid_constant__ SplitArgs p) {
   extern __shared__ uint8_t gs_smem_raw[];
@@ -100,8 +108,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   __shared__ float2 row_norm[RN > 0 ? RN : 1];
   volatile int *abort_flag = &abort_word;
   float *part = reinterpret_cast<float *>(tiles);  // [rn][128], over the ring once its last tile has been read
+  // LayerNorm scale and shift of this CTA's slice of K (times x_scale), behind the ring
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int rn = RN > 0 ? RN : p.rn;
   uint32_t S;
   asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(S));
@@ -110,7 +119,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   const int total_kb = (p.K + GP_BK - 1) / GP_BK;
   const int kb0 = (int)((long long)total_kb * rank / S), nkb = (int)((long long)total_kb * (rank + 1) / S) - kb0;
   const int stages = p.stages, stage_bytes = GS_W_BYTES + rn * (GP_BK * 4);
-  const uint32_t tmem_cols = rn <= 32 ? 32u : (rn <= 64 ? 64u : 128u);
+  float4 *gam = reinterpret_cast<float4 *>(tiles + (size_t)stages * stage_bytes), *bet = gam + nkb * (GP_BK / 4);
+  float2 *tile_st = reinterpret_cast<float2 *>(bet + nkb * (GP_BK / 4));  // [rows][x_tiles], as their producers left them
+  const uint32_t tmem_cols = rn <= 16 ? 32u : (rn <= 32 ? 64u : (rn <= 64 ? 128u : 256u));
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < stages; i++) {
@@ -128,6 +139,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     }
   }
   if (warp == 1) tmem_alloc(&tmem_slot, tmem_cols);
+  if (RN > 0) {
+    for (int i = threadIdx.x; i < nkb * (GP_BK / 4); i += GS_THREADS) {
+      const int col = kb0 * GP_BK + 4 * i;
+      const bool in = col < p.K;  // past the end both are zero, and so is what is multiplied
+      gam[i] = in ? scale4(__ldg(reinterpret_cast<const float4 *>(p.gamma + col)), p.x_scale) : make_float4(0.f, 0.f, 0.f, 0.f);
+      bet[i] = in ? scale4(__ldg(reinterpret_cast<const float4 *>(p.beta + col)), p.x_scale) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -168,42 +187,36 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = f16_idesc(128, rn), desc0 = umma_desc_lo(smem_addr(tiles));
-      const uint32_t x_plane = ((uint32_t)rn * (GP_BK * 2)) >> 4;
-      for (int j = 0; j < nkb; j++) {
-        const int s = j % stages, use = j / stages;
-        if (*abort_flag || !mbar_wait(&full_w[s], use & 1, TC_POLLS) || !mbar_wait(&full_x[s], use & 1, TC_POLLS)) {
-          *abort_flag = 1;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t w0 = desc0 + (uint32_t)s * ((uint32_t)stage_bytes >> 4), w1 = w0 + (GS_W_BYTES >> 5);
-        const uint32_t x0 = w0 + (GS_W_BYTES >> 4), x1 = x0 + x_plane;
+    // the whole warp runs this loop and one elected lane issues (see umma1_f16)
+    const uint32_t idesc = f16_idesc(128, rn), idesc2 = f16_idesc(128, 2 * rn), desc0 = umma_desc_lo(smem_addr(tiles));
+    for (int j = 0; j < nkb; j++) {
+      const int s = j % stages, use = j / stages;
+      if (!mbar_wait(&full_w[s], use & 1, TC_POLLS) || !mbar_wait(&full_x[s], use & 1, TC_POLLS)) *abort_flag = 1;
+      if (__any_sync(0xffffffffu, *abort_flag)) break;
+      tc_fence_after();
+      const uint32_t w0 = desc0 + (uint32_t)s * ((uint32_t)stage_bytes >> 4), w1 = w0 + (GS_W_BYTES >> 5);
+      const uint32_t x0 = w0 + (GS_W_BYTES >> 4);
 #pragma unroll
-        for (int k = 0; k < GP_BK / 16; k++) {
-          umma1_f16(tmem_acc, w0 + 2 * k, x0 + 2 * k, idesc, (j > 0 || k > 0) ? 1u : 0u);
-          umma1_f16(tmem_acc, w0 + 2 * k, x1 + 2 * k, idesc, 1u);
-          umma1_f16(tmem_acc, w1 + 2 * k, x0 + 2 * k, idesc, 1u);
-        }
-        umma_commit(&empty[s]);
+      for (int k = 0; k < GP_BK / 16; k++) {
+        umma1_f16(tmem_acc, w0 + 2 * k, x0 + 2 * k, idesc2, (j > 0 || k > 0) ? 1u : 0u);
+        umma1_f16(tmem_acc + (uint32_t)rn, w1 + 2 * k, x0 + 2 * k, idesc, 1u);
       }
-      umma_commit(&acc_full);  // (also reached after an abort)
+      umma_commit_elect(&empty[s]);
     }
-    __syncwarp();
+    umma_commit_elect(&acc_full);  // (also reached after an abort)
   } else if (RN > 0) {
     // ---------------- activations: 16 lanes per row (one float4 each), 12 rows per step ----------------
     constexpr int ITERS = RN > 0 ? (RN + 11) / 12 : 1, G = 12 / ITERS;  // G k-blocks of loads in flight together
     const int t = threadIdx.x - 64, k4 = t & 15, mrow = t >> 4;
     const int rows = min(RN, p.M - row0);
+    // the statistics first (every thread a few of them), then the rows: both are in flight together
+    for (int i = t; i < rows * p.x_tiles; i += GS_STAGERS) tile_st[i] = __ldcg(p.x_stats + (size_t)row0 * p.x_tiles + i);
     for (int j0 = 0; j0 < nkb; j0 += G) {
-      float4 v[G][ITERS], gm[G], bt[G];
+      float4 v[G][ITERS];
 #pragma unroll
       for (int g = 0; g < G; g++) {
         const int col = (kb0 + j0 + g) * GP_BK + 4 * k4;
         const bool in = j0 + g < nkb && col < p.K;
-        gm[g] = in ? __ldg(reinterpret_cast<const float4 *>(p.gamma + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
-        bt[g] = in ? __ldg(reinterpret_cast<const float4 *>(p.beta + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int i = 0; i < ITERS; i++) {
           const int m = mrow + 12 * i;
@@ -212,7 +225,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         }
       }
       if (j0 == 0) {
-        if (t < rows) row_norm[t] = merge_row_stats(p.x_stats + (size_t)(row0 + t) * p.x_tiles, p.x_tiles, p.K);
+        asm volatile("bar.sync 1, %0;" ::"n"(GS_STAGERS) : "memory");
+        if (t < rows) row_norm[t] = merge_row_stats(tile_st + t * p.x_tiles, p.x_tiles, p.K);
         asm volatile("bar.sync 1, %0;" ::"n"(GS_STAGERS) : "memory");
       }
 #pragma unroll
@@ -222,7 +236,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const int s = j % stages, use = j / stages;
         if (j >= stages && (*abort_flag || !mbar_wait(&empty[s], (use & 1) ^ 1, TC_POLLS))) { *abort_flag = 1; break; }
         const uint32_t xt = smem_addr(tiles + (size_t)s * stage_bytes) + GS_W_BYTES;
-        const float4 ga = scale4(gm[g], p.x_scale), be = scale4(bt[g], p.x_scale);
+        const float4 ga = gam[j * (GP_BK / 4) + k4], be = bet[j * (GP_BK / 4) + k4];
 #pragma unroll
         for (int i = 0; i < ITERS; i++) {
           const int m = mrow + 12 * i;
@@ -248,13 +262,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     if (!mbar_wait(&acc_full, 0, TC_POLLS << 2)) *abort_flag = 1;
     tc_fence_after();
     const int quad = warp & 3;
+    const uint32_t lanes = tmem_acc + ((uint32_t)(quad * 32) << 16);
 #pragma unroll 1
-    for (int c = 0; c < rn; c += 32) {
-      float v[32];
-      tmem_ld_32x32(tmem_acc + ((uint32_t)(quad * 32) << 16) + (uint32_t)c, v);
+    for (int c = 0; c < rn; c += 16) {
+      float v[16], w[16];
+      tmem_ld_2x16(lanes + (uint32_t)c, lanes + (uint32_t)(rn + c), v, w);
 #pragma unroll
-      for (int j = 0; j < 32; j++)
-        if (c + j < rn) part[(c + j) * 128 + quad * 32 + lane] = v[j];
+      for (int j = 0; j < 16; j++) part[(c + j) * 128 + quad * 32 + lane] = v[j] + w[j];
     }
     tc_fence_before();
   }
@@ -268,32 +282,42 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 
   const int cnt = min(128, p.N - f0);
   const uint32_t pbase = smem_addr(part) + (uint32_t)lane * 16u;
-  for (int r = r_beg + warp; r < r_end; r += GS_THREADS / 32) {
-    const int m = row0 + r;
-    if (m >= p.M) break;
-    float4 res = res_first;
-    if (r != r_beg + warp && e.residual != nullptr && n_live)
-      res = __ldcg(reinterpret_cast<const float4 *>(e.residual + (size_t)m * e.ld + n));
-    float4 q[8];
+  constexpr int NW = GS_THREADS / 32;
+  for (int r = r_beg + warp; r < r_end; r += 2 * NW) {  // two rows at a time: their remote reads are in flight together
+    const int m0 = row0 + r, m1 = m0 + NW;
+    if (m0 >= p.M) break;
+    const bool two = r + NW < r_end && m1 < p.M;
+    float4 res[2] = {res_first, make_float4(0.f, 0.f, 0.f, 0.f)};
+    if (e.residual != nullptr && n_live) {
+      if (r != r_beg + warp) res[0] = __ldcg(reinterpret_cast<const float4 *>(e.residual + (size_t)m0 * e.ld + n));
+      if (two) res[1] = __ldcg(reinterpret_cast<const float4 *>(e.residual + (size_t)m1 * e.ld + n));
+    }
+    float4 q[2][8];
     const uint32_t at = pbase + (uint32_t)r * 512u;
 #pragma unroll
     for (int s = 0; s < 8; s++)
       if (s < (int)S) {
         uint32_t ra;
         asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(at), "r"(s));
-        q[s] = dsmem_ld4(ra);
+        q[0][s] = dsmem_ld4(ra);
+        if (two) q[1][s] = dsmem_ld4(ra + NW * 512u);
       }
-    float4 v = q[0];
 #pragma unroll
-    for (int s = 1; s < 8; s++)
-      if (s < (int)S) v = add4(v, q[s]);
-    if (n_live) {
-      v = pair_epi_value4(e, v, cs, bs, res, m);
-      pair_epi_store4(e, v, m, n);
-    }
-    if (p.stats != nullptr) {
-      const float2 st = tile_row_stats(v, n_live, cnt);
-      if (lane == 0) p.stats[(size_t)m * p.f_tiles + ft] = st;
+    for (int u = 0; u < 2; u++) {
+      if (u == 1 && !two) break;
+      const int m = u == 0 ? m0 : m1;
+      float4 v = q[u][0];
+#pragma unroll
+      for (int s = 1; s < 8; s++)
+        if (s < (int)S) v = add4(v, q[u][s]);
+      if (n_live) {
+        v = pair_epi_value4(e, v, cs, bs, res[u], m);
+        pair_epi_store4(e, v, m, n);
+      }
+      if (p.stats != nullptr) {
+        const float2 st = tile_row_stats(v, n_live, cnt);
+        if (lane == 0) p.stats[(size_t)m * p.f_tiles + ft] = st;
+      }
     }
   }
   if (S > 1) {  // no CTA leaves while another may still read its partial tile (nothing is published by this barrier)
