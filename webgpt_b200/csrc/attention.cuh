@@ -103,25 +103,42 @@ attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict
 
   float m = -INFINITY, l = 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  // The trip count is the same for every lane of the warp (the shuffles below name all 32 lanes); a group whose
-  // position falls past the end of the slice runs the iteration with `valid` false and contributes nothing.
-#pragma unroll 2
-  for (int j0 = beg + warp * G; j0 < end; j0 += NW * G) {
-    const int j = j0 + g;
-    const bool valid = j < end;
-    const int jj = valid ? j : end - 1;  // in-bounds address for the idle group
-    float4 k4 = __ldcg(reinterpret_cast<const float4 *>(kb + (size_t)jj * ldkv));
-    float4 v4 = __ldcg(reinterpret_cast<const float4 *>(vb + (size_t)jj * ldkv));
-    float s = dot4(q4, k4);
+  // Four positions per group and step: eight cache rows in flight per thread (a step is one round trip to HBM, so with two
+  // the loop was a chain of twice as many), one maximum and one rescale for the four. The trip count is the same for
+  // every lane of the warp (the shuffles below name all 32 lanes); a position past the end of the slice reads an
+  // in-bounds row and contributes nothing.
+  constexpr int U = 4;
+  for (int j0 = beg + warp * G; j0 < end; j0 += NW * G * U) {
+    float4 k4[U], v4[U];
 #pragma unroll
-    for (int o = LPP / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (valid) {
-      s *= scale;
-      float mn = fmaxf(m, s);
-      float corr = expf(m - mn), p = expf(s - mn);  // m = -inf on the first key: corr = 0
-      l = l * corr + p;
-      acc.x = acc.x * corr + p * v4.x; acc.y = acc.y * corr + p * v4.y;
-      acc.z = acc.z * corr + p * v4.z; acc.w = acc.w * corr + p * v4.w;
+    for (int u = 0; u < U; u++) {
+      const int jj = min(j0 + u * NW * G + g, end - 1);
+      k4[u] = __ldcg(reinterpret_cast<const float4 *>(kb + (size_t)jj * ldkv));
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int jj = min(j0 + u * NW * G + g, end - 1);
+      v4[u] = __ldcg(reinterpret_cast<const float4 *>(vb + (size_t)jj * ldkv));
+    }
+    float s[U], mn = m;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      s[u] = dot4(q4, k4[u]);
+#pragma unroll
+      for (int o = LPP / 2; o > 0; o >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+      s[u] = j0 + u * NW * G + g < end ? s[u] * scale : -INFINITY;
+      mn = fmaxf(mn, s[u]);
+    }
+    if (mn != -INFINITY) {  // otherwise this group has seen no position yet
+      const float corr = expf(m - mn);  // m = -inf on the first step: 0
+      l *= corr;
+      acc.x *= corr; acc.y *= corr; acc.z *= corr; acc.w *= corr;
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const float pr = expf(s[u] - mn);  // exactly 0 for a position past the end
+        l += pr;
+        acc.x += pr * v4[u].x; acc.y += pr * v4[u].y; acc.z += pr * v4[u].z; acc.w += pr * v4[u].w;
+      }
       m = mn;
     }
   }

@@ -210,7 +210,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const int t = threadIdx.x - 64, k4 = t & 15, mrow = t >> 4;
     const int rows = min(RN, p.M - row0);
     // the statistics first (every thread a few of them), then the rows: both are in flight together
-    for (int i = t; i < rows * p.x_tiles; i += GS_STAGERS) tile_st[i] = __ldcg(p.x_stats + (size_t)row0 * p.x_tiles + i);
+    constexpr int NST = 4;
+    const int n_st = rows * p.x_tiles;
+    const float2 *st_src = p.x_stats + (size_t)row0 * p.x_tiles;
+    float2 st_pre[NST];
+#pragma unroll
+    for (int i = 0; i < NST; i++) st_pre[i] = t + GS_STAGERS * i < n_st ? __ldcg(st_src + t + GS_STAGERS * i) : make_float2(0.f, 0.f);
     for (int j0 = 0; j0 < nkb; j0 += G) {
       float4 v[G][ITERS];
 #pragma unroll
@@ -225,6 +230,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         }
       }
       if (j0 == 0) {
+#pragma unroll
+        for (int i = 0; i < NST; i++)
+          if (t + GS_STAGERS * i < n_st) tile_st[t + GS_STAGERS * i] = st_pre[i];
+        for (int i = t + GS_STAGERS * NST; i < n_st; i += GS_STAGERS) tile_st[i] = __ldcg(st_src + i);
         asm volatile("bar.sync 1, %0;" ::"n"(GS_STAGERS) : "memory");
         if (t < rows) row_norm[t] = merge_row_stats(tile_st + t * p.x_tiles, p.x_tiles, p.K);
         asm volatile("bar.sync 1, %0;" ::"n"(GS_STAGERS) : "memory");
