@@ -990,21 +990,33 @@ static bool attn_prefill_uses_mma(const wgpt_device *dev, int hs, int n_tok) {
   return hs == 64 && mma64 && dev->precision != WGPT_PRECISION_FP32 && n_tok >= 16;
 }
 
-// planes: the output as a pair (only where attn_prefill_uses_mma; the other kernels write FP32 to out).
+// Prefill attention of a pair model (head size 64, attn_prefill_uses_mma): output planes [2][rows][ldo]. Windows of more
+// than 64 tokens share each staged key tile among 128 query rows.
+static int32_t launch_attn_prefill_pair(wgpt_device *dev, const float *q, int ldq, const float *kc, const float *vc,
+                                        int ldkv, size_t kv_seq_stride, int n_tok, int n_seq, int H, const int *pos,
+                                        float scale, float s_qk, float s_v, __half *planes, size_t plane, int ldo) {
+  if (n_tok > 64)
+    LAUNCH_PDL(dev, attn_prefill64_pair_kernel<8>, dim3((n_tok + 127) / 128, H, n_seq), 256, 0, q, ldq, kc, vc, ldkv,
+               kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes, plane, ldo);
+  else
+    LAUNCH_PDL(dev, attn_prefill64_pair_kernel<4>, dim3((n_tok + 63) / 64, H, n_seq), 128, 0, q, ldq, kc, vc, ldkv,
+               kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes, plane, ldo);
+  return WGPT_OK;
+}
+
 static int32_t launch_attn_prefill(wgpt_device *dev, int hs, const float *q, int ldq, const float *kc, const float *vc,
                                    int ldkv, size_t kv_seq_stride, float *out, int ldo, int n_tok, int n_seq, int H,
-                                   const int *pos, float scale, __half *planes = nullptr, size_t plane = 0,
-                                   float pair_scale = 1.f) {
+                                   const int *pos, float scale) {
   static const bool tiled64 = [] { const char *ev = getenv("WGPT_ATTN_PREFILL64"); return !(ev && ev[0] == '0'); }();
   if (attn_prefill_uses_mma(dev, hs, n_tok) && (ldq % 4) == 0 && (ldkv % 4) == 0 && (ldo % 2) == 0) {
     // products in TF32 / 3xTF32: the warp-level tensor-core kernel; FP32 mode keeps the CUDA-core kernels below
     dim3 grid((n_tok + 63) / 64, H, n_seq);
     if (dev->precision == WGPT_PRECISION_TF32X3)
       LAUNCH(dev, attn_prefill64_mma_kernel<true>, grid, 128, 0, q, ldq, kc, vc, ldkv, kv_seq_stride, out, ldo, n_tok, pos,
-             scale, planes, plane, pair_scale);
+             scale);
     else
       LAUNCH(dev, attn_prefill64_mma_kernel<false>, grid, 128, 0, q, ldq, kc, vc, ldkv, kv_seq_stride, out, ldo, n_tok,
-             pos, scale, planes, plane, pair_scale);
+             pos, scale);
     return WGPT_OK;
   }
   if (hs == 64 && tiled64 && n_tok >= 16 && (ldq % 4) == 0 && (ldkv % 4) == 0 && (ldo % 4) == 0) {
@@ -2115,9 +2127,12 @@ static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
         ap.part = s->attn_part; ap.n_split = s->n_split; ap.H = H; ap.hs = hs;
         LAUNCH_PDL(dev, attn_merge_kernel, dim3((E / 4 + 127) / 128, M), 128, 0, ap, s->o, E);
       }
+    } else if (o_pair) {
+      TRY(launch_attn_prefill_pair(dev, s->q, E, kc, vc, E, (size_t)p.n_ctx, n_tok, s->n_seq, H, s->d_pos, m->scale,
+                                   L.s_qk, L.s_o, o, plane_e, E));
     } else {
       TRY(launch_attn_prefill(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, n_tok, s->n_seq, H, s->d_pos,
-                              m->scale, o_pair ? o : nullptr, plane_e, L.s_o));
+                              m->scale));
     }
     const __half *o_in = o;
     if (!o_pair) {  // an attention kernel that writes FP32 rows

@@ -7,6 +7,7 @@
 // j at base + (s*kv_seq_stride + j)*ldkv, same column convention (the reference's [T, E] K/V buffers).
 #pragma once
 #include "common.cuh"
+#include "pair.cuh"
 
 namespace wgpt {
 
@@ -525,8 +526,7 @@ template <bool X3>
 __global__ void __launch_bounds__(128)
 attn_prefill64_mma_kernel(const float *__restrict__ q, int ldq, const float *__restrict__ kc,
                           const float *__restrict__ vc, int ldkv, size_t kv_seq_stride, float *__restrict__ out,
-                          int ldo, int n_tok, const int *__restrict__ pos, float scale, __half *__restrict__ planes,
-                          size_t plane, float pair_scale) {
+                          int ldo, int n_tok, const int *__restrict__ pos, float scale) {
   constexpr int HS = 64, T = 64, KLD = kAttnMmaKLd, VLD = kAttnMmaVLd;
   __shared__ __align__(16) float Ks[T * KLD];
   __shared__ __align__(16) float Vs[T * VLD];
@@ -658,24 +658,226 @@ attn_prefill64_mma_kernel(const float *__restrict__ q, int ldq, const float *__r
   l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
   const float i0 = 1.f / l0, i1 = 1.f / l1;
-  // planes != nullptr: the output goes out as a pair of half-precision planes (pair.cuh), rows of ldo values
-  auto put = [&](int r, int d, float x, float y) {
-    const size_t at = ((size_t)seq * n_tok + t0 + r) * ldo + h * HS + d;
-    if (planes == nullptr) {
-      *reinterpret_cast<float2 *>(out + at) = make_float2(x, y);
-    } else {
-      x *= pair_scale;
-      y *= pair_scale;
-      const __half2 a = __floats2half2_rn(x, y);
-      const float2 f = __half22float2(a);
-      *reinterpret_cast<__half2 *>(planes + at) = a;
-      *reinterpret_cast<__half2 *>(planes + plane + at) = __floats2half2_rn(x - f.x, y - f.y);
-    }
-  };
 #pragma unroll
   for (int j = 0; j < 8; j++) {
-    if (r0 < nq) put(r0, 8 * j + 2 * t, o[j][0] * i0, o[j][1] * i0);
-    if (r1 < nq) put(r1, 8 * j + 2 * t, o[j][2] * i1, o[j][3] * i1);
+    if (r0 < nq)
+      *reinterpret_cast<float2 *>(out + ((size_t)seq * n_tok + t0 + r0) * ldo + h * HS + 8 * j + 2 * t) =
+          make_float2(o[j][0] * i0, o[j][1] * i0);
+    if (r1 < nq)
+      *reinterpret_cast<float2 *>(out + ((size_t)seq * n_tok + t0 + r1) * ldo + h * HS + 8 * j + 2 * t) =
+          make_float2(o[j][2] * i1, o[j][3] * i1);
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// The same for a model whose matrices are pairs of half-precision planes (pair.cuh): queries, keys, values and
+// probabilities are split into pairs (scaled by powers of two whose bounds are known at load; probabilities by 2^15) and
+// each product is h0 h0 + h0 h1 + h1 h0 through mma.sync.m16n8k16, half the instructions of the TF32 form at the same
+// terms. K and V tiles are split once, while they are staged, instead of by every warp at every fragment; fragments come
+// by ldmatrix; the score accumulators of two 8-key tiles are the A fragment of a 16-key value step as they are, so the
+// probabilities need no shuffles. 16 WARPS query rows per CTA share a staged 64-key tile. Output as a pair.
+constexpr int kAttnPairLd = 72;  // halves per staged row: 144 bytes, so that the eight rows of an ldmatrix hit all banks
+
+__device__ __forceinline__ void mma_f16_16x8x16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t saddr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr));
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t saddr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr));
+}
+// Two values as a half pair: the first planes' word, and the second planes'.
+__device__ __forceinline__ uint32_t pair_word(float x, float y, uint32_t &lo) {
+  const __half2 a = __floats2half2_rn(x, y);
+  const float2 f = __half22float2(a);
+  const __half2 b = __floats2half2_rn(x - f.x, y - f.y);
+  lo = *reinterpret_cast<const uint32_t *>(&b);
+  return *reinterpret_cast<const uint32_t *>(&a);
+}
+
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS)
+attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__restrict__ kc,
+                           const float *__restrict__ vc, int ldkv, size_t kv_seq_stride, int n_tok,
+                           const int *__restrict__ pos, float scale, float s_qk, float s_v,
+                           __half *__restrict__ planes, size_t plane, int ldo) {
+  constexpr int HS = 64, TQ = 16 * WARPS, T = 64, LD = kAttnPairLd, NT = 32 * WARPS;
+  __shared__ __align__(16) __half Ks[2][T * LD];
+  __shared__ __align__(16) __half Vs[2][T * LD];
+  const int h = blockIdx.y, seq = blockIdx.z;
+  const int t0 = (int)(gridDim.x - 1 - blockIdx.x) * TQ;  // the query tiles with the most keys first
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int pos0 = pos ? __ldcg(pos) : 0;
+  const int nq = min(TQ, n_tok - t0);
+  const int last_key = pos0 + t0 + nq - 1;  // newest key any query of this tile may see
+  const int r0 = 16 * warp + g, r1 = r0 + 8;
+  const int p0 = pos0 + t0 + min(r0, nq - 1), p1 = pos0 + t0 + min(r1, nq - 1);  // rows past the end shadow the last
+  const int warp_last = pos0 + t0 + min(16 * warp + 15, nq - 1);
+  const bool warp_live = 16 * warp < nq;
+
+  // ---- Q fragments: element (row, dim) pairs straight from global memory, once
+  uint32_t qh[4][4], ql[4][4];
+  {
+    const float *q0 = q + ((size_t)seq * n_tok + t0 + min(r0, nq - 1)) * ldq + h * HS + 2 * t;
+    const float *q1 = q + ((size_t)seq * n_tok + t0 + min(r1, nq - 1)) * ldq + h * HS + 2 * t;
+#pragma unroll
+    for (int ks = 0; ks < 4; ks++) {
+      const float2 a = __ldcg(reinterpret_cast<const float2 *>(q0 + 16 * ks)), b = __ldcg(reinterpret_cast<const float2 *>(q1 + 16 * ks));
+      const float2 c = __ldcg(reinterpret_cast<const float2 *>(q0 + 16 * ks + 8)), d = __ldcg(reinterpret_cast<const float2 *>(q1 + 16 * ks + 8));
+      qh[ks][0] = pair_word(a.x * s_qk, a.y * s_qk, ql[ks][0]);
+      qh[ks][1] = pair_word(b.x * s_qk, b.y * s_qk, ql[ks][1]);
+      qh[ks][2] = pair_word(c.x * s_qk, c.y * s_qk, ql[ks][2]);
+      qh[ks][3] = pair_word(d.x * s_qk, d.y * s_qk, ql[ks][3]);
+    }
+  }
+  const float *kb = kc + (size_t)seq * kv_seq_stride * ldkv + h * HS;
+  const float *vb = vc + (size_t)seq * kv_seq_stride * ldkv + h * HS;
+  const float score_scale = scale / (s_qk * s_qk);
+
+  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+  float o[8][4];
+#pragma unroll
+  for (int j = 0; j < 8; j++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) o[j][e] = 0.f;
+  // ldmatrix row addresses of this lane: keys (lane & 7) + 8 (lane >> 4), dims 8 ((lane >> 3) & 1) for K (two 8-key tiles
+  // x 16 dims); keys (lane & 15), dims 8 (lane >> 4) for V, transposed (16 keys x two 8-dim tiles)
+  const uint32_t k_row = smem_addr(&Ks[0][0]) + 2u * (uint32_t)(((lane & 7) + 8 * (lane >> 4)) * LD + 8 * ((lane >> 3) & 1));
+  const uint32_t v_row = smem_addr(&Vs[0][0]) + 2u * (uint32_t)((lane & 15) * LD + 8 * (lane >> 4));
+  constexpr uint32_t kPlane = 2u * T * LD;
+
+  for (int j0 = 0; j0 <= last_key; j0 += T) {
+    __syncthreads();  // the previous tile is no longer read
+    {
+      constexpr int PER = T * (HS / 4) / NT;  // float4 of K (and of V) per thread
+      float4 kv[PER], vv[PER];
+#pragma unroll
+      for (int i = 0; i < PER; i++) {
+        const int idx = tid + NT * i, r = idx >> 4, c4 = (idx & 15) * 4;
+        const size_t at = (size_t)min(j0 + r, last_key) * ldkv + c4;
+        kv[i] = __ldcg(reinterpret_cast<const float4 *>(kb + at));
+        vv[i] = __ldcg(reinterpret_cast<const float4 *>(vb + at));
+      }
+#pragma unroll
+      for (int i = 0; i < PER; i++) {
+        const int idx = tid + NT * i, r = idx >> 4, c4 = (idx & 15) * 4;
+        uint2 a, b;
+        pair_split4(scale4(kv[i], s_qk), a, b);
+        *reinterpret_cast<uint2 *>(&Ks[0][r * LD + c4]) = a;
+        *reinterpret_cast<uint2 *>(&Ks[1][r * LD + c4]) = b;
+        pair_split4(scale4(vv[i], s_v), a, b);
+        *reinterpret_cast<uint2 *>(&Vs[0][r * LD + c4]) = a;
+        *reinterpret_cast<uint2 *>(&Vs[1][r * LD + c4]) = b;
+      }
+    }
+    __syncthreads();
+    if (!warp_live || j0 > warp_last) continue;  // every key of the tile is masked for this warp's rows
+
+    // ---- scores: 16 rows x 64 keys as eight 16x8 accumulators, two per ldmatrix
+    float s[8][4];
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+#pragma unroll
+      for (int e = 0; e < 4; e++) s[j][e] = 0.f;
+#pragma unroll
+    for (int jp = 0; jp < 4; jp++) {
+#pragma unroll
+      for (int ks = 0; ks < 4; ks++) {
+        uint32_t kh[4], kl[4];
+        ldmatrix_x4(kh, k_row + 2u * (uint32_t)(16 * jp * LD + 16 * ks));
+        ldmatrix_x4(kl, k_row + kPlane + 2u * (uint32_t)(16 * jp * LD + 16 * ks));
+        mma_f16_16x8x16(s[2 * jp], qh[ks], kh[0], kh[1]);
+        mma_f16_16x8x16(s[2 * jp + 1], qh[ks], kh[2], kh[3]);
+        mma_f16_16x8x16(s[2 * jp], qh[ks], kl[0], kl[1]);
+        mma_f16_16x8x16(s[2 * jp + 1], qh[ks], kl[2], kl[3]);
+        mma_f16_16x8x16(s[2 * jp], ql[ks], kh[0], kh[1]);
+        mma_f16_16x8x16(s[2 * jp + 1], ql[ks], kh[2], kh[3]);
+      }
+    }
+    // ---- online softmax of rows r0 (elements 0, 1) and r1 (elements 2, 3); key of element e: j0 + 8j + 2t + (e & 1)
+    float mx0 = -INFINITY, mx1 = -INFINITY;
+    const bool masked = j0 + T - 1 > pos0 + t0 + 16 * warp;  // same for the whole warp: some key is beyond some row
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        s[j][e] *= score_scale;
+        if (masked) {
+          const int key = j0 + 8 * j + 2 * t + (e & 1);
+          if (key > (e < 2 ? p0 : p1)) s[j][e] = -INFINITY;
+        }
+      }
+      mx0 = fmaxf(mx0, fmaxf(s[j][0], s[j][1]));
+      mx1 = fmaxf(mx1, fmaxf(s[j][2], s[j][3]));
+    }
+    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1)); mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
+    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+    const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);  // finite: key 0 of the first tile is visible to every row
+    const float c0 = expf(m0 - mn0), c1 = expf(m1 - mn1);
+    float ps0 = 0.f, ps1 = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      s[j][0] = expf(s[j][0] - mn0);
+      s[j][1] = expf(s[j][1] - mn0);
+      s[j][2] = expf(s[j][2] - mn1);
+      s[j][3] = expf(s[j][3] - mn1);
+      ps0 += s[j][0] + s[j][1];
+      ps1 += s[j][2] + s[j][3];
+    }
+    l0 = l0 * c0 + ps0; m0 = mn0;  // l holds this lane's share of the row sum
+    l1 = l1 * c1 + ps1; m1 = mn1;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      o[j][0] *= c0; o[j][1] *= c0; o[j][2] *= c1; o[j][3] *= c1;
+    }
+    // ---- values
+#pragma unroll
+    for (int ks = 0; ks < 4; ks++) {
+      uint32_t ph[4], pl[4];
+      ph[0] = pair_word(s[2 * ks][0] * kPairTop, s[2 * ks][1] * kPairTop, pl[0]);
+      ph[1] = pair_word(s[2 * ks][2] * kPairTop, s[2 * ks][3] * kPairTop, pl[1]);
+      ph[2] = pair_word(s[2 * ks + 1][0] * kPairTop, s[2 * ks + 1][1] * kPairTop, pl[2]);
+      ph[3] = pair_word(s[2 * ks + 1][2] * kPairTop, s[2 * ks + 1][3] * kPairTop, pl[3]);
+#pragma unroll
+      for (int jp = 0; jp < 4; jp++) {
+        uint32_t vh[4], vl[4];
+        ldmatrix_x4_trans(vh, v_row + 2u * (uint32_t)(16 * ks * LD + 16 * jp));
+        ldmatrix_x4_trans(vl, v_row + kPlane + 2u * (uint32_t)(16 * ks * LD + 16 * jp));
+        mma_f16_16x8x16(o[2 * jp], ph, vh[0], vh[1]);
+        mma_f16_16x8x16(o[2 * jp + 1], ph, vh[2], vh[3]);
+        mma_f16_16x8x16(o[2 * jp], ph, vl[0], vl[1]);
+        mma_f16_16x8x16(o[2 * jp + 1], ph, vl[2], vl[3]);
+        mma_f16_16x8x16(o[2 * jp], pl, vh[0], vh[1]);
+        mma_f16_16x8x16(o[2 * jp + 1], pl, vh[2], vh[3]);
+      }
+    }
+  }
+  if (!warp_live) return;
+  l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+  l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+  // the values' own scale is also the output pair's
+  const float i0 = 1.f / (l0 * kPairTop), i1 = 1.f / (l1 * kPairTop);
+#pragma unroll
+  for (int j = 0; j < 8; j++) {
+    uint32_t lo;
+    if (r0 < nq) {
+      __half *at = planes + ((size_t)seq * n_tok + t0 + r0) * ldo + h * HS + 8 * j + 2 * t;
+      *reinterpret_cast<uint32_t *>(at) = pair_word(o[j][0] * i0, o[j][1] * i0, lo);
+      *reinterpret_cast<uint32_t *>(at + plane) = lo;
+    }
+    if (r1 < nq) {
+      __half *at = planes + ((size_t)seq * n_tok + t0 + r1) * ldo + h * HS + 8 * j + 2 * t;
+      *reinterpret_cast<uint32_t *>(at) = pair_word(o[j][2] * i1, o[j][3] * i1, lo);
+      *reinterpret_cast<uint32_t *>(at + plane) = lo;
+    }
   }
 }
 
