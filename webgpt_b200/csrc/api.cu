@@ -820,15 +820,21 @@ static int32_t make_pair_map(CUtensorMap *map, const __half *planes, uint64_t ro
 }
 
 // Tile width of gemm_pair_kernel: the multiple of 32 whose rounds over the pairs cost least, a tile costing
-// max(tensor pipe, shared memory) cycles per k-block (gemm_pair.cuh).
-static int pair_tile_columns(const wgpt_device *dev, int M, int N) {
+// max(tensor pipe, shared memory) cycles per k-block (gemm_pair.cuh). *cycles: the estimate with 40 bytes per cycle from
+// L2 as a third bound and 12 000 cycles for the first copies and the last epilogue, to compare with gemm_split_kernel.
+static int pair_tile_columns(const wgpt_device *dev, int M, int N, int K = 0, double *cycles = nullptr) {
   const int pairs = dev->sm_count / 2, m_tiles = (M + 255) / 256;
   int best = 256;
   long long best_cost = -1;
   for (int bn = 256; bn >= 64; bn -= 32) {
     const long long rounds = ((long long)m_tiles * ((N + bn - 1) / bn) + pairs - 1) / pairs;
     const long long cost = rounds * (6 * bn > 640 + 5 * bn / 2 ? 6 * bn : 640 + 5 * bn / 2);
-    if (best_cost < 0 || cost < best_cost) { best = bn; best_cost = cost; }
+    if (best_cost < 0 || cost < best_cost) {
+      best = bn;
+      best_cost = cost;
+      const double per_kb = fmax((double)cost / rounds, 820 + 3.2 * bn);
+      if (cycles) *cycles = rounds * per_kb * ((K + GP_BK - 1) / GP_BK) + 12000;
+    }
   }
   return best;
 }
@@ -926,6 +932,31 @@ static SplitShape split_shape_decode(const wgpt_device *dev, int M, int K, int N
   return sh;
 }
 
+// Any number of rows, activations as planes: row tiles of up to 128 and K slices by the same kind of estimate
+// (pair_tile_columns): a k-block costs max(6 RN tensor-core cycles, 32 KB + 256 RN bytes from L2 at 40 a cycle), a round
+// 9000 cycles of start, exchange and store and 60 more per row of the tile.
+static SplitShape split_shape_rows(const wgpt_device *dev, int M, int K, int N, double *cycles) {
+  SplitShape best = {};
+  const int ft = (N + 127) / 128, kb = (K + GP_BK - 1) / GP_BK, rt0 = (M + 127) / 128;
+  *cycles = 1e30;
+  for (int rt = rt0; rt <= rt0 + 2; rt++) {
+    const int rn = (((M + rt - 1) / rt) + 15) & ~15;
+    for (int S = 1; S <= 8 && S <= kb; S++) {
+      if (dev->max_clusters[S] < 1) continue;
+      const int rounds = (ft * rt + dev->max_clusters[S] - 1) / dev->max_clusters[S];
+      const double c = rounds * (((kb + S - 1) / S) * fmax(6.0 * rn, 820 + 6.4 * rn) + 9000 + 60.0 * rn);
+      if (c < *cycles) {
+        *cycles = c;
+        best.row_tiles = (M + rn - 1) / rn; best.rn = rn; best.S = S;
+        const int need = (kb + S - 1) / S, room = (int)((size_t(200) << 10) / (GS_W_BYTES + rn * (GP_BK * 4)));
+        best.stages = need < room ? need : room;
+        if (best.stages > GS_MAX_STAGES) best.stages = GS_MAX_STAGES;
+      }
+    }
+  }
+  return best;
+}
+
 // X: pair planes [2][M][K], or nullptr with the LayerNorm input described in a (kNorm, M <= 64).
 static int32_t launch_gemm_split(wgpt_device *dev, const SplitShape &sh, const __half *X, const __half *W, int M, int K,
                                  int N, const Epilogue &epi, SplitArgs a) {
@@ -955,6 +986,21 @@ static int32_t launch_gemm_split(wgpt_device *dev, const SplitShape &sh, const _
 #undef SPLIT_CASE
   dev->launches++;
   return WGPT_OK;
+}
+
+// A product of pairs with whichever kernel should be faster: CTA pairs on 256-row tiles, or 128-feature tiles with K split
+// over a cluster where the former would leave most pairs without a tile (GPT-2 at 333 rows: 0.98 against 1.24 ms per pass).
+static int32_t launch_pair_product(wgpt_device *dev, const __half *X, const __half *W, int M, int K, int N,
+                                   const Epilogue &epi, bool b_exact = false) {
+  double big = 0, split = 0;
+  pair_tile_columns(dev, M, N, K, &big);
+  const SplitShape sh = split_shape_rows(dev, M, K, N, &split);
+  if (split < big && N % 4 == 0 && (epi.ld & 3) == 0) {
+    SplitArgs a;
+    memset(&a, 0, sizeof a);
+    return launch_gemm_split(dev, sh, X, W, M, K, N, epi, a);
+  }
+  return launch_gemm_pair(dev, X, W, M, K, N, epi, b_exact);
 }
 
 // The reference-layout matmul used by the per-operator API: W is [K,N].
@@ -2102,7 +2148,7 @@ static int32_t forward_blocks_fused(wgpt_session *s, const uint32_t *ids) {
 // The transformer blocks of a pass of many rows on pairs (pair.cuh): both LayerNorms, the attention and the MLP
 // up-projection write the pair form that the product after them reads. s->h, s->o and s->f hold planes here (the same
 // bytes as the FP32 rows).
-constexpr int kPairMinRows = 300;
+constexpr int kPairMinRows = 8;
 static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
   wgpt_model *m = s->m;
   wgpt_device *dev = m->dev;
@@ -2118,7 +2164,7 @@ static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
     Epilogue e = plain_epi(s->q, E, L.bqkv);
     e.colscale = L.wqkv_p.cs;
     e.kc = kc; e.vc = vc; e.E = E; e.n_tok = n_tok; e.n_ctx = p.n_ctx; e.pos = s->d_pos;
-    TRY(launch_gemm_pair(dev, h, L.wqkv_p.p, M, E, 3 * E, e));
+    TRY(launch_pair_product(dev, h, L.wqkv_p.p, M, E, 3 * E, e));
     if (n_tok == 1) {
       TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, s->n_seq, H, s->n_split, s->d_pos,
                              m->scale, s->attn_part));
@@ -2143,17 +2189,17 @@ static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
     e = plain_epi(s->x, E, L.bo);
     e.colscale = L.wo_p.cs;
     e.residual = s->x;
-    TRY(launch_gemm_pair(dev, o_in, L.wo_p.p, M, E, E, e));
+    TRY(launch_pair_product(dev, o_in, L.wo_p.p, M, E, E, e));
     TRY(launch_layernorm(dev, s->x, (size_t)E, L.ln2_g, L.ln2_b, nullptr, (size_t)E, M, E, h, plane_e, L.s_h2));
     e = plain_epi(nullptr, F, L.bfc);
     e.colscale = L.wfc_p.cs;
     e.act = 1;
     e.pair = f; e.pair_plane = plane_f; e.pair_scale = L.s_f;
-    TRY(launch_gemm_pair(dev, h, L.wfc_p.p, M, E, F, e));
+    TRY(launch_pair_product(dev, h, L.wfc_p.p, M, E, F, e));
     e = plain_epi(s->x, E, L.bpr);
     e.colscale = L.wpr_p.cs;
     e.residual = s->x;
-    TRY(launch_gemm_pair(dev, f, L.wpr_p.p, M, F, E, e));
+    TRY(launch_pair_product(dev, f, L.wpr_p.p, M, F, E, e));
   }
   return WGPT_OK;
 }
@@ -2251,7 +2297,7 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
     return WGPT_OK;
   };
 
-  const bool pair = pair_mode && M > kPairMinRows;
+  const bool pair = pair_mode && M > kPairMinRows && !split;
   if (fused) TRY(forward_blocks_fused(s, ids));
   if (pair) TRY(forward_blocks_pair(s, n_tok));
   if (split) TRY(forward_blocks_split(s));
