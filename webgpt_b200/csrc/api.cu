@@ -10,8 +10,10 @@
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <set>
 #include <string>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #include "attention.cuh"
@@ -22,6 +24,7 @@
 #include "gemm_tc2.cuh"
 #include "gemm_pair.cuh"
 #include "gemm_split.cuh"
+#include "gemv_ring.cuh"
 #include "int8.cuh"
 #include "sampling.cuh"
 #include "matmul.cuh"
@@ -95,6 +98,29 @@ struct wgpt_device {
     (dev)->launches++;                                                    \
     CK(cudaGetLastError());                                               \
   } while (0)
+
+// Lets a kernel take all the dynamic shared memory that its static part leaves, once per kernel and device. The limit is
+// never lowered again: two threads that drive two devices handles share it, and one setting its own launch's size could
+// undercut the other's between that one's setting and its launch.
+static cudaError_t allow_smem_raw(const wgpt_device *dev, const void *kern, bool whole_carveout) {
+  static std::mutex mu;
+  static std::set<std::pair<const void *, int>> done;
+  std::lock_guard<std::mutex> lock(mu);
+  if (done.count({kern, dev->ordinal})) return cudaSuccess;
+  cudaFuncAttributes at;
+  cudaError_t e = cudaFuncGetAttributes(&at, kern);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(dev->smem_optin - at.sharedSizeBytes));
+  // the whole carveout, so that the next kernel's CTA fits on the SM beside this one's and fetches its weights early
+  if (e == cudaSuccess && whole_carveout)
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared);
+  if (e == cudaSuccess) done.insert({kern, dev->ordinal});
+  return e;
+}
+template <typename K>
+static cudaError_t allow_smem(const wgpt_device *dev, K kern, bool whole_carveout = false) {
+  return allow_smem_raw(dev, reinterpret_cast<const void *>(kern), whole_carveout);
+}
 
 // Launch for kernels that call pdl_wait() before touching anything an earlier kernel wrote: with dev->pdl they
 // carry the programmatic-serialisation attribute and may start while their predecessor is still running.
@@ -284,8 +310,7 @@ WGPT_EXPORT int32_t wgpt_device_create(int32_t ordinal, wgpt_device **out) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     dev->max_clusters[S] = 0;
-    if (cudaFuncSetAttribute(gemm_split_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg.dynamicSmemBytes) ==
-        cudaSuccess)
+    if (allow_smem(dev, gemm_split_kernel<0>) == cudaSuccess)
       cudaOccupancyMaxActiveClusters(&dev->max_clusters[S], gemm_split_kernel<0>, &cfg);
   }
   *out = dev;
@@ -501,7 +526,7 @@ static int32_t launch_gemv_nk_t(wgpt_device *dev, const float *x, size_t ldx, co
   constexpr int WC = 8 / WK;
   size_t smem = (size_t)M * K * 4 + (size_t)8 * CPW * M * 4;
   auto kern = gemv_nk_kernel<M, WK, CPW>;
-  if (smem > 48 * 1024) CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(allow_smem(dev, kern));
   int grid = (N + WC * CPW - 1) / (WC * CPW);
   // Weight slices are pulled towards L2 ahead of the dependency wait unless the matrix would flush L2 (the
   // de-embedding table is larger than L2 and is long enough to be bandwidth-bound on its own).
@@ -517,7 +542,7 @@ static int32_t launch_gemv_loop_t(wgpt_device *dev, const float *x, size_t ldx, 
   constexpr int CPW = M <= 4 ? 4 : 2;
   size_t smem = (size_t)M * K * 4;
   auto kern = gemv_loop_kernel<M, CPW>;
-  if (smem > 48 * 1024) CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(allow_smem(dev, kern));
   LAUNCH_PDL(dev, kern, 2 * dev->sm_count, 256, smem, x, ldx, gamma, beta, Wt, K, N, epi, gp, dev->d_work);
   return WGPT_OK;
 }
@@ -572,7 +597,7 @@ static int32_t launch_gemv_block_t(wgpt_device *dev, const float *x, size_t ldx,
                                    const float *Wt, int K, int N, int cols, int wk, size_t smem, const Epilogue &epi,
                                    const AttnPartials &ap) {
   auto kern = gemv_block_kernel<M>;
-  if (smem > 48 * 1024) CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(allow_smem(dev, kern));
   int grid = (N + cols - 1) / cols;
   LAUNCH_PDL(dev, kern, grid, kBlockGemvThreads, smem, x, ldx, gamma, beta, Wt, K, N, cols, wk, epi, dev->d_err, ap);
   return WGPT_OK;
@@ -615,6 +640,75 @@ static int32_t launch_gemv_nk(wgpt_device *dev, int M, const float *x, size_t ld
   return fail(WGPT_ERR_SHAPE, "gemv rows %d out of range", M);
 }
 
+// ---- FP32 products of one to eight rows through the shared-memory ring (gemv_ring.cuh) ----
+struct RingPlan {
+  int ft, S, kt, stages;
+  size_t smem;
+};
+static bool gemv_ring_plan(const wgpt_device *dev, int M, int K, int N, bool layernorm, RingPlan *pl) {
+  if (M < 1 || M > 8 || K % 4 != 0 || (layernorm && K > 2048)) return false;
+  const int mr = M <= 1 ? 1 : (M <= 2 ? 2 : (M <= 4 ? 4 : 8));
+  pl->S = 1;
+  // x in every CTA: beyond 32 KB the copies of it cost as much as the weights, and K is split over a cluster
+  while (!layernorm && pl->S < 8 && (size_t)mr * K * 4 / pl->S > (size_t(32) << 10)) pl->S *= 2;
+  for (;; pl->S /= 2) {
+    const int groups = pl->S == 1 ? dev->sm_count : dev->max_clusters[pl->S];
+    pl->ft = groups > 0 ? (N + groups - 1) / groups : 65;
+    if (pl->ft <= 64) break;
+    if (pl->S == 1) { pl->ft = 64; break; }
+  }
+  pl->kt = pl->ft < 24 ? 256 : 128;
+  const int chunks = (K + pl->kt - 1) / pl->kt;
+  if (pl->S > chunks) return false;
+  const size_t xbytes = (size_t)mr * ((chunks + pl->S - 1) / pl->S) * pl->kt * 4;
+  const size_t stage = (size_t)pl->ft * pl->kt * 4;
+  const size_t fixed = 128 + xbytes + (size_t)((pl->ft * mr + 3) & ~3) * 4 + (layernorm ? (size_t)K * 8 : 0);
+  const size_t room = size_t(222) << 10;  // one CTA per SM: 111 KB rings, two of them on an SM, took 1.95 / 2.81 ms at 1 / 4 rows
+  if (fixed + 2 * stage > room) return false;
+  pl->stages = (int)((room - fixed) / stage);
+  const int need = (chunks + pl->S - 1) / pl->S;
+  if (pl->stages > need) pl->stages = need;
+  if (pl->stages > GR_MAX_STAGES) pl->stages = GR_MAX_STAGES;
+  pl->smem = fixed + (size_t)pl->stages * stage;
+  return true;
+}
+
+static int32_t make_ring_map(CUtensorMap *map, const float *Wt, uint64_t N, uint64_t K, int ft, int kt);
+
+template <int M, int FPW>
+static int32_t launch_gemv_ring_t(wgpt_device *dev, const RingPlan &pl, const CUtensorMap &map, const RingArgs &a) {
+  auto kern = gemv_ring_kernel<M, FPW>;
+  CK(allow_smem(dev, kern, true));
+  const dim3 grid((unsigned)((a.N + pl.ft - 1) / pl.ft * pl.S));
+  CK(launch_ex_x(dev->pdl, pl.S, dev->stream, kern, grid, dim3(GR_THREADS), pl.smem, map, a));
+  dev->launches++;
+  return WGPT_OK;
+}
+
+static int32_t launch_gemv_ring(wgpt_device *dev, const RingPlan &pl, int M, const float *x, const float *gamma,
+                                const float *beta, const float *Wt, int K, int N, const Epilogue &epi) {
+  RingArgs a;
+  a.x = x; a.gamma = gamma; a.beta = beta;
+  a.rows = M; a.K = K; a.N = N; a.ft = pl.ft; a.kt = pl.kt; a.stages = pl.stages;
+  a.epi = epi;
+  a.err = dev->d_err;
+  CUtensorMap map;
+  TRY(make_ring_map(&map, Wt, (uint64_t)N, (uint64_t)K, pl.ft, pl.kt));
+  const int fpw = (pl.ft + GR_WARPS - 1) / GR_WARPS;
+#define RING_F(MV)                                                            \
+  do {                                                                        \
+    if (fpw <= 2) return launch_gemv_ring_t<MV, 2>(dev, pl, map, a);          \
+    if (fpw <= 4) return launch_gemv_ring_t<MV, 4>(dev, pl, map, a);          \
+    if (fpw <= 6) return launch_gemv_ring_t<MV, 6>(dev, pl, map, a);          \
+    return launch_gemv_ring_t<MV, 8>(dev, pl, map, a);                        \
+  } while (0)
+  if (M <= 1) RING_F(1);
+  if (M <= 2) RING_F(2);
+  if (M <= 4) RING_F(4);
+  RING_F(8);
+#undef RING_F
+}
+
 static int32_t launch_gemm_simt(wgpt_device *dev, bool b_nk, const float *A, size_t lda, const float *B, int M, int K,
                                 int N, const Epilogue &epi) {
   dim3 grid((N + 63) / 64, (M + 63) / 64);
@@ -655,6 +749,21 @@ static int32_t make_tile_map(CUtensorMap *map, const float *base, uint64_t rows,
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(base), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  REQUIRE(r == CUDA_SUCCESS, WGPT_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+  return WGPT_OK;
+}
+
+// Tensor map of a row-major FP32 weight [N, K]: boxes of kt x ft elements as they are, zero fill outside.
+static int32_t make_ring_map(CUtensorMap *map, const float *Wt, uint64_t N, uint64_t K, int ft, int kt) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  REQUIRE(fn != nullptr, WGPT_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t dims[2] = {K, N};
+  cuuint64_t strides[1] = {K * 4};
+  cuuint32_t box[2] = {(cuuint32_t)kt, (cuuint32_t)ft};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(Wt), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   REQUIRE(r == CUDA_SUCCESS, WGPT_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
   return WGPT_OK;
@@ -738,12 +847,12 @@ static int32_t launch_gemm_tc(wgpt_device *dev, bool x3, const float *A, size_t 
     dim3 grid2(2 * pairs);
     if (x3) {
       auto kern = gemm_tc2_kernel<true>;
-      CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcPlan<true>::kSmemBytes));
+      CK(allow_smem(dev, kern));
       LAUNCH_PDL(dev, kern, grid2, TcPlan<true>::kThreads, TcPlan<true>::kSmemBytes, ma, mb, M, K, N, epi,
                  dev->d_err);
     } else {
       auto kern = gemm_tc2_kernel<false>;
-      CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcPlan<false>::kSmemBytes));
+      CK(allow_smem(dev, kern));
       LAUNCH_PDL(dev, kern, grid2, TcPlan<false>::kThreads, TcPlan<false>::kSmemBytes, ma, mb, M, K, N, epi,
                  dev->d_err);
     }
@@ -751,12 +860,12 @@ static int32_t launch_gemm_tc(wgpt_device *dev, bool x3, const float *A, size_t 
   }
   if (x3) {
     auto kern = gemm_tc_kernel<true>;
-    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcPlan<true>::kSmemBytes));
+    CK(allow_smem(dev, kern));
     LAUNCH_PDL(dev, kern, grid, TcPlan<true>::kThreads, TcPlan<true>::kSmemBytes, m_first, m_second, km, K, kn, epi,
                dev->d_err, kb_per_split, splits, split_out, static_op, exchanged ? 1 : 0, b_exact && !exchanged ? 1 : 0);
   } else {
     auto kern = gemm_tc_kernel<false>;
-    CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TcPlan<false>::kSmemBytes));
+    CK(allow_smem(dev, kern));
     LAUNCH_PDL(dev, kern, grid, TcPlan<false>::kThreads, TcPlan<false>::kSmemBytes, m_first, m_second, km, K, kn, epi,
                dev->d_err, kb_per_split, splits, split_out, static_op, exchanged ? 1 : 0, 0);
   }
@@ -850,7 +959,7 @@ static int32_t launch_gemm_pair(wgpt_device *dev, const __half *A, const __half 
   const int work = ((M + 255) / 256) * ((N + bn - 1) / bn);
   int pairs = dev->sm_count / 2;
   if (pairs > work) pairs = work;
-  CK(cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM_BYTES));
+  CK(allow_smem(dev, gemm_pair_kernel));
   LAUNCH_PDL(dev, gemm_pair_kernel, 2 * pairs, GP_THREADS, GP_SMEM_BYTES, ma, mb, M, K, N, bn, b_exact ? 1 : 0, epi,
              dev->d_err);
   return WGPT_OK;
@@ -876,7 +985,7 @@ static int32_t launch_gemv_kn_t(wgpt_device *dev, const float *x, const float *W
   int klen_max = ((K / 4 + ksplit - 1) / ksplit + 1) * 4;
   size_t smem = (size_t)M * klen_max * 4 + (size_t)8 * M * 32 * 16;
   auto kern = gemv_kn_partial_kernel<M>;
-  if (smem > 48 * 1024) CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(allow_smem(dev, kern));
   dim3 grid((N + 127) / 128, ksplit);
   LAUNCH(dev, kern, grid, 256, smem, x, W, K, N, part);
   return WGPT_OK;
@@ -974,7 +1083,7 @@ static int32_t launch_gemm_split(wgpt_device *dev, const SplitShape &sh, const _
   const dim3 grid(sh.row_tiles * a.f_tiles * sh.S);
 #define SPLIT_CASE(RNV)                                                                                              \
   do {                                                                                                               \
-    CK(cudaFuncSetAttribute(gemm_split_kernel<RNV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));        \
+    CK(allow_smem(dev, gemm_split_kernel<RNV>));        \
     CK(launch_ex_x(dev->pdl, sh.S, dev->stream, gemm_split_kernel<RNV>, grid, dim3(GS_THREADS), smem, mw, mx, a));   \
   } while (0)
   if (X != nullptr) SPLIT_CASE(0);
@@ -1025,7 +1134,7 @@ static int32_t launch_attn_prefill_t(wgpt_device *dev, const float *q, int ldq, 
                                      const int *pos, float scale) {
   size_t smem = attn_prefill_smem_bytes(HS);
   auto kern = attn_prefill_kernel<HS>;
-  if (smem > 48 * 1024) CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(allow_smem(dev, kern));
   dim3 grid((n_tok + 31) / 32, H, n_seq);
   LAUNCH(dev, kern, grid, 128, smem, q, ldq, kc, vc, ldkv, kv_seq_stride, out, ldo, n_tok, pos, scale);
   return WGPT_OK;
@@ -1067,7 +1176,7 @@ static int32_t launch_attn_prefill(wgpt_device *dev, int hs, const float *q, int
   }
   if (hs == 64 && tiled64 && n_tok >= 16 && (ldq % 4) == 0 && (ldkv % 4) == 0 && (ldo % 4) == 0) {
     const size_t smem = attn_prefill64_smem_bytes();
-    CK(cudaFuncSetAttribute(attn_prefill64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CK(allow_smem(dev, attn_prefill64_kernel));
     dim3 grid((n_tok + kAttn64Tile - 1) / kAttn64Tile, H, n_seq);
     LAUNCH(dev, attn_prefill64_kernel, grid, 256, smem, q, ldq, kc, vc, ldkv, kv_seq_stride, out, ldo, n_tok, pos, scale);
     return WGPT_OK;
@@ -1336,7 +1445,7 @@ static int32_t launch_int8_gemv_t(wgpt_device *dev, const float *x, const uint32
   int klen_max = ((K / 4 + ksplit - 1) / ksplit + 1) * 4;
   size_t smem = (size_t)M * klen_max * 4 + (size_t)8 * M * 32 * 4 * VEC * 4;
   auto kern = int8_gemv_partial_kernel<M, VEC>;
-  if (smem > 48 * 1024) CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(allow_smem(dev, kern));
   dim3 grid((N + 128 * VEC - 1) / (128 * VEC), ksplit);
   LAUNCH(dev, kern, grid, 256, smem, x, Bq, K, N, part);
   return WGPT_OK;
@@ -1450,9 +1559,7 @@ static int32_t launch_int8_block_t(wgpt_device *dev, const wgpt_int8_weight *w, 
   const size_t smem = (size_t)cols * K + ((size_t)M * K + ((red + 3) & ~size_t(3))) * 4 + 16;
   if (smem > dev->smem_optin - 2048) return WGPT_ERR_UNSUPPORTED;  // caller falls back (no message: not an error)
   auto kern = int8_block_gemv_kernel<M>;
-  if (smem > 48 * 1024) CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  // the whole carveout, so that the next launch's CTA fits beside this one and fetches its codes early
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+  CK(allow_smem(dev, kern, true));
   LAUNCH_PDL(dev, kern, (N + cols - 1) / cols, kInt8BlockThreads, smem, A, (const uint8_t *)w->bytes,
              (const float *)w->scale, K, N, cols, wk, out, dev->d_err);
   return WGPT_OK;
@@ -1667,10 +1774,7 @@ template <int HS, int CS>
 static int32_t attn_block_launch_t(wgpt_device *dev, const FusedPlan &fp, int H, const AttnBlockParams &a,
                                    int *max_clusters) {
   auto kern = attn_block_kernel<HS, CS>;
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp.smem_a));
-  // the whole shared-memory carveout: the next kernel's CTA must fit on the SM beside this one to fetch its
-  // weights while this one runs
-  CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+  CK(allow_smem(dev, kern, true));
   if (max_clusters != nullptr) {  // planning: how many clusters of this shape can be resident at once
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof cfg);
@@ -1746,8 +1850,7 @@ static int32_t fused_plan(wgpt_model *m) {
     if (fp.n_mlp_rows > (kAttnBlockThreads / 32) * kAttnSumRows || H > 2 * kMlpSumRows ||
         (E / 4) / kMlpCluster > 16 * (kMlpBlockThreads / 32))
       return WGPT_OK;
-    CK(cudaFuncSetAttribute(mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp.smem_b));
-    CK(cudaFuncSetAttribute(mlp, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+    CK(allow_smem(dev, mlp, true));
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof cfg);
     cfg.gridDim = dim3(fp.n_mlp);
@@ -2103,8 +2206,7 @@ static int32_t forward_blocks_fused(wgpt_session *s, const uint32_t *ids) {
   const int E = p.n_embd, F = 4 * E, H = p.n_head;
   const size_t kv_layer = (size_t)p.n_ctx * E;
   auto mlp = mlp_block_kernel;
-  if (fp.smem_b > 48 * 1024) CK(cudaFuncSetAttribute(mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fp.smem_b));
-  CK(cudaFuncSetAttribute(mlp, cudaFuncAttributePreferredSharedMemoryCarveout, (int)cudaSharedmemCarveoutMaxShared));
+  if (fp.smem_b > 48 * 1024) CK(allow_smem(dev, mlp, true));
   for (int l = 0; l < p.n_layer; l++) {
     const LayerWeights &L = m->layers[l];
     AttnBlockParams a;
@@ -2204,6 +2306,7 @@ static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
   return WGPT_OK;
 }
 
+constexpr int kSplitMinRows = 6;
 // The transformer blocks of a decode step of up to 64 sequences as five kernels per block (gemm_split.cuh): both LayerNorms
 // ride on the products that consume them, the attention finishes its own output, and every product is complete in one
 // launch.
@@ -2249,6 +2352,49 @@ static int32_t forward_blocks_split(wgpt_session *s) {
   return WGPT_OK;
 }
 
+// The transformer blocks of a decode step of a few sequences as five FP32 kernels per block (gemv_ring.cuh), for models
+// whose weights do not fit the block form (every product does in GPT-2 117M, and the block form then is faster: 0.318
+// against 0.367 ms per pass at two sequences; XL at one / two / four 1.93 / 2.15 / 2.50 ms against 2.71 / 3.52 / 5.14 in the
+// register-streaming kernels). False in *done: nothing has been launched.
+static int32_t forward_blocks_ring(wgpt_session *s, bool *done) {
+  wgpt_model *m = s->m;
+  wgpt_device *dev = m->dev;
+  const wgpt_params &p = m->p;
+  const int E = p.n_embd, F = 4 * E, H = p.n_head, hs = m->hs, M = s->n_seq;
+  const size_t kv_layer = (size_t)s->n_seq * p.n_ctx * E;
+  RingPlan pq, po, pf, pp;
+  *done = false;
+  if (dev->block_gemv) {
+    int c, w;
+    size_t b;
+    if (gemv_block_plan(dev, M, E, 3 * E, true, &c, &w, &b) && gemv_block_plan(dev, M, E, F, true, &c, &w, &b) &&
+        gemv_block_plan(dev, M, F, E, false, &c, &w, &b))
+      return WGPT_OK;
+  }
+  *done = gemv_ring_plan(dev, M, E, 3 * E, true, &pq) && gemv_ring_plan(dev, M, E, E, false, &po) &&
+          gemv_ring_plan(dev, M, E, F, true, &pf) && gemv_ring_plan(dev, M, F, E, false, &pp);
+  if (!*done) return WGPT_OK;
+  for (int l = 0; l < p.n_layer; l++) {
+    const LayerWeights &L = m->layers[l];
+    float *kc = s->kc + (size_t)l * kv_layer, *vc = s->vc + (size_t)l * kv_layer;
+    Epilogue e = plain_epi(s->q, E, L.bqkv);
+    e.kc = kc; e.vc = vc; e.E = E; e.n_tok = 1; e.n_ctx = p.n_ctx; e.pos = s->d_pos;
+    TRY(launch_gemv_ring(dev, pq, M, s->x, L.ln1_g, L.ln1_b, L.wqkv_t, E, 3 * E, e));
+    TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, M, H, s->n_split, s->d_pos, m->scale,
+                           nullptr, nullptr, true));
+    e = plain_epi(s->x, E, L.bo);
+    e.residual = s->x;
+    TRY(launch_gemv_ring(dev, po, M, s->o, nullptr, nullptr, L.wo_t, E, E, e));
+    e = plain_epi(s->f, F, L.bfc);
+    e.act = 1;
+    TRY(launch_gemv_ring(dev, pf, M, s->x, L.ln2_g, L.ln2_b, L.wfc_t, E, F, e));
+    e = plain_epi(s->x, E, L.bpr);
+    e.residual = s->x;
+    TRY(launch_gemv_ring(dev, pp, M, s->f, nullptr, nullptr, L.wpr_t, F, E, e));
+  }
+  return WGPT_OK;
+}
+
 // With pick, the greedy choice of every sequence is also made (next_ids, out_ids) and the position advanced.
 static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pick = false) {
   wgpt_model *m = s->m;
@@ -2259,7 +2405,10 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
 
   const bool fused = n_tok == 1 && s->n_seq == 1 && m->fused.ok && s->fx_a != nullptr;
   const bool pair_mode = m->pair_ok && dev->precision == WGPT_PRECISION_TF32X3;
-  const bool split = pair_mode && n_tok == 1 && M > 8 && M <= 64;
+  // From six sequences on, where the de-embedding leaves the FP32 kernels too (logits of a decode step against double
+  // precision, 2-norm: GPT-2 2.9e-6, XL 6.0e-6; five sequences in FP32 4e-7, and eight with FP32 blocks and the 3xTF32
+  // de-embedding 6.3e-6 and 1.45e-5). Decode pass of eight sequences 0.369 ms (FP32 blocks 0.489), XL 2.21 (5.08).
+  const bool split = pair_mode && n_tok == 1 && M >= kSplitMinRows && M <= 64;
   if (!fused)
     LAUNCH_PDL(dev, embed_kernel, M, 128, 0, ids, m->wte, m->wpe, s->x, M, n_tok, E, p.vocab_size,
                (const int *)s->d_pos, dev->d_err, split ? s->stats : nullptr);
@@ -2301,7 +2450,9 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
   if (fused) TRY(forward_blocks_fused(s, ids));
   if (pair) TRY(forward_blocks_pair(s, n_tok));
   if (split) TRY(forward_blocks_split(s));
-  for (int l = 0; l < (fused || pair || split ? 0 : p.n_layer); l++) {
+  bool ring = false;
+  if (!fused && !pair && !split && n_tok == 1 && M <= 8) TRY(forward_blocks_ring(s, &ring));
+  for (int l = 0; l < (fused || pair || split || ring ? 0 : p.n_layer); l++) {
     const LayerWeights &L = m->layers[l];
     float *kc = s->kc + (size_t)l * kv_layer, *vc = s->vc + (size_t)l * kv_layer;
     SplitHandoff qkv_slices;
@@ -2462,8 +2613,7 @@ static int32_t launch_sample_topk(wgpt_device *dev, const float *logits, int n_r
   const size_t smem = (kSampleThreads + cap) * sizeof(unsigned long long);
   REQUIRE(smem <= size_t(200) << 10, WGPT_ERR_SHAPE,
           "top_k %d with a vocabulary of %d needs %zu bytes of shared memory for the candidate list", top_k, V, smem);
-  if (smem > 40 * 1024)  // the kernel's static arrays count against the 48 KB default as well
-    CK(cudaFuncSetAttribute(sample_topk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(allow_smem(dev, sample_topk_kernel));
   LAUNCH_PDL(dev, sample_topk_kernel, n_rows, kSampleThreads, smem, logits, V, top_k, temperature, uniforms, (int)cap,
              next_ids, out_ids, out_stride, pos, step, n_tok, counter);
   return WGPT_OK;
