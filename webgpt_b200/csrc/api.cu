@@ -914,12 +914,13 @@ static int32_t launch_layernorm(wgpt_device *dev, const float *in, size_t ld_in,
 // ---- products of pair operands (pair.cuh) ----
 // Tensor map of both planes of a pair matrix [2][rows][K]: boxes of {64 halves, box_rows, 2}, 128-byte swizzle, zero
 // fill outside. K % 8 == 0 (16-byte row and plane strides).
-static int32_t make_pair_map(CUtensorMap *map, const __half *planes, uint64_t rows, uint64_t K, int box_rows) {
+static int32_t make_pair_map(CUtensorMap *map, const __half *planes, uint64_t rows, uint64_t K, int box_rows,
+                             int n_planes = 2) {
   EncodeTiledFn fn = encode_tiled_fn();
   REQUIRE(fn != nullptr, WGPT_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-  cuuint64_t dims[3] = {K, rows, 2};
+  cuuint64_t dims[3] = {K, rows, (cuuint64_t)n_planes};
   cuuint64_t strides[2] = {K * 2, rows * K * 2};
-  cuuint32_t box[3] = {(cuuint32_t)GP_BK, (cuuint32_t)box_rows, 2};
+  cuuint32_t box[3] = {(cuuint32_t)GP_BK, (cuuint32_t)box_rows, (cuuint32_t)n_planes};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half *>(planes), dims, strides, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -955,7 +956,7 @@ static int32_t launch_gemm_pair(wgpt_device *dev, const __half *A, const __half 
   const int bn = pair_tile_columns(dev, M, N);
   CUtensorMap ma, mb;
   TRY(make_pair_map(&ma, A, (uint64_t)M, (uint64_t)K, GP_BM));
-  TRY(make_pair_map(&mb, W, (uint64_t)N, (uint64_t)K, bn / 2));
+  TRY(make_pair_map(&mb, W, (uint64_t)N, (uint64_t)K, bn / 2, b_exact ? 1 : 2));
   const int work = ((M + 255) / 256) * ((N + bn - 1) / bn);
   int pairs = dev->sm_count / 2;
   if (pairs > work) pairs = work;
@@ -1073,12 +1074,13 @@ static int32_t launch_gemm_split(wgpt_device *dev, const SplitShape &sh, const _
   a.rn = sh.rn; a.f_tiles = (N + 127) / 128; a.stages = sh.stages;
   a.epi = epi;
   a.err = dev->d_err;
+  if (a.w_planes == 0) a.w_planes = 2;
   CUtensorMap mw, mx;
-  TRY(make_pair_map(&mw, W, (uint64_t)N, (uint64_t)K, 128));
+  TRY(make_pair_map(&mw, W, (uint64_t)N, (uint64_t)K, 128, a.w_planes));
   mx = mw;
   if (X != nullptr) TRY(make_pair_map(&mx, X, (uint64_t)M, (uint64_t)K, sh.rn));
   const int kb = (K + GP_BK - 1) / GP_BK;
-  const size_t smem = 1024 + (size_t)sh.stages * (GS_W_BYTES + sh.rn * (GP_BK * 4)) +
+  const size_t smem = 1024 + (size_t)sh.stages * (a.w_planes * (GS_W_BYTES / 2) + sh.rn * (GP_BK * 4)) +
                       (X == nullptr ? (size_t)((kb + sh.S - 1) / sh.S) * GP_BK * 8 + (size_t)sh.rn * a.x_tiles * 8 : 0);
   const dim3 grid(sh.row_tiles * a.f_tiles * sh.S);
 #define SPLIT_CASE(RNV)                                                                                              \
@@ -1097,20 +1099,52 @@ static int32_t launch_gemm_split(wgpt_device *dev, const SplitShape &sh, const _
   return WGPT_OK;
 }
 
+// Operands of per-operator products as pairs (pair_operands_kernel): fills in the launch-shape fields.
+static int32_t launch_pair_operands(wgpt_device *dev, PairOperands &p) {
+  const int S = p.n_w == 0 ? 1 : (p.K >= 512 ? 8 : (p.K >= 128 ? 4 : 1));
+  p.klen = ((p.K + S - 1) / S + 7) & ~7;
+  p.block_rows = p.K <= 8192 && p.M <= 1024 ? 1 : 0;
+  p.x_ctas = p.block_rows ? p.M : (p.M + 7) / 8;
+  p.x_ctas = (p.x_ctas + S - 1) / S * S;
+  const size_t smem = p.n_w == 0 ? 0 : (size_t)p.klen * 33 * 4;
+  REQUIRE(smem <= (size_t(200) << 10), WGPT_ERR_SHAPE, "shared dimension %d too long", p.K);
+  CK(allow_smem(dev, pair_operands_kernel));
+  CK(launch_ex_x(dev->pdl, S, dev->stream, pair_operands_kernel, dim3(p.x_ctas + p.n_w * ((p.N + 31) / 32) * S), dim3(256),
+                 smem, p));
+  dev->launches++;
+  return WGPT_OK;
+}
+// Reference-layout products that can go this way: TMA strides, and a column strip that fits shared memory.
+static bool pair_operands_fit(int K) { return K % 8 == 0 && K <= 8 * 1536; }
+
 // A product of pairs with whichever kernel should be faster: CTA pairs on 256-row tiles, or 128-feature tiles with K split
 // over a cluster where the former would leave most pairs without a tile (GPT-2 at 333 rows: 0.98 against 1.24 ms per pass).
 static int32_t launch_pair_product(wgpt_device *dev, const __half *X, const __half *W, int M, int K, int N,
-                                   const Epilogue &epi, bool b_exact = false) {
+                                   const Epilogue &epi, bool dyn = false, bool b_exact = false) {
   double big = 0, split = 0;
   pair_tile_columns(dev, M, N, K, &big);
   const SplitShape sh = split_shape_rows(dev, M, K, N, &split);
   if (split < big && N % 4 == 0 && (epi.ld & 3) == 0) {
     SplitArgs a;
     memset(&a, 0, sizeof a);
+    a.dyn = dyn ? 1 : 0;
+    a.w_planes = b_exact ? 1 : 2;
     return launch_gemm_split(dev, sh, X, W, M, K, N, epi, a);
   }
   return launch_gemm_pair(dev, X, W, M, K, N, epi, b_exact);
 }
+
+// Pieces of the workspace, each 256-byte aligned; first pass (base == nullptr) counts.
+struct Carve {
+  char *base;
+  size_t used = 0;
+  template <typename T>
+  T *take(size_t n) {
+    T *p = base ? reinterpret_cast<T *>(base + used) : nullptr;
+    used += (n * sizeof(T) + 255) & ~size_t(255);
+    return p;
+  }
+};
 
 // The reference-layout matmul used by the per-operator API: W is [K,N].
 static int32_t matmul_kn(wgpt_device *dev, int M, int K, int N, const float *in, const float *W, const Epilogue &epi) {
@@ -1119,9 +1153,31 @@ static int32_t matmul_kn(wgpt_device *dev, int M, int K, int N, const float *in,
     TRY(scratch_reserve(dev, (size_t)ksplit * M * N * 4));
     return gemv_kn_with_scratch(dev, M, in, W, K, N, ksplit, static_cast<float *>(dev->scratch), epi);
   }
+  if (dev->precision == WGPT_PRECISION_TF32X3 && M >= 32 && pair_operands_fit(K)) {
+    // Both operands to half-precision pairs in one pass, then the product; 128 x 768 x 768: 11 us against 21 us for
+    // transposition, split-K 3xTF32 product and its second stage.
+    PairOperands p;
+    memset(&p, 0, sizeof p);
+    Epilogue e = epi;
+    __half *xp = nullptr, *wp = nullptr;
+    float *xd = nullptr, *wd = nullptr;
+    for (int pass = 0; pass < 2; pass++) {
+      Carve c{pass ? static_cast<char *>(dev->scratch) : nullptr};
+      xp = c.take<__half>((size_t)2 * M * K);
+      wp = c.take<__half>((size_t)2 * N * K);
+      xd = c.take<float>(M);
+      wd = c.take<float>(N);
+      if (!pass) TRY(scratch_reserve(dev, c.used));
+    }
+    p.x = in; p.M = M; p.K = K; p.xp = xp; p.x_descale = xd;
+    p.n_w = 1; p.N = N; p.w[0] = W; p.wp[0] = wp; p.plane[0] = (size_t)N * K; p.descale[0] = wd;
+    TRY(launch_pair_operands(dev, p));
+    e.colscale = wd;
+    e.rowscale = xd;
+    return launch_pair_product(dev, xp, wp, M, K, N, e, true);
+  }
   if (dev->precision != WGPT_PRECISION_FP32 && M >= 32) {
-    // Tensor cores behind the reference layout: W[K,N] is transposed into the workspace (one pass over the weight,
-    // a few microseconds against a product of more than a hundred) and the [N,K] kernel runs on the copy.
+    // Tensor cores behind the reference layout: W[K,N] is transposed into the workspace and the [N,K] kernel runs on it.
     TRY(scratch_reserve(dev, (size_t)K * N * 4));
     return gemm_kn_via_transpose(dev, in, (size_t)K, W, M, K, N, epi, static_cast<float *>(dev->scratch));
   }
@@ -1149,13 +1205,14 @@ static bool attn_prefill_uses_mma(const wgpt_device *dev, int hs, int n_tok) {
 // than 64 tokens share each staged key tile among 128 query rows.
 static int32_t launch_attn_prefill_pair(wgpt_device *dev, const float *q, int ldq, const float *kc, const float *vc,
                                         int ldkv, size_t kv_seq_stride, int n_tok, int n_seq, int H, const int *pos,
-                                        float scale, float s_qk, float s_v, __half *planes, size_t plane, int ldo) {
+                                        float scale, float s_qk, float s_v, __half *planes, size_t plane, int ldo,
+                                        const AttnScaleSrc &src = AttnScaleSrc()) {
   if (n_tok > 64)
     LAUNCH_PDL(dev, attn_prefill64_pair_kernel<8>, dim3((n_tok + 127) / 128, H, n_seq), 256, 0, q, ldq, kc, vc, ldkv,
-               kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes, plane, ldo);
+               kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes, plane, ldo, src);
   else
     LAUNCH_PDL(dev, attn_prefill64_pair_kernel<4>, dim3((n_tok + 63) / 64, H, n_seq), 128, 0, q, ldq, kc, vc, ldkv,
-               kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes, plane, ldo);
+               kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes, plane, ldo, src);
   return WGPT_OK;
 }
 
@@ -1302,7 +1359,7 @@ WGPT_EXPORT int32_t wgpt_residual(wgpt_device *dev, int32_t rows, int32_t cols, 
   REQUIRE(cols % 4 == 0, WGPT_ERR_SHAPE, "Cols must be divisible by 4.");  // instructions.js:337
   REQUIRE(aligned16(a) && aligned16(b) && aligned16(out), WGPT_ERR_ALIGN, "buffers must be 16-byte aligned");
   size_t n4 = (size_t)rows * cols / 4;
-  LAUNCH(dev, residual_kernel, grid_for(n4, 256, dev->sm_count), 256, 0, reinterpret_cast<const float4 *>(a),
+  LAUNCH_PDL(dev, residual_kernel, grid_for(n4, 256, dev->sm_count), 256, 0, reinterpret_cast<const float4 *>(a),
          reinterpret_cast<const float4 *>(b), reinterpret_cast<float4 *>(out), n4);
   return WGPT_OK;
 }
@@ -1314,7 +1371,7 @@ WGPT_EXPORT int32_t wgpt_gelu(wgpt_device *dev, int32_t rows, int32_t cols, cons
   REQUIRE(cols % 4 == 0, WGPT_ERR_SHAPE, "Cols must be divisible by 4.");  // instructions.js:684
   REQUIRE(aligned16(in) && aligned16(out), WGPT_ERR_ALIGN, "buffers must be 16-byte aligned");
   size_t n4 = (size_t)rows * cols / 4;
-  LAUNCH(dev, gelu_kernel, grid_for(n4, 256, dev->sm_count), 256, 0, reinterpret_cast<const float4 *>(in),
+  LAUNCH_PDL(dev, gelu_kernel, grid_for(n4, 256, dev->sm_count), 256, 0, reinterpret_cast<const float4 *>(in),
          reinterpret_cast<float4 *>(out), n4);
   return WGPT_OK;
 }
@@ -1391,6 +1448,65 @@ WGPT_EXPORT int32_t wgpt_deembed(wgpt_device *dev, int32_t n_embd, int32_t vocab
                         plain_epi(logits, vocab_size, nullptr));
 }
 
+// wgpt_attention on half-precision pairs, four kernels: all four weights and the rows to pairs; q | k | v as one product;
+// attention (scales from the norms the first pass left, |q| <= |x| |w| + |b|), its output as a pair; output projection.
+// The passes it replaces were thirteen kernels (a transposition, a split-K product and its second stage per weight).
+static int32_t attention_pair(wgpt_device *dev, int T, int E, float scale, int H, int hs, const float *in, const float *qW,
+                              const float *qB, const float *kW, const float *kB, const float *vW, const float *vB,
+                              const float *linW, const float *linB, float *out) {
+  const size_t te = (size_t)T * E;
+  const int nblk = (E + 31) / 32;
+  __half *xp = nullptr, *op = nullptr, *wp = nullptr, *wo = nullptr;
+  float *qkv = nullptr, *o = nullptr, *xd = nullptr, *od = nullptr, *wd = nullptr, *wod = nullptr, *bias = nullptr,
+        *xn = nullptr, *wn = nullptr;
+  const bool mma = attn_prefill_uses_mma(dev, hs, T);
+  for (int pass = 0; pass < 2; pass++) {
+    Carve c{pass ? static_cast<char *>(dev->scratch) : nullptr};
+    xp = c.take<__half>(2 * te);
+    op = c.take<__half>(2 * te);
+    wp = c.take<__half>((size_t)2 * 3 * E * E);
+    wo = c.take<__half>((size_t)2 * E * E);
+    qkv = c.take<float>(3 * te);
+    if (!mma) o = c.take<float>(te);
+    xd = c.take<float>(T); od = c.take<float>(T); wd = c.take<float>((size_t)3 * E); wod = c.take<float>(E);
+    bias = c.take<float>((size_t)3 * E); xn = c.take<float>((size_t)T + 8); wn = c.take<float>((size_t)6 * nblk);
+    if (!pass) TRY(scratch_reserve(dev, c.used));
+  }
+  PairOperands p;
+  memset(&p, 0, sizeof p);
+  p.x = in; p.M = T; p.K = E; p.xp = xp; p.x_descale = xd; p.x_norm = xn;
+  p.n_w = 4; p.N = E;
+  const float *w[4] = {qW, kW, vW, linW}, *b[3] = {qB, kB, vB};
+  for (int i = 0; i < 4; i++) {
+    p.w[i] = w[i];
+    p.wp[i] = i < 3 ? wp + (size_t)i * E * E : wo;
+    p.plane[i] = i < 3 ? (size_t)3 * E * E : (size_t)E * E;
+    p.descale[i] = i < 3 ? wd + (size_t)i * E : wod;
+    if (i < 3) {
+      p.bias[i] = b[i];
+      p.bias_out[i] = bias + (size_t)i * E;
+      p.norm[i] = wn + (size_t)2 * i * nblk;
+    }
+  }
+  TRY(launch_pair_operands(dev, p));
+  Epilogue e = plain_epi(qkv, 3 * E, bias);
+  e.colscale = wd;
+  e.rowscale = xd;
+  TRY(launch_pair_product(dev, xp, wp, T, E, 3 * E, e, true));
+  if (mma) {
+    AttnScaleSrc src{xn, wn, p.x_ctas, nblk, od};
+    TRY(launch_attn_prefill_pair(dev, qkv, 3 * E, qkv + E, qkv + 2 * E, 3 * E, 0, T, 1, H, nullptr, scale, 1.f, 1.f, op, te, E,
+                                 src));
+  } else {
+    TRY(launch_attn_prefill(dev, hs, qkv, 3 * E, qkv + E, qkv + 2 * E, 3 * E, 0, o, E, T, 1, H, nullptr, scale));
+    LAUNCH_PDL(dev, pair_rows_kernel, (T + 7) / 8, 256, 0, (const float *)o, (size_t)E, T, E, op, od, (float *)nullptr);
+  }
+  e = plain_epi(out, E, linB);
+  e.colscale = wod;
+  e.rowscale = od;
+  return launch_pair_product(dev, op, wo, T, E, E, e, true);
+}
+
 WGPT_EXPORT int32_t wgpt_attention(wgpt_device *dev, int32_t T, int32_t E, float scale, int32_t H, int32_t hs,
                                    const float *in, const float *qW, const float *qB, const float *kW, const float *kB,
                                    const float *vW, const float *vB, const float *linW, const float *linB, float *out) {
@@ -1402,6 +1518,8 @@ WGPT_EXPORT int32_t wgpt_attention(wgpt_device *dev, int32_t T, int32_t E, float
   REQUIRE(aligned16(in) && aligned16(qW) && aligned16(kW) && aligned16(vW) && aligned16(linW) && aligned16(out) &&
               aligned16(qB) && aligned16(kB) && aligned16(vB) && aligned16(linB),
           WGPT_ERR_ALIGN, "buffers must be 16-byte aligned");
+  if (dev->precision == WGPT_PRECISION_TF32X3 && T >= 32 && pair_operands_fit(E) && E % 32 == 0)
+    return attention_pair(dev, T, E, scale, H, hs, in, qW, qB, kW, kB, vW, vB, linW, linB, out);
   // workspace: q, k, v, o [T,E] + split-K partials
   size_t te = (size_t)T * E;
   int ksplit = T <= 8 ? kn_ksplit(dev, T, E, (E + 127) / 128) : 0;
@@ -1506,6 +1624,7 @@ struct wgpt_int8_weight {
   int K, N;
   uint32_t *words;   // [K, N/4], the prototype's packing (copy)
   uint8_t *bytes;    // [N, K], K contiguous; nullptr when K % 16 != 0
+  __half *halves;    // [N, K]: the codes as half-precision values (exact), for the tensor cores; nullptr as bytes
   float *scale;      // [N]
 };
 
@@ -1518,21 +1637,24 @@ WGPT_EXPORT int32_t wgpt_int8_weight_create(wgpt_device *dev, int32_t K, int32_t
   REQUIRE(K >= 4 && N >= 8 && N % 8 == 0 && K % 4 == 0, WGPT_ERR_SHAPE, "N must be divisible by 8 and K by 4");
   REQUIRE(aligned16(Bq) && aligned16(scale), WGPT_ERR_ALIGN, "buffers must be 16-byte aligned");
   wgpt_int8_weight *w = new wgpt_int8_weight();
-  w->dev = dev; w->K = K; w->N = N; w->words = nullptr; w->bytes = nullptr; w->scale = nullptr;
+  w->dev = dev; w->K = K; w->N = N; w->words = nullptr; w->bytes = nullptr; w->halves = nullptr; w->scale = nullptr;
   const size_t nbytes = (size_t)K * N;
   cudaError_t e = cudaMalloc(&w->words, nbytes);
   if (e == cudaSuccess) e = cudaMalloc(&w->scale, (size_t)N * 4);
   if (e == cudaSuccess && K % 16 == 0) e = cudaMalloc(&w->bytes, nbytes);
+  if (e == cudaSuccess && K % 16 == 0) e = cudaMalloc(&w->halves, 2 * nbytes);
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->words, Bq, nbytes, cudaMemcpyDeviceToDevice, dev->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->scale, scale, (size_t)N * 4, cudaMemcpyDeviceToDevice, dev->stream);
   if (e != cudaSuccess) {
-    cudaFree(w->words); cudaFree(w->scale); cudaFree(w->bytes);
+    cudaFree(w->words); cudaFree(w->scale); cudaFree(w->bytes); cudaFree(w->halves);
     delete w;
     return fail(e == cudaErrorMemoryAllocation ? WGPT_ERR_OOM : WGPT_ERR_CUDA, "int8 weight: %s", cudaGetErrorString(e));
   }
   if (w->bytes) {
     dim3 grid((N / 4 + 31) / 32, (K + 31) / 32);
     LAUNCH(dev, int8_relayout_nk_kernel, grid, 256, 0, (const uint32_t *)w->words, K, N, w->bytes);
+    const size_t n16 = (size_t)N * K / 16;
+    LAUNCH(dev, int8_half_kernel, grid_for(n16, 256, dev->sm_count), 256, 0, (const uint8_t *)w->bytes, n16, w->halves);
   }
   CK(cudaStreamSynchronize(dev->stream));
   *out = w;
@@ -1544,7 +1666,7 @@ WGPT_EXPORT int32_t wgpt_int8_weight_destroy(wgpt_int8_weight *w) {
   TRY(use(w->dev));
   NOT_RECORDING(w->dev, "wgpt_int8_weight_destroy");
   CK(cudaStreamSynchronize(w->dev->stream));
-  cudaFree(w->words); cudaFree(w->scale); cudaFree(w->bytes);
+  cudaFree(w->words); cudaFree(w->scale); cudaFree(w->bytes); cudaFree(w->halves);
   delete w;
   return WGPT_OK;
 }
@@ -1583,17 +1705,26 @@ WGPT_EXPORT int32_t wgpt_int8_matmul_w(wgpt_device *dev, int32_t M, const wgpt_i
     }
     if (rc != WGPT_ERR_UNSUPPORTED) return rc;
   }
-  if (w->bytes != nullptr && M > 16 && dev->precision != WGPT_PRECISION_FP32) {
-    // many rows: the codes are expanded to an FP32 [N,K] weight in the workspace (exact; one coalesced pass) and the
-    // tcgen05 product runs on it with the scales in its epilogue
-    TRY(scratch_reserve(dev, (size_t)N * K * 4));
-    float *wt = static_cast<float *>(dev->scratch);
-    const size_t n16 = (size_t)N * K / 16;
-    LAUNCH(dev, int8_expand_bytes_kernel, grid_for(n16, 256, dev->sm_count), 256, 0, (const uint8_t *)w->bytes, n16, wt);
+  if (w->halves != nullptr && M > 16 && dev->precision != WGPT_PRECISION_FP32) {
+    // Many rows: the codes are exact in half precision, the rows become pairs (pair.cuh), the scales are in the epilogue of
+    // a two-MMA product. 256 x 3072 x 768: 24.6 us when the codes were expanded to an FP32 weight on every call and the
+    // TF32 product left its K slices to a second stage.
+    __half *xp = nullptr;
+    float *xd = nullptr;
+    for (int pass = 0; pass < 2; pass++) {
+      Carve c{pass ? static_cast<char *>(dev->scratch) : nullptr};
+      xp = c.take<__half>((size_t)2 * M * K);
+      xd = c.take<float>(M);
+      if (!pass) TRY(scratch_reserve(dev, c.used));
+    }
+    PairOperands p;
+    memset(&p, 0, sizeof p);
+    p.x = A; p.M = M; p.K = K; p.xp = xp; p.x_descale = xd;
+    TRY(launch_pair_operands(dev, p));
     Epilogue e = plain_epi(out, N, nullptr);
     e.colscale = w->scale;
-    return launch_gemm_tc(dev, dev->precision == WGPT_PRECISION_TF32X3, A, (size_t)K, wt, M, K, N, e, nullptr, false,
-                          nullptr, true);
+    e.rowscale = xd;
+    return launch_pair_product(dev, xp, w->halves, M, K, N, e, false, true);
   }
   return wgpt_int8_matmul(dev, M, K, N, A, w->words, w->scale, out);
 }

@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(32 * WARPS)
 attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__restrict__ kc,
                            const float *__restrict__ vc, int ldkv, size_t kv_seq_stride, int n_tok,
                            const int *__restrict__ pos, float scale, float s_qk, float s_v,
-                           __half *__restrict__ planes, size_t plane, int ldo) {
+                           __half *__restrict__ planes, size_t plane, int ldo, AttnScaleSrc src) {
   constexpr int HS = 64, TQ = 16 * WARPS, T = 64, LD = kAttnPairLd, NT = 32 * WARPS;
   __shared__ __align__(16) __half Ks[2][T * LD];
   __shared__ __align__(16) __half Vs[2][T * LD];
@@ -717,6 +717,12 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
   pdl_wait();
   const int pos0 = pos ? __ldcg(pos) : 0;
   const int nq = min(TQ, n_tok - t0);
+  if (src.x_norm != nullptr) {  // no bounds known at load: the per-operator attention
+    const float2 sc = attn_pair_scales(src);
+    s_qk = sc.x;
+    s_v = sc.y;
+    if (h == 0 && tid < nq) src.o_descale[t0 + tid] = 1.f / s_v;
+  }
   const int last_key = pos0 + t0 + nq - 1;  // newest key any query of this tile may see
   const int r0 = 16 * warp + g, r1 = r0 + 8;
   const int p0 = pos0 + t0 + min(r0, nq - 1), p1 = pos0 + t0 + min(r1, nq - 1);  // rows past the end shadow the last

@@ -11,8 +11,10 @@ __global__ void residual_kernel(const float4 *__restrict__ a, const float4 *__re
                                 size_t n4) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   size_t stride = (size_t)gridDim.x * blockDim.x;
+  pdl_launch_dependents();
+  pdl_wait();
   for (; i < n4; i += stride) {
-    float4 x = a[i], y = b[i];
+    const float4 x = __ldcg(a + i), y = __ldcg(b + i);
     out[i] = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
   }
 }
@@ -21,8 +23,10 @@ __global__ void residual_kernel(const float4 *__restrict__ a, const float4 *__re
 __global__ void gelu_kernel(const float4 *__restrict__ in, float4 *__restrict__ out, size_t n4) {
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   size_t stride = (size_t)gridDim.x * blockDim.x;
+  pdl_launch_dependents();
+  pdl_wait();
   for (; i < n4; i += stride) {
-    float4 x = in[i];
+    const float4 x = __ldcg(in + i);
     out[i] = make_float4(gelu_f(x.x), gelu_f(x.y), gelu_f(x.z), gelu_f(x.w));
   }
 }

@@ -85,12 +85,12 @@ __host__ __device__ constexpr uint32_t f16_idesc(int m, int n) {
 
 // gridDim.x = 2 x pairs, cluster (2,1,1). Pair p walks the 256 x bn tiles p, p + pairs, ... (row tile fastest).
 // map_a: box of 128 rows; map_b: box of bn/2 rows. bn % 32 == 0, bn <= 256.
-// b_exact: the weight's second plane is zero (integers of at most 11 bits); the product with it is not issued.
+// b_exact: the weight is exact in one plane (integers of at most 11 bits) and has no second one (map_b: one plane).
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int K,
                  int N, int bn, int b_exact, Epilogue epi, int *err) {
   // narrower tiles leave room for a fourth stage (a copy takes about 3000 cycles to arrive under load)
-  const int stage_bytes = GP_A_BYTES + bn * (GP_BK * 2);
+  const int stage_bytes = GP_A_BYTES + bn * (b_exact ? GP_BK : GP_BK * 2);
   const int S = 4 * stage_bytes <= GP_RING_BYTES ? 4 : 3;
   extern __shared__ uint8_t gp_smem_raw[];
   uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(gp_smem_raw) + 1023) & ~uintptr_t(1023));

@@ -40,6 +40,8 @@ struct SplitArgs {
   int stages;          // ring stages (<= GS_MAX_STAGES); stages * stage_bytes >= rn * 512
   Epilogue epi;
   float2 *stats;       // [M][f_tiles] or nullptr
+  int dyn;             // the weight and its scales were written by the previous kernel: nothing is read ahead of the wait
+  int w_planes;        // 2, or 1 for a weight that is exact in one plane (small integers)
   // kNorm
   const float *x;      // [M][K] FP32
   const float2 *x_stats;  // [M][x_tiles]: mean and sum of squared deviations of columns 128 t ..
@@ -118,7 +120,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   const int tile = blockIdx.x / S, ft = tile % p.f_tiles, row0 = (tile / p.f_tiles) * rn, f0 = ft * 128;
   const int total_kb = (p.K + GP_BK - 1) / GP_BK;
   const int kb0 = (int)((long long)total_kb * rank / S), nkb = (int)((long long)total_kb * (rank + 1) / S) - kb0;
-  const int stages = p.stages, stage_bytes = GS_W_BYTES + rn * (GP_BK * 4);
+  const int stages = p.stages, w_bytes = p.w_planes * (GS_W_BYTES / 2);
+  const int stage_bytes = w_bytes + rn * (GP_BK * 4);
   float4 *gam = reinterpret_cast<float4 *>(tiles + (size_t)stages * stage_bytes), *bet = gam + nkb * (GP_BK / 4);
   float2 *tile_st = reinterpret_cast<float2 *>(bet + nkb * (GP_BK / 4));  // [rows][x_tiles], as their producers left them
   const uint32_t tmem_cols = rn <= 16 ? 32u : (rn <= 32 ? 64u : (rn <= 64 ? 128u : 256u));
@@ -132,9 +135,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     mbar_init(&acc_full, 1);
     abort_word = 0;
     fence_async_smem();
+    if (p.dyn) pdl_wait();
     const int pre = min(stages, nkb);
     for (int j = 0; j < pre; j++) {  // weights: ahead of the dependency wait
-      mbar_expect_tx(&full_w[j], GS_W_BYTES);
+      mbar_expect_tx(&full_w[j], (uint32_t)w_bytes);
       tma_load_3d(tiles + (size_t)j * stage_bytes, &map_w, (kb0 + j) * GP_BK, f0, &full_w[j]);
     }
   }
@@ -156,9 +160,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   const int n = f0 + lane * 4;
   const bool n_live = n < p.N;
   float4 cs = make_float4(1.f, 1.f, 1.f, 1.f), bs = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (n_live && e.colscale != nullptr) cs = __ldg(reinterpret_cast<const float4 *>(e.colscale + n));
-  if (n_live && e.bias != nullptr) bs = __ldg(reinterpret_cast<const float4 *>(e.bias + n));
   pdl_launch_dependents();
+  if (p.dyn) pdl_wait();
+  if (n_live && e.colscale != nullptr) cs = __ldcg(reinterpret_cast<const float4 *>(e.colscale + n));
+  if (n_live && e.bias != nullptr) bs = __ldcg(reinterpret_cast<const float4 *>(e.bias + n));
   pdl_wait();  // the activations come from the previous kernel
   if (e.kc != nullptr && e.pos != nullptr) {
     e.pos_base = __ldcg(e.pos);
@@ -176,12 +181,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         uint8_t *st = tiles + (size_t)s * stage_bytes;
         if (j >= stages) {
           if (*abort_flag || !mbar_wait(&empty[s], (use & 1) ^ 1, TC_POLLS)) { *abort_flag = 1; break; }
-          mbar_expect_tx(&full_w[s], GS_W_BYTES);
+          mbar_expect_tx(&full_w[s], (uint32_t)w_bytes);
           tma_load_3d(st, &map_w, (kb0 + j) * GP_BK, f0, &full_w[s]);
         }
         if (RN == 0) {
           mbar_expect_tx(&full_x[s], (uint32_t)rn * (GP_BK * 4));
-          tma_load_3d(st + GS_W_BYTES, &map_x, (kb0 + j) * GP_BK, row0, &full_x[s]);
+          tma_load_3d(st + w_bytes, &map_x, (kb0 + j) * GP_BK, row0, &full_x[s]);
         }
       }
     }
@@ -195,11 +200,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       if (__any_sync(0xffffffffu, *abort_flag)) break;
       tc_fence_after();
       const uint32_t w0 = desc0 + (uint32_t)s * ((uint32_t)stage_bytes >> 4), w1 = w0 + (GS_W_BYTES >> 5);
-      const uint32_t x0 = w0 + (GS_W_BYTES >> 4);
+      const uint32_t x0 = w0 + ((uint32_t)w_bytes >> 4);
 #pragma unroll
       for (int k = 0; k < GP_BK / 16; k++) {
         umma1_f16(tmem_acc, w0 + 2 * k, x0 + 2 * k, idesc2, (j > 0 || k > 0) ? 1u : 0u);
-        umma1_f16(tmem_acc + (uint32_t)rn, w1 + 2 * k, x0 + 2 * k, idesc, 1u);
+        if (p.w_planes == 2) umma1_f16(tmem_acc + (uint32_t)rn, w1 + 2 * k, x0 + 2 * k, idesc, 1u);
       }
       umma_commit_elect(&empty[s]);
     }
@@ -244,7 +249,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         if (j >= nkb) break;
         const int s = j % stages, use = j / stages;
         if (j >= stages && (*abort_flag || !mbar_wait(&empty[s], (use & 1) ^ 1, TC_POLLS))) { *abort_flag = 1; break; }
-        const uint32_t xt = smem_addr(tiles + (size_t)s * stage_bytes) + GS_W_BYTES;
+        const uint32_t xt = smem_addr(tiles + (size_t)s * stage_bytes) + (uint32_t)w_bytes;
         const float4 ga = gam[j * (GP_BK / 4) + k4], be = bet[j * (GP_BK / 4) + k4];
 #pragma unroll
         for (int i = 0; i < ITERS; i++) {

@@ -250,18 +250,22 @@ int8_relayout_nk_kernel(const uint32_t *__restrict__ Bq, int K, int N, uint8_t *
   }
 }
 
-// Bytes [N, K] -> FP32 [N, K] (exact), for the tensor-core product of many rows.
-__global__ void int8_expand_bytes_kernel(const uint8_t *__restrict__ q, size_t n16, float *__restrict__ out) {
+// Bytes [N, K] -> half-precision [N, K] (exact), for the tensor-core product of many rows. Load time.
+__global__ void int8_half_kernel(const uint8_t *__restrict__ q, size_t n16, __half *__restrict__ out) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += (size_t)gridDim.x * blockDim.x) {
     const uint4 w = ldg_stream4u(reinterpret_cast<const uint4 *>(q) + i);
     const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
-    float4 *o = reinterpret_cast<float4 *>(out) + 4 * i;
+    uint2 o[4];
 #pragma unroll
     for (int v = 0; v < 4; v++) {
       float f[4];
       unpack_int8x4(ws[v], f);
-      o[v] = make_float4(f[0], f[1], f[2], f[3]);
+      const __half2 a = __floats2half2_rn(f[0], f[1]), b = __floats2half2_rn(f[2], f[3]);
+      o[v] = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
     }
+    uint4 *dst = reinterpret_cast<uint4 *>(out + 16 * i);
+    dst[0] = make_uint4(o[0].x, o[0].y, o[1].x, o[1].y);
+    dst[1] = make_uint4(o[2].x, o[2].y, o[3].x, o[3].y);
   }
 }
 

@@ -43,7 +43,7 @@ __device__ __forceinline__ float4 scale4(float4 v, float s) { return make_float4
 // Epilogue of the kernels that multiply pairs: four raw sums of row m, columns n..n+3, with the columns' constants and
 // the residual already in registers -> the finished values, and their store.
 __device__ __forceinline__ float4 pair_epi_value4(const Epilogue &e, float4 v, float4 cs, float4 bs, float4 res, int m) {
-  if (e.rowscale != nullptr) v = scale4(v, __ldg(e.rowscale + m));
+  if (e.rowscale != nullptr) v = scale4(v, __ldcg(e.rowscale + m));
   v = make_float4(v.x * cs.x + bs.x, v.y * cs.y + bs.y, v.z * cs.z + bs.z, v.w * cs.w + bs.w);
   if (e.act == 1) v = make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
   return make_float4(v.x + res.x, v.y + res.y, v.z + res.z, v.w + res.w);
@@ -67,7 +67,7 @@ __device__ __forceinline__ void pair_epi_store4(const Epilogue &e, float4 v, int
 __device__ __forceinline__ void pair_epi_block(const Epilogue &e, const float *pad, int row0, int sub_r, int col4, int n,
                                                int M) {
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-  const float4 cs = e.colscale != nullptr ? __ldg(reinterpret_cast<const float4 *>(e.colscale + n)) : make_float4(1.f, 1.f, 1.f, 1.f);
+  const float4 cs = e.colscale != nullptr ? __ldcg(reinterpret_cast<const float4 *>(e.colscale + n)) : make_float4(1.f, 1.f, 1.f, 1.f);
   const float4 bs = e.bias != nullptr ? __ldg(reinterpret_cast<const float4 *>(e.bias + n)) : zero4;
   if (e.act == 0 && e.pair == nullptr) {
     float4 res[8];
@@ -83,7 +83,7 @@ __device__ __forceinline__ void pair_epi_block(const Epilogue &e, const float *p
       const float *src = pad + r * 33 + col4;
       float4 v = make_float4(src[0], src[1], src[2], src[3]);
       if (m >= M) continue;
-      if (e.rowscale != nullptr) v = scale4(v, __ldg(e.rowscale + m));
+      if (e.rowscale != nullptr) v = scale4(v, __ldcg(e.rowscale + m));
       *reinterpret_cast<float4 *>(epi_addr(e, m, n)) =
           make_float4(v.x * cs.x + bs.x + res[it].x, v.y * cs.y + bs.y + res[it].y, v.z * cs.z + bs.z + res[it].z,
                       v.w * cs.w + bs.w + res[it].w);
@@ -100,7 +100,7 @@ __device__ __forceinline__ void pair_epi_block(const Epilogue &e, const float *p
   }
 }
 __device__ __forceinline__ void pair_epi1(const Epilogue &e, float v, int m, int n) {  // N % 4 != 0: never a pair out
-  if (e.rowscale) v *= __ldg(e.rowscale + m);
+  if (e.rowscale) v *= __ldcg(e.rowscale + m);
   epi_store(e, v, m, n);
 }
 
@@ -153,6 +153,234 @@ pair_convert_kernel(const float *__restrict__ in, size_t n, float scale, __half 
     reinterpret_cast<uint2 *>(planes)[i] = a;
     reinterpret_cast<uint2 *>(planes + n)[i] = b;
   }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Operands of one per-operator product (or the four of an attention) as pairs, in one launch: activations X[M,K] row by row,
+// weights W[K,N] in the reference layout (instructions.js:219-224) transposed on the way, one exponent per column.
+//
+// A cluster of S CTAs takes 32 columns of a weight, each CTA a slice of K held in shared memory: the column maxima are
+// exchanged through distributed shared memory, so the weight is read once, and it may be read before the dependency wait
+// (parameter buffers are constants); only the writes wait. HBM-bound: 8 bytes per value. The transposition, split-K
+// product and second stage this prepares for took 21-26 us for GPT-2's products at 128 rows; this pass and the product
+// that finishes in its cluster take about half.
+struct PairOperands {
+  // activations
+  const float *x;
+  int M, K;
+  __half *xp;         // [2][M][K]
+  float *x_descale;   // [M]
+  float *x_norm;      // [x_ctas] largest row norm of each CTA's rows, or nullptr
+  int x_ctas;         // a multiple of the cluster size
+  int block_rows;     // 1: a CTA per row (K <= 8192), 0: a warp per row
+  // weights [K,N]
+  int n_w, N, klen;   // klen: rows of K per CTA of a cluster, a multiple of 8
+  const float *w[4], *bias[4];
+  __half *wp[4];      // plane 0 of the weight's first column, rows of K
+  size_t plane[4];
+  float *descale[4];  // [N]
+  float *bias_out[4]; // [N] copy of bias (zero where there is none), or nullptr
+  float *norm[4];     // [ceil(N / 32)][2]: largest column norm, largest |bias| of 32 columns, or nullptr
+};
+
+__device__ __forceinline__ void pair_operand_rows(const PairOperands &p) {
+  __shared__ float red[2][8];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, K4 = p.K >> 2;
+  float top = 0.f;
+  if (p.block_rows) {
+    constexpr int V = 8;
+    for (int row = blockIdx.x; row < p.M; row += p.x_ctas) {
+      const float4 *x = reinterpret_cast<const float4 *>(p.x + (size_t)row * p.K);
+      float4 v[V];
+      float m = 0.f, q = 0.f;
+#pragma unroll
+      for (int j = 0; j < V; j++) v[j] = tid + 256 * j < K4 ? __ldcg(x + tid + 256 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < V; j++) {
+        m = fmaxf(m, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
+        q += dot4(v[j], v[j]);
+      }
+      m = warp_max(m);
+      q = warp_sum(q);
+      if (lane == 0) { red[0][warp] = m; red[1][warp] = q; }
+      __syncthreads();
+      m = 0.f; q = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; w++) { m = fmaxf(m, red[0][w]); q += red[1][w]; }
+      __syncthreads();
+      const float s = pair_scale_for(m);
+      if (tid == 0) p.x_descale[row] = 1.f / s;
+      top = fmaxf(top, sqrtf(q));
+      uint2 *o0 = reinterpret_cast<uint2 *>(p.xp + (size_t)row * p.K);
+      uint2 *o1 = reinterpret_cast<uint2 *>(p.xp + ((size_t)p.M + row) * p.K);
+#pragma unroll
+      for (int j = 0; j < V; j++)
+        if (tid + 256 * j < K4) {
+          uint2 a, b;
+          pair_split4(scale4(v[j], s), a, b);
+          o0[tid + 256 * j] = a;
+          o1[tid + 256 * j] = b;
+        }
+    }
+  } else {
+    for (int row = blockIdx.x * 8 + warp; row < p.M; row += p.x_ctas * 8) {
+      const float4 *x = reinterpret_cast<const float4 *>(p.x + (size_t)row * p.K);
+      float m = 0.f, q = 0.f;
+#pragma unroll 8
+      for (int i = lane; i < K4; i += 32) {
+        const float4 v = __ldcg(x + i);
+        m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+        q += dot4(v, v);
+      }
+      m = warp_max(m);
+      top = fmaxf(top, sqrtf(warp_sum(q)));
+      const float s = pair_scale_for(m);
+      if (lane == 0) p.x_descale[row] = 1.f / s;
+      uint2 *o0 = reinterpret_cast<uint2 *>(p.xp + (size_t)row * p.K);
+      uint2 *o1 = reinterpret_cast<uint2 *>(p.xp + ((size_t)p.M + row) * p.K);
+#pragma unroll 8
+      for (int i = lane; i < K4; i += 32) {
+        uint2 a, b;
+        pair_split4(scale4(__ldcg(x + i), s), a, b);
+        o0[i] = a;
+        o1[i] = b;
+      }
+    }
+    if (lane == 0) red[0][warp] = top;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < 8; w++) top = fmaxf(top, red[0][w]);
+  }
+  if (p.x_norm != nullptr && tid == 0) p.x_norm[blockIdx.x] = top;
+}
+
+// grid = x_ctas + n_w ceil(N / 32) S, cluster (S,1,1), 256 threads; dynamic shared memory klen x 33 floats.
+__global__ void __launch_bounds__(256)
+pair_operands_kernel(const __grid_constant__ PairOperands p) {
+  extern __shared__ __align__(16) float po_tile[];  // [klen][33]
+  __shared__ float own[2][32], stat[8][2][32], scl[32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  pdl_launch_dependents();
+  if ((int)blockIdx.x < p.x_ctas) {  // whole clusters
+    pdl_wait();
+    pair_operand_rows(p);
+    return;
+  }
+  uint32_t S;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(S));
+  const int rank = (int)cluster_ctarank(), cl = (int)((blockIdx.x - p.x_ctas) / S);
+  const int nblk = (p.N + 31) >> 5, wi = cl / nblk, blk = cl - wi * nblk, n0 = blk * 32;
+  const int kb = min(p.K, rank * p.klen), kn = min(p.K, kb + p.klen) - kb;
+  cluster_arrive();
+  {
+    const int c4 = (tid & 7) * 4, r0 = tid >> 3;
+    const bool in = n0 + c4 < p.N;  // N % 4 == 0
+    const float *src = p.w[wi] + (size_t)kb * p.N + n0 + c4;
+    for (int r = r0; r < kn; r += 128) {
+      float4 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        v[u] = in && r + 32 * u < kn ? ldg_stream4(reinterpret_cast<const float4 *>(src + (size_t)(r + 32 * u) * p.N))
+                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (r + 32 * u < kn) {
+          float *t = po_tile + (r + 32 * u) * 33 + c4;
+          t[0] = v[u].x; t[1] = v[u].y; t[2] = v[u].z; t[3] = v[u].w;
+        }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int c = 4 * warp + i;
+    float m = 0.f, q = 0.f;
+#pragma unroll 4
+    for (int r = lane; r < kn; r += 32) {
+      const float v = po_tile[r * 33 + c];
+      m = fmaxf(m, fabsf(v));
+      q += v * v;
+    }
+    m = warp_max(m);
+    q = warp_sum(q);
+    if (lane == 0) { own[0][c] = m; own[1][c] = q; }
+  }
+  __syncthreads();
+  cluster_wait();  // every CTA of the cluster is running
+  if (tid < 64) {
+    const int c = tid & 31, h = tid >> 5;
+    for (int r = 0; r < (int)S; r++) dsmem_st(dsmem_addr(&stat[rank][h][c], (uint32_t)r), own[h][c]);
+  }
+  cluster_arrive();
+  cluster_wait();
+  pdl_wait();  // what this kernel writes may still be read by earlier ones
+  if (tid < 32) {
+    float m = 0.f, q = 0.f;
+    for (int r = 0; r < (int)S; r++) { m = fmaxf(m, stat[r][0][tid]); q += stat[r][1][tid]; }
+    const float s = pair_scale_for(m);
+    scl[tid] = s;
+    if (rank == 0) {
+      const int n = n0 + tid;
+      const float b = n < p.N && p.bias[wi] != nullptr ? p.bias[wi][n] : 0.f;
+      if (n < p.N) {
+        p.descale[wi][n] = 1.f / s;
+        if (p.bias_out[wi] != nullptr) p.bias_out[wi][n] = b;
+      }
+      if (p.norm[wi] != nullptr) {
+        const float qm = warp_max(sqrtf(q)), bm = warp_max(fabsf(b));
+        if (tid == 0) { p.norm[wi][2 * blk] = qm; p.norm[wi][2 * blk + 1] = bm; }
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; i++) {
+    const int c = 4 * warp + i;
+    if (n0 + c >= p.N) continue;
+    const float s = scl[c];
+    __half2 *o0 = reinterpret_cast<__half2 *>(p.wp[wi] + (size_t)(n0 + c) * p.K + kb);
+    __half2 *o1 = reinterpret_cast<__half2 *>(p.wp[wi] + p.plane[wi] + (size_t)(n0 + c) * p.K + kb);
+#pragma unroll 2
+    for (int k2 = lane; 2 * k2 < kn; k2 += 32) {  // K % 8 == 0 and klen % 8 == 0: pairs are whole
+      const float x = po_tile[2 * k2 * 33 + c] * s, y = po_tile[(2 * k2 + 1) * 33 + c] * s;
+      const __half2 a = __floats2half2_rn(x, y);
+      const float2 f = __half22float2(a);
+      o0[k2] = a;
+      o1[k2] = __floats2half2_rn(x - f.x, y - f.y);
+    }
+  }
+}
+
+// Bounds of an attention's queries / keys and values from what pair_operands_kernel left (|w x + b| <= |w| |x| + |b|), as
+// the powers of two they are scaled by. Every thread of the CTA gets them.
+struct AttnScaleSrc {
+  const float *x_norm;   // [x_ctas]
+  const float *w_norm;   // [3 blocks][2]: q | k | v blocks of 32 columns
+  int x_ctas, blocks;    // blocks: per matrix
+  float *o_descale;      // [rows]: 1 / (the values' scale), for the product that reads the attention's output
+};
+__device__ __forceinline__ float2 attn_pair_scales(const AttnScaleSrc &a) {
+  __shared__ float red[32][3];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+  float x = 0.f, qk = 0.f, v = 0.f, bqk = 0.f, bv = 0.f;
+  for (int i = tid; i < a.x_ctas; i += blockDim.x) x = fmaxf(x, __ldcg(a.x_norm + i));
+  for (int i = tid; i < 3 * a.blocks; i += blockDim.x) {
+    const float2 w = __ldcg(reinterpret_cast<const float2 *>(a.w_norm) + i);
+    if (i < 2 * a.blocks) { qk = fmaxf(qk, w.x); bqk = fmaxf(bqk, w.y); }
+    else { v = fmaxf(v, w.x); bv = fmaxf(bv, w.y); }
+  }
+  x = warp_max(x);
+  if (lane == 0) red[warp][0] = x;
+  __syncthreads();
+  x = 0.f;
+  for (int w = 0; w < nw; w++) x = fmaxf(x, red[w][0]);
+  qk = warp_max(qk) * x + warp_max(bqk);  // >= every thread's own bound
+  v = warp_max(v) * x + warp_max(bv);
+  if (lane == 0) { red[warp][1] = qk; red[warp][2] = v; }
+  __syncthreads();
+  qk = 0.f; v = 0.f;
+  for (int w = 0; w < nw; w++) { qk = fmaxf(qk, red[w][1]); v = fmaxf(v, red[w][2]); }
+  return make_float2(pair_scale_for(1.01f * qk), pair_scale_for(1.01f * v));
 }
 
 }  // namespace wgpt
