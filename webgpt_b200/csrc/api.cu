@@ -1101,7 +1101,11 @@ static int32_t launch_gemm_split(wgpt_device *dev, const SplitShape &sh, const _
 
 // Operands of per-operator products as pairs (pair_operands_kernel): fills in the launch-shape fields.
 static int32_t launch_pair_operands(wgpt_device *dev, PairOperands &p) {
-  const int S = p.n_w == 0 ? 1 : (p.K >= 512 ? 8 : (p.K >= 128 ? 4 : 1));
+  int S = 1;
+  if (p.n_w > 0) {  // 192 rows of a strip per CTA: pass list of GPT-2 at 128 tokens 1.05 ms, 96 rows 1.17, 384 rows 1.10
+    S = (p.K + 191) / 192;
+    if (S > 8) S = 8;
+  }
   p.klen = ((p.K + S - 1) / S + 7) & ~7;
   p.block_rows = p.K <= 8192 && p.M <= 1024 ? 1 : 0;
   p.x_ctas = p.block_rows ? p.M : (p.M + 7) / 8;
@@ -1207,7 +1211,7 @@ static int32_t launch_attn_prefill_pair(wgpt_device *dev, const float *q, int ld
                                         int ldkv, size_t kv_seq_stride, int n_tok, int n_seq, int H, const int *pos,
                                         float scale, float s_qk, float s_v, __half *planes, size_t plane, int ldo,
                                         const AttnScaleSrc &src = AttnScaleSrc()) {
-  if (n_tok > 64)
+  if (n_tok > 64 && (long long)((n_tok + 127) / 128) * H * n_seq * 2 > dev->sm_count)
     LAUNCH_PDL(dev, attn_prefill64_pair_kernel<8>, dim3((n_tok + 127) / 128, H, n_seq), 256, 0, q, ldq, kc, vc, ldkv,
                kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes, plane, ldo, src);
   else
@@ -1671,20 +1675,43 @@ WGPT_EXPORT int32_t wgpt_int8_weight_destroy(wgpt_int8_weight *w) {
   return WGPT_OK;
 }
 
+template <int M, int CG>
+static int32_t launch_int8_block_cg(wgpt_device *dev, const wgpt_int8_weight *w, const float *A, float *out, int cols, int wk,
+                                    size_t smem) {
+  auto kern = int8_block_gemv_kernel<M, CG>;
+  CK(allow_smem(dev, kern, true));
+  LAUNCH_PDL(dev, kern, (w->N + cols - 1) / cols, kInt8BlockThreads, smem, A, (const uint8_t *)w->bytes,
+             (const float *)w->scale, w->K, w->N, cols, wk, out, dev->d_err);
+  return WGPT_OK;
+}
+
 template <int M>
 static int32_t launch_int8_block_t(wgpt_device *dev, const wgpt_int8_weight *w, const float *A, float *out) {
   const int K = w->K, N = w->N, nw = kInt8BlockThreads / 32;
   const int cols = (N + dev->sm_count - 1) / dev->sm_count;
-  int wk = 1;
-  while (cols * wk < 2 * nw && wk < 8 && (K / 16) / (wk * 2) >= 32) wk *= 2;
+  // Columns per work item and K slices: the pair with the smallest sum of shared-memory cycles (a 128-bit load is four),
+  // issue cycles (four a cycle) and the busiest warp's own path. 1600 x 6400 has 44 columns per CTA: items of four columns
+  // left five of the sixteen warps without one, three columns leave one; with more rows the row loads decide, which the
+  // columns of an item share.
+  int cg = 1, wk = 1;
+  long long best = -1;
+  for (int c = 1; c <= (M <= 4 ? 4 : 3); c++)
+    for (int k = 1; k <= 8; k *= 2) {
+      const int groups = (cols + c - 1) / c, rounds = (groups * k + nw - 1) / nw, steps = ((K / 16 + k - 1) / k + 31) / 32;
+      const long long work = (long long)groups * k * steps, instr = c * (28 + 8 * M);
+      const long long cost = work * ((c + 4 * M) * 4 + instr / 4) + rounds * (steps * (instr + 60) + 20 * c * M + 60);
+      if (best < 0 || cost < best) { best = cost; cg = c; wk = k; }
+    }
   const size_t red = (size_t)(cols * wk > nw ? cols * wk : nw) * M;
   const size_t smem = (size_t)cols * K + ((size_t)M * K + ((red + 3) & ~size_t(3))) * 4 + 16;
   if (smem > dev->smem_optin - 2048) return WGPT_ERR_UNSUPPORTED;  // caller falls back (no message: not an error)
-  auto kern = int8_block_gemv_kernel<M>;
-  CK(allow_smem(dev, kern, true));
-  LAUNCH_PDL(dev, kern, (N + cols - 1) / cols, kInt8BlockThreads, smem, A, (const uint8_t *)w->bytes,
-             (const float *)w->scale, K, N, cols, wk, out, dev->d_err);
-  return WGPT_OK;
+  switch (cg) {
+    case 1: return launch_int8_block_cg<M, 1>(dev, w, A, out, cols, wk, smem);
+    case 2: return launch_int8_block_cg<M, 2>(dev, w, A, out, cols, wk, smem);
+    case 3: return launch_int8_block_cg<M, 3>(dev, w, A, out, cols, wk, smem);
+    case 4: if constexpr (M <= 4) return launch_int8_block_cg<M, 4>(dev, w, A, out, cols, wk, smem); break;
+  }
+  return WGPT_ERR_UNSUPPORTED;
 }
 
 WGPT_EXPORT int32_t wgpt_int8_matmul_w(wgpt_device *dev, int32_t M, const wgpt_int8_weight *w, const float *A,
@@ -1695,9 +1722,13 @@ WGPT_EXPORT int32_t wgpt_int8_matmul_w(wgpt_device *dev, int32_t M, const wgpt_i
   REQUIRE(M >= 1, WGPT_ERR_SHAPE, "empty int8 matmul");
   REQUIRE(aligned16(A) && aligned16(out), WGPT_ERR_ALIGN, "buffers must be 16-byte aligned");
   const int K = w->K, N = w->N;
-  if (w->bytes != nullptr && M <= 4) {
+  if (w->bytes != nullptr && M <= 8) {
     int32_t rc = WGPT_ERR_UNSUPPORTED;
     switch (M) {
+      case 5: rc = launch_int8_block_t<5>(dev, w, A, out); break;
+      case 6: rc = launch_int8_block_t<6>(dev, w, A, out); break;
+      case 7: rc = launch_int8_block_t<7>(dev, w, A, out); break;
+      case 8: rc = launch_int8_block_t<8>(dev, w, A, out); break;
       case 1: rc = launch_int8_block_t<1>(dev, w, A, out); break;
       case 2: rc = launch_int8_block_t<2>(dev, w, A, out); break;
       case 3: rc = launch_int8_block_t<3>(dev, w, A, out); break;

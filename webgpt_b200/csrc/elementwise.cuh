@@ -44,12 +44,23 @@ layernorm_kernel(const float *__restrict__ in, size_t ld_in, const float *__rest
                  __half *__restrict__ planes, size_t plane, float scale) {
   int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   int lane = threadIdx.x & 31;
+  const int n4 = N >> 2;
+  constexpr int R = V > 0 ? V : 1;
   pdl_launch_dependents();
+  const float4 *g4 = reinterpret_cast<const float4 *>(gamma);
+  const float4 *b4 = reinterpret_cast<const float4 *>(beta);
+  float4 gv[R], bv[R];
+  if (V > 0) {  // scale and shift are weights: ahead of the dependency wait
+#pragma unroll
+    for (int j = 0; j < R; j++) {
+      const int i = lane + 32 * j;
+      gv[j] = i < n4 ? __ldg(g4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      bv[j] = i < n4 ? __ldg(b4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
   pdl_wait();  // the rows come from the previous kernel (read through L2, see common.cuh)
   if (row >= rows) return;
   const float4 *x = reinterpret_cast<const float4 *>(in + (size_t)row * ld_in);
-  const int n4 = N >> 2;
-  constexpr int R = V > 0 ? V : 1;
   float4 v[R];
   float s = 0.f;
   if (V > 0) {
@@ -80,10 +91,7 @@ layernorm_kernel(const float *__restrict__ in, size_t ld_in, const float *__rest
     }
   }
   const float sd = sqrtf(warp_sum(q) / (float)N + 1e-5f);
-  const float4 *g4 = reinterpret_cast<const float4 *>(gamma);
-  const float4 *b4 = reinterpret_cast<const float4 *>(beta);
-  auto put = [&](int i, float4 t) {
-    const float4 g = __ldg(g4 + i), b = __ldg(b4 + i);
+  auto put = [&](int i, float4 t, float4 g, float4 b) {
     const float4 y = make_float4(g.x * ((t.x - mean) / sd) + b.x, g.y * ((t.y - mean) / sd) + b.y,
                                  g.z * ((t.z - mean) / sd) + b.z, g.w * ((t.w - mean) / sd) + b.w);
     if (planes != nullptr) {
@@ -98,9 +106,9 @@ layernorm_kernel(const float *__restrict__ in, size_t ld_in, const float *__rest
   if (V > 0) {
 #pragma unroll
     for (int j = 0; j < R; j++)
-      if (lane + 32 * j < n4) put(lane + 32 * j, v[j]);
+      if (lane + 32 * j < n4) put(lane + 32 * j, v[j], gv[j], bv[j]);
   } else {
-    for (int i = lane; i < n4; i += 32) put(i, __ldcg(x + i));
+    for (int i = lane; i < n4; i += 32) put(i, __ldcg(x + i), __ldg(g4 + i), __ldg(b4 + i));
   }
 }
 

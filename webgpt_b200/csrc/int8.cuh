@@ -16,18 +16,6 @@ __device__ __forceinline__ void unpack_int8x4(uint32_t word, float (&f)[4]) {
   f[3] = (float)(v >> 24);
 }
 
-// The same four integers as unpack_int8x4, as floats, without integer-to-float conversions (a quarter-rate
-// instruction): byte b as an unsigned u = b ^ 0x80 is dropped into the mantissa of 2^23 (bits 0x4B000000 | u =
-// 2^23 + u exactly) and 2^23 + 128 is subtracted, which leaves u - 128 = the signed code, exactly.
-__device__ __forceinline__ float4 unpack_int8x4_fast(uint32_t word) {
-  const uint32_t u = word ^ 0x80808080u;
-  const float bias = 8388736.0f;  // 2^23 + 128
-  return make_float4(__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7650)) - bias,
-                     __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7651)) - bias,
-                     __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7652)) - bias,
-                     __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7653)) - bias);
-}
-
 // quantizeMatrix, other/int8-gemm.js:25-46, on the device. Pass 1: |w| maxima per output column of the row-major
 // [K, N] matrix (the prototype's header asks for vector-wise scales, :4), one thread per column per k slice,
 // partial maxima [gridDim.y][N]. The maximum is order-independent, so no fixed order is needed for exactness.
@@ -85,6 +73,37 @@ __global__ void int8_pack_kernel(const float *__restrict__ w, const float *__res
     }
     packed[i] = word;
   }
+}
+
+// Two FP32 operations per instruction (each rounded on its own).
+__device__ __forceinline__ unsigned long long pack2(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float sum2(unsigned long long a) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+  return x + y;
+}
+// The same four integers as unpack_int8x4, as two packed pairs of floats, without integer-to-float conversions (a
+// quarter-rate instruction): byte b as an unsigned u = b ^ 0x80 is dropped into the mantissa of 2^23 (bits 0x4B000000 | u =
+// 2^23 + u exactly) and 2^23 + 128 is subtracted, which leaves u - 128 = the signed code, exactly.
+__device__ __forceinline__ void unpack_int8x4_pairs(uint32_t word, unsigned long long &lo, unsigned long long &hi) {
+  const uint32_t u = word ^ 0x80808080u;
+  const unsigned long long bias = pack2(-8388736.0f, -8388736.0f);  // -(2^23 + 128)
+  lo = add2(pack2(__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7650)), __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7651))), bias);
+  hi = add2(pack2(__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7652)), __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7653))), bias);
 }
 
 // M <= 16 rows. Lane owns 4*VEC consecutive columns (VEC 32-bit words per load: VEC = 4 is a 128-bit load);
@@ -269,15 +288,16 @@ __global__ void int8_half_kernel(const uint8_t *__restrict__ q, size_t n16, __ha
   }
 }
 
-// Up to four activation rows against a re-laid-out weight (bytes [N, K]): the int8 counterpart of
+// Up to eight activation rows against a re-laid-out weight (bytes [N, K]): the int8 counterpart of
 // gemv_block_kernel. One CTA per SM owns `cols` consecutive columns, i.e. one contiguous run of cols*K bytes,
 // fetched into shared memory by bulk copies issued before the dependency wait. Work items are (column, K slice);
 // a lane takes 16 codes per step (one 128-bit load), unpacks them exactly as the prototype does
 // ((int32(word) << (24-8j)) >> 24, other/int8-gemm.js:126-131) and multiplies with the matching 16 activations;
 // slices are summed in a fixed order and the per-column scale multiplies the finished sum.
-// HBM-bound: bytes = K*N + 4*N + 4*M*(K+N). K % 16 == 0.
+// HBM-bound: bytes = K*N + 4*N + 4*M*(K+N); in practice the instructions that unpack and multiply (two codes or two products
+// each) and the hand-off between dependent launches. K % 16 == 0.
 constexpr int kInt8BlockThreads = 512;
-template <int M>
+template <int M, int CG>
 __global__ void __launch_bounds__(kInt8BlockThreads)
 int8_block_gemv_kernel(const float *__restrict__ x, const uint8_t *__restrict__ Wq, const float *__restrict__ scale,
                        int K, int N, int cols, int wk, float *__restrict__ out, int *err) {
@@ -322,35 +342,33 @@ int8_block_gemv_kernel(const float *__restrict__ x, const uint8_t *__restrict__ 
     mbar_wait(bar, 0, 1u << 22);
     return;
   }
-  const float4 *x4 = reinterpret_cast<const float4 *>(xs);
-  constexpr int CG = M == 1 ? 4 : 2;  // columns per work item: they share the activation loads
-  const int groups = (ncol + CG - 1) / CG;
+  const ulonglong2 *x4 = reinterpret_cast<const ulonglong2 *>(xs);  // a float4 as two pairs
+  const int groups = (ncol + CG - 1) / CG;  // work item: CG columns, which share the activation loads
   for (int it = warp; it < (groups << wk_log2); it += NW) {
     const int g = it >> wk_log2;
     const uint4 *w16[CG];
 #pragma unroll
     for (int q = 0; q < CG; q++) w16[q] = reinterpret_cast<const uint4 *>(wbuf + (size_t)min(g * CG + q, ncol - 1) * K);
-    float acc[CG][M];
+    unsigned long long acc[CG][M];
 #pragma unroll
     for (int q = 0; q < CG; q++)
 #pragma unroll
-      for (int m = 0; m < M; m++) acc[q][m] = 0.f;
-#pragma unroll 2
+      for (int m = 0; m < M; m++) acc[q][m] = 0ull;
     for (int i = beg + lane; i < end; i += 32) {
-      float4 xv[M][4];
+      uint4 w[CG];
 #pragma unroll
-      for (int m = 0; m < M; m++)
+      for (int q = 0; q < CG; q++) w[q] = w16[q][i];
 #pragma unroll
-        for (int v = 0; v < 4; v++) xv[m][v] = x4[(size_t)m * (K >> 2) + v * K16 + i];
+      for (int v = 0; v < 4; v++) {
+        ulonglong2 xv[M];
 #pragma unroll
-      for (int q = 0; q < CG; q++) {
-        const uint4 w = w16[q][i];
-        const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+        for (int m = 0; m < M; m++) xv[m] = x4[(size_t)m * (K >> 2) + v * K16 + i];
 #pragma unroll
-        for (int v = 0; v < 4; v++) {
-          const float4 wf = unpack_int8x4_fast(ws[v]);
+        for (int q = 0; q < CG; q++) {
+          unsigned long long lo, hi;
+          unpack_int8x4_pairs(v == 0 ? w[q].x : (v == 1 ? w[q].y : (v == 2 ? w[q].z : w[q].w)), lo, hi);
 #pragma unroll
-          for (int m = 0; m < M; m++) acc[q][m] += dot4(wf, xv[m][v]);
+          for (int m = 0; m < M; m++) acc[q][m] = fma2(hi, xv[m].y, fma2(lo, xv[m].x, acc[q][m]));
         }
       }
     }
@@ -358,7 +376,7 @@ int8_block_gemv_kernel(const float *__restrict__ x, const uint8_t *__restrict__ 
     for (int q = 0; q < CG; q++)
 #pragma unroll
       for (int m = 0; m < M; m++) {
-        const float v = warp_sum(acc[q][m]);
+        const float v = warp_sum(sum2(acc[q][m]));
         if (lane == 0 && g * CG + q < ncol) red[((g * CG + q) * wk + ks) * M + m] = v;
       }
   }

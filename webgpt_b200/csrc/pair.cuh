@@ -276,14 +276,15 @@ pair_operands_kernel(const __grid_constant__ PairOperands p) {
     const int c4 = (tid & 7) * 4, r0 = tid >> 3;
     const bool in = n0 + c4 < p.N;  // N % 4 == 0
     const float *src = p.w[wi] + (size_t)kb * p.N + n0 + c4;
-    for (int r = r0; r < kn; r += 128) {
-      float4 v[4];
+    constexpr int U = 6;
+    for (int r = r0; r < kn; r += 32 * U) {
+      float4 v[U];
 #pragma unroll
-      for (int u = 0; u < 4; u++)
+      for (int u = 0; u < U; u++)
         v[u] = in && r + 32 * u < kn ? ldg_stream4(reinterpret_cast<const float4 *>(src + (size_t)(r + 32 * u) * p.N))
                                      : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int u = 0; u < 4; u++)
+      for (int u = 0; u < U; u++)
         if (r + 32 * u < kn) {
           float *t = po_tile + (r + 32 * u) * 33 + c4;
           t[0] = v[u].x; t[1] = v[u].y; t[2] = v[u].z; t[3] = v[u].w;

@@ -209,8 +209,18 @@ class GPT:
         self.computePasses = []
 
         def push(inst):
+            # model.js:245-257 replays the list once it is complete; a pass only enqueues, so each is started as it is
+            # added and the device works while the rest of the list is built
             self.computePasses.extend(inst["passes"])
+            for ps in inst["passes"]:
+                start(ps)
             return inst["resultBuffer"]
+
+        def start(ps):
+            if ps["flag"] == "compute":
+                ps["run"]()
+            elif ps["flag"] == "copy":
+                self.device.copy(ps["src"], ps["srcOffset"], ps["dst"], ps["dstOffset"], ps["size"])
 
         intermediate = push(G.EmbedBlock.newInstance(idx, seq_length, n_embd, p["vocab_chunk_size"],
                                                      m["embeddingsBuffers"], m["posEmbdBuffer"], G.ResidualBlock))
@@ -233,18 +243,15 @@ class GPT:
                                                               b["secondLayerWeightsBuffer"], b["secondLayerBiasBuffer"]))
             intermediate = residual = push(G.ResidualBlock.newInstance(seq_length, n_embd, intermediate, residual))
         if self.externalBuffer is not None:  # model.js:211-222
-            self.computePasses.append({"flag": "copy", "src": intermediate, "srcOffset": 0, "dst": self.externalBuffer,
-                                       "dstOffset": 0, "size": self.bufferSize(seq_length, n_embd)})
+            tap = {"flag": "copy", "src": intermediate, "srcOffset": 0, "dst": self.externalBuffer, "dstOffset": 0,
+                   "size": self.bufferSize(seq_length, n_embd)}
+            self.computePasses.append(tap)
+            start(tap)
         intermediate = push(G.LayerNormBlock.newInstance(seq_length, n_embd, intermediate, m["normGammaBuffer"],
                                                          m["normBetaBuffer"]))
         result = push(G.DeEmbedBlock.newInstance(n_embd, p["vocab_size"],
                                                  p["vocab_chunk_size"] * p["vocab_chunk_instances"], seq_length,
                                                  p["vocab_chunk_size"], intermediate, m["deEmbeddingsBuffers"]))
-        for ps in self.computePasses:  # model.js:245-257
-            if ps["flag"] == "compute":
-                ps["run"]()
-            elif ps["flag"] == "copy":
-                self.device.copy(ps["src"], ps["srcOffset"], ps["dst"], ps["dstOffset"], ps["size"])
         out = result.read(np.float32, p["vocab_size"])  # model.js:261-263
         G.clearOperationCache()
         return out
