@@ -250,6 +250,8 @@ attn_block_kernel(AttnBlockParams p) {
     g_first = reinterpret_cast<const float4 *>(p.gamma)[tid];
     b_first = reinterpret_cast<const float4 *>(p.beta)[tid];
   }
+  float4 bias_x = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (tid < ncol4 && p.bias_in) bias_x = reinterpret_cast<const float4 *>(p.bias_in + col0)[tid];
   const float *kb = p.kc + h * HS, *vb = p.vc + h * HS;
   {  // ask for this CTA's slice of the cache in L2, from the position as it stands now (possibly one step old)
     const int Ls = __ldcg(p.pos) + 1;
@@ -298,7 +300,7 @@ attn_block_kernel(AttnBlockParams p) {
       } else {
         x0 = __ldcg(reinterpret_cast<const float4 *>(p.xin + col0) + tid);
       }
-      if (p.bias_in) x0 = add4(x0, reinterpret_cast<const float4 *>(p.bias_in + col0)[tid]);
+      x0 = add4(x0, bias_x);
     }
     if (lane < ncol4) reinterpret_cast<float4 *>(red)[warp * 32 + lane] = part;
     // the first positions of this CTA's cache slice, requested here: they land while the row is exchanged and normalised
@@ -315,13 +317,24 @@ attn_block_kernel(AttnBlockParams p) {
     }
     __syncthreads();
     cluster_wait();
-    if (tid < ncol4) {
+    if (warp == 0) {  // ncol4 <= 32
+      const bool has = lane < ncol4;
       float4 x = x0;
+      if (has) {
 #pragma unroll
-      for (int w = 0; w < NW; w++) x = add4(x, reinterpret_cast<const float4 *>(red)[w * 32 + tid]);
+        for (int w = 0; w < NW; w++) x = add4(x, reinterpret_cast<const float4 *>(red)[w * 32 + lane]);
 #pragma unroll
-      for (int cc = 0; cc < CS; cc++) dsmem_st4(dsmem_addr(xs + col0 + 4 * tid, (uint32_t)cc), x);
+        for (int cc = 0; cc < CS; cc++) dsmem_st4(dsmem_addr(xs + col0 + 4 * lane, (uint32_t)cc), x);
+      }
       x_keep = x;
+      // this share's part of the LayerNorm statistics goes with it (in a merge record's padding), so that no block-wide
+      // sums follow the barrier
+      const float2 st = tile_row_stats(x, has, ncolA);
+      if (lane < CS) {
+        const uint32_t at = dsmem_addr(mrg + (int)rank * MS + HS + 2, (uint32_t)lane);
+        dsmem_st(at, st.x);
+        dsmem_st(at + 4, st.y);
+      }
     }
   }
   trace(8, 2);
@@ -331,10 +344,21 @@ attn_block_kernel(AttnBlockParams p) {
 
   // ---- LayerNorm (normStats + norm, instructions.js:451-550): thread t holds elements 4t..4t+3
   {
-    const bool has = tid < E4;
-    const float4 v = has ? reinterpret_cast<const float4 *>(xs)[tid] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 y = block_layernorm4<NT>(v, has, E, g_first, b_first, red);
-    if (has) reinterpret_cast<float4 *>(hn)[tid] = y;
+    float mean = 0.f, q = 0.f;
+#pragma unroll
+    for (int r = 0; r < CS; r++) mean += mrg[r * MS + HS + 2];
+    mean *= 1.0f / CS;  // equal shares
+#pragma unroll
+    for (int r = 0; r < CS; r++) {
+      const float d = mrg[r * MS + HS + 2] - mean;
+      q += mrg[r * MS + HS + 3] + (float)ncolA * d * d;
+    }
+    const float rsd = 1.0f / sqrtf(q / (float)E + 1e-5f);
+    if (tid < E4) {
+      const float4 v = reinterpret_cast<const float4 *>(xs)[tid], g = g_first, b = b_first;
+      reinterpret_cast<float4 *>(hn)[tid] = make_float4(g.x * ((v.x - mean) * rsd) + b.x, g.y * ((v.y - mean) * rsd) + b.y,
+                                                        g.z * ((v.z - mean) * rsd) + b.z, g.w * ((v.w - mean) * rsd) + b.w);
+    }
     __syncthreads();
   }
   trace(8, 4);
@@ -603,10 +627,14 @@ mlp_block_kernel(MlpBlockParams p) {
   const int items = nu << wk_log2;
   float bias_u = 0.f;
   if (tid < nu) bias_u = p.bfc[j0 + tid];
-  float4 g_first = make_float4(0.f, 0.f, 0.f, 0.f), b_first = g_first;
-  if (tid < E4) {
-    g_first = reinterpret_cast<const float4 *>(p.gamma)[tid];
-    b_first = reinterpret_cast<const float4 *>(p.beta)[tid];
+  // one half-warp per 16 float4 columns of the row (both halves of a warp hold the same ones)
+  const int xc = warp * 16 + (lane & 15), xcols = min(16, max(E4 - warp * 16, 0));
+  const bool has = (lane & 15) < xcols;
+  float4 g_x = make_float4(0.f, 0.f, 0.f, 0.f), b_x = g_x, bias_x = g_x;
+  if (has) {
+    g_x = reinterpret_cast<const float4 *>(p.gamma)[xc];
+    b_x = reinterpret_cast<const float4 *>(p.beta)[xc];
+    bias_x = reinterpret_cast<const float4 *>(p.bias_in)[xc];
   }
   cluster_arrive();  // pairs with the wait below: every CTA of the cluster is running before any remote store
   if (tid == 0) {
@@ -615,46 +643,55 @@ mlp_block_kernel(MlpBlockParams p) {
   pdl_wait();
   trace(9, 1);
 
-  // ---- residual stream: xin + bias + the per-head partial results for this CTA's share of the columns
+  // ---- residual stream: xin + bias + the per-head partial results, the whole row in every CTA. Sharing the columns in
+  // the cluster halved these loads but cost an exchange through distributed shared memory and its barrier; a round trip
+  // to L2 takes as long for twelve warps as for six.
   float4 x_keep = make_float4(0.f, 0.f, 0.f, 0.f);
-  int x_col = -1;
   {
-    const int cbase = (int)rank * nq4;
-    const int c = warp * 16 + (lane & 15);  // one warp per 16 columns, its two halves take alternate rows
-    const bool mine = c < nq4 && lane < 16;
     // The second weight block is requested only here, behind this kernel's own loads of the partial results: requested
     // ahead of the wait together with the first, its 9.4 MB were still arriving when these loads were issued, and they
-    // waited behind it (2.9 us instead of 1.6 us from the wait to the exchange).
+    // waited behind it (2.9 us instead of 1.6 us).
     const float4 sum = halfwarp_rows_sum<kMlpSumRows>(
-        reinterpret_cast<const float4 *>(p.part_in) + cbase + warp * 16, min(16, max(nq4 - warp * 16, 0)), (size_t)E4,
-        p.n_part, lane, [&] {
+        reinterpret_cast<const float4 *>(p.part_in) + warp * 16, xcols, (size_t)E4, p.n_part, lane, [&] {
           if (tid == 0)
             bulk_g2s_block(wdn, p.wpr_kn + (size_t)j0 * E, (uint32_t)nu * (uint32_t)E * 4u, &bars[1]);
         });
-    float4 x0 = make_float4(0.f, 0.f, 0.f, 0.f);
-    x_col = cbase + c;
-    if (mine)
-      x0 = add4(__ldcg(reinterpret_cast<const float4 *>(p.xin) + cbase + c),
-                reinterpret_cast<const float4 *>(p.bias_in)[cbase + c]);
-    cluster_wait();
-    if (mine) {
-      const float4 x = add4(x0, sum);
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (has) x = add4(add4(__ldcg(reinterpret_cast<const float4 *>(p.xin) + xc), bias_x), sum);
+    x_keep = x;  // CTA 0 stores it after the last cluster barrier (see attn_block_kernel)
+    // LayerNorm (instructions.js:451-550): mean and squared deviations of this warp's 64 columns, merged by everybody
+    float2 *st = reinterpret_cast<float2 *>(red);
+    const float cnt = (float)(4 * xcols);
+    float t = (x.x + x.y) + (x.z + x.w);
 #pragma unroll
-      for (int cc = 0; cc < CS; cc++) dsmem_st4(dsmem_addr(xs + 4 * (cbase + c), (uint32_t)cc), x);
-      if (blockIdx.x < CS) x_keep = x;  // stored after the last cluster barrier (see attn_block_kernel)
-      else x_col = -1;
-    } else {
-      x_col = -1;
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    const float mt = xcols > 0 ? t / cnt : 0.f;
+    float q = 0.f;
+    if (has) {
+      const float a = x.x - mt, b = x.y - mt, c = x.z - mt, d = x.w - mt;
+      q = (a * a + b * b) + (c * c + d * d);
     }
-  }
-  cluster_arrive();
-  cluster_wait();
-  trace(9, 2);
-  {
-    const bool has = tid < E4;
-    const float4 v = has ? reinterpret_cast<const float4 *>(xs)[tid] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 y = block_layernorm4<NT>(v, has, E, g_first, b_first, red);
-    if (has) reinterpret_cast<float4 *>(xs)[tid] = y;  // in place: v was read before the barriers inside
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+    if (lane == 0) st[warp] = make_float2(mt, q);
+    __syncthreads();
+    trace(9, 2);
+    // lane w (and w + 16) holds warp w's record: two butterflies of four steps, few registers (merging all sixteen in
+    // every thread took 104 of them and left no room for the next attention kernel's CTA beside this one)
+    const float2 rec = st[lane & 15];
+    const float rc = (float)min(64, max(E - 64 * (lane & 15), 0));
+    float mean = rec.x * rc;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) mean += __shfl_xor_sync(0xffffffffu, mean, o);
+    mean /= (float)E;
+    float qs = rec.y + rc * (rec.x - mean) * (rec.x - mean);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) qs += __shfl_xor_sync(0xffffffffu, qs, o);
+    const float rsd = 1.0f / sqrtf(qs / (float)E + 1e-5f);
+    if (has && lane < 16)
+      reinterpret_cast<float4 *>(xs)[xc] =
+          make_float4(g_x.x * ((x.x - mean) * rsd) + b_x.x, g_x.y * ((x.y - mean) * rsd) + b_x.y,
+                      g_x.z * ((x.z - mean) * rsd) + b_x.z, g_x.w * ((x.w - mean) * rsd) + b_x.w);
   }
   trace(9, 3);
 
@@ -730,6 +767,7 @@ mlp_block_kernel(MlpBlockParams p) {
       if (part > 0) dsum[(part - 1) * E4 + c4] = a;
     }
     __syncthreads();
+    cluster_wait();  // every CTA of the cluster has started (it has, long since)
     if (part == 0) {
       for (int q = 1; q < p.down_parts; q++) a = add4(a, dsum[(q - 1) * E4 + c4]);
       const int owner = c4 / nq4, cc = c4 - owner * nq4;
@@ -745,7 +783,7 @@ mlp_block_kernel(MlpBlockParams p) {
     for (int r = 1; r < CS; r++) a = add4(a, x4[r * nq4 + tid]);
     reinterpret_cast<float4 *>(p.part_out + (size_t)(blockIdx.x / CS) * E)[(int)rank * nq4 + tid] = a;
   }
-  if (x_col >= 0) reinterpret_cast<float4 *>(p.x_out)[x_col] = x_keep;
+  if (blockIdx.x == 0 && has && lane < 16) reinterpret_cast<float4 *>(p.x_out)[xc] = x_keep;
   trace(9, 7);
 }
 
