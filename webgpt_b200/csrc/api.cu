@@ -13,6 +13,7 @@
 #include <set>
 #include <string>
 #include <thread>
+#include <unordered_map>
 #include <utility>
 #include <vector>
 
@@ -914,8 +915,34 @@ static int32_t launch_layernorm(wgpt_device *dev, const float *in, size_t ld_in,
 // ---- products of pair operands (pair.cuh) ----
 // Tensor map of both planes of a pair matrix [2][rows][K]: boxes of {64 halves, box_rows, 2}, 128-byte swizzle, zero
 // fill outside. K % 8 == 0 (16-byte row and plane strides).
+// Encoded maps are kept (a prefill uses the same hundred over and over and a launch-bound one waits for the host): the
+// arguments determine the map. At most 4096 of them, then the store starts over.
 static int32_t make_pair_map(CUtensorMap *map, const __half *planes, uint64_t rows, uint64_t K, int box_rows,
                              int n_planes = 2) {
+  struct Key {
+    const void *p;
+    uint64_t rows, K;
+    int box, planes;
+    bool operator==(const Key &o) const {
+      return p == o.p && rows == o.rows && K == o.K && box == o.box && planes == o.planes;
+    }
+  };
+  struct Hash {
+    size_t operator()(const Key &k) const {
+      return (reinterpret_cast<uintptr_t>(k.p) >> 4) * 0x9E3779B97F4A7C15ull ^ (k.rows << 20) ^ (k.K << 4) ^ (uint64_t)(k.box * 2 + k.planes);
+    }
+  };
+  static std::mutex mu;
+  static std::unordered_map<Key, CUtensorMap, Hash> kept;
+  const Key key{planes, rows, K, box_rows, n_planes};
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    const auto it = kept.find(key);
+    if (it != kept.end()) {
+      *map = it->second;
+      return WGPT_OK;
+    }
+  }
   EncodeTiledFn fn = encode_tiled_fn();
   REQUIRE(fn != nullptr, WGPT_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
   cuuint64_t dims[3] = {K, rows, (cuuint64_t)n_planes};
@@ -926,6 +953,9 @@ static int32_t make_pair_map(CUtensorMap *map, const __half *planes, uint64_t ro
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   REQUIRE(r == CUDA_SUCCESS, WGPT_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+  std::lock_guard<std::mutex> lock(mu);
+  if (kept.size() >= 4096) kept.clear();
+  kept.emplace(key, *map);
   return WGPT_OK;
 }
 
@@ -1205,7 +1235,12 @@ static bool attn_prefill_uses_mma(const wgpt_device *dev, int hs, int n_tok) {
   return hs == 64 && mma64 && dev->precision != WGPT_PRECISION_FP32 && n_tok >= 16;
 }
 
-// Prefill attention of a pair model (head size 64, attn_prefill_uses_mma): output planes [2][rows][ldo]. Windows of more
+// Prefill attention on half-precision pairs: head size 64 in 3xTF32 mode, any number of tokens.
+static bool attn_prefill_pair_ok(const wgpt_device *dev, int hs) {
+  return attn_prefill_uses_mma(dev, hs, 64) && dev->precision == WGPT_PRECISION_TF32X3;
+}
+
+// Prefill attention of a pair model (attn_prefill_pair_ok): output planes [2][rows][ldo]. Windows of more
 // than 64 tokens share each staged key tile among 128 query rows.
 static int32_t launch_attn_prefill_pair(wgpt_device *dev, const float *q, int ldq, const float *kc, const float *vc,
                                         int ldkv, size_t kv_seq_stride, int n_tok, int n_seq, int H, const int *pos,
@@ -1463,7 +1498,7 @@ static int32_t attention_pair(wgpt_device *dev, int T, int E, float scale, int H
   __half *xp = nullptr, *op = nullptr, *wp = nullptr, *wo = nullptr;
   float *qkv = nullptr, *o = nullptr, *xd = nullptr, *od = nullptr, *wd = nullptr, *wod = nullptr, *bias = nullptr,
         *xn = nullptr, *wn = nullptr;
-  const bool mma = attn_prefill_uses_mma(dev, hs, T);
+  const bool mma = attn_prefill_pair_ok(dev, hs);
   for (int pass = 0; pass < 2; pass++) {
     Carve c{pass ? static_cast<char *>(dev->scratch) : nullptr};
     xp = c.take<__half>(2 * te);
@@ -2420,7 +2455,7 @@ static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
   const int E = p.n_embd, F = 4 * E, H = p.n_head, hs = m->hs, M = s->n_seq * n_tok;
   const size_t kv_layer = (size_t)s->n_seq * p.n_ctx * E, plane_e = (size_t)M * E, plane_f = (size_t)M * F;
   __half *h = reinterpret_cast<__half *>(s->h), *o = reinterpret_cast<__half *>(s->o), *f = reinterpret_cast<__half *>(s->f);
-  const bool o_pair = n_tok > 1 && attn_prefill_uses_mma(dev, hs, n_tok);
+  const bool o_pair = n_tok > 1 && attn_prefill_pair_ok(dev, hs);
   for (int l = 0; l < p.n_layer; l++) {
     const LayerWeights &L = m->layers[l];
     float *kc = s->kc + (size_t)l * kv_layer, *vc = s->vc + (size_t)l * kv_layer;
@@ -2469,14 +2504,14 @@ static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
 }
 
 constexpr int kSplitMinRows = 6;
-// The transformer blocks of a decode step of up to 64 sequences as five kernels per block (gemm_split.cuh): both LayerNorms
-// ride on the products that consume them, the attention finishes its own output, and every product is complete in one
-// launch.
-static int32_t forward_blocks_split(wgpt_session *s) {
+// The transformer blocks of a pass of up to 64 rows (a decode step, a short prompt) as five kernels per block
+// (gemm_split.cuh): both LayerNorms ride on the products that consume them, the attention finishes its own output, and
+// every product is complete in one launch.
+static int32_t forward_blocks_split(wgpt_session *s, int n_tok) {
   wgpt_model *m = s->m;
   wgpt_device *dev = m->dev;
   const wgpt_params &p = m->p;
-  const int E = p.n_embd, F = 4 * E, H = p.n_head, hs = m->hs, M = s->n_seq, xt = (E + 127) / 128;
+  const int E = p.n_embd, F = 4 * E, H = p.n_head, hs = m->hs, M = s->n_seq * n_tok, xt = (E + 127) / 128;
   const size_t kv_layer = (size_t)s->n_seq * p.n_ctx * E, plane_e = (size_t)M * E, plane_f = (size_t)M * F;
   __half *o = reinterpret_cast<__half *>(s->o), *f = reinterpret_cast<__half *>(s->f);
   const SplitShape sh_qkv = split_shape_decode(dev, M, E, 3 * E), sh_o = split_shape_decode(dev, M, E, E),
@@ -2491,15 +2526,27 @@ static int32_t forward_blocks_split(wgpt_session *s) {
     float *kc = s->kc + (size_t)l * kv_layer, *vc = s->vc + (size_t)l * kv_layer;
     Epilogue e = plain_epi(s->q, E, L.bqkv);
     e.colscale = L.wqkv_p.cs;
-    e.kc = kc; e.vc = vc; e.E = E; e.n_tok = 1; e.n_ctx = p.n_ctx; e.pos = s->d_pos;
+    e.kc = kc; e.vc = vc; e.E = E; e.n_tok = n_tok; e.n_ctx = p.n_ctx; e.pos = s->d_pos;
     norm.gamma = L.ln1_g; norm.beta = L.ln1_b; norm.x_scale = L.s_h1;
     TRY(launch_gemm_split(dev, sh_qkv, nullptr, L.wqkv_p.p, M, E, 3 * E, e, norm));
-    TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, nullptr, E, M, H, s->n_split, s->d_pos, m->scale,
-                           nullptr, nullptr, true, o, plane_e, L.s_o));
+    const __half *o_in = o;
+    if (n_tok == 1) {
+      TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, nullptr, E, M, H, s->n_split, s->d_pos, m->scale,
+                             nullptr, nullptr, true, o, plane_e, L.s_o));
+    } else if (attn_prefill_pair_ok(dev, hs)) {
+      TRY(launch_attn_prefill_pair(dev, s->q, E, kc, vc, E, (size_t)p.n_ctx, n_tok, s->n_seq, H, s->d_pos, m->scale,
+                                   L.s_qk, L.s_o, o, plane_e, E));
+    } else {
+      TRY(launch_attn_prefill(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, n_tok, s->n_seq, H, s->d_pos,
+                              m->scale));
+      o_in = reinterpret_cast<const __half *>(s->h);
+      LAUNCH_PDL(dev, pair_convert_kernel, grid_for(plane_e / 4, 256, dev->sm_count), 256, 0, (const float *)s->o, plane_e,
+                 L.s_o, reinterpret_cast<__half *>(s->h));
+    }
     e = plain_epi(s->x, E, L.bo);
     e.colscale = L.wo_p.cs;
     e.residual = s->x;
-    TRY(launch_gemm_split(dev, sh_o, o, L.wo_p.p, M, E, E, e, plain));
+    TRY(launch_gemm_split(dev, sh_o, o_in, L.wo_p.p, M, E, E, e, plain));
     e = plain_epi(nullptr, F, L.bfc);
     e.colscale = L.wfc_p.cs;
     e.act = 1;
@@ -2570,7 +2617,8 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
   // From six sequences on, where the de-embedding leaves the FP32 kernels too (logits of a decode step against double
   // precision, 2-norm: GPT-2 2.9e-6, XL 6.0e-6; five sequences in FP32 4e-7, and eight with FP32 blocks and the 3xTF32
   // de-embedding 6.3e-6 and 1.45e-5). Decode pass of eight sequences 0.369 ms (FP32 blocks 0.489), XL 2.21 (5.08).
-  const bool split = pair_mode && n_tok == 1 && M >= kSplitMinRows && M <= 64;
+  // Prompts: from nine rows on (up to eight stay in FP32).
+  const bool split = pair_mode && M <= 64 && (n_tok == 1 ? M >= kSplitMinRows : M > 8);
   if (!fused)
     LAUNCH_PDL(dev, embed_kernel, M, 128, 0, ids, m->wte, m->wpe, s->x, M, n_tok, E, p.vocab_size,
                (const int *)s->d_pos, dev->d_err, split ? s->stats : nullptr);
@@ -2611,7 +2659,7 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
   const bool pair = pair_mode && M > kPairMinRows && !split;
   if (fused) TRY(forward_blocks_fused(s, ids));
   if (pair) TRY(forward_blocks_pair(s, n_tok));
-  if (split) TRY(forward_blocks_split(s));
+  if (split) TRY(forward_blocks_split(s, n_tok));
   bool ring = false;
   if (!fused && !pair && !split && n_tok == 1 && M <= 8) TRY(forward_blocks_ring(s, &ring));
   for (int l = 0; l < (fused || pair || split || ring ? 0 : p.n_layer); l++) {
