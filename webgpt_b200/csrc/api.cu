@@ -643,12 +643,12 @@ static int32_t launch_gemv_nk(wgpt_device *dev, int M, const float *x, size_t ld
 
 // ---- FP32 products of one to eight rows through the shared-memory ring (gemv_ring.cuh) ----
 struct RingPlan {
-  int ft, S, kt, stages;
+  int ft, S, stages;
   size_t smem;
 };
 static bool gemv_ring_plan(const wgpt_device *dev, int M, int K, int N, bool layernorm, RingPlan *pl) {
   if (M < 1 || M > 8 || K % 4 != 0 || (layernorm && K > 2048)) return false;
-  const int mr = M <= 1 ? 1 : (M <= 2 ? 2 : (M <= 4 ? 4 : 8));
+  const int mr = M <= 2 ? M : (M <= 4 ? 4 : (M <= 5 ? 5 : 8));
   pl->S = 1;
   // x in every CTA: beyond 32 KB the copies of it cost as much as the weights, and K is split over a cluster
   while (!layernorm && pl->S < 8 && (size_t)mr * K * 4 / pl->S > (size_t(32) << 10)) pl->S *= 2;
@@ -658,11 +658,10 @@ static bool gemv_ring_plan(const wgpt_device *dev, int M, int K, int N, bool lay
     if (pl->ft <= 64) break;
     if (pl->S == 1) { pl->ft = 64; break; }
   }
-  pl->kt = pl->ft < 24 ? 256 : 128;
-  const int chunks = (K + pl->kt - 1) / pl->kt;
+  const int chunks = (K + GR_KT - 1) / GR_KT;
   if (pl->S > chunks) return false;
-  const size_t xbytes = (size_t)mr * ((chunks + pl->S - 1) / pl->S) * pl->kt * 4;
-  const size_t stage = (size_t)pl->ft * pl->kt * 4;
+  const size_t xbytes = (size_t)mr * ((chunks + pl->S - 1) / pl->S) * GR_KT * 4;
+  const size_t stage = (size_t)pl->ft * GR_KT * 4;
   const size_t fixed = 128 + xbytes + (size_t)((pl->ft * mr + 3) & ~3) * 4 + (layernorm ? (size_t)K * 8 : 0);
   const size_t room = size_t(222) << 10;  // one CTA per SM: 111 KB rings, two of them on an SM, took 1.95 / 2.81 ms at 1 / 4 rows
   if (fixed + 2 * stage > room) return false;
@@ -690,11 +689,11 @@ static int32_t launch_gemv_ring(wgpt_device *dev, const RingPlan &pl, int M, con
                                 const float *beta, const float *Wt, int K, int N, const Epilogue &epi) {
   RingArgs a;
   a.x = x; a.gamma = gamma; a.beta = beta;
-  a.rows = M; a.K = K; a.N = N; a.ft = pl.ft; a.kt = pl.kt; a.stages = pl.stages;
+  a.rows = M; a.K = K; a.N = N; a.ft = pl.ft; a.stages = pl.stages;
   a.epi = epi;
   a.err = dev->d_err;
   CUtensorMap map;
-  TRY(make_ring_map(&map, Wt, (uint64_t)N, (uint64_t)K, pl.ft, pl.kt));
+  TRY(make_ring_map(&map, Wt, (uint64_t)N, (uint64_t)K, pl.ft, GR_KT));
   const int fpw = (pl.ft + GR_WARPS - 1) / GR_WARPS;
 #define RING_F(MV)                                                            \
   do {                                                                        \
@@ -706,6 +705,7 @@ static int32_t launch_gemv_ring(wgpt_device *dev, const RingPlan &pl, int M, con
   if (M <= 1) RING_F(1);
   if (M <= 2) RING_F(2);
   if (M <= 4) RING_F(4);
+  if (M <= 5) RING_F(5);
   RING_F(8);
 #undef RING_F
 }

@@ -24,12 +24,13 @@ namespace wgpt {
 constexpr int GR_WARPS = 8;
 constexpr int GR_THREADS = 32 * (GR_WARPS + 1);
 constexpr int GR_MAX_STAGES = 16;
+constexpr int GR_KT = 256;  // K values per stage: with 128 the warps spent more time at the barriers than reading
 constexpr uint32_t GR_POLLS = 1u << 20;
 
 struct RingArgs {
   const float *x;             // [rows][K]
   const float *gamma, *beta;  // LayerNorm of x, or nullptr (only then may S exceed 1)
-  int rows, K, N, ft, kt, stages;  // kt: K values per stage, 128 or 256
+  int rows, K, N, ft, stages;
   Epilogue epi;
   int *err;
 };
@@ -93,11 +94,11 @@ __device__ __forceinline__ void ring_layernorm(const float *__restrict__ x, int 
   }
 }
 
-// grid = ceil(N / ft) * S, cluster (S,1,1). M: rows rounded up to 1, 2, 4 or 8; FPW: columns per warp (ft <= 8 FPW).
+// grid = ceil(N / ft) * S, cluster (S,1,1). M: rows rounded up to 1, 2, 4, 5 or 8; FPW: columns per warp (ft <= 8 FPW).
 // Dynamic shared memory: ring [stages][ft][kt] (128-byte aligned), x [M][K slice padded to kt], sums [ft][M] (padded to a
 // multiple of 4), and with a LayerNorm gamma [K], beta [K].
 template <int M, int FPW>
-__global__ void __launch_bounds__(GR_THREADS, 2)
+__global__ void __launch_bounds__(GR_THREADS, 1)
 gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ RingArgs p) {
   extern __shared__ uint8_t gr_smem_raw[];
   __shared__ uint64_t full[GR_MAX_STAGES], empty[GR_MAX_STAGES];
@@ -110,11 +111,11 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(S));
   const int rank = (int)cluster_ctarank();
   const int col0 = (int)(blockIdx.x / S) * p.ft, ncol = min(p.ft, p.N - col0);
-  const int chunks_all = (p.K + p.kt - 1) / p.kt;
+  const int chunks_all = (p.K + GR_KT - 1) / GR_KT;
   const int ch0 = (int)((long long)chunks_all * rank / S), nch = (int)((long long)chunks_all * (rank + 1) / S) - ch0;
-  const int stage_floats = p.ft * p.kt;
+  const int stage_floats = p.ft * GR_KT;
   float *xs = ring + (size_t)p.stages * stage_floats;
-  const int xld = ((chunks_all + (int)S - 1) / (int)S) * p.kt;  // row stride of xs
+  const int xld = ((chunks_all + (int)S - 1) / (int)S) * GR_KT;  // row stride of xs
   float *sums = xs + (size_t)M * xld;
   float4 *gam = reinterpret_cast<float4 *>(sums + ((p.ft * M + 3) & ~3)), *bet = gam + (p.K >> 2);
 
@@ -132,7 +133,7 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     const int pre = min(p.stages, nch);
     for (int i = 0; i < pre; i++) {  // weights: ahead of the dependency wait
       mbar_expect_tx(&full[i], tx);
-      tma_load_2d(ring + (size_t)i * stage_floats, &map_w, (ch0 + i) * p.kt, col0, &full[i]);
+      tma_load_2d(ring + (size_t)i * stage_floats, &map_w, (ch0 + i) * GR_KT, col0, &full[i]);
     }
   }
   // the output this thread will finish (a second round of them is rare): its bias ahead of the wait, the rest right after
@@ -162,15 +163,15 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
       for (int i = p.stages, s = 0, ph = 0; i < nch; i++) {
         if (*abort_flag || !mbar_wait(&empty[s], ph, GR_POLLS)) { *abort_flag = 1; break; }
         mbar_expect_tx(&full[s], tx);
-        tma_load_2d(ring + (size_t)s * stage_floats, &map_w, (ch0 + i) * p.kt, col0, &full[s]);
+        tma_load_2d(ring + (size_t)s * stage_floats, &map_w, (ch0 + i) * GR_KT, col0, &full[s]);
         if (++s == p.stages) { s = 0; ph ^= 1; }
       }
     }
     __syncwarp();
   } else {
-    const int k_lo = ch0 * p.kt, k_len = min(nch * p.kt, p.K - k_lo);
+    const int k_lo = ch0 * GR_KT, k_len = min(nch * GR_KT, p.K - k_lo);
     if (p.gamma != nullptr) {
-      ring_layernorm<M>(p.x, p.rows, p.K, gam, bet, xs, xld, ln_red, warp, lane);
+      ring_layernorm<(M <= 2 ? M : (M <= 4 ? 4 : 8))>(p.x, p.rows, p.K, gam, bet, xs, xld, ln_red, warp, lane);
     } else {
       // eight loads in flight per thread, whatever rows they fall into; every CTA reads the same rows at the same time,
       // so each starts at another place
@@ -203,20 +204,20 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     for (int f = 0; f < FPW; f++)
 #pragma unroll
       for (int m = 0; m < M; m++) acc[f][m] = 0.f;
-    const int steps = p.kt >> 7;
     int s = 0, ph = 0;
     for (int i = 0; i < nch; i++) {
       const bool ok = mbar_wait(&full[s], ph, GR_POLLS);
       if (!__all_sync(0xffffffffu, ok)) { *abort_flag = 1; break; }
       const float4 *w4 = reinterpret_cast<const float4 *>(ring + (size_t)s * stage_floats) + lane;
-      const float4 *x4 = reinterpret_cast<const float4 *>(xs + (size_t)i * p.kt) + lane;
-      for (int t = 0; t < steps; t++) {
+      const float4 *x4 = reinterpret_cast<const float4 *>(xs + (size_t)i * GR_KT) + lane;
+#pragma unroll
+      for (int t = 0; t < GR_KT / 128; t++) {
         float4 xv[M];
 #pragma unroll
         for (int m = 0; m < M; m++) xv[m] = x4[(size_t)min(m, p.rows - 1) * (xld >> 2) + 32 * t];
 #pragma unroll
         for (int f = 0; f < FPW; f++) {
-          const float4 w = w4[min(warp + GR_WARPS * f, p.ft - 1) * (p.kt >> 2) + 32 * t];
+          const float4 w = w4[min(warp + GR_WARPS * f, p.ft - 1) * (GR_KT >> 2) + 32 * t];
 #pragma unroll
           for (int m = 0; m < M; m++) acc[f][m] += dot4(w, xv[m]);
         }
