@@ -170,9 +170,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     e.pos = nullptr;
   }
   const int r_beg = rn * rank / (int)S, r_end = rn * (rank + 1) / (int)S;
-  float4 res_first = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (e.residual != nullptr && n_live && r_beg + warp < r_end && row0 + r_beg + warp < p.M)
-    res_first = __ldcg(reinterpret_cast<const float4 *>(e.residual + (size_t)(row0 + r_beg + warp) * e.ld + n));
+  // the residual of this warp's first two rows: a round trip to L2 that would otherwise follow the exchange
+  float4 res_first[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int r = r_beg + warp + u * (GS_THREADS / 32);
+    if (e.residual != nullptr && n_live && r < r_end && row0 + r < p.M)
+      res_first[u] = __ldcg(reinterpret_cast<const float4 *>(e.residual + (size_t)(row0 + r) * e.ld + n));
+  }
 
   if (warp == 0) {
     if (lane == 0) {
@@ -301,9 +306,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     const int m0 = row0 + r, m1 = m0 + NW;
     if (m0 >= p.M) break;
     const bool two = r + NW < r_end && m1 < p.M;
-    float4 res[2] = {res_first, make_float4(0.f, 0.f, 0.f, 0.f)};
-    if (e.residual != nullptr && n_live) {
-      if (r != r_beg + warp) res[0] = __ldcg(reinterpret_cast<const float4 *>(e.residual + (size_t)m0 * e.ld + n));
+    float4 res[2] = {res_first[0], res_first[1]};
+    if (e.residual != nullptr && n_live && r != r_beg + warp) {
+      res[0] = __ldcg(reinterpret_cast<const float4 *>(e.residual + (size_t)m0 * e.ld + n));
       if (two) res[1] = __ldcg(reinterpret_cast<const float4 *>(e.residual + (size_t)m1 * e.ld + n));
     }
     float4 q[2][8];
