@@ -1240,18 +1240,25 @@ static bool attn_prefill_pair_ok(const wgpt_device *dev, int hs) {
   return attn_prefill_uses_mma(dev, hs, 64) && dev->precision == WGPT_PRECISION_TF32X3;
 }
 
-// Prefill attention of a pair model (attn_prefill_pair_ok): output planes [2][rows][ldo]. Windows of more
-// than 64 tokens share each staged key tile among 128 query rows.
+// Prefill attention of a pair model (attn_prefill_pair_ok): output planes [2][rows][ldo].
 static int32_t launch_attn_prefill_pair(wgpt_device *dev, const float *q, int ldq, const float *kc, const float *vc,
                                         int ldkv, size_t kv_seq_stride, int n_tok, int n_seq, int H, const int *pos,
                                         float scale, float s_qk, float s_v, __half *planes, size_t plane, int ldo,
                                         const AttnScaleSrc &src = AttnScaleSrc()) {
-  if (n_tok > 64 && (long long)((n_tok + 127) / 128) * H * n_seq * 2 > dev->sm_count)
-    LAUNCH_PDL(dev, attn_prefill64_pair_kernel<8>, dim3((n_tok + 127) / 128, H, n_seq), 256, 0, q, ldq, kc, vc, ldkv,
-               kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes, plane, ldo, src);
-  else
-    LAUNCH_PDL(dev, attn_prefill64_pair_kernel<4>, dim3((n_tok + 63) / 64, H, n_seq), 128, 0, q, ldq, kc, vc, ldkv,
-               kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes, plane, ldo, src);
+  // Two groups of warps per 64 query rows, alternating key tiles, up to 2.5 CTAs per SM (GPT-2 at 333 / 1024 tokens 0.85 /
+  // 1.64 ms per pass against 1.00 / 1.95 with one group and 0.94 / 1.79 with 128 query rows per CTA; GPT-2 XL at 1024, 400
+  // CTAs: no difference); one group beyond that (64 x 128 tokens, 1536 CTAs: 4.46 against 4.8 ms) and for a single tile.
+  const long long ctas = (long long)((n_tok + 63) / 64) * H * n_seq;
+#define PAIR_ATTN(W, G)                                                                                                  \
+  do {                                                                                                                   \
+    CK(allow_smem(dev, attn_prefill64_pair_kernel<W, G>));                                                               \
+    LAUNCH_PDL(dev, (attn_prefill64_pair_kernel<W, G>), dim3((n_tok + 16 * W - 1) / (16 * W), H, n_seq), 32 * W * G,     \
+               attn_pair_smem_bytes(G), q, ldq, kc, vc, ldkv, kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes, plane, \
+               ldo, src);                                                                                                \
+  } while (0)
+  if (n_tok > 64 && 2 * ctas <= 5 * dev->sm_count) PAIR_ATTN(4, 2);
+  else PAIR_ATTN(4, 1);
+#undef PAIR_ATTN
   return WGPT_OK;
 }
 

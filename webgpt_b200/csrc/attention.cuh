@@ -675,7 +675,9 @@ attn_prefill64_mma_kernel(const float *__restrict__ q, int ldq, const float *__r
 // each product is h0 h0 + h0 h1 + h1 h0 through mma.sync.m16n8k16, half the instructions of the TF32 form at the same
 // terms. K and V tiles are split once, while they are staged, instead of by every warp at every fragment; fragments come
 // by ldmatrix; the score accumulators of two 8-key tiles are the A fragment of a 16-key value step as they are, so the
-// probabilities need no shuffles. 16 WARPS query rows per CTA share a staged 64-key tile. Output as a pair.
+// probabilities need no shuffles. 16 WARPS query rows per CTA share a staged 64-key tile. KG > 1: KG groups of WARPS warps
+// take the same rows and alternate key tiles (staged together), their results merged at the end - for grids that leave SMs
+// idle, where the serial chain of a row's key tiles is what the kernel takes. Output as a pair.
 constexpr int kAttnPairLd = 72;  // halves per staged row: 144 bytes, so that the eight rows of an ldmatrix hit all banks
 
 __device__ __forceinline__ void mma_f16_16x8x16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -701,18 +703,21 @@ __device__ __forceinline__ uint32_t pair_word(float x, float y, uint32_t &lo) {
   return *reinterpret_cast<const uint32_t *>(&a);
 }
 
-template <int WARPS>
-__global__ void __launch_bounds__(32 * WARPS)
+constexpr size_t attn_pair_smem_bytes(int kg) { return (size_t)4 * kg * 64 * kAttnPairLd * 2; }
+
+template <int WARPS, int KG>
+__global__ void __launch_bounds__(32 * WARPS * KG)
 attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__restrict__ kc,
                            const float *__restrict__ vc, int ldkv, size_t kv_seq_stride, int n_tok,
                            const int *__restrict__ pos, float scale, float s_qk, float s_v,
                            __half *__restrict__ planes, size_t plane, int ldo, AttnScaleSrc src) {
-  constexpr int HS = 64, TQ = 16 * WARPS, T = 64, LD = kAttnPairLd, NT = 32 * WARPS;
-  __shared__ __align__(16) __half Ks[2][T * LD];
-  __shared__ __align__(16) __half Vs[2][T * LD];
+  constexpr int HS = 64, TQ = 16 * WARPS, T = 64, LD = kAttnPairLd, NT = 32 * WARPS * KG;
+  extern __shared__ __align__(16) __half attn_pair_smem[];
+  __half *Ks = attn_pair_smem, *Vs = attn_pair_smem + 2 * KG * T * LD;  // [plane][KG tiles of T keys][LD]
   const int h = blockIdx.y, seq = blockIdx.z;
   const int t0 = (int)(gridDim.x - 1 - blockIdx.x) * TQ;  // the query tiles with the most keys first
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int warp = (tid >> 5) % WARPS, kg = (tid >> 5) / WARPS;
   pdl_launch_dependents();
   pdl_wait();
   const int pos0 = pos ? __ldcg(pos) : 0;
@@ -756,19 +761,20 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
     for (int e = 0; e < 4; e++) o[j][e] = 0.f;
   // ldmatrix row addresses of this lane: keys (lane & 7) + 8 (lane >> 4), dims 8 ((lane >> 3) & 1) for K (two 8-key tiles
   // x 16 dims); keys (lane & 15), dims 8 (lane >> 4) for V, transposed (16 keys x two 8-dim tiles)
-  const uint32_t k_row = smem_addr(&Ks[0][0]) + 2u * (uint32_t)(((lane & 7) + 8 * (lane >> 4)) * LD + 8 * ((lane >> 3) & 1));
-  const uint32_t v_row = smem_addr(&Vs[0][0]) + 2u * (uint32_t)((lane & 15) * LD + 8 * (lane >> 4));
-  constexpr uint32_t kPlane = 2u * T * LD;
+  const uint32_t k_row = smem_addr(Ks) + 2u * (uint32_t)((kg * T + (lane & 7) + 8 * (lane >> 4)) * LD + 8 * ((lane >> 3) & 1));
+  const uint32_t v_row = smem_addr(Vs) + 2u * (uint32_t)((kg * T + (lane & 15)) * LD + 8 * (lane >> 4));
+  constexpr uint32_t kPlane = 2u * KG * T * LD;
 
-  for (int j0 = 0; j0 <= last_key; j0 += T) {
+  for (int jb = 0; jb <= last_key; jb += KG * T) {
+    const int j0 = jb + kg * T;
     __syncthreads();  // the previous tile is no longer read
     {
-      constexpr int PER = T * (HS / 4) / NT;  // float4 of K (and of V) per thread
+      constexpr int PER = KG * T * (HS / 4) / NT;  // float4 of K (and of V) per thread
       float4 kv[PER], vv[PER];
 #pragma unroll
       for (int i = 0; i < PER; i++) {
         const int idx = tid + NT * i, r = idx >> 4, c4 = (idx & 15) * 4;
-        const size_t at = (size_t)min(j0 + r, last_key) * ldkv + c4;
+        const size_t at = (size_t)min(jb + r, last_key) * ldkv + c4;
         kv[i] = __ldcg(reinterpret_cast<const float4 *>(kb + at));
         vv[i] = __ldcg(reinterpret_cast<const float4 *>(vb + at));
       }
@@ -777,11 +783,11 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
         const int idx = tid + NT * i, r = idx >> 4, c4 = (idx & 15) * 4;
         uint2 a, b;
         pair_split4(scale4(kv[i], s_qk), a, b);
-        *reinterpret_cast<uint2 *>(&Ks[0][r * LD + c4]) = a;
-        *reinterpret_cast<uint2 *>(&Ks[1][r * LD + c4]) = b;
+        *reinterpret_cast<uint2 *>(Ks + r * LD + c4) = a;
+        *reinterpret_cast<uint2 *>(Ks + (KG * T + r) * LD + c4) = b;
         pair_split4(scale4(vv[i], s_v), a, b);
-        *reinterpret_cast<uint2 *>(&Vs[0][r * LD + c4]) = a;
-        *reinterpret_cast<uint2 *>(&Vs[1][r * LD + c4]) = b;
+        *reinterpret_cast<uint2 *>(Vs + r * LD + c4) = a;
+        *reinterpret_cast<uint2 *>(Vs + (KG * T + r) * LD + c4) = b;
       }
     }
     __syncthreads();
@@ -826,15 +832,18 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
     }
     mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1)); mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
     mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-    const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);  // finite: key 0 of the first tile is visible to every row
-    const float c0 = expf(m0 - mn0), c1 = expf(m1 - mn1);
+    float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);  // finite with KG == 1: every row sees key 0 of its first tile
+    m0 = KG > 1 && mn0 == -INFINITY ? 0.f : m0;        // a row that has seen no key yet: everything below gives zero
+    m1 = KG > 1 && mn1 == -INFINITY ? 0.f : m1;
+    const float b0 = KG > 1 && mn0 == -INFINITY ? 0.f : mn0, b1 = KG > 1 && mn1 == -INFINITY ? 0.f : mn1;
+    const float c0 = expf(m0 - b0), c1 = expf(m1 - b1);
     float ps0 = 0.f, ps1 = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
-      s[j][0] = expf(s[j][0] - mn0);
-      s[j][1] = expf(s[j][1] - mn0);
-      s[j][2] = expf(s[j][2] - mn1);
-      s[j][3] = expf(s[j][3] - mn1);
+      s[j][0] = expf(s[j][0] - b0);
+      s[j][1] = expf(s[j][1] - b0);
+      s[j][2] = expf(s[j][2] - b1);
+      s[j][3] = expf(s[j][3] - b1);
       ps0 += s[j][0] + s[j][1];
       ps1 += s[j][2] + s[j][3];
     }
@@ -863,6 +872,36 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
         mma_f16_16x8x16(o[2 * jp + 1], ph, vl[2], vl[3]);
         mma_f16_16x8x16(o[2 * jp], pl, vh[0], vh[1]);
         mma_f16_16x8x16(o[2 * jp + 1], pl, vh[2], vh[3]);
+      }
+    }
+  }
+  if (KG > 1) {  // merge the groups' results, in group order
+    constexpr int REC = 36;
+    float *mg = reinterpret_cast<float *>(attn_pair_smem);  // [KG - 1][WARPS][REC][32]
+    __syncthreads();
+    if (kg > 0) {
+      float *r = mg + (size_t)((kg - 1) * WARPS + warp) * REC * 32 + lane;
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) r[(4 * j + e) * 32] = o[j][e];
+      r[32 * 32] = m0; r[33 * 32] = m1; r[34 * 32] = l0; r[35 * 32] = l1;
+    }
+    __syncthreads();
+    if (kg > 0) return;
+#pragma unroll 1
+    for (int k = 0; k < KG - 1; k++) {
+      const float *r = mg + (size_t)(k * WARPS + warp) * REC * 32 + lane;
+      const float n0 = r[32 * 32], n1 = r[33 * 32];
+      const float x0 = fmaxf(m0, n0), x1 = fmaxf(m1, n1);  // finite: group 0 has seen key 0
+      const float a0 = expf(m0 - x0), a1 = expf(m1 - x1), d0 = expf(n0 - x0), d1 = expf(n1 - x1);
+      l0 = l0 * a0 + r[34 * 32] * d0;
+      l1 = l1 * a1 + r[35 * 32] * d1;
+      m0 = x0; m1 = x1;
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        o[j][0] = o[j][0] * a0 + r[(4 * j) * 32] * d0; o[j][1] = o[j][1] * a0 + r[(4 * j + 1) * 32] * d0;
+        o[j][2] = o[j][2] * a1 + r[(4 * j + 2) * 32] * d1; o[j][3] = o[j][3] * a1 + r[(4 * j + 3) * 32] * d1;
       }
     }
   }
