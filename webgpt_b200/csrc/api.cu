@@ -1668,7 +1668,7 @@ WGPT_EXPORT int32_t wgpt_int8_matmul(wgpt_device *dev, int32_t M, int32_t K, int
 struct wgpt_int8_weight {
   wgpt_device *dev;
   int K, N;
-  uint32_t *words;   // [K, N/4], the prototype's packing (copy)
+  uint32_t *words;   // [K, N/4], the prototype's packing (copy); owns the allocation of all four
   uint8_t *bytes;    // [N, K], K contiguous; nullptr when K % 16 != 0
   __half *halves;    // [N, K]: the codes as half-precision values (exact), for the tensor cores; nullptr as bytes
   float *scale;      // [N]
@@ -1685,14 +1685,20 @@ WGPT_EXPORT int32_t wgpt_int8_weight_create(wgpt_device *dev, int32_t K, int32_t
   wgpt_int8_weight *w = new wgpt_int8_weight();
   w->dev = dev; w->K = K; w->N = N; w->words = nullptr; w->bytes = nullptr; w->halves = nullptr; w->scale = nullptr;
   const size_t nbytes = (size_t)K * N;
-  cudaError_t e = cudaMalloc(&w->words, nbytes);
-  if (e == cudaSuccess) e = cudaMalloc(&w->scale, (size_t)N * 4);
-  if (e == cudaSuccess && K % 16 == 0) e = cudaMalloc(&w->bytes, nbytes);
-  if (e == cudaSuccess && K % 16 == 0) e = cudaMalloc(&w->halves, 2 * nbytes);
+  const size_t a256 = (nbytes + 255) & ~size_t(255), s256 = ((size_t)N * 4 + 255) & ~size_t(255);
+  const bool relaid = K % 16 == 0;
+  char *base = nullptr;  // one allocation: words | scale | bytes | halves
+  cudaError_t e = cudaMalloc(&base, a256 + s256 + (relaid ? 3 * a256 : 0));
+  w->words = reinterpret_cast<uint32_t *>(base);
+  w->scale = reinterpret_cast<float *>(base + a256);
+  if (relaid) {
+    w->bytes = reinterpret_cast<uint8_t *>(base + a256 + s256);
+    w->halves = reinterpret_cast<__half *>(base + 2 * a256 + s256);
+  }
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->words, Bq, nbytes, cudaMemcpyDeviceToDevice, dev->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->scale, scale, (size_t)N * 4, cudaMemcpyDeviceToDevice, dev->stream);
   if (e != cudaSuccess) {
-    cudaFree(w->words); cudaFree(w->scale); cudaFree(w->bytes); cudaFree(w->halves);
+    cudaFree(w->words);
     delete w;
     return fail(e == cudaErrorMemoryAllocation ? WGPT_ERR_OOM : WGPT_ERR_CUDA, "int8 weight: %s", cudaGetErrorString(e));
   }
@@ -1712,7 +1718,7 @@ WGPT_EXPORT int32_t wgpt_int8_weight_destroy(wgpt_int8_weight *w) {
   TRY(use(w->dev));
   NOT_RECORDING(w->dev, "wgpt_int8_weight_destroy");
   CK(cudaStreamSynchronize(w->dev->stream));
-  cudaFree(w->words); cudaFree(w->scale); cudaFree(w->bytes); cudaFree(w->halves);
+  cudaFree(w->words);
   delete w;
   return WGPT_OK;
 }
@@ -2825,6 +2831,13 @@ static int32_t reserve_out_ids(wgpt_session *s, int n_new) {
 static int32_t launch_sample_topk(wgpt_device *dev, const float *logits, int n_rows, int V, int top_k,
                                   double temperature, const double *uniforms, uint32_t *next_ids, uint32_t *out_ids,
                                   int out_stride, int *pos, int *step, int n_tok, unsigned int *counter) {
+  const int C = V > 4096 ? kPickCluster : 1;
+  if (top_k <= kPickTopK && V <= C * kPickThreads * kPickVals) {
+    CK(launch_ex_x(dev->pdl, C, dev->stream, sample_pick_kernel, dim3(C * n_rows), dim3(kPickThreads), 0, logits, V, top_k,
+                   temperature, uniforms, next_ids, out_ids, out_stride, pos, step, n_tok, counter));
+    dev->launches++;
+    return WGPT_OK;
+  }
   const int per_thread = (V + kSampleThreads - 1) / kSampleThreads;
   const size_t cap = (size_t)top_k * per_thread;
   const size_t smem = (kSampleThreads + cap) * sizeof(unsigned long long);
