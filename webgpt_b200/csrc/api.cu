@@ -2857,8 +2857,11 @@ static int32_t pick_and_advance(wgpt_session *s, int n_tok) {
     s->len += n_tok;
     return WGPT_OK;
   }
-  LAUNCH_PDL(s->m->dev, argmax_kernel, s->n_seq, 1024, 0, (const float *)s->logits, s->m->p.vocab_size, s->next_ids,
-             s->out_ids, s->out_cap, s->d_pos, s->d_step, n_tok, s->attn_cnt + (size_t)s->n_seq * s->m->p.n_head);
+  const int C = s->m->p.vocab_size > 4096 ? 8 : 1;
+  CK(launch_ex_x(s->m->dev->pdl, C, s->m->dev->stream, argmax_kernel, dim3(C * s->n_seq), dim3(C > 1 ? 512 : 1024), 0,
+                 (const float *)s->logits, s->m->p.vocab_size, s->next_ids, s->out_ids, s->out_cap, s->d_pos, s->d_step, n_tok,
+                 s->attn_cnt + (size_t)s->n_seq * s->m->p.n_head));
+  s->m->dev->launches++;
   s->len += n_tok;
   return WGPT_OK;
 }

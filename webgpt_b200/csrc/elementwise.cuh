@@ -175,21 +175,29 @@ __global__ void embed_kernel(const uint32_t *__restrict__ idx, const float *__re
 // with top_k = 1). Writes the id as the next input token and into the output list at *step. The last block to
 // finish then advances the session's position by n_tok and its step counter by one (every block has read
 // *step before it can be counted as finished). done_counter must be zero on entry and is left zero.
+// The CTAs of a cluster share a sequence's logits (a decode step waits for this kernel: one CTA per row of 50257 took 8.3 us).
 __global__ void argmax_kernel(const float *__restrict__ logits, int V, uint32_t *__restrict__ next_ids,
                               uint32_t *__restrict__ out_ids, int out_stride, int *__restrict__ pos,
                               int *__restrict__ step, int n_tok, unsigned int *__restrict__ done_counter) {
+  uint32_t C;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(C));
+  const int rank = (int)cluster_ctarank(), rows = gridDim.x / C;
+  __shared__ float cv[8];
+  __shared__ int ci[8];
+  cluster_arrive();  // pairs with the wait ahead of the remote stores
   pdl_launch_dependents();
   pdl_wait();
-  int seq = blockIdx.x;
+  int seq = blockIdx.x / C;
   const int my_step = __ldcg(step);
   const float *x = logits + (size_t)seq * V;
+  const int share = (V + (int)C - 1) / (int)C, first = rank * share, last = min(V, first + share);
   float best = -INFINITY;
   int bi = 0x7fffffff;
   // eight loads in flight per thread (few CTAs run: the row scan is bound by latency, not bandwidth); a thread's
   // indices ascend, so a strict > keeps its lowest index among equal values
-  int i = threadIdx.x;
+  int i = first + threadIdx.x;
   const int stride = blockDim.x;
-  for (; i + 7 * stride < V; i += 8 * stride) {
+  for (; i + 7 * stride < last; i += 8 * stride) {
     float v[8];
 #pragma unroll
     for (int u = 0; u < 8; u++) v[u] = __ldcg(x + i + u * stride);
@@ -197,7 +205,7 @@ __global__ void argmax_kernel(const float *__restrict__ logits, int V, uint32_t 
     for (int u = 0; u < 8; u++)
       if (v[u] > best) { best = v[u]; bi = i + u * stride; }
   }
-  for (; i < V; i += stride) {
+  for (; i < last; i += stride) {
     float v = __ldcg(x + i);
     if (v > best) { best = v; bi = i; }
   }
@@ -222,13 +230,28 @@ __global__ void argmax_kernel(const float *__restrict__ logits, int V, uint32_t 
       int oi = __shfl_xor_sync(0xffffffffu, bi, o);
       if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
     }
+    cluster_wait();
     if (lane == 0) {
+      dsmem_st(dsmem_addr(&cv[rank], 0), best);
+      dsmem_st(dsmem_addr(&ci[rank], 0), __int_as_float(bi));
+    }
+  } else {
+    cluster_wait();
+  }
+  cluster_arrive();
+  cluster_wait();
+  if (rank == 0 && warp == 0) {
+    if (lane == 0) {
+      best = cv[0];
+      bi = ci[0];
+      for (int r = 1; r < (int)C; r++)  // shares ascend: a later one has to be greater
+        if (cv[r] > best || (bi == 0x7fffffff && ci[r] != 0x7fffffff)) { best = cv[r]; bi = ci[r]; }
       if (bi == 0x7fffffff) bi = 0;  // a row of NaNs compares false everywhere: report index 0
       next_ids[seq] = (uint32_t)bi;
       if (out_ids) out_ids[(size_t)seq * out_stride + my_step] = (uint32_t)bi;
       __threadfence();
       unsigned int prev = atomicAdd(done_counter, 1u);
-      if (prev == gridDim.x - 1) {
+      if (prev == (unsigned int)rows - 1) {
         *pos = __ldcg(pos) + n_tok;
         *step = my_step + 1;
         *done_counter = 0u;
