@@ -595,38 +595,30 @@ static bool gemv_block_plan(const wgpt_device *dev, int M, int K, int N, bool la
 
 template <int M>
 static int32_t launch_gemv_block_t(wgpt_device *dev, const float *x, size_t ldx, const float *gamma, const float *beta,
-                                   const float *Wt, int K, int N, int cols, int wk, size_t smem, const Epilogue &epi,
-                                   const AttnPartials &ap) {
+                                   const float *Wt, int K, int N, int cols, int wk, size_t smem, const Epilogue &epi) {
   auto kern = gemv_block_kernel<M>;
   CK(allow_smem(dev, kern));
   int grid = (N + cols - 1) / cols;
-  LAUNCH_PDL(dev, kern, grid, kBlockGemvThreads, smem, x, ldx, gamma, beta, Wt, K, N, cols, wk, epi, dev->d_err, ap);
+  LAUNCH_PDL(dev, kern, grid, kBlockGemvThreads, smem, x, ldx, gamma, beta, Wt, K, N, cols, wk, epi, dev->d_err);
   return WGPT_OK;
 }
 
 static int32_t launch_gemv_nk(wgpt_device *dev, int M, const float *x, size_t ldx, const float *gamma,
                               const float *beta, const float *Wt, int K, int N, const Epilogue &epi,
-                              const GreedyPick &gp = no_pick(), const AttnPartials *partials = nullptr) {
-  AttnPartials ap;
-  memset(&ap, 0, sizeof ap);
-  if (partials) ap = *partials;
+                              const GreedyPick &gp = no_pick()) {
   int cols = 0, wk = 0;
   size_t smem = 0;
   if (gp.pval == nullptr && dev->block_gemv && gemv_block_plan(dev, M, K, N, gamma != nullptr, &cols, &wk, &smem)) {
     switch (M) {
-      case 1: return launch_gemv_block_t<1>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi, ap);
-      case 2: return launch_gemv_block_t<2>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi, ap);
-      case 3: return launch_gemv_block_t<3>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi, ap);
-      case 4: return launch_gemv_block_t<4>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi, ap);
-      case 5: return launch_gemv_block_t<5>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi, ap);
-      case 6: return launch_gemv_block_t<6>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi, ap);
-      case 7: return launch_gemv_block_t<7>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi, ap);
-      case 8: return launch_gemv_block_t<8>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi, ap);
+      case 1: return launch_gemv_block_t<1>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi);
+      case 2: return launch_gemv_block_t<2>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi);
+      case 3: return launch_gemv_block_t<3>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi);
+      case 4: return launch_gemv_block_t<4>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi);
+      case 5: return launch_gemv_block_t<5>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi);
+      case 6: return launch_gemv_block_t<6>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi);
+      case 7: return launch_gemv_block_t<7>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi);
+      case 8: return launch_gemv_block_t<8>(dev, x, ldx, gamma, beta, Wt, K, N, cols, wk, smem, epi);
     }
-  }
-  if (ap.part != nullptr) {  // the register-streaming kernel reads merged rows: merge into x first
-    dim3 mg((ap.H * ap.hs / 4 + 127) / 128, M);
-    LAUNCH_PDL(dev, attn_merge_kernel, mg, 128, 0, ap, const_cast<float *>(x), (int)ldx);
   }
   switch (M) {
     case 1: return launch_gemv_nk_m<1>(dev, x, ldx, gamma, beta, Wt, K, N, epi, gp);
@@ -1293,45 +1285,26 @@ static int32_t launch_attn_prefill(wgpt_device *dev, int hs, const float *q, int
   return fail(WGPT_ERR_UNSUPPORTED, "head_size %d: supported sizes are 4, 8, 16, 32, 64, 128", hs);
 }
 
+// The slices of a (sequence, head) are a cluster along z that merges them; the output may be a pair (planes).
 static int32_t launch_attn_decode(wgpt_device *dev, int hs, const float *q, int ldq, const float *kc, const float *vc,
                                   int ldkv, size_t kv_seq_stride, float *out, int ldo, int n_seq, int H, int n_split,
-                                  const int *pos, float scale, float *part, const QkvPartials *qp = nullptr,
-                                  bool merge_here = false, __half *planes = nullptr, size_t plane = 0,
-                                  float pair_scale = 1.f) {
+                                  const int *pos, float scale, const QkvPartials *qp = nullptr, __half *planes = nullptr,
+                                  size_t plane = 0, float pair_scale = 1.f) {
   dim3 grid(H, n_seq, n_split);
-  if (merge_here) {  // the slices of a (sequence, head) merge inside their cluster; the output may be a pair
-#define CASE_M(HSV)                                                                                                  \
-  case HSV:                                                                                                          \
-    CK(launch_ex(dev->pdl, n_split, dev->stream, (attn_decode_kernel<HSV>), grid, dim3(256), 0, q, ldq, kc, vc, ldkv, \
-                 kv_seq_stride, out, ldo, pos, scale, part, QkvPartials(), n_split > 1 ? 1 : 0, planes, plane,       \
-                 pair_scale));                                                                                       \
-    dev->launches++;                                                                                                 \
+#define CASE(HSV, FROM)                                                                                               \
+  case HSV:                                                                                                           \
+    CK(launch_ex(dev->pdl, n_split, dev->stream, (attn_decode_kernel<HSV, FROM>), grid, dim3(256), 0, q, ldq, kc, vc, \
+                 ldkv, kv_seq_stride, out, ldo, pos, scale, qp ? *qp : QkvPartials(), planes, plane, pair_scale));    \
+    dev->launches++;                                                                                                  \
     return WGPT_OK;
-    switch (hs) {
-      CASE_M(4) CASE_M(8) CASE_M(16) CASE_M(32) CASE_M(64) CASE_M(128)
-    }
-#undef CASE_M
-    return fail(WGPT_ERR_UNSUPPORTED, "head_size %d: supported sizes are 4, 8, 16, 32, 64, 128", hs);
-  }
   if (qp != nullptr) {  // the attention CTAs are the QKV product's second stage (one position slice, 3*hs <= 256)
     switch (hs) {
-#define CASE_Q(HSV)                                                                                                  \
-  case HSV:                                                                                                          \
-    LAUNCH_PDL(dev, (attn_decode_kernel<HSV, true>), grid, 256, 0, q, ldq, kc, vc, ldkv, kv_seq_stride, out, ldo, pos, \
-               scale, part, *qp, 0, (__half *)nullptr, (size_t)0, 1.f);                                               \
-    return WGPT_OK;
-      CASE_Q(4) CASE_Q(8) CASE_Q(16) CASE_Q(32) CASE_Q(64)
-#undef CASE_Q
+      CASE(4, true) CASE(8, true) CASE(16, true) CASE(32, true) CASE(64, true)
     }
     return fail(WGPT_ERR_UNSUPPORTED, "head_size %d with fused QKV second stage", hs);
   }
-#define CASE(HSV)                                                                                                   \
-  case HSV:                                                                                                         \
-    LAUNCH_PDL(dev, attn_decode_kernel<HSV>, grid, 256, 0, q, ldq, kc, vc, ldkv, kv_seq_stride, out, ldo, pos, scale, \
-               part, QkvPartials(), 0, (__half *)nullptr, (size_t)0, 1.f);                                          \
-    return WGPT_OK;
   switch (hs) {
-    CASE(4) CASE(8) CASE(16) CASE(32) CASE(64) CASE(128)
+    CASE(4, false) CASE(8, false) CASE(16, false) CASE(32, false) CASE(64, false) CASE(128, false)
   }
 #undef CASE
   return fail(WGPT_ERR_UNSUPPORTED, "head_size %d: supported sizes are 4, 8, 16, 32, 64, 128", hs);
@@ -2258,7 +2231,6 @@ struct wgpt_session {
   float *kc, *vc;  // [n_layer][n_seq][n_ctx][E]
   float *fx_a = nullptr, *fx_b = nullptr;     // fused decode: residual stream entering the attention / MLP kernel
   float *fpart_a = nullptr, *fpart_b = nullptr;  // fused decode: partial results [n_head][E] and [mlp CTAs][E]
-  float *attn_part;  // decode-attention partials, [n_seq][n_head][n_split][hs + 4]
   unsigned int *attn_cnt;
   uint32_t *ids, *next_ids, *out_ids;
   float *pick_val;  // [n_seq][vocab] per-CTA arg-max candidates of the fused greedy pick
@@ -2342,7 +2314,6 @@ WGPT_EXPORT int32_t wgpt_session_create(wgpt_model *m, int32_t n_seq, wgpt_sessi
   cudaError_t e = cudaMalloc(&s->kc, kv * 4);
   if (e == cudaSuccess) e = cudaMalloc(&s->vc, kv * 4);
   if (e == cudaSuccess) e = cudaMalloc(&s->logits, (size_t)n_seq * p.vocab_size * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&s->attn_part, (size_t)n_seq * p.n_head * kMaxAttnSplit * (m->hs + 4) * 4);
   if (e == cudaSuccess) e = cudaMalloc(&s->attn_cnt, ((size_t)n_seq * p.n_head + 1) * 4);  // + arg-max done counter
   if (e == cudaSuccess) e = cudaMalloc(&s->next_ids, (size_t)n_seq * 4);
   if (e == cudaSuccess) e = cudaMalloc(&s->pick_val, (size_t)n_seq * p.vocab_size * 4);
@@ -2360,7 +2331,7 @@ WGPT_EXPORT int32_t wgpt_session_create(wgpt_model *m, int32_t n_seq, wgpt_sessi
   if (e == cudaSuccess) e = cudaMemsetAsync(s->attn_cnt, 0, ((size_t)n_seq * p.n_head + 1) * 4, m->dev->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(s->d_pos, 0, 2 * sizeof(int), m->dev->stream);
   if (e != cudaSuccess) {
-    cudaFree(s->kc); cudaFree(s->vc); cudaFree(s->logits); cudaFree(s->attn_part); cudaFree(s->attn_cnt);
+    cudaFree(s->kc); cudaFree(s->vc); cudaFree(s->logits); cudaFree(s->attn_cnt);
     cudaFree(s->next_ids); cudaFree(s->d_pos); cudaFree(s->pick_val); cudaFree(s->pick_idx); cudaFree(s->pick_keys);
     cudaFree(s->fx_a); cudaFree(s->fx_b); cudaFree(s->fpart_a); cudaFree(s->fpart_b);
     delete s;
@@ -2379,7 +2350,7 @@ WGPT_EXPORT int32_t wgpt_session_destroy(wgpt_session *s) {
   cudaStreamSynchronize(s->m->dev->stream);
   drop_step_graph(s);
   session_free_act(s);
-  cudaFree(s->kc); cudaFree(s->vc); cudaFree(s->logits); cudaFree(s->attn_part); cudaFree(s->attn_cnt);
+  cudaFree(s->kc); cudaFree(s->vc); cudaFree(s->logits); cudaFree(s->attn_cnt);
   cudaFree(s->next_ids); cudaFree(s->out_ids); cudaFree(s->d_pos); cudaFree(s->pick_val); cudaFree(s->pick_idx); cudaFree(s->pick_keys);
   cudaFree(s->d_uniform);
   cudaFree(s->fx_a); cudaFree(s->fx_b); cudaFree(s->fpart_a); cudaFree(s->fpart_b);
@@ -2468,7 +2439,7 @@ static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
   const int E = p.n_embd, F = 4 * E, H = p.n_head, hs = m->hs, M = s->n_seq * n_tok;
   const size_t kv_layer = (size_t)s->n_seq * p.n_ctx * E, plane_e = (size_t)M * E, plane_f = (size_t)M * F;
   __half *h = reinterpret_cast<__half *>(s->h), *o = reinterpret_cast<__half *>(s->o), *f = reinterpret_cast<__half *>(s->f);
-  const bool o_pair = n_tok > 1 && attn_prefill_pair_ok(dev, hs);
+  const bool o_pair = n_tok == 1 || attn_prefill_pair_ok(dev, hs);
   for (int l = 0; l < p.n_layer; l++) {
     const LayerWeights &L = m->layers[l];
     float *kc = s->kc + (size_t)l * kv_layer, *vc = s->vc + (size_t)l * kv_layer;
@@ -2478,13 +2449,8 @@ static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
     e.kc = kc; e.vc = vc; e.E = E; e.n_tok = n_tok; e.n_ctx = p.n_ctx; e.pos = s->d_pos;
     TRY(launch_pair_product(dev, h, L.wqkv_p.p, M, E, 3 * E, e));
     if (n_tok == 1) {
-      TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, s->n_seq, H, s->n_split, s->d_pos,
-                             m->scale, s->attn_part));
-      if (s->n_split > 1) {
-        AttnPartials ap;
-        ap.part = s->attn_part; ap.n_split = s->n_split; ap.H = H; ap.hs = hs;
-        LAUNCH_PDL(dev, attn_merge_kernel, dim3((E / 4 + 127) / 128, M), 128, 0, ap, s->o, E);
-      }
+      TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, nullptr, E, s->n_seq, H, s->n_split, s->d_pos,
+                             m->scale, nullptr, o, plane_e, L.s_o));
     } else if (o_pair) {
       TRY(launch_attn_prefill_pair(dev, s->q, E, kc, vc, E, (size_t)p.n_ctx, n_tok, s->n_seq, H, s->d_pos, m->scale,
                                    L.s_qk, L.s_o, o, plane_e, E));
@@ -2545,7 +2511,7 @@ static int32_t forward_blocks_split(wgpt_session *s, int n_tok) {
     const __half *o_in = o;
     if (n_tok == 1) {
       TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, nullptr, E, M, H, s->n_split, s->d_pos, m->scale,
-                             nullptr, nullptr, true, o, plane_e, L.s_o));
+                             nullptr, o, plane_e, L.s_o));
     } else if (attn_prefill_pair_ok(dev, hs)) {
       TRY(launch_attn_prefill_pair(dev, s->q, E, kc, vc, E, (size_t)p.n_ctx, n_tok, s->n_seq, H, s->d_pos, m->scale,
                                    L.s_qk, L.s_o, o, plane_e, E));
@@ -2603,7 +2569,7 @@ static int32_t forward_blocks_ring(wgpt_session *s, bool *done) {
     e.kc = kc; e.vc = vc; e.E = E; e.n_tok = 1; e.n_ctx = p.n_ctx; e.pos = s->d_pos;
     TRY(launch_gemv_ring(dev, pq, M, s->x, L.ln1_g, L.ln1_b, L.wqkv_t, E, 3 * E, e));
     TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, M, H, s->n_split, s->d_pos, m->scale,
-                           nullptr, nullptr, true));
+                           nullptr));
     e = plain_epi(s->x, E, L.bo);
     e.residual = s->x;
     TRY(launch_gemv_ring(dev, po, M, s->o, nullptr, nullptr, L.wo_t, E, E, e));
@@ -2690,30 +2656,17 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
     if (n_tok == 1 && qkv_slices.taken) {
       QkvPartials qp{qkv_slices.part, L.bqkv, qkv_slices.splits, M, E};
       TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, s->n_seq, H, s->n_split, s->d_pos,
-                             m->scale, s->attn_part, &qp));
-    } else if (n_tok == 1)
+                             m->scale, &qp));
+    } else if (n_tok == 1)  // the slices of a (sequence, head) merge in their cluster
       TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, s->n_seq, H, s->n_split, s->d_pos,
-                             m->scale, s->attn_part));
+                             m->scale));
     else
       TRY(launch_attn_prefill(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, n_tok, s->n_seq, H, s->d_pos,
                               m->scale));
     {  // attention output projection + residual
       Epilogue e = plain_epi(s->x, E, L.bo);
       e.residual = s->x;
-      if (n_tok == 1 && s->n_split > 1) {
-        // the decode attention left per-slice partials; the projection merges them while staging its input
-        AttnPartials ap;
-        ap.part = s->attn_part; ap.n_split = s->n_split; ap.H = H; ap.hs = hs;
-        if (gemv_nk_fits(dev, M, E)) {
-          TRY(launch_gemv_nk(dev, M, s->o, (size_t)E, nullptr, nullptr, L.wo_t, E, E, e, no_pick(), &ap));
-        } else {
-          dim3 mg((E / 4 + 127) / 128, M);
-          LAUNCH_PDL(dev, attn_merge_kernel, mg, 128, 0, ap, s->o, E);
-          TRY(mm(s->o, nullptr, nullptr, L.wo_t, E, E, e, L.ln2_g, L.ln2_b));
-        }
-      } else {
-        TRY(mm(s->o, nullptr, nullptr, L.wo_t, E, E, e, L.ln2_g, L.ln2_b));
-      }
+      TRY(mm(s->o, nullptr, nullptr, L.wo_t, E, E, e, L.ln2_g, L.ln2_b));
     }
     {  // LN2 + MLP up-projection + GELU
       Epilogue e = plain_epi(s->f, F, L.bfc);

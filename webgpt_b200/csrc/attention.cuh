@@ -14,9 +14,9 @@ namespace wgpt {
 // ------------------------------------------------------------------------------------------------
 // Decode: one query row per sequence at position *pos (keys 0..*pos). grid = (H, n_seq, n_split): the CTAs along
 // z share one (sequence, head) and each takes a slice of the positions. A CTA (8 warps) runs an online softmax
-// over its slice. With n_split == 1 it writes the head's output; otherwise it writes an un-normalised partial
-// (acc[HS], max, sum, 2 pad) to scratch, part[((seq*H + h)*n_split + split)*(HS+4)], and the consumer merges the
-// slices in slice order while it stages its input (attn_merged_value below): no atomics, no extra pass.
+// over its slice; with n_split > 1 the slices' CTAs are a cluster and the first one merges their un-normalised results
+// (acc, max, sum) in slice order. Left to the consumer, the merge cost every CTA of the output projection the partial
+// results of every row (GPT-2 pass of 2 / 4 / 5 sequences 319 / 397 / 466 us, merged here 298 / 354 / 409).
 // HBM-bound: reads 2*HS*4 bytes per position per head. Before the dependency wait the CTA asks for its slice of
 // the cache in L2, computed from the position counter as it stands then (possibly one step old: the rows of
 // earlier positions never change, so a stale bound only misses the newest row).
@@ -46,8 +46,7 @@ template <int HS, bool FROM_QKV_PART = false>
 __global__ void __launch_bounds__(256)
 attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict__ kc, const float *__restrict__ vc,
                    int ldkv, size_t kv_seq_stride, float *__restrict__ out, int ldo, const int *__restrict__ pos,
-                   float scale, float *__restrict__ part, QkvPartials qp = QkvPartials(), int merge_here = 0,
-                   __half *__restrict__ planes = nullptr, size_t plane = 0, float pair_scale = 1.f) {
+                   float scale, QkvPartials qp, __half *__restrict__ planes, size_t plane, float pair_scale) {
   constexpr int LPP = HS / 4;      // lanes per position (one float4 each)
   constexpr int G = 32 / LPP;      // positions per warp iteration
   constexpr int NW = 8;
@@ -58,7 +57,7 @@ attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict
   const float *vb = vc + (size_t)seq * kv_seq_stride * ldkv + h * HS;
   TRACE_BEGIN(3);
   trace(3, 0);
-  if (merge_here) cluster_arrive();  // pairs with the wait ahead of the first remote store
+  if (n_split > 1) cluster_arrive();  // pairs with the wait ahead of the first remote store
   pdl_launch_dependents();
   {
     const int Ls = __ldcg(pos) + 1;
@@ -180,17 +179,13 @@ attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict
     }
     if (n_split == 1) {
       attn_put(out, planes, plane, pair_scale, (size_t)seq * ldo + h * HS + tid, a / ll);
-    } else if (merge_here) {
+    } else {
       keep_a = a;
       keep_m = mm;
       keep_l = ll;
-    } else {
-      float *my = part + ((size_t)(seq * H + h) * n_split + split) * (HS + 4);
-      my[tid] = a;
-      if (tid == 0) { my[HS] = mm; my[HS + 1] = ll; }
     }
   }
-  if (merge_here && n_split > 1) {
+  if (n_split > 1) {
     // The slices of a (sequence, head) are a cluster along z: every CTA hands its record to the first one, which merges
     // them in slice order and finishes the output, so no consumer has to (and no merge pass stands before it).
     __shared__ float mrg[8][HS + 2];
@@ -214,55 +209,6 @@ attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict
     }
   }
   trace(3, 4);
-}
-
-// Description of attention partials left by attn_decode_kernel with n_split > 1, for consumers that merge them
-// while staging their input. part == nullptr: no merge, the input is read as is.
-struct AttnPartials {
-  const float *part;
-  int n_split, H, hs;
-};
-
-// Elements c..c+3 (c % 4 == 0, all in one head) of the attention output of sequence `seq`: the slices'
-// partials combined in slice order.
-__device__ __forceinline__ float4 attn_merged_value4(const AttnPartials &ap, int seq, int c) {
-  const int h = c / ap.hs, d = c - h * ap.hs;
-  const int stride = ap.hs + 4;
-  const float *p0 = ap.part + (size_t)(seq * ap.H + h) * ap.n_split * stride;
-  float pm[8], pl[8];
-  float4 pa[8];
-#pragma unroll
-  for (int r = 0; r < 8; r++) {
-    if (r < ap.n_split) {
-      const float *pr = p0 + (size_t)r * stride;
-      pa[r] = __ldcg(reinterpret_cast<const float4 *>(pr + d));
-      float2 ml = __ldcg(reinterpret_cast<const float2 *>(pr + ap.hs));
-      pm[r] = ml.x;
-      pl[r] = ml.y;
-    } else {
-      pm[r] = -INFINITY; pl[r] = 0.f; pa[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
-  float mm = pm[0];
-#pragma unroll
-  for (int r = 1; r < 8; r++) mm = fmaxf(mm, pm[r]);
-  float ll = 0.f;
-  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-  for (int r = 0; r < 8; r++) {
-    float c2 = (pm[r] == -INFINITY) ? 0.f : expf(pm[r] - mm);
-    ll += pl[r] * c2;
-    a.x += pa[r].x * c2; a.y += pa[r].y * c2; a.z += pa[r].z * c2; a.w += pa[r].w * c2;
-  }
-  return make_float4(a.x / ll, a.y / ll, a.z / ll, a.w / ll);
-}
-
-// Stand-alone merge for consumers that cannot merge on the fly: out[seq, c] for c in [0, H*hs).
-__global__ void attn_merge_kernel(AttnPartials ap, float *__restrict__ out, int ldo) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int seq = blockIdx.y, c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
-  if (c < ap.H * ap.hs) *reinterpret_cast<float4 *>(out + (size_t)seq * ldo + c) = attn_merged_value4(ap, seq, c);
 }
 
 // ------------------------------------------------------------------------------------------------

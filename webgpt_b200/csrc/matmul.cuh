@@ -577,7 +577,7 @@ template <int M>
 __global__ void __launch_bounds__(kBlockGemvThreads)
 gemv_block_kernel(const float *__restrict__ x, size_t ldx, const float *__restrict__ gamma,
                   const float *__restrict__ beta, const float *__restrict__ Wt, int K, int N, int cols, int wk,
-                  Epilogue epi, int *err, AttnPartials ap) {
+                  Epilogue epi, int *err) {
   extern __shared__ __align__(128) float smem[];
   // Rows-in-lanes form (more than four rows, see below): eight lanes read the same float4 position of eight
   // rows at once, so the rows are padded by one float4 to fall into different banks.
@@ -634,11 +634,7 @@ gemv_block_kernel(const float *__restrict__ x, size_t ldx, const float *__restri
     float4 *xs4w = reinterpret_cast<float4 *>(xs);
     const size_t ldx4 = ldx >> 2;
     const float4 *x4 = reinterpret_cast<const float4 *>(x);
-    if (ap.part != nullptr) {  // the input rows are attention outputs still split into position slices
-#pragma unroll
-      for (int m = 0; m < M; m++)
-        for (int i = tid; i < K4; i += NT) xs4w[(size_t)m * RS4 + i] = attn_merged_value4(ap, m, 4 * i);
-    } else if (M > 1) {
+    if (M > 1) {
       // Every CTA reads the same rows at the same time; starting each CTA at a different offset spreads the
       // requests over L2 instead of having all SMs ask for the same lines at once.
       const int total = M * K4;
