@@ -2275,18 +2275,17 @@ static int32_t session_reserve(wgpt_session *s, int n_tok) {
   return WGPT_OK;
 }
 
-// Position slices per (sequence, head) of the decode attention: 1, 2, 4 or 8 CTAs share a head's cache rows.
-// Doubled while the grid stays within a CTA budget: about two CTAs per SM for up to eight sequences with a short
-// context (the projection that follows merges the slices of every row in every CTA, so slices are not free
-// there), about five per SM for more sequences or a long context, where the attention itself is what costs.
-// Measured per decode pass, chosen / other: GPT-2 117M 16 rows 0.606 (4) / 0.645 (1), 32 rows 0.683 (2) / 0.711 (1),
-// 64 rows 0.791 (1) / 0.820 (2), 8 rows 0.574 (2) / 0.584 (8); GPT-2 XL at 768+ positions 8 sequences 6.57 (4) /
-// 7.46 (1), 16 sequences 6.70 (2) / 7.66 (1), 32 sequences 8.23 (1) / 8.28 (4) ms.
+// Position slices per (sequence, head) of the decode attention: 1, 2, 4 or 8 CTAs of a cluster share a head's cache rows.
+// Doubled while the grid stays within about 5.5 CTAs per SM (what is resident at once) and a slice keeps the positions that
+// a CTA has in flight in one step (4096 / head size), for the context as it is when the step is captured plus 64 for what
+// is generated from there. Per pass, chosen (slices) / others: GPT-2 16 sequences at 128 positions 0.414 (2) / 0.432 (4),
+// 8 at 64 0.362 (2) / 0.400 (8), 4 at 500 0.379 (8) / 0.437 (2); GPT-2 XL 4 at 200 2.25 (4) / 2.39 (2) / 2.47 (8) ms.
 constexpr int kMaxAttnSplit = 8;
-static int attn_split_for(const wgpt_device *dev, int n_head, int n_seq, int context_len) {
-  const int budget = (n_seq > 8 || context_len >= 512) ? (11 * dev->sm_count) / 2 : 2 * dev->sm_count;
+static int attn_split_for(const wgpt_device *dev, int n_head, int n_seq, int head_size, int context_len) {
+  const int step = 4096 / head_size;
   int split = 1;
-  while (split < kMaxAttnSplit && n_head * n_seq * split * 2 <= budget) split *= 2;
+  while (split < kMaxAttnSplit && 2 * n_head * n_seq * split * 2 <= 11 * dev->sm_count && context_len + 64 >= 2 * split * step)
+    split *= 2;
   return split;
 }
 
@@ -2310,7 +2309,7 @@ WGPT_EXPORT int32_t wgpt_session_create(wgpt_model *m, int32_t n_seq, wgpt_sessi
       s->split_forced = true;
     }
   }
-  if (!s->split_forced) s->n_split = attn_split_for(m->dev, p.n_head, n_seq, 0);
+  if (!s->split_forced) s->n_split = attn_split_for(m->dev, p.n_head, n_seq, m->hs, 0);
   cudaError_t e = cudaMalloc(&s->kc, kv * 4);
   if (e == cudaSuccess) e = cudaMalloc(&s->vc, kv * 4);
   if (e == cudaSuccess) e = cudaMalloc(&s->logits, (size_t)n_seq * p.vocab_size * 4);
@@ -2825,7 +2824,7 @@ static int32_t decode_step(wgpt_session *s) {
   wgpt_device *dev = s->m->dev;
   // the slice count follows the context length as it is when the step is (re)captured
   if (!s->split_forced && (!dev->graphs || s->step_graph == nullptr))
-    s->n_split = attn_split_for(dev, s->m->p.n_head, s->n_seq, s->len);
+    s->n_split = attn_split_for(dev, s->m->p.n_head, s->n_seq, s->m->hs, s->len);
   if (!dev->graphs) {
     return forward(s, s->next_ids, 1, true);
   }
