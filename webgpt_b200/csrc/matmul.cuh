@@ -473,7 +473,8 @@ gemv_loop_kernel(const float *__restrict__ x, size_t ldx, const float *__restric
 template <int M>
 __device__ __forceinline__ void cta_layernorm_rows(const float *raw, float *normed, int K,
                                                    const float *__restrict__ gamma, const float *__restrict__ beta,
-                                                   float4 g_first, float4 b_first, int rs4) {
+                                                   float4 g_first, float4 b_first, int rs4, const float4 *g_sm,
+                                                   const float4 *b_sm) {
   // rs4: row stride of raw and normed in float4 (K/4, or more when the rows are padded against bank conflicts)
   const int tid = threadIdx.x, lane = tid & 31;
   const int K4 = K >> 2;
@@ -488,9 +489,9 @@ __device__ __forceinline__ void cta_layernorm_rows(const float *raw, float *norm
     const int warp = tid >> 5, nw = (int)blockDim.x >> 5;
     // gamma and beta of this lane's first eight positions, requested before the statistics so that their L2
     // latency overlaps them (loaded one by one inside the last loop they cost a round trip per position)
-    constexpr int GP = 8;
+    constexpr int GP = M <= 4 ? 8 : 1;
     float4 gpre[GP], bpre[GP];
-    if (warp < M) {
+    if (M <= 4 && warp < M) {
 #pragma unroll
       for (int j = 0; j < GP; j++) {
         const int i = lane + 32 * j;
@@ -514,6 +515,19 @@ __device__ __forceinline__ void cta_layernorm_rows(const float *raw, float *norm
         q += (a * a + b * b) + (c * c + d * d);
       }
       const float rsd = 1.0f / sqrtf(warp_sum(q) / (float)K + 1e-5f);
+      if (M > 4) {
+        // five and more rows: scale and shift from shared memory, where the caller put them ahead of the dependency wait
+        // (GPT-2 at five rows 409 -> 390 us per pass). With up to four rows registers are faster (351 against 376 us at
+        // four): they also keep a second of these kernels off the SM, whose weights would arrive in the middle of this
+        // one's exchanges, and a later release of it did not make up for that (369 us).
+#pragma unroll 2
+        for (int i = lane; i < K4; i += 32) {
+          const float4 v = x4[(size_t)m * rs4 + i], g = g_sm[i], b = b_sm[i];
+          o4[(size_t)m * rs4 + i] = make_float4(g.x * ((v.x - mean) * rsd) + b.x, g.y * ((v.y - mean) * rsd) + b.y,
+                                               g.z * ((v.z - mean) * rsd) + b.z, g.w * ((v.w - mean) * rsd) + b.w);
+        }
+        continue;
+      }
 #pragma unroll
       for (int j = 0; j < GP; j++) {
         const int i = lane + 32 * j;
@@ -569,7 +583,7 @@ __device__ __forceinline__ void cta_layernorm_rows(const float *raw, float *norm
 // keeps the same K slice for all its items and handles three columns at a time; the K slices of a column are
 // summed in a fixed order.
 // Dynamic shared memory: [cols*K] weights, [M*K] input rows (twice with LayerNorm), [max(cols*wk, 16)*M]
-// partial sums, one mbarrier.
+// partial sums, with a LayerNorm of more than four rows its scale and shift [2*K], one mbarrier.
 // *err is set (and nothing stored) if the copies do not land within the poll limit.
 constexpr int kBlockGemvThreads = 512;
 
@@ -589,7 +603,10 @@ gemv_block_kernel(const float *__restrict__ x, size_t ldx, const float *__restri
   float *red = xn + (size_t)M * RS4 * 4;
   constexpr int NT = kBlockGemvThreads, NW = NT / 32;
   const int red_floats = ((kRowsInLanes ? NW * cols : max(cols * wk, NW)) * M + 3) & ~3;
-  uint64_t *bar = reinterpret_cast<uint64_t *>(red + red_floats);
+  float4 *g_sm = reinterpret_cast<float4 *>(red + red_floats);  // LayerNorm scale and shift (more than four rows)
+  const int ln4 = M > 4 && gamma != nullptr ? K >> 2 : 0;
+  float4 *b_sm = g_sm + ln4;
+  uint64_t *bar = reinterpret_cast<uint64_t *>(b_sm + ln4);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int K4 = K >> 2;
   const int col0 = blockIdx.x * cols;
@@ -621,9 +638,13 @@ gemv_block_kernel(const float *__restrict__ x, size_t ldx, const float *__restri
   const int end = (int)(((unsigned)K4 * (unsigned)(ks + 1)) >> wk_log2);
   const int items = ncol << wk_log2;
   float4 g_first = make_float4(0.f, 0.f, 0.f, 0.f), b_first = g_first;
-  if (gamma != nullptr && tid < K4) {
+  if (M == 1 && gamma != nullptr && tid < K4) {
     g_first = reinterpret_cast<const float4 *>(gamma)[tid];
     b_first = reinterpret_cast<const float4 *>(beta)[tid];
+  }
+  for (int i = tid; i < ln4; i += NT) {
+    g_sm[i] = reinterpret_cast<const float4 *>(gamma)[i];
+    b_sm[i] = reinterpret_cast<const float4 *>(beta)[i];
   }
   pdl_launch_dependents();
   pdl_wait();
@@ -654,7 +675,7 @@ gemv_block_kernel(const float *__restrict__ x, size_t ldx, const float *__restri
   }
   __syncthreads();  // also makes the mbarrier initialisation visible to every thread
   trace(2, 2);
-  if (gamma != nullptr) cta_layernorm_rows<M>(xs, xn, K, gamma, beta, g_first, b_first, RS4);
+  if (gamma != nullptr) cta_layernorm_rows<M>(xs, xn, K, gamma, beta, g_first, b_first, RS4, g_sm, b_sm);
 
   // Bounded wait for the weights. On expiry: flag the error, give the copies one more bounded chance to land
   // (shared memory must not be released under them), and leave without storing.
