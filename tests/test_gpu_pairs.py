@@ -1,0 +1,193 @@
+"""GPU parity of the kernels on half-precision pairs, of the ring GEMV and of the cluster sampling kernel, at the sizes
+where their tiles, slices and dispatch rules have edges."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import rel_err
+from webgpt_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    from webgpt_b200 import Device
+    d = Device(0)
+    yield d
+    d.destroy()
+
+
+def matmul(dev, A, W, b=None):
+    from webgpt_b200 import _lib
+    M, K = A.shape
+    N = W.shape[1]
+    a_d, w_d, o_d = dev.tensor(A), dev.tensor(W), dev.buffer(M * N * 4)
+    b_d = dev.tensor(b) if b is not None else None
+    _lib.call("wgpt_matmul", dev.handle, M, N, K, a_d.ptr, w_d.ptr, b_d.ptr if b_d else None, o_d.ptr)
+    _lib.call("wgpt_device_check", dev.handle)
+    return o_d.read(np.float32, M * N).reshape(M, N)
+
+
+# (rows, K, N): one row tile and its neighbours, 256-row tiles, N off every tile width, K off 16, 64 and the cluster's
+# slices (a strip of more than 8 x 192 rows of K, fewer k-blocks than slices)
+SHAPES = [(32, 8, 8), (33, 72, 40), (64, 768, 136), (65, 200, 264), (127, 1600, 128), (128, 3072, 8), (129, 64, 4800),
+          (255, 1544, 520), (257, 768, 768), (513, 136, 2312), (1100, 768, 3072)]
+
+
+@pytest.mark.parametrize("M,K,N", SHAPES)
+def test_product_of_pairs_error_bound(dev, M, K, N):
+    """Elementwise bound from the representation. Per product: each operand is off by at most 2^-22 of itself, the dropped
+    h1 g1 is at most 2^-22, so 3 * 2^-22. Per accumulation: the FP32 accumulator of an MMA step is truncated, 2^-23 of the
+    sum so far, 3 K / 16 steps. Both against sum |x w|; 2^-23 more for what is stored. (Operands below 2^-17 of their row's
+    largest carry the absolute error 2^-40 of it, K terms of that at most.)"""
+    rng = np.random.default_rng(M + 7 * K + N)
+    A = rng.standard_normal((M, K), dtype=np.float32)
+    W = (rng.standard_normal((K, N), dtype=np.float32) * np.exp2(rng.integers(-6, 7, N))).astype(np.float32)
+    ref = A.astype(np.float64) @ W.astype(np.float64)
+    mag = np.abs(A).astype(np.float64) @ np.abs(W).astype(np.float64)
+    top = np.abs(A).max(1)[:, None].astype(np.float64) * np.abs(W).max(0)[None, :] * K
+    bound = (3 * 2.0 ** -22 + (3 * K / 16 + 2) * 2.0 ** -23) * mag + 2.0 ** -39 * top
+    got = matmul(dev, A, W)
+    assert (np.abs(got - ref) <= bound).all()
+    assert np.array_equal(matmul(dev, A, W), got)  # deterministic
+    # powers of two per row and per column pass through exactly
+    r, c = np.exp2(rng.integers(-30, 31, M)), np.exp2(rng.integers(-30, 31, N))
+    scaled = matmul(dev, (A * r[:, None]).astype(np.float32), (W * c[None, :]).astype(np.float32))
+    assert np.array_equal(scaled, (got * r[:, None] * c[None, :]).astype(np.float32))
+
+
+@pytest.mark.parametrize("M,K,N", [(40, 96, 264), (300, 776, 200)])
+def test_product_of_pairs_integers_are_exact(dev, M, K, N):
+    """Integers of at most 11 bits are exact in the first plane and their sums in FP32: any misplaced element shows."""
+    A = ((np.arange(M)[:, None] * 7 + np.arange(K)[None, :] * 3) % 11 - 5).astype(np.float32)
+    W = ((np.arange(K)[:, None] * 5 + np.arange(N)[None, :]) % 13 - 6).astype(np.float32)
+    b = np.arange(N, dtype=np.float32)
+    assert np.array_equal(matmul(dev, A, W, b).astype(np.float64), A.astype(np.float64) @ W + b)
+
+
+@pytest.mark.parametrize("T,E,H", [(32, 128, 2), (63, 64, 1), (65, 128, 2), (128, 192, 3), (129, 128, 2), (200, 128, 4),
+                                   (321, 64, 1)])
+def test_attention_operator_on_pairs(dev, oracle, T, E, H):
+    """Query tiles of 64, key tiles shared by two warp groups, head sizes with and without the pair attention."""
+    from webgpt_b200 import _lib
+    rng = np.random.default_rng(T + E)
+    x = rng.standard_normal((T, E), dtype=np.float32)
+    ws = [(rng.standard_normal((E, E), dtype=np.float32) * 0.15).astype(np.float32) for _ in range(4)]
+    bs = [rng.standard_normal(E, dtype=np.float32) for _ in range(4)]
+    scale = float(np.float32(1 / np.sqrt(E // H)))
+    d = [dev.tensor(a) for pair in zip(ws, bs) for a in pair]
+    x_d, o_d = dev.tensor(x), dev.buffer(T * E * 4)
+    _lib.call("wgpt_attention", dev.handle, T, E, scale, H, E // H, x_d.ptr, *[t.ptr for t in d], o_d.ptr)
+    _lib.call("wgpt_device_check", dev.handle)
+    ref = oracle.attention(x, H, scale, ws[0], bs[0], ws[1], bs[1], ws[2], bs[2], ws[3], bs[3])
+    # three products behind one another, each within ~1e-6 of its largest value at these K; 2e-5 is the operators' bound
+    assert rel_err(o_d.read(np.float32, T * E).reshape(T, E), ref) < 2e-5
+
+
+@pytest.fixture(scope="module")
+def model64(oracle):
+    """Head size 64, two layers: every prefill and decode path of the model takes it."""
+    from webgpt_b200 import GPT
+    params = dict(n_layer=2, n_head=3, n_embd=192, n_ctx=384, vocab_size=4104)
+    w = synth.make_weights(params, seed=17, std=0.08, ln_random=True)
+    gpt = GPT(None, params=params, weights=w)
+    gpt.initialize()
+    yield gpt, oracle.Model(params, synth.weight_list(params, w)), params
+    gpt.destroy()
+
+
+@pytest.mark.parametrize("n", [8, 9, 16, 63, 64, 65, 128, 129, 300, 384])
+def test_prompt_lengths(model64, n):
+    gpt, m, p = model64
+    ids = synth.make_tokens(p["vocab_size"], n, seed=n)
+    assert rel_err(gpt.run(ids), m.run(ids)) < 2e-5  # two layers of the products above
+
+
+@pytest.mark.parametrize("n_seq", [2, 5, 6, 16, 17, 48, 49, 64, 65, 70])
+def test_decode_rows(model64, n_seq):
+    """Row tiles of 16, 32, 48 and 64, the step to the planes of more rows, ragged last tiles; greedy ids of the first and
+    last sequence, and logits of one more step behind a chunked prompt."""
+    gpt, m, p = model64
+    prompts = np.stack([synth.make_tokens(p["vocab_size"], 9, seed=90, stream=i) for i in range(n_seq)])
+    s = gpt.session(n_seq)
+    got = s.generate_greedy(prompts, 6)
+    for i in (0, n_seq - 1):
+        assert np.array_equal(got[i], m.kv_generate_greedy(prompts[i], 6)), i
+    s.reset()
+    s.forward(prompts[:, :4], want_logits=False)
+    s.forward(prompts[:, 4:], want_logits=False)
+    lg = s.forward(got[:, :1])
+    for i in (0, n_seq - 1):
+        assert rel_err(lg[i], m.run(np.concatenate([prompts[i], got[i, :1]]))) < 2e-5
+
+
+@pytest.mark.parametrize("n_seq", [1, 2, 3, 5, 8])
+def test_ring_gemv_rows(oracle, n_seq):
+    """Layers that do not fit shared memory (n_embd 1600): FP32 through the ring for up to five sequences, and for eight
+    in FP32 mode; K = 1600 is no multiple of a stage's 256.
+
+    Bound: the reference adds each product's K terms one after another in FP32. For terms of random sign a rounding is at
+    most 2^-24 of a running sum that grows like sqrt(k), uniformly spread (1/sqrt(3)), so the error of a sum is about
+    sqrt(K / 2) 2^-24 / sqrt(3) of its size, 1.9e-6 at the longest K of 6400; four of these is 8e-6. The kernel's own sums,
+    split over lanes and warps, add far less."""
+    from webgpt_b200 import GPT, _lib
+    params = dict(n_layer=1, n_head=25, n_embd=1600, n_ctx=24, vocab_size=512)
+    w = synth.make_weights(params, seed=41, std=0.04, ln_random=True)
+    m = oracle.Model(params, synth.weight_list(params, w))
+    gpt = GPT(None, params=params, weights=w)
+    gpt.initialize()
+    try:
+        if n_seq == 8:
+            gpt.device.set_precision(_lib.PRECISION_FP32)
+        prompts = np.stack([synth.make_tokens(512, 5, seed=5, stream=i) for i in range(n_seq)])
+        s = gpt.session(n_seq)
+        for t in range(5):  # token by token: every pass is a decode pass
+            lg = s.forward(prompts[:, t:t + 1])
+        for i in (0, n_seq - 1):
+            assert rel_err(lg[i], m.run(prompts[i])) < 8e-6
+    finally:
+        gpt.destroy()
+
+
+@pytest.mark.parametrize("K,N", [(48, 40), (768, 136), (1616, 152), (3072, 768)])
+def test_int8_handle_rows(dev, oracle, K, N):
+    """Up to eight rows in the block kernel (columns per item 1-4, K slices 1-8), above 16 rows as pairs against the exact
+    codes: error bound as above with one inexact operand and two MMAs per step."""
+    from webgpt_b200 import _lib
+    h = C.c_void_p()
+    _, q, packed, scale = synth.make_int8_case(1, K, N)
+    p_d, s_d = dev.tensor(packed), dev.tensor(scale)
+    _lib.call("wgpt_int8_weight_create", dev.handle, K, N, p_d.ptr, s_d.ptr, C.byref(h))
+    try:
+        for M in (1, 2, 3, 4, 5, 7, 8, 9, 16, 17, 33, 129, 257):
+            A = np.random.default_rng(M).standard_normal((M, K), dtype=np.float32)
+            a_d, o_d = dev.tensor(A), dev.buffer(M * N * 4)
+            _lib.call("wgpt_int8_matmul_w", dev.handle, M, h, a_d.ptr, o_d.ptr)
+            _lib.call("wgpt_device_check", dev.handle)
+            Wf = q.astype(np.float64) * scale.astype(np.float64)
+            ref, mag = A.astype(np.float64) @ Wf, np.abs(A).astype(np.float64) @ np.abs(Wf)
+            steps = K if M <= 16 else 2 * K / 16 + 2  # CUDA cores: one rounding per term at most
+            bound = (2.0 ** -22 + (steps + 2) * 2.0 ** -23) * mag + 2.0 ** -39 * np.abs(A).max() * np.abs(Wf).max() * K
+            assert (np.abs(o_d.read(np.float32, M * N).reshape(M, N) - ref) <= bound).all(), M
+    finally:
+        _lib.call("wgpt_int8_weight_destroy", h)
+
+
+@pytest.mark.parametrize("V", [48, 4096, 4097, 50257, 65536, 65540])
+def test_sampling_kernel_edges(dev, oracle, V):
+    """One CTA or a cluster, the largest vocabulary its registers hold and the one beyond, top_k at its limit and beyond;
+    an all-equal row has more values at the bound than a list holds, a falling one has them all in one CTA."""
+    from webgpt_b200 import _lib
+    rng = np.random.default_rng(V)
+    rows = np.stack([rng.standard_normal(V).astype(np.float32), np.zeros(V, np.float32),
+                     -np.arange(V, dtype=np.float32), np.where(np.arange(V) % 128 < 8, 5.0, -5.0).astype(np.float32)])
+    u = rng.random(len(rows))
+    r_d, u_d, o_d = dev.tensor(rows), dev.tensor(u), dev.buffer(4 * len(rows))
+    for top_k in (1, 2, 31, 47, 48, 49):
+        if top_k > V:
+            continue
+        _lib.call("wgpt_sample_topk", dev.handle, r_d.ptr, len(rows), V, top_k, 1.3, u_d.ptr, o_d.ptr)
+        got = o_d.read(np.uint32, len(rows))
+        assert [int(t) for t in got] == [oracle.sample_topk(rows[i], top_k, 1.3, u[i]) for i in range(len(rows))], top_k
