@@ -45,12 +45,14 @@ enum {
 };
 
 /* Arithmetic used by matrix products with more than 8 rows (prefill, batched decode, wgpt_matmul_nk; wgpt_matmul and
- * wgpt_attention on reference-layout weights from 32 rows on, through a transposed copy of the weight in the
- * workspace). Products with up to 8 rows always run in FP32 on the CUDA cores. A new device starts in
- * WGPT_PRECISION_TF32X3. */
+ * wgpt_attention on reference-layout weights from 32 rows on) and by a model's decode passes of more than 5 sequences.
+ * The other products of up to 8 rows always run in FP32 on the CUDA cores. A new device starts in
+ * WGPT_PRECISION_TF32X3, in which every tensor-core product is three products of operands split in two: models, wgpt_matmul,
+ * wgpt_attention and the int8 weight handles split an operand into two half-precision values and a power of two per row
+ * (22 significant bits), the others into two TF32 values (21 bits). */
 enum {
   WGPT_PRECISION_FP32 = 0,   /* FP32 FMA on the CUDA cores */
-  WGPT_PRECISION_TF32X3 = 1, /* tensor cores, three TF32 products per FP32 product (error 1e-6..2e-5, growing with K) */
+  WGPT_PRECISION_TF32X3 = 1, /* tensor cores, three products per FP32 product (error 1e-6..2e-5, growing with K) */
   WGPT_PRECISION_TF32 = 2    /* tensor cores, single TF32 product (error ~1e-3) */
 };
 
@@ -206,7 +208,7 @@ int32_t wgpt_int8_matmul(wgpt_device *dev, int32_t M, int32_t K, int32_t N, cons
  * dispatches against it, other/int8-gemm.js:101-113): the handle owns a copy of Bq [K, N/4] and scale [N] (both
  * device memory) and, when K % 16 == 0, a re-laid-out copy with each output column's codes contiguous, which the
  * kernels stream with 128-bit loads. wgpt_int8_matmul_w computes what wgpt_int8_matmul computes, out[M,N] =
- * A[M,K] . (f32(q) * scale[n]): up to 4 rows in one weight-streaming kernel, more than 16 rows on the tensor cores
+ * A[M,K] . (f32(q) * scale[n]): up to 16 rows by a weight-streaming kernel, 8 rows a launch, more than 16 rows on the tensor cores
  * (device precision mode), otherwise through wgpt_int8_matmul. */
 typedef struct wgpt_int8_weight wgpt_int8_weight;
 int32_t wgpt_int8_weight_create(wgpt_device *dev, int32_t K, int32_t N, const uint32_t *Bq, const float *scale,

@@ -1697,43 +1697,54 @@ WGPT_EXPORT int32_t wgpt_int8_weight_destroy(wgpt_int8_weight *w) {
   return WGPT_OK;
 }
 
+constexpr int kInt8BlockGroups = 3;
+struct Int8BlockPlan {
+  int cols, cg, wk;  // columns per CTA, columns per work item, K slices
+  size_t smem;       // 0: the rows and the CTA's columns do not fit shared memory
+};
+
+// Columns per work item and K slices: the pair with the smallest sum of shared-memory cycles (a 128-bit load is four),
+// issue cycles (four a cycle) and the busiest warp's own path. 1600 x 6400 has 44 columns per CTA: items of four columns
+// left five of the sixteen warps without one, three columns leave one; with more rows the row loads decide, which the
+// columns of an item share.
+static Int8BlockPlan int8_block_plan(const wgpt_device *dev, int K, int N, int M) {
+  const int nw = kInt8BlockThreads / 32;
+  Int8BlockPlan p{(N + dev->sm_count - 1) / dev->sm_count, 1, 1, 0};
+  long long best = -1;
+  for (int c = 1; c <= (M <= 4 ? 4 : 3); c++)
+    for (int k = 1; k <= 8; k *= 2) {
+      const int groups = (p.cols + c - 1) / c, rounds = (groups * k + nw - 1) / nw, steps = ((K / 16 + k - 1) / k + 31) / 32;
+      const long long work = (long long)groups * k * steps, instr = c * (28 + 8 * M);
+      const long long cost = work * ((c + 4 * M) * 4 + instr / 4) + rounds * (steps * (instr + 60) + 20 * c * M + 60);
+      if (best < 0 || cost < best) { best = cost; p.cg = c; p.wk = k; }
+    }
+  const size_t red = (size_t)(p.cols * p.wk > nw ? p.cols * p.wk : nw) * M;
+  p.smem = (size_t)p.cols * K + ((size_t)M * K + ((red + 3) & ~size_t(3))) * 4 + 16;
+  if (p.smem > dev->smem_optin - 2048) p.smem = 0;
+  return p;
+}
+
 template <int M, int CG>
-static int32_t launch_int8_block_cg(wgpt_device *dev, const wgpt_int8_weight *w, const float *A, float *out, int cols, int wk,
-                                    size_t smem) {
+static int32_t launch_int8_block_cg(wgpt_device *dev, const wgpt_int8_weight *w, const float *A, float *out,
+                                    const Int8BlockPlan &p) {
   auto kern = int8_block_gemv_kernel<M, CG>;
   CK(allow_smem(dev, kern, true));
-  LAUNCH_PDL(dev, kern, (w->N + cols - 1) / cols, kInt8BlockThreads, smem, A, (const uint8_t *)w->bytes,
-             (const float *)w->scale, w->K, w->N, cols, wk, out, dev->d_err);
+  LAUNCH_PDL(dev, kern, (w->N + p.cols - 1) / p.cols, kInt8BlockThreads, p.smem, A, (const uint8_t *)w->bytes,
+             (const float *)w->scale, w->K, w->N, p.cols, p.wk, out, dev->d_err);
   return WGPT_OK;
 }
 
 template <int M>
-static int32_t launch_int8_block_t(wgpt_device *dev, const wgpt_int8_weight *w, const float *A, float *out) {
-  const int K = w->K, N = w->N, nw = kInt8BlockThreads / 32;
-  const int cols = (N + dev->sm_count - 1) / dev->sm_count;
-  // Columns per work item and K slices: the pair with the smallest sum of shared-memory cycles (a 128-bit load is four),
-  // issue cycles (four a cycle) and the busiest warp's own path. 1600 x 6400 has 44 columns per CTA: items of four columns
-  // left five of the sixteen warps without one, three columns leave one; with more rows the row loads decide, which the
-  // columns of an item share.
-  int cg = 1, wk = 1;
-  long long best = -1;
-  for (int c = 1; c <= (M <= 4 ? 4 : 3); c++)
-    for (int k = 1; k <= 8; k *= 2) {
-      const int groups = (cols + c - 1) / c, rounds = (groups * k + nw - 1) / nw, steps = ((K / 16 + k - 1) / k + 31) / 32;
-      const long long work = (long long)groups * k * steps, instr = c * (28 + 8 * M);
-      const long long cost = work * ((c + 4 * M) * 4 + instr / 4) + rounds * (steps * (instr + 60) + 20 * c * M + 60);
-      if (best < 0 || cost < best) { best = cost; cg = c; wk = k; }
-    }
-  const size_t red = (size_t)(cols * wk > nw ? cols * wk : nw) * M;
-  const size_t smem = (size_t)cols * K + ((size_t)M * K + ((red + 3) & ~size_t(3))) * 4 + 16;
-  if (smem > dev->smem_optin - 2048) return WGPT_ERR_UNSUPPORTED;  // caller falls back (no message: not an error)
-  switch (cg) {
-    case 1: return launch_int8_block_cg<M, 1>(dev, w, A, out, cols, wk, smem);
-    case 2: return launch_int8_block_cg<M, 2>(dev, w, A, out, cols, wk, smem);
-    case 3: return launch_int8_block_cg<M, 3>(dev, w, A, out, cols, wk, smem);
-    case 4: if constexpr (M <= 4) return launch_int8_block_cg<M, 4>(dev, w, A, out, cols, wk, smem); break;
+static int32_t launch_int8_block_t(wgpt_device *dev, const wgpt_int8_weight *w, const float *A, float *out,
+                                   const Int8BlockPlan &p) {
+  switch (p.cg) {
+    case 1: return launch_int8_block_cg<M, 1>(dev, w, A, out, p);
+    case 2: return launch_int8_block_cg<M, 2>(dev, w, A, out, p);
+    case 3: return launch_int8_block_cg<M, 3>(dev, w, A, out, p);
+    default:
+      if constexpr (M <= 4) return launch_int8_block_cg<M, 4>(dev, w, A, out, p);
+      return fail(WGPT_ERR_SHAPE, "int8 block plan of %d columns per item", p.cg);
   }
-  return WGPT_ERR_UNSUPPORTED;
 }
 
 WGPT_EXPORT int32_t wgpt_int8_matmul_w(wgpt_device *dev, int32_t M, const wgpt_int8_weight *w, const float *A,
@@ -1744,19 +1755,33 @@ WGPT_EXPORT int32_t wgpt_int8_matmul_w(wgpt_device *dev, int32_t M, const wgpt_i
   REQUIRE(M >= 1, WGPT_ERR_SHAPE, "empty int8 matmul");
   REQUIRE(aligned16(A) && aligned16(out), WGPT_ERR_ALIGN, "buffers must be 16-byte aligned");
   const int K = w->K, N = w->N;
-  if (w->bytes != nullptr && M <= 8) {
-    int32_t rc = WGPT_ERR_UNSUPPORTED;
-    switch (M) {
-      case 5: rc = launch_int8_block_t<5>(dev, w, A, out); break;
-      case 6: rc = launch_int8_block_t<6>(dev, w, A, out); break;
-      case 7: rc = launch_int8_block_t<7>(dev, w, A, out); break;
-      case 8: rc = launch_int8_block_t<8>(dev, w, A, out); break;
-      case 1: rc = launch_int8_block_t<1>(dev, w, A, out); break;
-      case 2: rc = launch_int8_block_t<2>(dev, w, A, out); break;
-      case 3: rc = launch_int8_block_t<3>(dev, w, A, out); break;
-      case 4: rc = launch_int8_block_t<4>(dev, w, A, out); break;
+  if (w->bytes != nullptr && M <= 16) {
+    // Rows in equal groups of at most eight, or of what fits shared memory beside the weight (five at K = 6400); the groups
+    // after the first find the weight in L2. Against the kernel on the packed words, 9 / 12 / 16 rows: 768 x 3072 6.8 / 8.1 /
+    // 9.1 us (9.9 / 11.6 / 12.9), 1600 x 6400 13.3 / 15.9 / 19.2 (17.5 / 20.4 / 24.2), 6400 x 1600 in two and three groups
+    // 16.9 / 20.3 (20.3 / 23.2); four groups there are no faster (16 rows 27.8 / 27.5), which sets the limit.
+    int most = M < 8 ? M : 8;
+    while (most > 0 && int8_block_plan(dev, K, N, most).smem == 0) most--;
+    if (most > 0 && (M + most - 1) / most <= kInt8BlockGroups) {
+      for (int m = 0, left = (M + most - 1) / most; left > 0; left--) {
+        const int rows = (M - m + left - 1) / left;
+        const float *a = A + (size_t)m * K;
+        float *o = out + (size_t)m * N;
+        const Int8BlockPlan p = int8_block_plan(dev, K, N, rows);
+        switch (rows) {
+          case 1: TRY(launch_int8_block_t<1>(dev, w, a, o, p)); break;
+          case 2: TRY(launch_int8_block_t<2>(dev, w, a, o, p)); break;
+          case 3: TRY(launch_int8_block_t<3>(dev, w, a, o, p)); break;
+          case 4: TRY(launch_int8_block_t<4>(dev, w, a, o, p)); break;
+          case 5: TRY(launch_int8_block_t<5>(dev, w, a, o, p)); break;
+          case 6: TRY(launch_int8_block_t<6>(dev, w, a, o, p)); break;
+          case 7: TRY(launch_int8_block_t<7>(dev, w, a, o, p)); break;
+          case 8: TRY(launch_int8_block_t<8>(dev, w, a, o, p)); break;
+        }
+        m += rows;
+      }
+      return WGPT_OK;
     }
-    if (rc != WGPT_ERR_UNSUPPORTED) return rc;
   }
   if (w->halves != nullptr && M > 16 && dev->precision != WGPT_PRECISION_FP32) {
     // Many rows: the codes are exact in half precision, the rows become pairs (pair.cuh), the scales are in the epilogue of

@@ -197,7 +197,7 @@ attn_block_kernel(AttnBlockParams p) {
   const int E = p.E, E4 = E >> 2;
   const int ncolA = E / CS, ncol4 = ncolA >> 2;
   float *wbuf = smem;                       // q/k/v weight rows, later the projection slice [HS][ncolA]
-  float *xs = wbuf + (size_t)NC * E;        // residual stream (filled by all CTAs of the cluster), then normalised
+  float *xs = wbuf + (size_t)NC * E;        // residual stream, then normalised
   float *hn = xs;                           // in place: every thread holds its elements in registers in between
   float *red = xs + E;
   float *qfull = red + p.red_floats;        // filled by all CTAs of the cluster
@@ -590,19 +590,18 @@ __host__ __device__ inline size_t mlp_block_smem_floats(int E, int units, int re
          ((units + 3) & ~3) + red_floats + 8;
 }
 
-// grid = kMlpCluster * clusters; CTA c owns hidden units [F*c/grid, F*(c+1)/grid). Inside a cluster each CTA sums
-// its share of the residual stream's columns and hands it to the others, and the cluster's partial results of the
-// down-projection are added (in rank order) by the CTA that owns the columns, so the next kernel reads one row per
-// cluster.
+// grid = kMlpCluster * clusters; CTA c owns hidden units [F*c/grid, F*(c+1)/grid). Every CTA sums
+// the whole residual stream for itself; the cluster's partial results of the down-projection are added (in rank order)
+// by the CTA that owns the columns, so the next kernel reads one row per cluster.
 __global__ void __launch_bounds__(kMlpBlockThreads)
 mlp_block_kernel(MlpBlockParams p) {
   constexpr int NT = kMlpBlockThreads, NW = NT / 32, CS = kMlpCluster;
   extern __shared__ __align__(128) float smem[];
   const int E = p.E, E4 = E >> 2, U = p.units;
-  const int nq4 = E4 / CS;                 // float4 columns of the residual stream this CTA sums and owns
+  const int nq4 = E4 / CS;                 // float4 columns of the down-projection this CTA adds up and stores
   float *wfc = smem;                       // [U][E]; re-used for the down-projection's slice sums
   float *wdn = wfc + (size_t)U * E;        // [U][E]
-  float *xs = wdn + (size_t)U * E;         // residual stream (filled by all CTAs of the cluster), then normalised
+  float *xs = wdn + (size_t)U * E;         // residual stream, then normalised
   float *xch = xs + E;                     // [CS][E/CS]: the cluster's partial results for this CTA's columns
   float *gs = xch + E;                     // GELU outputs of this CTA's units
   float *red = gs + ((U + 3) & ~3);
