@@ -1004,30 +1004,46 @@ static int kn_ksplit(const wgpt_device *dev, int M, int K, int col_groups, size_
 }
 
 template <int M>
-static int32_t launch_gemv_kn_t(wgpt_device *dev, const float *x, const float *W, int K, int N, int ksplit,
+static int32_t launch_gemv_kn_t(wgpt_device *dev, const float *x, const float *W, int rows, int K, int N, int ksplit,
                                 float *part) {
   int klen_max = ((K / 4 + ksplit - 1) / ksplit + 1) * 4;
   size_t smem = (size_t)M * klen_max * 4 + (size_t)8 * M * 32 * 16;
   auto kern = gemv_kn_partial_kernel<M>;
   CK(allow_smem(dev, kern));
-  dim3 grid((N + 127) / 128, ksplit);
-  LAUNCH(dev, kern, grid, 256, smem, x, W, K, N, part);
+  dim3 grid((N + 127) / 128, ksplit, (rows + M - 1) / M);
+  LAUNCH(dev, kern, grid, 256, smem, x, W, rows, K, N, part);
   return WGPT_OK;
 }
 
-// out = x[M,K] . W[K,N] (+ epilogue) for M <= 8, split-K with the partial sums in `part`
+// Rows of a reference-layout product below the tensor cores' 32, and how many of them a CTA takes: all of up to eight, above
+// that 12 or 16 in one or two groups (16 float4 sums are what a thread's registers hold). 9 to 31 rows used to run on the
+// 64 x 64 tiles of gemm_simt_kernel, 12 CTAs for 768 columns: the operators of a GPT-2 pass took 6.4 ms, now 1.3 to 1.5.
+constexpr int kKnMaxRows = 31;
+static int kn_rows(int M) {
+  if (M <= 8) return M;
+  const int groups = (M + 15) / 16;
+  return (M + groups - 1) / groups <= 12 ? 12 : 16;
+}
+static int kn_split(const wgpt_device *dev, int M, int K, int N) {
+  const int r = kn_rows(M);
+  return kn_ksplit(dev, r, K, (N + 127) / 128 * ((M + r - 1) / r));
+}
+
+// out = x[M,K] . W[K,N] (+ epilogue) for M <= kKnMaxRows, split-K with the partial sums in `part`
 // ([ksplit][M][N] floats, caller-provided).
 static int32_t gemv_kn_with_scratch(wgpt_device *dev, int M, const float *x, const float *W, int K, int N, int ksplit,
                                     float *part, const Epilogue &epi) {
-  switch (M) {
-    case 1: TRY(launch_gemv_kn_t<1>(dev, x, W, K, N, ksplit, part)); break;
-    case 2: TRY(launch_gemv_kn_t<2>(dev, x, W, K, N, ksplit, part)); break;
-    case 3: TRY(launch_gemv_kn_t<3>(dev, x, W, K, N, ksplit, part)); break;
-    case 4: TRY(launch_gemv_kn_t<4>(dev, x, W, K, N, ksplit, part)); break;
-    case 5: TRY(launch_gemv_kn_t<5>(dev, x, W, K, N, ksplit, part)); break;
-    case 6: TRY(launch_gemv_kn_t<6>(dev, x, W, K, N, ksplit, part)); break;
-    case 7: TRY(launch_gemv_kn_t<7>(dev, x, W, K, N, ksplit, part)); break;
-    case 8: TRY(launch_gemv_kn_t<8>(dev, x, W, K, N, ksplit, part)); break;
+  switch (kn_rows(M)) {
+    case 1: TRY(launch_gemv_kn_t<1>(dev, x, W, M, K, N, ksplit, part)); break;
+    case 2: TRY(launch_gemv_kn_t<2>(dev, x, W, M, K, N, ksplit, part)); break;
+    case 3: TRY(launch_gemv_kn_t<3>(dev, x, W, M, K, N, ksplit, part)); break;
+    case 4: TRY(launch_gemv_kn_t<4>(dev, x, W, M, K, N, ksplit, part)); break;
+    case 5: TRY(launch_gemv_kn_t<5>(dev, x, W, M, K, N, ksplit, part)); break;
+    case 6: TRY(launch_gemv_kn_t<6>(dev, x, W, M, K, N, ksplit, part)); break;
+    case 7: TRY(launch_gemv_kn_t<7>(dev, x, W, M, K, N, ksplit, part)); break;
+    case 8: TRY(launch_gemv_kn_t<8>(dev, x, W, M, K, N, ksplit, part)); break;
+    case 12: TRY(launch_gemv_kn_t<12>(dev, x, W, M, K, N, ksplit, part)); break;
+    case 16: TRY(launch_gemv_kn_t<16>(dev, x, W, M, K, N, ksplit, part)); break;
     default: return fail(WGPT_ERR_SHAPE, "gemv rows %d out of range", M);
   }
   int n4 = M * (N / 4);
@@ -1175,8 +1191,8 @@ struct Carve {
 
 // The reference-layout matmul used by the per-operator API: W is [K,N].
 static int32_t matmul_kn(wgpt_device *dev, int M, int K, int N, const float *in, const float *W, const Epilogue &epi) {
-  if (M <= 8) {
-    int ksplit = kn_ksplit(dev, M, K, (N + 127) / 128);
+  if (M <= kKnMaxRows) {
+    int ksplit = kn_split(dev, M, K, N);
     TRY(scratch_reserve(dev, (size_t)ksplit * M * N * 4));
     return gemv_kn_with_scratch(dev, M, in, W, K, N, ksplit, static_cast<float *>(dev->scratch), epi);
   }
@@ -1542,14 +1558,14 @@ WGPT_EXPORT int32_t wgpt_attention(wgpt_device *dev, int32_t T, int32_t E, float
     return attention_pair(dev, T, E, scale, H, hs, in, qW, qB, kW, kB, vW, vB, linW, linB, out);
   // workspace: q, k, v, o [T,E] + split-K partials
   size_t te = (size_t)T * E;
-  int ksplit = T <= 8 ? kn_ksplit(dev, T, E, (E + 127) / 128) : 0;
+  int ksplit = T <= kKnMaxRows ? kn_split(dev, T, E, E) : 0;
   const bool tc = dev->precision != WGPT_PRECISION_FP32 && T >= 32;
   size_t part_floats = tc ? (size_t)E * E : (size_t)ksplit * T * E;  // split-K partials, or a transposed weight
   TRY(scratch_reserve(dev, (4 * te + part_floats) * 4));
   float *q = static_cast<float *>(dev->scratch), *k = q + te, *v = k + te, *o = v + te, *part = o + te;
   auto mm = [&](const float *a, const float *W, const float *b, float *dst) -> int32_t {
     Epilogue e = plain_epi(dst, E, b);
-    if (T <= 8) return gemv_kn_with_scratch(dev, T, a, W, E, E, ksplit, part, e);
+    if (T <= kKnMaxRows) return gemv_kn_with_scratch(dev, T, a, W, E, E, ksplit, part, e);
     if (tc) return gemm_kn_via_transpose(dev, a, (size_t)E, W, T, E, E, e, part);
     return launch_gemm_simt(dev, false, a, (size_t)E, W, T, E, E, e);
   };

@@ -792,10 +792,13 @@ gemv_block_kernel(const float *__restrict__ x, size_t ldx, const float *__restri
 // ------------------------------------------------------------------------------------------------
 // Weight in the reference layout W[K,N]. Thread owns 4 consecutive columns; a warp covers 128 columns of one
 // k row per load (512 contiguous bytes); the CTA's 8 warps and gridDim.y CTAs split K.
-// part receives [gridDim.y][M][N] partial sums (scratch); gemv_kn_reduce_kernel adds them in order.
+// part receives [gridDim.y][rows][N] partial sums (scratch); gemv_kn_reduce_kernel adds them in order.
+// blockIdx.z takes M of the `rows` rows; the last group's missing ones are staged as zeros and not stored. With 12 and 16 rows
+// a weight element meets enough of them that the multiply-adds (4 M per warp and 128-bit load, against M broadcast loads
+// from shared memory) and not HBM decide: 768 x 3072 takes ~1 us of them on 148 SMs, under the launch and the second stage.
 template <int M>
 __global__ void __launch_bounds__(256)
-gemv_kn_partial_kernel(const float *__restrict__ x, const float *__restrict__ W, int K, int N,
+gemv_kn_partial_kernel(const float *__restrict__ x, const float *__restrict__ W, int rows, int K, int N,
                        float *__restrict__ part) {
   extern __shared__ __align__(128) float smem[];  // xs[M][kslice] + red[8][M][128]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -805,9 +808,10 @@ gemv_kn_partial_kernel(const float *__restrict__ x, const float *__restrict__ W,
   const int klen = kend - kbeg;
   float *xs = smem;
   float4 *red = reinterpret_cast<float4 *>(smem + (size_t)M * ((klen + 3) & ~3));
+  const int m0 = blockIdx.z * M, live = min(M, rows - m0);
   for (int i = tid; i < M * klen; i += 256) {
     int m = i / klen, k = i - m * klen;
-    xs[m * klen + k] = x[(size_t)m * K + kbeg + k];
+    xs[m * klen + k] = m < live ? x[(size_t)(m0 + m) * K + kbeg + k] : 0.f;
   }
   __syncthreads();
   const int n = blockIdx.x * 128 + lane * 4;
@@ -832,14 +836,14 @@ gemv_kn_partial_kernel(const float *__restrict__ x, const float *__restrict__ W,
   for (int i = tid; i < M * 32; i += 256) {
     int m = i / 32, l = i % 32;
     int nn = blockIdx.x * 128 + l * 4;
-    if (nn >= N) continue;
+    if (nn >= N || m >= live) continue;
     float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int w = 0; w < 8; w++) {
       float4 v = red[(w * M + m) * 32 + l];
       s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
     }
-    *reinterpret_cast<float4 *>(part + ((size_t)blockIdx.y * M + m) * N + nn) = s;
+    *reinterpret_cast<float4 *>(part + ((size_t)blockIdx.y * rows + m0 + m) * N + nn) = s;
   }
 }
 
