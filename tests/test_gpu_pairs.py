@@ -58,8 +58,24 @@ def test_product_of_pairs_error_bound(dev, M, K, N):
     assert np.array_equal(scaled, (got * r[:, None] * c[None, :]).astype(np.float32))
 
 
-@pytest.mark.parametrize("M,K,N", [(40, 96, 264), (300, 776, 200)])
-def test_product_of_pairs_integers_are_exact(dev, M, K, N):
+@pytest.mark.parametrize("M,K,N", [(9, 768, 136), (12, 3072, 768), (13, 72, 40), (16, 40, 2304), (17, 1600, 128), (24, 8, 8),
+                                   (25, 768, 768), (31, 3080, 72)])
+def test_product_of_9_to_31_rows_is_fp32(dev, M, K, N):
+    """One or two row groups of 12 or 16, the last one ragged, K slices of uneven length. FP32 sums: at most one rounding of
+    2^-24 per term and per addition of a partial sum."""
+    rng = np.random.default_rng(M + K + N)
+    A = rng.standard_normal((M, K), dtype=np.float32)
+    W = rng.standard_normal((K, N), dtype=np.float32)
+    b = rng.standard_normal(N, dtype=np.float32)
+    ref = A.astype(np.float64) @ W.astype(np.float64) + b
+    bound = (K + 20) * 2.0 ** -24 * (np.abs(A).astype(np.float64) @ np.abs(W).astype(np.float64) + np.abs(b))
+    got = matmul(dev, A, W, b)
+    assert (np.abs(got - ref) <= bound).all()
+    assert rel_err(got, ref) < 4e-6  # and not a product of split operands: sqrt(K / 3) 2^-24 of a sum, four times over
+
+
+@pytest.mark.parametrize("M,K,N", [(9, 64, 72), (31, 96, 264), (40, 96, 264), (300, 776, 200)])
+def test_products_of_integers_are_exact(dev, M, K, N):
     """Integers of at most 11 bits are exact in the first plane and their sums in FP32: any misplaced element shows."""
     A = ((np.arange(M)[:, None] * 7 + np.arange(K)[None, :] * 3) % 11 - 5).astype(np.float32)
     W = ((np.arange(K)[:, None] * 5 + np.arange(N)[None, :]) % 13 - 6).astype(np.float32)
@@ -123,7 +139,7 @@ def test_decode_rows(model64, n_seq):
         assert rel_err(lg[i], m.run(np.concatenate([prompts[i], got[i, :1]]))) < 2e-5
 
 
-@pytest.mark.parametrize("n_seq", [1, 2, 3, 5, 8])
+@pytest.mark.parametrize("n_seq", [1, 2, 3, 5, 7, 8])
 def test_ring_gemv_rows(oracle, n_seq):
     """Layers that do not fit shared memory (n_embd 1600): FP32 through the ring for up to five sequences, and for eight
     in FP32 mode; K = 1600 is no multiple of a stage's 256.
@@ -147,6 +163,12 @@ def test_ring_gemv_rows(oracle, n_seq):
             lg = s.forward(prompts[:, t:t + 1])
         for i in (0, n_seq - 1):
             assert rel_err(lg[i], m.run(prompts[i])) < 8e-6
+        # the same rows as a prompt of n_seq tokens, in two passes (from six rows on these are products of pairs)
+        s1 = gpt.session(1)
+        s1.reset()  # the session of one sequence is the one above when n_seq is 1
+        s1.forward(prompts[0], want_logits=False)
+        ids = np.concatenate([prompts[0], synth.make_tokens(512, n_seq, seed=6)])
+        assert rel_err(s1.forward(ids[5:])[0], m.run(ids)) < 8e-6
     finally:
         gpt.destroy()
 

@@ -2581,25 +2581,27 @@ static int32_t forward_blocks_split(wgpt_session *s, int n_tok) {
   return WGPT_OK;
 }
 
-// The transformer blocks of a decode step of a few sequences as five FP32 kernels per block (gemv_ring.cuh), for models
+// Every layer product of M rows fits the shared-memory block GEMV (gemv_block_kernel).
+static bool layers_fit_block_form(const wgpt_device *dev, int M, int E) {
+  int c, w;
+  size_t b;
+  return dev->block_gemv && gemv_block_plan(dev, M, E, 3 * E, true, &c, &w, &b) &&
+         gemv_block_plan(dev, M, E, 4 * E, true, &c, &w, &b) && gemv_block_plan(dev, M, 4 * E, E, false, &c, &w, &b);
+}
+
+// The transformer blocks of a pass of a few rows as five FP32 kernels per block (gemv_ring.cuh), for models
 // whose weights do not fit the block form (every product does in GPT-2 117M, and the block form then is faster: 0.318
 // against 0.367 ms per pass at two sequences; XL at one / two / four 1.93 / 2.15 / 2.50 ms against 2.71 / 3.52 / 5.14 in the
-// register-streaming kernels). False in *done: nothing has been launched.
-static int32_t forward_blocks_ring(wgpt_session *s, bool *done) {
+// register-streaming kernels; a prompt of three tokens 4.06 -> 2.52). False in *done: nothing has been launched.
+static int32_t forward_blocks_ring(wgpt_session *s, int n_tok, bool *done) {
   wgpt_model *m = s->m;
   wgpt_device *dev = m->dev;
   const wgpt_params &p = m->p;
-  const int E = p.n_embd, F = 4 * E, H = p.n_head, hs = m->hs, M = s->n_seq;
+  const int E = p.n_embd, F = 4 * E, H = p.n_head, hs = m->hs, M = s->n_seq * n_tok;
   const size_t kv_layer = (size_t)s->n_seq * p.n_ctx * E;
   RingPlan pq, po, pf, pp;
   *done = false;
-  if (dev->block_gemv) {
-    int c, w;
-    size_t b;
-    if (gemv_block_plan(dev, M, E, 3 * E, true, &c, &w, &b) && gemv_block_plan(dev, M, E, F, true, &c, &w, &b) &&
-        gemv_block_plan(dev, M, F, E, false, &c, &w, &b))
-      return WGPT_OK;
-  }
+  if (layers_fit_block_form(dev, M, E)) return WGPT_OK;
   *done = gemv_ring_plan(dev, M, E, 3 * E, true, &pq) && gemv_ring_plan(dev, M, E, E, false, &po) &&
           gemv_ring_plan(dev, M, E, F, true, &pf) && gemv_ring_plan(dev, M, F, E, false, &pp);
   if (!*done) return WGPT_OK;
@@ -2607,10 +2609,13 @@ static int32_t forward_blocks_ring(wgpt_session *s, bool *done) {
     const LayerWeights &L = m->layers[l];
     float *kc = s->kc + (size_t)l * kv_layer, *vc = s->vc + (size_t)l * kv_layer;
     Epilogue e = plain_epi(s->q, E, L.bqkv);
-    e.kc = kc; e.vc = vc; e.E = E; e.n_tok = 1; e.n_ctx = p.n_ctx; e.pos = s->d_pos;
+    e.kc = kc; e.vc = vc; e.E = E; e.n_tok = n_tok; e.n_ctx = p.n_ctx; e.pos = s->d_pos;
     TRY(launch_gemv_ring(dev, pq, M, s->x, L.ln1_g, L.ln1_b, L.wqkv_t, E, 3 * E, e));
-    TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, M, H, s->n_split, s->d_pos, m->scale,
-                           nullptr));
+    if (n_tok == 1)
+      TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, M, H, s->n_split, s->d_pos, m->scale,
+                             nullptr));
+    else
+      TRY(launch_attn_prefill(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, s->o, E, n_tok, s->n_seq, H, s->d_pos, m->scale));
     e = plain_epi(s->x, E, L.bo);
     e.residual = s->x;
     TRY(launch_gemv_ring(dev, po, M, s->o, nullptr, nullptr, L.wo_t, E, E, e));
@@ -2637,8 +2642,9 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
   // From six sequences on, where the de-embedding leaves the FP32 kernels too (logits of a decode step against double
   // precision, 2-norm: GPT-2 2.9e-6, XL 6.0e-6; five sequences in FP32 4e-7, and eight with FP32 blocks and the 3xTF32
   // de-embedding 6.3e-6 and 1.45e-5). Decode pass of eight sequences 0.369 ms (FP32 blocks 0.489), XL 2.21 (5.08).
-  // Prompts: from nine rows on (up to eight stay in FP32).
-  const bool split = pair_mode && M <= 64 && (n_tok == 1 ? M >= kSplitMinRows : M > 8);
+  // Prompts: from nine rows on; up to eight stay in FP32 where the products fit the block form, as they always have.
+  const bool split = pair_mode && M <= 64 &&
+                     (n_tok == 1 ? M >= kSplitMinRows : M > 8 || (M >= kSplitMinRows && !layers_fit_block_form(dev, M, E)));
   if (!fused)
     LAUNCH_PDL(dev, embed_kernel, M, 128, 0, ids, m->wte, m->wpe, s->x, M, n_tok, E, p.vocab_size,
                (const int *)s->d_pos, dev->d_err, split ? s->stats : nullptr);
@@ -2681,7 +2687,7 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
   if (pair) TRY(forward_blocks_pair(s, n_tok));
   if (split) TRY(forward_blocks_split(s, n_tok));
   bool ring = false;
-  if (!fused && !pair && !split && n_tok == 1 && M <= 8) TRY(forward_blocks_ring(s, &ring));
+  if (!fused && !pair && !split && M <= 8) TRY(forward_blocks_ring(s, n_tok, &ring));
   for (int l = 0; l < (fused || pair || split || ring ? 0 : p.n_layer); l++) {
     const LayerWeights &L = m->layers[l];
     float *kc = s->kc + (size_t)l * kv_layer, *vc = s->vc + (size_t)l * kv_layer;
