@@ -876,7 +876,8 @@ static int32_t launch_gemm_tc(wgpt_device *dev, bool x3, const float *A, size_t 
       ln->done = true;
     } else {
       int n4 = M * (N / 4);
-      LAUNCH_PDL(dev, gemv_kn_reduce_kernel, (n4 + 255) / 256, 256, 0, (const float *)split_out, splits, M, N, epi, tw);
+      LAUNCH_PDL(dev, gemv_kn_reduce_kernel, (n4 + 255) / 256, 256, 0, (const float *)split_out, splits, M, N, epi, tw,
+                 KnWeights{});
     }
   }
   return WGPT_OK;
@@ -1004,20 +1005,20 @@ static int kn_ksplit(const wgpt_device *dev, int M, int K, int col_groups, size_
 }
 
 template <int M>
-static int32_t launch_gemv_kn_t(wgpt_device *dev, const float *x, const float *W, int rows, int K, int N, int ksplit,
+static int32_t launch_gemv_kn_t(wgpt_device *dev, const float *x, const KnWeights &W, int rows, int K, int N, int ksplit,
                                 float *part) {
   int klen_max = ((K / 4 + ksplit - 1) / ksplit + 1) * 4;
   size_t smem = (size_t)M * klen_max * 4 + (size_t)8 * M * 32 * 16;
   auto kern = gemv_kn_partial_kernel<M>;
   CK(allow_smem(dev, kern));
   dim3 grid((N + 127) / 128, ksplit, (rows + M - 1) / M);
-  LAUNCH(dev, kern, grid, 256, smem, x, W, rows, K, N, part);
+  LAUNCH_PDL(dev, kern, grid, 256, smem, x, W, rows, K, N, part);
   return WGPT_OK;
 }
 
 // Rows of a reference-layout product below the tensor cores' 32, and how many of them a CTA takes: all of up to eight, above
 // that 12 or 16 in one or two groups (16 float4 sums are what a thread's registers hold). 9 to 31 rows used to run on the
-// 64 x 64 tiles of gemm_simt_kernel, 12 CTAs for 768 columns: the operators of a GPT-2 pass took 6.4 ms, now 1.3 to 1.5.
+// 64 x 64 tiles of gemm_simt_kernel, 12 CTAs for 768 columns: the operators of a GPT-2 pass took 6.4 ms, now 1.1 to 1.2.
 constexpr int kKnMaxRows = 31;
 static int kn_rows(int M) {
   if (M <= 8) return M;
@@ -1030,9 +1031,9 @@ static int kn_split(const wgpt_device *dev, int M, int K, int N) {
 }
 
 // out = x[M,K] . W[K,N] (+ epilogue) for M <= kKnMaxRows, split-K with the partial sums in `part`
-// ([ksplit][M][N] floats, caller-provided).
-static int32_t gemv_kn_with_scratch(wgpt_device *dev, int M, const float *x, const float *W, int K, int N, int ksplit,
-                                    float *part, const Epilogue &epi) {
+// ([ksplit][M][N] floats, caller-provided). W may be several weights side by side, with their own biases.
+static int32_t gemv_kn_with_scratch(wgpt_device *dev, int M, const float *x, const KnWeights &W, int K, int N, int ksplit,
+                                    float *part, const Epilogue &epi, const KnWeights &bias = KnWeights{}) {
   switch (kn_rows(M)) {
     case 1: TRY(launch_gemv_kn_t<1>(dev, x, W, M, K, N, ksplit, part)); break;
     case 2: TRY(launch_gemv_kn_t<2>(dev, x, W, M, K, N, ksplit, part)); break;
@@ -1047,7 +1048,7 @@ static int32_t gemv_kn_with_scratch(wgpt_device *dev, int M, const float *x, con
     default: return fail(WGPT_ERR_SHAPE, "gemv rows %d out of range", M);
   }
   int n4 = M * (N / 4);
-  LAUNCH_PDL(dev, gemv_kn_reduce_kernel, (n4 + 255) / 256, 256, 0, part, ksplit, M, N, epi, N);
+  LAUNCH_PDL(dev, gemv_kn_reduce_kernel, (n4 + 255) / 256, 256, 0, part, ksplit, M, N, epi, N, bias);
   return WGPT_OK;
 }
 
@@ -1194,7 +1195,7 @@ static int32_t matmul_kn(wgpt_device *dev, int M, int K, int N, const float *in,
   if (M <= kKnMaxRows) {
     int ksplit = kn_split(dev, M, K, N);
     TRY(scratch_reserve(dev, (size_t)ksplit * M * N * 4));
-    return gemv_kn_with_scratch(dev, M, in, W, K, N, ksplit, static_cast<float *>(dev->scratch), epi);
+    return gemv_kn_with_scratch(dev, M, in, KnWeights{{W}, N}, K, N, ksplit, static_cast<float *>(dev->scratch), epi);
   }
   if (dev->precision == WGPT_PRECISION_TF32X3 && M >= 32 && pair_operands_fit(K)) {
     // Both operands to half-precision pairs in one pass, then the product; 128 x 768 x 768: 11 us against 21 us for
@@ -1556,16 +1557,26 @@ WGPT_EXPORT int32_t wgpt_attention(wgpt_device *dev, int32_t T, int32_t E, float
           WGPT_ERR_ALIGN, "buffers must be 16-byte aligned");
   if (dev->precision == WGPT_PRECISION_TF32X3 && T >= 32 && pair_operands_fit(E) && E % 32 == 0)
     return attention_pair(dev, T, E, scale, H, hs, in, qW, qB, kW, kB, vW, vB, linW, linB, out);
-  // workspace: q, k, v, o [T,E] + split-K partials
+  if (T <= kKnMaxRows) {
+    // Workspace: q | k | v rows [T,3E], o [T,E], split-K partial sums. The three projections are one product.
+    // (The operators of a GPT-2 pass of 8 / 16 tokens: 1.22 / 1.40 -> 0.94 / 1.10 ms, with the first stage launched
+    // ahead of its predecessor's end.)
+    const int ks3 = kn_split(dev, T, E, 3 * E), ks1 = kn_split(dev, T, E, E);
+    const size_t te = (size_t)T * E, part_floats = te * (3 * ks3 > ks1 ? 3 * ks3 : ks1);
+    TRY(scratch_reserve(dev, (4 * te + part_floats) * 4));
+    float *qkv = static_cast<float *>(dev->scratch), *o = qkv + 3 * te, *part = o + te;
+    TRY(gemv_kn_with_scratch(dev, T, in, KnWeights{{qW, kW, vW}, E}, E, 3 * E, ks3, part, plain_epi(qkv, 3 * E, nullptr),
+                             KnWeights{{qB, kB, vB}, E}));
+    TRY(launch_attn_prefill(dev, hs, qkv, 3 * E, qkv + E, qkv + 2 * E, 3 * E, 0, o, E, T, 1, H, nullptr, scale));
+    return gemv_kn_with_scratch(dev, T, o, KnWeights{{linW}, E}, E, E, ks1, part, plain_epi(out, E, linB));
+  }
+  // workspace: q, k, v, o [T,E] + a transposed weight
   size_t te = (size_t)T * E;
-  int ksplit = T <= kKnMaxRows ? kn_split(dev, T, E, E) : 0;
-  const bool tc = dev->precision != WGPT_PRECISION_FP32 && T >= 32;
-  size_t part_floats = tc ? (size_t)E * E : (size_t)ksplit * T * E;  // split-K partials, or a transposed weight
-  TRY(scratch_reserve(dev, (4 * te + part_floats) * 4));
+  const bool tc = dev->precision != WGPT_PRECISION_FP32;
+  TRY(scratch_reserve(dev, (4 * te + (tc ? (size_t)E * E : 0)) * 4));
   float *q = static_cast<float *>(dev->scratch), *k = q + te, *v = k + te, *o = v + te, *part = o + te;
   auto mm = [&](const float *a, const float *W, const float *b, float *dst) -> int32_t {
     Epilogue e = plain_epi(dst, E, b);
-    if (T <= kKnMaxRows) return gemv_kn_with_scratch(dev, T, a, W, E, E, ksplit, part, e);
     if (tc) return gemm_kn_via_transpose(dev, a, (size_t)E, W, T, E, E, e, part);
     return launch_gemm_simt(dev, false, a, (size_t)E, W, T, E, E, e);
   };
@@ -1649,7 +1660,7 @@ WGPT_EXPORT int32_t wgpt_int8_matmul(wgpt_device *dev, int32_t M, int32_t K, int
 #undef CASE_W
 #undef CASE_N
   int n4 = M * (N / 4);
-  LAUNCH_PDL(dev, gemv_kn_reduce_kernel, (n4 + 255) / 256, 256, 0, part, ksplit, M, N, e, N);
+  LAUNCH_PDL(dev, gemv_kn_reduce_kernel, (n4 + 255) / 256, 256, 0, part, ksplit, M, N, e, N, KnWeights{});
   return WGPT_OK;
 }
 
@@ -3177,7 +3188,7 @@ WGPT_EXPORT int32_t wgpt_matmul_static(wgpt_device *dev, int32_t rows, int32_t c
   TRY(static_scratch_for(dev, &part));
   // Every element of the [ksplit][rows][cols] partial block is written by the first kernel before the second
   // reads it, so nothing left over from an earlier call is ever read and nothing needs clearing.
-  return gemv_kn_with_scratch(dev, rows, in, W, shared, cols, ksplit, part, plain_epi(out, cols, bias));
+  return gemv_kn_with_scratch(dev, rows, in, KnWeights{{W}, cols}, shared, cols, ksplit, part, plain_epi(out, cols, bias));
 }
 
 #ifdef WGPT_TRACE

@@ -796,10 +796,16 @@ gemv_block_kernel(const float *__restrict__ x, size_t ldx, const float *__restri
 // blockIdx.z takes M of the `rows` rows; the last group's missing ones are staged as zeros and not stored. With 12 and 16 rows
 // a weight element meets enough of them that the multiply-adds (4 M per warp and 128-bit load, against M broadcast loads
 // from shared memory) and not HBM decide: 768 x 3072 takes ~1 us of them on 148 SMs, under the launch and the second stage.
+// Up to three weights of the same shape [K, wn] stand side by side (N = 3 wn: an attention's q, k and v in one launch).
+// The dependents are released after the wait, not ahead of it: the second stage reads its biases before it waits, and a
+// caller's kernel in front of this one may have written them.
+struct KnWeights {
+  const float *w[3];
+  int wn;  // columns of each
+};
 template <int M>
 __global__ void __launch_bounds__(256)
-gemv_kn_partial_kernel(const float *__restrict__ x, const float *__restrict__ W, int rows, int K, int N,
-                       float *__restrict__ part) {
+gemv_kn_partial_kernel(const float *__restrict__ x, KnWeights W, int rows, int K, int N, float *__restrict__ part) {
   extern __shared__ __align__(128) float smem[];  // xs[M][kslice] + red[8][M][128]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ksplit = gridDim.y;
@@ -809,9 +815,11 @@ gemv_kn_partial_kernel(const float *__restrict__ x, const float *__restrict__ W,
   float *xs = smem;
   float4 *red = reinterpret_cast<float4 *>(smem + (size_t)M * ((klen + 3) & ~3));
   const int m0 = blockIdx.z * M, live = min(M, rows - m0);
+  pdl_wait();
+  pdl_launch_dependents();
   for (int i = tid; i < M * klen; i += 256) {
     int m = i / klen, k = i - m * klen;
-    xs[m * klen + k] = m < live ? x[(size_t)(m0 + m) * K + kbeg + k] : 0.f;
+    xs[m * klen + k] = m < live ? __ldcg(x + (size_t)(m0 + m) * K + kbeg + k) : 0.f;
   }
   __syncthreads();
   const int n = blockIdx.x * 128 + lane * 4;
@@ -819,10 +827,11 @@ gemv_kn_partial_kernel(const float *__restrict__ x, const float *__restrict__ W,
 #pragma unroll
   for (int m = 0; m < M; m++) acc[m] = make_float4(0.f, 0.f, 0.f, 0.f);
   if (n < N) {
-    const float *wp = W + (size_t)kbeg * N + n;
+    const int seg = n / W.wn;  // columns come in fours and wn is a multiple of four
+    const float *wp = (seg == 0 ? W.w[0] : seg == 1 ? W.w[1] : W.w[2]) + (size_t)kbeg * W.wn + (n - seg * W.wn);
 #pragma unroll 8
     for (int k = warp; k < klen; k += 8) {
-      float4 w = ldg_stream4(reinterpret_cast<const float4 *>(wp + (size_t)k * N));
+      float4 w = ldg_stream4(reinterpret_cast<const float4 *>(wp + (size_t)k * W.wn));
 #pragma unroll
       for (int m = 0; m < M; m++) {
         float a = xs[m * klen + k];
@@ -848,7 +857,9 @@ gemv_kn_partial_kernel(const float *__restrict__ x, const float *__restrict__ W,
 }
 
 // part: [ksplit][N / tw column tiles][M][tw] (tw = N: plain [ksplit][M][N]); tw % 4 == 0.
-__global__ void gemv_kn_reduce_kernel(const float *__restrict__ part, int ksplit, int M, int N, Epilogue epi, int tw) {
+// bias.wn != 0: the columns' biases, wn at a time, in place of epi.bias.
+__global__ void gemv_kn_reduce_kernel(const float *__restrict__ part, int ksplit, int M, int N, Epilogue epi, int tw,
+                                      KnWeights bias) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;  // float4 index over [M, N/4]
   int N4 = N >> 2;
   TRACE_BEGIN(6);
@@ -857,6 +868,11 @@ __global__ void gemv_kn_reduce_kernel(const float *__restrict__ part, int ksplit
   const int m = live ? i / N4 : 0, n = live ? (i - m * N4) * 4 : 0;
   float4 bias_pre = make_float4(0.f, 0.f, 0.f, 0.f), res_pre = bias_pre;
   if (live && epi.bias) bias_pre = *reinterpret_cast<const float4 *>(epi.bias + n);  // a weight: ahead of the wait
+  if (live && bias.wn) {
+    const int seg = n / bias.wn;
+    const float *b = seg == 0 ? bias.w[0] : seg == 1 ? bias.w[1] : bias.w[2];
+    if (b) bias_pre = *reinterpret_cast<const float4 *>(b + (n - seg * bias.wn));
+  }
   pdl_launch_dependents();
   pdl_wait();  // the partial sums come from the previous kernel
   trace(6, 1);
