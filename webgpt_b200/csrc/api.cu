@@ -1255,18 +1255,19 @@ static int32_t launch_attn_prefill_pair(wgpt_device *dev, const float *q, int ld
                                         int ldkv, size_t kv_seq_stride, int n_tok, int n_seq, int H, const int *pos,
                                         float scale, float s_qk, float s_v, __half *planes, size_t plane, int ldo,
                                         const AttnScaleSrc &src = AttnScaleSrc()) {
-  // Two groups of warps per 64 query rows, alternating key tiles, up to 2.5 CTAs per SM (GPT-2 at 333 / 1024 tokens 0.85 /
-  // 1.64 ms per pass against 1.00 / 1.95 with one group and 0.94 / 1.79 with 128 query rows per CTA; GPT-2 XL at 1024, 400
-  // CTAs: no difference); one group beyond that (64 x 128 tokens, 1536 CTAs: 4.46 against 4.8 ms) and for a single tile.
+  // Two groups of warps per 64 query rows, alternating key tiles, while all CTAs are resident at once, up to three per SM
+  // (GPT-2 at 333 / 1024 tokens 0.85 / 1.64 ms per pass against 1.00 / 1.95 with one group; with the CTAs' order balanced over
+  // the SMs 1024 tokens take 1.55, XL 12.15 against 12.5, and XL with one group 12.8); one group beyond that (64 x 128 tokens,
+  // 1536 CTAs: 4.46 against 4.8 ms) and for a single tile.
   const long long ctas = (long long)((n_tok + 63) / 64) * H * n_seq;
 #define PAIR_ATTN(W, G)                                                                                                  \
   do {                                                                                                                   \
     CK(allow_smem(dev, attn_prefill64_pair_kernel<W, G>));                                                               \
-    LAUNCH_PDL(dev, (attn_prefill64_pair_kernel<W, G>), dim3((n_tok + 16 * W - 1) / (16 * W), H, n_seq), 32 * W * G,     \
+    LAUNCH_PDL(dev, (attn_prefill64_pair_kernel<W, G>), (n_tok + 16 * W - 1) / (16 * W) * H * n_seq, 32 * W * G,          \
                attn_pair_smem_bytes(G), q, ldq, kc, vc, ldkv, kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes, plane, \
-               ldo, src);                                                                                                \
+               ldo, src, H, dev->sm_count);                                                                              \
   } while (0)
-  if (n_tok > 64 && 2 * ctas <= 5 * dev->sm_count) PAIR_ATTN(4, 2);
+  if (n_tok > 64 && ctas <= 3 * dev->sm_count) PAIR_ATTN(4, 2);
   else PAIR_ATTN(4, 1);
 #undef PAIR_ATTN
   return WGPT_OK;
