@@ -197,6 +197,27 @@ def test_int8_handle_rows(dev, oracle, K, N):
         _lib.call("wgpt_int8_weight_destroy", h)
 
 
+@pytest.mark.parametrize("M,K,N", [(323, 16, 8), (129, 16, 6400), (206, 336, 768), (323, 208, 768), (1024, 464, 256)])
+def test_int8_handle_one_k_block_per_slice(dev, M, K, N):
+    """Row tiles of more than 64 rows with one k-block per CTA of the cluster: the FP32 partial tile is larger than the one
+    stage it lies over. Bound as in test_int8_handle_rows."""
+    from webgpt_b200 import _lib
+    h = C.c_void_p()
+    A, q, packed, scale = synth.make_int8_case(M, K, N)
+    p_d, s_d, a_d, o_d = dev.tensor(packed), dev.tensor(scale), dev.tensor(A), dev.buffer(M * N * 4)
+    _lib.call("wgpt_int8_weight_create", dev.handle, K, N, p_d.ptr, s_d.ptr, C.byref(h))
+    try:
+        _lib.call("wgpt_int8_matmul_w", dev.handle, M, h, a_d.ptr, o_d.ptr)
+        _lib.call("wgpt_device_check", dev.handle)
+        got = o_d.read(np.float32, M * N).reshape(M, N)
+    finally:
+        _lib.call("wgpt_int8_weight_destroy", h)
+    Wf = q.astype(np.float64) * scale.astype(np.float64)
+    ref, mag = A.astype(np.float64) @ Wf, np.abs(A).astype(np.float64) @ np.abs(Wf)
+    bound = (2.0 ** -22 + (2 * K / 16 + 4) * 2.0 ** -23) * mag + 2.0 ** -39 * np.abs(A).max() * np.abs(Wf).max() * K
+    assert (np.abs(got - ref) <= bound).all()
+
+
 @pytest.mark.parametrize("V", [48, 4096, 4097, 50257, 65536, 65540])
 def test_sampling_kernel_edges(dev, oracle, V):
     """One CTA or a cluster, the largest vocabulary its registers hold and the one beyond, top_k at its limit and beyond;

@@ -1061,51 +1061,7 @@ static int32_t gemm_kn_via_transpose(wgpt_device *dev, const float *A, size_t ld
   return launch_gemm_tc(dev, dev->precision == WGPT_PRECISION_TF32X3, A, lda, wt, M, K, N, epi, nullptr, false);
 }
 
-// Launch shape of gemm_split_kernel.
-struct SplitShape {
-  int row_tiles, rn, S, stages;
-};
-// One row tile of RN rows (kNorm / decode): the smallest number of K slices with the shortest longest slice, among those
-// whose clusters are all resident at once with one CTA per SM (a second round would double the product's time).
-static SplitShape split_shape_decode(const wgpt_device *dev, int M, int K, int N) {
-  SplitShape sh;
-  sh.row_tiles = 1;
-  sh.rn = (M + 15) & ~15;
-  const int ft = (N + 127) / 128, kb = (K + GP_BK - 1) / GP_BK;
-  sh.S = 1;
-  for (int S = 2; S <= 8 && S <= kb; S++)
-    if (ft <= dev->max_clusters[S] && (kb + S - 1) / S < (kb + sh.S - 1) / sh.S) sh.S = S;
-  const int stage_bytes = GS_W_BYTES + sh.rn * (GP_BK * 4);
-  const int need = (kb + sh.S - 1) / sh.S, room = (int)((size_t(200) << 10) / stage_bytes);
-  sh.stages = need < room ? need : room;
-  if (sh.stages > GS_MAX_STAGES) sh.stages = GS_MAX_STAGES;
-  return sh;
-}
-
-// Any number of rows, activations as planes: row tiles of up to 128 and K slices by the same kind of estimate
-// (pair_tile_columns): a k-block costs max(6 RN tensor-core cycles, 32 KB + 256 RN bytes from L2 at 40 a cycle), a round
-// 9000 cycles of start, exchange and store and 60 more per row of the tile.
-static SplitShape split_shape_rows(const wgpt_device *dev, int M, int K, int N, double *cycles) {
-  SplitShape best = {};
-  const int ft = (N + 127) / 128, kb = (K + GP_BK - 1) / GP_BK, rt0 = (M + 127) / 128;
-  *cycles = 1e30;
-  for (int rt = rt0; rt <= rt0 + 2; rt++) {
-    const int rn = (((M + rt - 1) / rt) + 15) & ~15;
-    for (int S = 1; S <= 8 && S <= kb; S++) {
-      if (dev->max_clusters[S] < 1) continue;
-      const int rounds = (ft * rt + dev->max_clusters[S] - 1) / dev->max_clusters[S];
-      const double c = rounds * (((kb + S - 1) / S) * fmax(6.0 * rn, 820 + 6.4 * rn) + 9000 + 60.0 * rn);
-      if (c < *cycles) {
-        *cycles = c;
-        best.row_tiles = (M + rn - 1) / rn; best.rn = rn; best.S = S;
-        const int need = (kb + S - 1) / S, room = (int)((size_t(200) << 10) / (GS_W_BYTES + rn * (GP_BK * 4)));
-        best.stages = need < room ? need : room;
-        if (best.stages > GS_MAX_STAGES) best.stages = GS_MAX_STAGES;
-      }
-    }
-  }
-  return best;
-}
+static SplitLimits split_limits(const wgpt_device *dev) { return SplitLimits{dev->max_clusters}; }
 
 // X: pair planes [2][M][K], or nullptr with the LayerNorm input described in a (kNorm, M <= 64).
 static int32_t launch_gemm_split(wgpt_device *dev, const SplitShape &sh, const __half *X, const __half *W, int M, int K,
@@ -1115,18 +1071,18 @@ static int32_t launch_gemm_split(wgpt_device *dev, const SplitShape &sh, const _
   a.epi = epi;
   a.err = dev->d_err;
   if (a.w_planes == 0) a.w_planes = 2;
+  const size_t ring = sh.stages * split_stage_bytes(sh.rn, a.w_planes), part = (size_t)sh.rn * 512;
+  REQUIRE(sh.stages >= 1 && sh.smem >= 1024 + (ring > part ? ring : part) + (X == nullptr ? split_norm_bytes(K, sh.rn, sh.S) : 0),
+          WGPT_ERR_SHAPE, "no launch shape for a product of %d x %d x %d", M, K, N);
   CUtensorMap mw, mx;
   TRY(make_pair_map(&mw, W, (uint64_t)N, (uint64_t)K, 128, a.w_planes));
   mx = mw;
   if (X != nullptr) TRY(make_pair_map(&mx, X, (uint64_t)M, (uint64_t)K, sh.rn));
-  const int kb = (K + GP_BK - 1) / GP_BK;
-  const size_t smem = 1024 + (size_t)sh.stages * (a.w_planes * (GS_W_BYTES / 2) + sh.rn * (GP_BK * 4)) +
-                      (X == nullptr ? (size_t)((kb + sh.S - 1) / sh.S) * GP_BK * 8 + (size_t)sh.rn * a.x_tiles * 8 : 0);
   const dim3 grid(sh.row_tiles * a.f_tiles * sh.S);
 #define SPLIT_CASE(RNV)                                                                                              \
   do {                                                                                                               \
-    CK(allow_smem(dev, gemm_split_kernel<RNV>));        \
-    CK(launch_ex_x(dev->pdl, sh.S, dev->stream, gemm_split_kernel<RNV>, grid, dim3(GS_THREADS), smem, mw, mx, a));   \
+    CK(allow_smem(dev, gemm_split_kernel<RNV>));                                                                       \
+    CK(launch_ex_x(dev->pdl, sh.S, dev->stream, gemm_split_kernel<RNV>, grid, dim3(GS_THREADS), sh.smem, mw, mx, a)); \
   } while (0)
   if (X != nullptr) SPLIT_CASE(0);
   else if (sh.rn == 16) SPLIT_CASE(16);
@@ -1167,7 +1123,7 @@ static int32_t launch_pair_product(wgpt_device *dev, const __half *X, const __ha
                                    const Epilogue &epi, bool dyn = false, bool b_exact = false) {
   double big = 0, split = 0;
   pair_tile_columns(dev, M, N, K, &big);
-  const SplitShape sh = split_shape_rows(dev, M, K, N, &split);
+  const SplitShape sh = split_shape_rows(split_limits(dev), M, K, N, b_exact ? 1 : 2, &split);
   if (split < big && N % 4 == 0 && (epi.ld & 3) == 0) {
     SplitArgs a;
     memset(&a, 0, sizeof a);
@@ -2546,8 +2502,9 @@ static int32_t forward_blocks_split(wgpt_session *s, int n_tok) {
   const int E = p.n_embd, F = 4 * E, H = p.n_head, hs = m->hs, M = s->n_seq * n_tok, xt = (E + 127) / 128;
   const size_t kv_layer = (size_t)s->n_seq * p.n_ctx * E, plane_e = (size_t)M * E, plane_f = (size_t)M * F;
   __half *o = reinterpret_cast<__half *>(s->o), *f = reinterpret_cast<__half *>(s->f);
-  const SplitShape sh_qkv = split_shape_decode(dev, M, E, 3 * E), sh_o = split_shape_decode(dev, M, E, E),
-                   sh_fc = split_shape_decode(dev, M, E, F), sh_pr = split_shape_decode(dev, M, F, E);
+  const SplitLimits lim = split_limits(dev);
+  const SplitShape sh_qkv = split_shape_decode(lim, M, E, 3 * E, true), sh_o = split_shape_decode(lim, M, E, E, false),
+                   sh_fc = split_shape_decode(lim, M, E, F, true), sh_pr = split_shape_decode(lim, M, F, E, false);
   SplitArgs norm, plain;
   memset(&norm, 0, sizeof norm);
   memset(&plain, 0, sizeof plain);

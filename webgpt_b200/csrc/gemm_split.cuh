@@ -25,19 +25,20 @@
 // Every wait is bounded; on expiry the CTA sets *err = 3 and carries on through its cluster barriers (the result is void).
 #pragma once
 #include "gemm_pair.cuh"
+#include "split_plan.h"
 
 namespace wgpt {
 
 constexpr int GS_THREADS = 256;        // warp 0 TMA, warp 1 MMA, warps 2-7 staging, warps 4-7 accumulator read-back
 constexpr int GS_STAGERS = 192;
-constexpr int GS_MAX_STAGES = 6;
 constexpr int GS_W_BYTES = GP_A_BYTES;  // both planes of a 128 x 64 weight tile
+static_assert(GS_W_BYTES == 2 * GS_PLANE_BYTES && GP_BK == GS_BK, "the launch shapes are planned for these tiles");
 
 struct SplitArgs {
   int M, K, N;
   int rn;              // activation rows per CTA: a multiple of 16, at most 128 (kPlanes) / RN (kNorm)
   int f_tiles;         // ceil(N / 128)
-  int stages;          // ring stages (<= GS_MAX_STAGES); stages * stage_bytes >= rn * 512
+  int stages;          // ring stages (<= GS_MAX_STAGES); max(stages * stage_bytes, rn * 512) bytes of ring (split_plan.h)
   Epilogue epi;
   float2 *stats;       // [M][f_tiles] or nullptr
   int dyn;             // the weight and its scales were written by the previous kernel: nothing is read ahead of the wait
