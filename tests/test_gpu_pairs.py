@@ -173,6 +173,27 @@ def test_ring_gemv_rows(oracle, n_seq):
         gpt.destroy()
 
 
+def test_decode_rows_of_a_wide_model(oracle):
+    """n_embd 3072: LayerNorm scale, shift and row statistics leave the normalising product fewer ring stages than its slice
+    of K asks for, at 32 and at 64 rows. Two tokens as decode passes; bound as in test_decode_rows."""
+    from webgpt_b200 import GPT
+    params = dict(n_layer=1, n_head=48, n_embd=3072, n_ctx=8, vocab_size=256)
+    w = synth.make_weights(params, seed=23, std=0.02, ln_random=True)
+    m = oracle.Model(params, synth.weight_list(params, w))
+    gpt = GPT(None, params=params, weights=w)
+    gpt.initialize()
+    try:
+        for n_seq in (24, 64):
+            prompts = np.stack([synth.make_tokens(256, 2, seed=8, stream=i) for i in range(n_seq)])
+            s = gpt.session(n_seq)
+            s.forward(prompts[:, :1], want_logits=False)
+            lg = s.forward(prompts[:, 1:])
+            for i in (0, n_seq - 1):
+                assert rel_err(lg[i], m.run(prompts[i])) < 2e-5, n_seq
+    finally:
+        gpt.destroy()
+
+
 @pytest.mark.parametrize("K,N", [(48, 40), (768, 136), (1616, 152), (3072, 768)])
 def test_int8_handle_rows(dev, oracle, K, N):
     """Up to eight rows in the block kernel (columns per item 1-4, K slices 1-8), above 16 rows as pairs against the exact

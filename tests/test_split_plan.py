@@ -1,6 +1,6 @@
 """CPU checks of the launch shapes of the cluster split-K product (csrc/split_plan.h): what a CTA keeps in shared memory
-fits what is asked for, and that fits an SM. The limits are a B200's: 227 KB per CTA, of which 2 KB are left to the
-kernel's static arrays, and clusters of one to eight CTAs, one per SM, on 148 SMs in groups of 16 or fewer."""
+fits what is asked for, and what is asked for fits an SM. The limits are a B200's: 227 KB per CTA, of which 2 KB are left
+to the kernel's static arrays, and clusters of one to eight CTAs, one per SM, on 148 SMs in groups of 16 or fewer."""
 import ctypes as C
 import os
 import subprocess
@@ -18,12 +18,12 @@ using namespace wgpt;
 static void put(const SplitShape &sh, long long *out) {
   out[0] = sh.row_tiles; out[1] = sh.rn; out[2] = sh.S; out[3] = sh.stages; out[4] = (long long)sh.smem;
 }
-extern "C" void decode(const int *clusters, int M, int K, int N, int norm, long long *out) {
-  put(split_shape_decode(SplitLimits{clusters}, M, K, N, norm != 0), out);
+extern "C" void decode(const int *clusters, long long smem, int M, int K, int N, int norm, long long *out) {
+  put(split_shape_decode(SplitLimits{clusters, (size_t)smem}, M, K, N, norm != 0), out);
 }
-extern "C" void rows(const int *clusters, int M, int K, int N, int w_planes, long long *out) {
+extern "C" void rows(const int *clusters, long long smem, int M, int K, int N, int w_planes, long long *out) {
   double cycles;
-  put(split_shape_rows(SplitLimits{clusters}, M, K, N, w_planes, &cycles), out);
+  put(split_shape_rows(SplitLimits{clusters, (size_t)smem}, M, K, N, w_planes, &cycles), out);
 }
 """
 
@@ -40,7 +40,7 @@ def plan(tmp_path_factory):
 
     def call(fn, *args):
         out = (C.c_longlong * 5)()
-        getattr(so, fn)(clusters, *args, out)
+        getattr(so, fn)(clusters, C.c_longlong(SMEM), *args, out)
         return dict(zip(("row_tiles", "rn", "S", "stages", "smem"), out))
 
     return call
@@ -61,6 +61,25 @@ def test_partial_tile_fits_the_ring(plan, w_planes, N):
             assert sh["stages"] >= 1 and sh["rn"] % 16 == 0 and sh["rn"] <= 128 and sh["row_tiles"] * sh["rn"] >= M
             assert sh["smem"] <= SMEM
             assert sh["smem"] >= 1024 + max(ring_bytes(sh, w_planes), sh["rn"] * 512), (M, K, N, sh)
+
+
+@pytest.mark.parametrize("M", [9, 16, 17, 32, 33, 48, 49, 64])
+def test_normalising_form_fits_or_is_refused(plan, M):
+    """Scale, shift and row statistics lie behind the ring; a width at which nothing fits is refused (smem 0) and the
+    caller takes another path. Everything up to 8192 has to fit."""
+    for E in list(range(64, 1665, 32)) + [2048, 2560, 2688, 2880, 3072, 3200, 4096, 5120, 8192, 12288, 16384]:
+        kb = (E + 63) // 64
+        for N in (3 * E, 4 * E):
+            sh = plan("decode", M, E, N, 1)
+            if sh["smem"] == 0:
+                assert E > 8192
+                continue
+            behind = -(-kb // sh["S"]) * 512 + sh["rn"] * ((E + 127) // 128) * 8
+            assert sh["stages"] >= 1 and sh["smem"] <= SMEM
+            assert sh["smem"] >= 1024 + max(ring_bytes(sh, 2), sh["rn"] * 512) + behind
+        for K, N in ((E, E), (4 * E, E)):
+            sh = plan("decode", M, K, N, 0)
+            assert sh["stages"] >= 1 and 1024 + max(ring_bytes(sh, 2), sh["rn"] * 512) <= sh["smem"] <= SMEM
 
 
 def test_ring_keeps_its_share_where_everything_fits(plan):

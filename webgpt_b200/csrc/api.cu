@@ -1061,7 +1061,7 @@ static int32_t gemm_kn_via_transpose(wgpt_device *dev, const float *A, size_t ld
   return launch_gemm_tc(dev, dev->precision == WGPT_PRECISION_TF32X3, A, lda, wt, M, K, N, epi, nullptr, false);
 }
 
-static SplitLimits split_limits(const wgpt_device *dev) { return SplitLimits{dev->max_clusters}; }
+static SplitLimits split_limits(const wgpt_device *dev) { return SplitLimits{dev->max_clusters, dev->smem_optin - 2048}; }
 
 // X: pair planes [2][M][K], or nullptr with the LayerNorm input described in a (kNorm, M <= 64).
 static int32_t launch_gemm_split(wgpt_device *dev, const SplitShape &sh, const __half *X, const __half *W, int M, int K,
@@ -1124,7 +1124,7 @@ static int32_t launch_pair_product(wgpt_device *dev, const __half *X, const __ha
   double big = 0, split = 0;
   pair_tile_columns(dev, M, N, K, &big);
   const SplitShape sh = split_shape_rows(split_limits(dev), M, K, N, b_exact ? 1 : 2, &split);
-  if (split < big && N % 4 == 0 && (epi.ld & 3) == 0) {
+  if (sh.smem > 0 && split < big && N % 4 == 0 && (epi.ld & 3) == 0) {
     SplitArgs a;
     memset(&a, 0, sizeof a);
     a.dyn = dyn ? 1 : 0;
@@ -2491,6 +2491,20 @@ static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
   return WGPT_OK;
 }
 
+// The four products of a block in the split form; ok: all of them fit shared memory (the LayerNorm's scale, shift and row
+// statistics grow with the width, see split_plan.h).
+struct SplitBlockShapes {
+  SplitShape qkv, o, fc, pr;
+  bool ok;
+};
+static SplitBlockShapes split_block_shapes(const wgpt_device *dev, int M, int E) {
+  const SplitLimits lim = split_limits(dev);
+  SplitBlockShapes b = {split_shape_decode(lim, M, E, 3 * E, true), split_shape_decode(lim, M, E, E, false),
+                        split_shape_decode(lim, M, E, 4 * E, true), split_shape_decode(lim, M, 4 * E, E, false), false};
+  b.ok = b.qkv.smem > 0 && b.o.smem > 0 && b.fc.smem > 0 && b.pr.smem > 0;
+  return b;
+}
+
 constexpr int kSplitMinRows = 6;
 // The transformer blocks of a pass of up to 64 rows (a decode step, a short prompt) as five kernels per block
 // (gemm_split.cuh): both LayerNorms ride on the products that consume them, the attention finishes its own output, and
@@ -2502,9 +2516,7 @@ static int32_t forward_blocks_split(wgpt_session *s, int n_tok) {
   const int E = p.n_embd, F = 4 * E, H = p.n_head, hs = m->hs, M = s->n_seq * n_tok, xt = (E + 127) / 128;
   const size_t kv_layer = (size_t)s->n_seq * p.n_ctx * E, plane_e = (size_t)M * E, plane_f = (size_t)M * F;
   __half *o = reinterpret_cast<__half *>(s->o), *f = reinterpret_cast<__half *>(s->f);
-  const SplitLimits lim = split_limits(dev);
-  const SplitShape sh_qkv = split_shape_decode(lim, M, E, 3 * E, true), sh_o = split_shape_decode(lim, M, E, E, false),
-                   sh_fc = split_shape_decode(lim, M, E, F, true), sh_pr = split_shape_decode(lim, M, F, E, false);
+  const SplitBlockShapes sh = split_block_shapes(dev, M, E);
   SplitArgs norm, plain;
   memset(&norm, 0, sizeof norm);
   memset(&plain, 0, sizeof plain);
@@ -2517,7 +2529,7 @@ static int32_t forward_blocks_split(wgpt_session *s, int n_tok) {
     e.colscale = L.wqkv_p.cs;
     e.kc = kc; e.vc = vc; e.E = E; e.n_tok = n_tok; e.n_ctx = p.n_ctx; e.pos = s->d_pos;
     norm.gamma = L.ln1_g; norm.beta = L.ln1_b; norm.x_scale = L.s_h1;
-    TRY(launch_gemm_split(dev, sh_qkv, nullptr, L.wqkv_p.p, M, E, 3 * E, e, norm));
+    TRY(launch_gemm_split(dev, sh.qkv, nullptr, L.wqkv_p.p, M, E, 3 * E, e, norm));
     const __half *o_in = o;
     if (n_tok == 1) {
       TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, nullptr, E, M, H, s->n_split, s->d_pos, m->scale,
@@ -2535,17 +2547,17 @@ static int32_t forward_blocks_split(wgpt_session *s, int n_tok) {
     e = plain_epi(s->x, E, L.bo);
     e.colscale = L.wo_p.cs;
     e.residual = s->x;
-    TRY(launch_gemm_split(dev, sh_o, o_in, L.wo_p.p, M, E, E, e, plain));
+    TRY(launch_gemm_split(dev, sh.o, o_in, L.wo_p.p, M, E, E, e, plain));
     e = plain_epi(nullptr, F, L.bfc);
     e.colscale = L.wfc_p.cs;
     e.act = 1;
     e.pair = f; e.pair_plane = plane_f; e.pair_scale = L.s_f;
     norm.gamma = L.ln2_g; norm.beta = L.ln2_b; norm.x_scale = L.s_h2;
-    TRY(launch_gemm_split(dev, sh_fc, nullptr, L.wfc_p.p, M, E, F, e, norm));
+    TRY(launch_gemm_split(dev, sh.fc, nullptr, L.wfc_p.p, M, E, F, e, norm));
     e = plain_epi(s->x, E, L.bpr);
     e.colscale = L.wpr_p.cs;
     e.residual = s->x;
-    TRY(launch_gemm_split(dev, sh_pr, f, L.wpr_p.p, M, F, E, e, plain));
+    TRY(launch_gemm_split(dev, sh.pr, f, L.wpr_p.p, M, F, E, e, plain));
   }
   return WGPT_OK;
 }
@@ -2613,7 +2625,8 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
   // de-embedding 6.3e-6 and 1.45e-5). Decode pass of eight sequences 0.369 ms (FP32 blocks 0.489), XL 2.21 (5.08).
   // Prompts: from nine rows on; up to eight stay in FP32 where the products fit the block form, as they always have.
   const bool split = pair_mode && M <= 64 &&
-                     (n_tok == 1 ? M >= kSplitMinRows : M > 8 || (M >= kSplitMinRows && !layers_fit_block_form(dev, M, E)));
+                     (n_tok == 1 ? M >= kSplitMinRows : M > 8 || (M >= kSplitMinRows && !layers_fit_block_form(dev, M, E))) &&
+                     split_block_shapes(dev, M, E).ok;
   if (!fused)
     LAUNCH_PDL(dev, embed_kernel, M, 128, 0, ids, m->wte, m->wpe, s->x, M, n_tok, E, p.vocab_size,
                (const int *)s->d_pos, dev->d_err, split ? s->stats : nullptr);

@@ -14,12 +14,14 @@ constexpr size_t GS_RING_BYTES = size_t(200) << 10;
 
 struct SplitShape {
   int row_tiles, rn, S, stages;
-  size_t smem;  // dynamic
+  size_t smem;  // dynamic; 0: does not fit
 };
 
-// What the shapes depend on: clusters of S CTAs that are resident at once with one CTA per SM.
+// What the shapes depend on: clusters of S CTAs that are resident at once with one CTA per SM, and the dynamic shared
+// memory that a CTA may ask for.
 struct SplitLimits {
   const int *max_clusters;  // [9]
+  size_t smem;
 };
 
 // Bytes of one ring stage: w_planes planes of a weight tile and both planes of rn activation rows.
@@ -32,14 +34,21 @@ inline size_t split_norm_bytes(int K, int rn, int S) {
   return (size_t)((kb + S - 1) / S) * GS_BK * 8 + (size_t)rn * ((K + 127) / 128) * 8;
 }
 
-// As many stages as a CTA's slice of K has k-blocks and the ring's share of shared memory holds. The partial tile [rn][128]
-// lies over the ring once that has been read, so the ring is never smaller than it: a slice of one k-block against a
-// one-plane weight has a stage of 16 KB + 256 rn and a tile of 512 rn.
-inline void split_place(SplitShape &sh, int K, int w_planes, bool norm) {
+// As many stages as a CTA's slice of K has k-blocks, as the ring's share of shared memory holds, and as the whole fits.
+// The partial tile [rn][128] lies over the ring once that has been read, so the ring is never smaller than it: a slice of
+// one k-block against a one-plane weight has a stage of 16 KB + 256 rn and a tile of 512 rn.
+inline void split_place(SplitShape &sh, const SplitLimits &lim, int K, int w_planes, bool norm) {
   const int kb = (K + GS_BK - 1) / GS_BK;
   const size_t stage = split_stage_bytes(sh.rn, w_planes), part = (size_t)sh.rn * 512;
-  sh.stages = (int)std::min<size_t>({(size_t)((kb + sh.S - 1) / sh.S), GS_RING_BYTES / stage, (size_t)GS_MAX_STAGES});
-  sh.smem = 1024 + std::max(sh.stages * stage, part) + (norm ? split_norm_bytes(K, sh.rn, sh.S) : 0);
+  const size_t fixed = 1024 + (norm ? split_norm_bytes(K, sh.rn, sh.S) : 0);
+  sh.stages = 0;
+  sh.smem = 0;
+  if (fixed >= lim.smem) return;
+  const size_t room = std::min(lim.smem - fixed, GS_RING_BYTES);
+  sh.stages = (int)std::min<size_t>({(size_t)((kb + sh.S - 1) / sh.S), room / stage, (size_t)GS_MAX_STAGES});
+  const size_t ring = std::max(sh.stages * stage, part);
+  if (sh.stages < 1 || fixed + ring > lim.smem) return;
+  sh.smem = fixed + ring;
 }
 
 // One row tile of RN rows (kNorm / decode): the smallest number of K slices with the shortest longest slice, among those
@@ -52,7 +61,7 @@ inline SplitShape split_shape_decode(const SplitLimits &lim, int M, int K, int N
   sh.S = 1;
   for (int S = 2; S <= 8 && S <= kb; S++)
     if (ft <= lim.max_clusters[S] && (kb + S - 1) / S < (kb + sh.S - 1) / sh.S) sh.S = S;
-  split_place(sh, K, 2, norm);
+  split_place(sh, lim, K, 2, norm);
   return sh;
 }
 
@@ -75,7 +84,7 @@ inline SplitShape split_shape_rows(const SplitLimits &lim, int M, int K, int N, 
       }
     }
   }
-  if (best.S > 0) split_place(best, K, w_planes, false);
+  if (best.S > 0) split_place(best, lim, K, w_planes, false);
   return best;
 }
 
