@@ -139,6 +139,75 @@ def test_decode_rows(model64, n_seq):
         assert rel_err(lg[i], m.run(np.concatenate([prompts[i], got[i, :1]]))) < 2e-5
 
 
+@pytest.fixture(scope="module")
+def model8(oracle):
+    """Head size 8: a head's output is a quarter of a warp."""
+    from webgpt_b200 import GPT
+    params = dict(n_layer=2, n_head=8, n_embd=64, n_ctx=96, vocab_size=264)
+    w = synth.make_weights(params, seed=19, std=0.1, ln_random=True)
+    gpt = GPT(None, params=params, weights=w)
+    gpt.initialize()
+    yield gpt, oracle.Model(params, synth.weight_list(params, w)), params
+    gpt.destroy()
+
+
+@pytest.mark.parametrize("n_seq", [2, 6])
+@pytest.mark.parametrize("slices", [2, 4, 8])
+@pytest.mark.parametrize("fixture", ["model64", "model8"])
+def test_decode_attention_slices(request, monkeypatch, fixture, slices, n_seq):
+    """The cluster merge of 2, 4 and 8 slices, f32 output (2 sequences) and pairs (6), at contexts from one position on:
+    up to seven slices without a position, slices of unequal length, and one that takes several steps."""
+    gpt, m, p = request.getfixturevalue(fixture)
+    monkeypatch.setenv("WGPT_ATTN_SPLIT", str(slices))
+    ids = np.stack([synth.make_tokens(p["vocab_size"], 90, seed=51, stream=i) for i in range(n_seq)])
+    from webgpt_b200.model import Session
+    s = Session(gpt, n_seq)
+    try:
+        for t in range(13):
+            lg = s.forward(ids[:, t:t + 1])
+            for i in (0, n_seq - 1):
+                assert rel_err(lg[i], m.run(ids[i, :t + 1])) < 2e-5, t
+        s.forward(ids[:, 13:88], want_logits=False)
+        for t in (88, 89):
+            lg = s.forward(ids[:, t:t + 1])
+            for i in (0, n_seq - 1):
+                assert rel_err(lg[i], m.run(ids[i, :t + 1])) < 2e-5, t
+    finally:
+        s.destroy()
+
+
+def test_decode_slices_follow_the_context(model64, monkeypatch):
+    """Sums over another number of slices differ in their last bits, so equal logits show which number ran: one-token
+    forwards take it from the context they meet, and a captured completion changes it as it grows (at 64 and 192 positions
+    for these sizes), so that both leave the same cache."""
+    from webgpt_b200.model import Session
+    gpt, _, p = model64
+    ids = np.stack([synth.make_tokens(p["vocab_size"], 301, seed=52, stream=i) for i in range(2)])
+
+    def logits(n, slices):
+        monkeypatch.setenv("WGPT_ATTN_SPLIT", slices)
+        s = Session(gpt, 2)
+        s.forward(ids[:, :n], want_logits=False)
+        out = s.forward(ids[:, n:n + 1])
+        s.destroy()
+        return out
+
+    for n, want in ((30, "1"), (100, "2"), (300, "4")):
+        by_context = logits(n, "0")
+        assert [k for k in "1248" if np.array_equal(logits(n, k), by_context)] == [want], n
+    monkeypatch.setenv("WGPT_ATTN_SPLIT", "0")
+    s, t = Session(gpt, 2), Session(gpt, 2)
+    try:
+        new = s.generate_greedy(ids[:, :16], 300)
+        t.forward(ids[:, :16], want_logits=False)
+        for i in range(299):
+            t.forward(new[:, i:i + 1], want_logits=False)
+        assert np.array_equal(s.forward(new[:, 299:]), t.forward(new[:, 299:]))
+    finally:
+        s.destroy()
+        t.destroy()
+
+
 @pytest.mark.parametrize("n_seq", [1, 2, 3, 5, 7, 8])
 def test_ring_gemv_rows(oracle, n_seq):
     """Layers that do not fit shared memory (n_embd 1600): FP32 through the ring for up to five sequences, and for eight

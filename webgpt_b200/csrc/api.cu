@@ -2234,8 +2234,9 @@ struct wgpt_session {
   int cap_tok;   // tokens per forward the activation buffers are sized for
   int out_cap;   // capacity (per sequence) of d_out_ids
   int last_rows; // rows of the most recent forward (for the tap)
-  int n_split;        // position slices of the decode attention (attn_split_for), fixed while a step graph lives
-  bool split_forced;  // set by WGPT_ATTN_SPLIT
+  int n_split = 1;       // position slices of the decode attention of the pass at hand
+  int forced_split = 0;  // WGPT_ATTN_SPLIT, 0: by the context (context_split)
+  int step_split = 0;    // slices of this completion's newest decode step, 0: none yet
   float *x, *h, *q, *o, *f, *logits;
   float2 *stats = nullptr;  // [rows][n_embd / 128] (mean, squared deviations) of the residual stream's tiles
   float *kc, *vc;  // [n_layer][n_seq][n_ctx][E]
@@ -2255,8 +2256,8 @@ struct wgpt_session {
   double sample_temp = 1.0;
   double *d_uniform = nullptr;
   size_t uniform_cap = 0;  // doubles
-  cudaGraphExec_t step_graph;  // one captured decode step (pointers of this session baked in)
-  uint64_t step_graph_launches;
+  cudaGraphExec_t step_graph[4];  // one captured decode step (pointers of this session baked in) per slice count 1, 2, 4, 8
+  uint64_t step_graph_launches[4];
   bool step_warm;
 };
 
@@ -2287,9 +2288,10 @@ static int32_t session_reserve(wgpt_session *s, int n_tok) {
 
 // Position slices per (sequence, head) of the decode attention: 1, 2, 4 or 8 CTAs of a cluster share a head's cache rows.
 // Doubled while the grid stays within about 5.5 CTAs per SM (what is resident at once) and a slice keeps the positions that
-// a CTA has in flight in one step (4096 / head size), for the context as it is when the step is captured plus 64 for what
-// is generated from there. Per pass, chosen (slices) / others: GPT-2 16 sequences at 128 positions 0.414 (2) / 0.432 (4),
-// 8 at 64 0.362 (2) / 0.400 (8), 4 at 500 0.379 (8) / 0.437 (2); GPT-2 XL 4 at 200 2.25 (4) / 2.39 (2) / 2.47 (8) ms.
+// a CTA has in flight in one step (4096 / head size), for the context at hand plus the 64 positions it may grow by before
+// the next look. Per pass with 1 / 2 / 4 / 8 slices, GPT-2 2 sequences at 100 positions 359 / 346 / 342 / 349, at 300
+// 418 / 379 / 360 / 357, at 900 643 / 488 / 413 / 377 us, 16 at 192 486 / 472 / 489 / 546, at 900 737 / 709 / 638 / 639; GPT-2
+// XL 1 sequence at 900 2710 / 2175 / 1943 / 1984, 4 at 448 3248 / 2847 / 2638 / 2658.
 constexpr int kMaxAttnSplit = 8;
 static int attn_split_for(const wgpt_device *dev, int n_head, int n_seq, int head_size, int context_len) {
   const int step = 4096 / head_size;
@@ -2311,15 +2313,10 @@ WGPT_EXPORT int32_t wgpt_session_create(wgpt_model *m, int32_t n_seq, wgpt_sessi
   s->n_seq = n_seq;
   const wgpt_params &p = m->p;
   size_t kv = (size_t)p.n_layer * n_seq * p.n_ctx * p.n_embd;
-  s->split_forced = false;
   if (const char *ev = getenv("WGPT_ATTN_SPLIT")) {  // tuning override: 1, 2, 4 or 8
     int v = atoi(ev);
-    if (v == 1 || v == 2 || v == 4 || v == 8) {
-      s->n_split = v;
-      s->split_forced = true;
-    }
+    if (v == 1 || v == 2 || v == 4 || v == 8) s->forced_split = v;
   }
-  if (!s->split_forced) s->n_split = attn_split_for(m->dev, p.n_head, n_seq, m->hs, 0);
   cudaError_t e = cudaMalloc(&s->kc, kv * 4);
   if (e == cudaSuccess) e = cudaMalloc(&s->vc, kv * 4);
   if (e == cudaSuccess) e = cudaMalloc(&s->logits, (size_t)n_seq * p.vocab_size * 4);
@@ -2610,15 +2607,26 @@ static int32_t forward_blocks_ring(wgpt_session *s, int n_tok, bool *done) {
   return WGPT_OK;
 }
 
-// With pick, the greedy choice of every sequence is also made (next_ids, out_ids) and the position advanced.
-static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pick = false) {
+// A decode step of this session runs on the two fused kernels per block (their clusters share a head's positions).
+static bool decodes_fused(const wgpt_session *s) { return s->n_seq == 1 && s->m->fused.ok && s->fx_a != nullptr; }
+
+// The attention slices of a decode pass over the context as it is now.
+static int context_split(const wgpt_session *s) {
+  if (s->forced_split > 0) return s->forced_split;
+  return decodes_fused(s) ? 1 : attn_split_for(s->m->dev, s->m->p.n_head, s->n_seq, s->m->hs, s->len);
+}
+
+// With pick, the greedy choice of every sequence is also made (next_ids, out_ids) and the position advanced. slices: of a
+// decode pass's attention, 0: by the context.
+static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pick = false, int slices = 0) {
+  s->n_split = slices > 0 ? slices : context_split(s);
   wgpt_model *m = s->m;
   wgpt_device *dev = m->dev;
   const wgpt_params &p = m->p;
   const int E = p.n_embd, F = 4 * E, H = p.n_head, hs = m->hs, M = s->n_seq * n_tok;
   const size_t kv_layer = (size_t)s->n_seq * p.n_ctx * E;
 
-  const bool fused = n_tok == 1 && s->n_seq == 1 && m->fused.ok && s->fx_a != nullptr;
+  const bool fused = n_tok == 1 && decodes_fused(s);
   const bool pair_mode = m->pair_ok && dev->precision == WGPT_PRECISION_TF32X3;
   // From six sequences on, where the de-embedding leaves the FP32 kernels too (logits of a decode step against double
   // precision, 2-norm: GPT-2 2.9e-6, XL 6.0e-6; five sequences in FP32 4e-7, and eight with FP32 blocks and the 3xTF32
@@ -2849,51 +2857,59 @@ static int32_t pick_and_advance(wgpt_session *s, int n_tok) {
 }
 
 // One decode step (newest token of every sequence -> next token), replayed as a CUDA graph: all position- and
-// step-dependent values are read from device memory, so one captured step serves every position.
-static int32_t decode_step(wgpt_session *s) {
+// step-dependent values are read from device memory, so one captured step serves every position that the same number of
+// attention slices suits. `left`: steps of this completion from here on, this one included.
+static int32_t decode_step(wgpt_session *s, int left) {
   wgpt_device *dev = s->m->dev;
-  // the slice count follows the context length as it is when the step is (re)captured
-  if (!s->split_forced && (!dev->graphs || s->step_graph == nullptr))
-    s->n_split = attn_split_for(dev, s->m->p.n_head, s->n_seq, s->m->hs, s->len);
-  if (!dev->graphs) {
-    return forward(s, s->next_ids, 1, true);
-  }
-  if (s->step_graph == nullptr) {
+  int slices = context_split(s);
+  if (!dev->graphs) return forward(s, s->next_ids, 1, true, slices);
+  auto slot = [](int n) { return n >= 8 ? 3 : n >> 1; };
+  // Another slice count gains some 2 to 6 % of a step, and to capture a step takes as long as a few of them: with fewer
+  // than kRecaptureSteps to go, a completion keeps the one it has.
+  constexpr int kRecaptureSteps = 64;
+  if (left < kRecaptureSteps && s->step_split > 0 && s->step_graph[slot(slices)] == nullptr &&
+      s->step_graph[slot(s->step_split)] != nullptr)
+    slices = s->step_split;
+  s->step_split = slices;
+  const int g = slot(slices);
+  if (s->step_graph[g] == nullptr) {
     // The first step runs eagerly (it also sets every kernel's shared-memory attribute); the second is captured.
     if (!s->step_warm) {
       s->step_warm = true;
-      return forward(s, s->next_ids, 1, true);
+      return forward(s, s->next_ids, 1, true, slices);
     }
     uint64_t before = dev->launches;
     int len_before = s->len;
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(dev->stream, cudaStreamCaptureModeRelaxed));
-    int32_t rc = forward(s, s->next_ids, 1, true);
+    int32_t rc = forward(s, s->next_ids, 1, true, slices);
     cudaError_t e = cudaStreamEndCapture(dev->stream, &graph);
     s->len = len_before;  // capturing enqueued nothing
-    s->step_graph_launches = dev->launches - before;
+    s->step_graph_launches[g] = dev->launches - before;
     dev->launches = before;
     if (rc != WGPT_OK) {
       if (graph) cudaGraphDestroy(graph);
       return rc;
     }
     if (e != cudaSuccess) return fail(WGPT_ERR_CUDA, "cudaStreamEndCapture: %s", cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&s->step_graph, graph, 0);
+    e = cudaGraphInstantiate(&s->step_graph[g], graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) {
-      s->step_graph = nullptr;
+      s->step_graph[g] = nullptr;
       return fail(WGPT_ERR_CUDA, "cudaGraphInstantiate: %s", cudaGetErrorString(e));
     }
   }
-  CK(cudaGraphLaunch(s->step_graph, dev->stream));
-  dev->launches += s->step_graph_launches;
+  CK(cudaGraphLaunch(s->step_graph[g], dev->stream));
+  dev->launches += s->step_graph_launches[g];
   s->len += 1;
   return WGPT_OK;
 }
 
 static void drop_step_graph(wgpt_session *s) {
-  if (s->step_graph) cudaGraphExecDestroy(s->step_graph);
-  s->step_graph = nullptr;
+  for (cudaGraphExec_t &g : s->step_graph) {
+    if (g) cudaGraphExecDestroy(g);
+    g = nullptr;
+  }
   s->step_warm = false;
 }
 
@@ -2977,6 +2993,7 @@ static int32_t generate(wgpt_session *s, int32_t n_new) {
   // (Re)start from the prompt window held in s->ids by set_prompts; a repeated call regenerates from the prompt.
   CK(cudaMemsetAsync(s->d_pos, 0, 2 * sizeof(int), dev->stream));
   s->len = 0;
+  s->step_split = 0;
   if (s->ids_dirty) {
     for (int q = 0; q < n_seq; q++)
       CK(cudaMemcpyAsync(s->ids + (size_t)q * first, s->prompts.data() + (size_t)q * n_prompt + (n_prompt - first),
@@ -2988,7 +3005,7 @@ static int32_t generate(wgpt_session *s, int32_t n_new) {
   const int i_start = 1;
   for (int i = i_start; i < n_new; i++) {
     if (s->len + 1 <= n_ctx) {
-      TRY(decode_step(s));
+      TRY(decode_step(s, n_new - i));
       continue;
     }
     // Window slides: every position index shifts, so the cache is void; recompute the newest n_ctx tokens
