@@ -324,3 +324,17 @@ def test_sampling_kernel_edges(dev, oracle, V):
         _lib.call("wgpt_sample_topk", dev.handle, r_d.ptr, len(rows), V, top_k, 1.3, u_d.ptr, o_d.ptr)
         got = o_d.read(np.uint32, len(rows))
         assert [int(t) for t in got] == [oracle.sample_topk(rows[i], top_k, 1.3, u[i]) for i in range(len(rows))], top_k
+
+
+@pytest.mark.parametrize("n_rows,V,ks", [(12, 8192, (32, 33)), (13, 8191, (8, 9)), (32, 32000, (32, 33)), (33, 50257, (20, 21)),
+                                         (49, 50257, (1,)), (2, 257, (32, 33, 40)), (2, 383, (47, 48)), (2, 384, (48,))])
+def test_sampling_on_both_sides_of_the_cluster_rule(dev, oracle, n_rows, V, ks):
+    """Rows, vocabularies and kept logits at which one kernel hands over to the other: the same picks."""
+    from webgpt_b200 import _lib
+    rng = np.random.default_rng(V + n_rows)
+    rows, u = rng.standard_normal((n_rows, V), dtype=np.float32), rng.random(n_rows)
+    r_d, u_d, o_d = dev.tensor(rows), dev.tensor(u), dev.buffer(4 * n_rows)
+    for top_k in ks:
+        _lib.call("wgpt_sample_topk", dev.handle, r_d.ptr, n_rows, V, top_k, 0.8, u_d.ptr, o_d.ptr)
+        got = o_d.read(np.uint32, n_rows)
+        assert [int(t) for t in got] == [oracle.sample_topk(rows[i], top_k, 0.8, u[i]) for i in range(n_rows)], top_k

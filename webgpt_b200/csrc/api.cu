@@ -2816,13 +2816,30 @@ static int32_t reserve_out_ids(wgpt_session *s, int n_new) {
   return WGPT_OK;
 }
 
+// Where the cluster form of the pick (sample_pick_kernel) is the faster one. Its time grows with the rows, once their CTAs
+// share SMs, and with the candidates that the kept logits leave; that of the kernel of one CTA a row with the vocabulary. One
+// CTA / cluster, us per call: 50257 logits, 1 row top_k 3 22.6 / 12.3, 40 26.1 / 18.5, 48 26.5 / 26.7; 12 rows 40 26.7 / 20.5;
+// 16 rows 32 26.1 / 21.3, 40 26.6 / 26.6; 32 rows 32 26.5 / 20.6, 40 26.7 / 26.7; 48 rows 20 24.6 / 24.3, 32 26.6 / 27.5; 64
+// rows 3 22.6 / 24.6, 48 26.8 / 50.4. 20000 logits, 8 rows 40 21.3 / 19.8; 32 rows 20 20.5 / 18.5, 32 20.8 / 21.5; 40 rows 3
+// 18.6 / 19.8. 8192 logits, 8 rows 32 18.5 / 16.8, 40 18.6 / 20.5; 32 rows 20 18.5 / 18.3. 4100 logits, 32 rows 8 16.5 / 16.4,
+// 20 17.5 / 18.3. Up to 4096 logits a cluster is one CTA and always faster (4096, 64 rows, 48: 18.5 / 15.8), unless fewer
+// groups of eight have a value than are kept: then every value is a candidate, more than the list holds (300 logits, 40:
+// 14.6 / 47.1).
+static bool pick_in_cluster(int n_rows, int V, int top_k) {
+  if (V <= 4096) return top_k <= kPickTopK && (V <= kPickCap || V >= 8 * top_k);
+  if (V > kPickCluster * kPickThreads * kPickVals) return false;
+  if (n_rows <= 12) return top_k <= (V >= 16384 ? 40 : 32);
+  if (n_rows <= 32) return top_k <= (V >= 32000 ? 32 : V >= 8192 ? 20 : 8);
+  return n_rows <= 48 && V >= 49152 && top_k <= 20;
+}
+
 // Arg-max of the newest logits of every sequence -> next input ids and output list; the same kernel then advances
 // the session's position by n_tok and its step counter by one.
 static int32_t launch_sample_topk(wgpt_device *dev, const float *logits, int n_rows, int V, int top_k,
                                   double temperature, const double *uniforms, uint32_t *next_ids, uint32_t *out_ids,
                                   int out_stride, int *pos, int *step, int n_tok, unsigned int *counter) {
-  const int C = V > 4096 ? kPickCluster : 1;
-  if (top_k <= kPickTopK && V <= C * kPickThreads * kPickVals) {
+  if (pick_in_cluster(n_rows, V, top_k)) {
+    const int C = V > 4096 ? kPickCluster : 1;
     CK(launch_ex_x(dev->pdl, C, dev->stream, sample_pick_kernel, dim3(C * n_rows), dim3(kPickThreads), 0, logits, V, top_k,
                    temperature, uniforms, next_ids, out_ids, out_stride, pos, step, n_tok, counter));
     dev->launches++;

@@ -164,7 +164,8 @@ sample_topk_kernel(const float *__restrict__ logits, int V, int top_k, double te
 }
 
 // ------------------------------------------------------------------------------------------------
-// The same pick for top_k <= 48 by a cluster of C CTAs per sequence, each holding its share of the logits in registers. A
+// The same pick for top_k <= 48 by a cluster of C CTAs per sequence, each holding its share of the logits in registers (for
+// few rows; pick_in_cluster in api.cu has the limits). A
 // decode step waits for this kernel, and what it takes is a chain of latencies: one CTA reading the row twice and sorting
 // 1024 maxima (55 barriers) took 10.6 us per token at 50257 logits; this form takes 8 us off the step (GPT-2, top_k 3 / 20: 235.8 / 238.8 -> 221 / 223).
 //   1. every thread reads its logits once, all loads in flight; the 64 groups of eight lanes leave their best keys in shared
