@@ -58,6 +58,24 @@ def test_product_of_pairs_error_bound(dev, M, K, N):
     assert np.array_equal(scaled, (got * r[:, None] * c[None, :]).astype(np.float32))
 
 
+@pytest.mark.parametrize("M,N,a,w", [(40, 72, 128, -124), (40, 72, -124, 128), (600, 520, 128, -124), (40, 72, 114, 10),
+                                     (40, 72, -60, -60)])
+def test_product_of_pairs_at_the_ends_of_the_exponent_range(dev, M, N, a, w):
+    """Operands of up to 2^a and 2^w, the largest FP32 number among them, whose products are finite: bound as above. The
+    largest values fit the scaled form, and a row's and a column's power of two come back without passing infinity."""
+    rng = np.random.default_rng(M + N + abs(a))
+    K, one = 136, 1 - 2.0 ** -24
+    A, W = (rng.standard_normal((M, K)) / 8).clip(-one, one), (rng.standard_normal((K, N)) / 8).clip(-one, one)
+    A[3, 5], W[7, 6] = one, -one
+    A, W = (A * 2.0 ** a).astype(np.float32), (W * 2.0 ** w).astype(np.float32)
+    assert np.isfinite(A).all() and np.isfinite(W).all()
+    ref = A.astype(np.float64) @ W.astype(np.float64)
+    mag = np.abs(A).astype(np.float64) @ np.abs(W).astype(np.float64)
+    top = np.abs(A).max(1)[:, None].astype(np.float64) * np.abs(W).max(0)[None, :].astype(np.float64) * K
+    got = matmul(dev, A, W)
+    assert (np.abs(got - ref) <= (3 * 2.0 ** -22 + (3 * K / 16 + 2) * 2.0 ** -23) * mag + 2.0 ** -39 * top).all()
+
+
 @pytest.mark.parametrize("M,K,N", [(9, 768, 136), (12, 3072, 768), (13, 72, 40), (16, 40, 2304), (17, 1600, 128), (24, 8, 8),
                                    (25, 768, 768), (31, 3080, 72)])
 def test_product_of_9_to_31_rows_is_fp32(dev, M, K, N):

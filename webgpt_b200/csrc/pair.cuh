@@ -12,6 +12,9 @@
 // Both planes together are 4 bytes per value, as the FP32 value itself: nothing more is streamed from HBM, and no
 // operand has to be split by CUDA threads between shared memory and the tensor core.
 #pragma once
+#include <cmath>
+#include <cstring>
+
 #include "common.cuh"
 
 namespace wgpt {
@@ -22,12 +25,20 @@ constexpr float kPairTop = 32768.f;  // scaled values stay below this (the half 
 // of zero, an infinity or a NaN gives 1 (an infinite or NaN element then turns the products it enters into NaN, as
 // hi + lo = inf + (inf - inf) did).
 __host__ __device__ inline float pair_scale_for(float bound) {
-  if (!(bound > 0.f) || !(bound < 3.0e38f)) return 1.f;
-  int ex;
-  const float m = frexpf(bound, &ex);            // bound = m 2^ex, m in [1/2, 1)
-  int e = 15 - (m == 0.5f ? ex - 1 : ex);        // bound 2^e <= 2^15
-  e = e < -110 ? -110 : (e > 110 ? 110 : e);     // 2^e and 2^-e stay normal; rows below 2^-95 lose low bits only
-  return ldexpf(1.f, e);
+#ifdef __CUDA_ARCH__
+  const uint32_t b = __float_as_uint(bound);
+#else
+  uint32_t b;
+  memcpy(&b, &bound, 4);
+#endif
+  if (b == 0u || b >= 0x7F800000u) return 1.f;  // zero, negative, infinite, NaN
+  int e = 141 - (int)(b >> 23) + ((b & 0x7FFFFFu) == 0u ? 1 : 0);  // bound 2^e <= 2^15; -113 at the largest number
+  e = e > 126 ? 126 : e;  // 2^-e stays normal; even a row of 2^-126 keeps 25 bits
+#ifdef __CUDA_ARCH__
+  return __uint_as_float((uint32_t)(e + 127) << 23);
+#else
+  return std::ldexp(1.f, e);
+#endif
 }
 
 // Four scaled values -> the four halves of each plane, packed for one 8-byte store.
@@ -40,11 +51,18 @@ __device__ __forceinline__ void pair_split4(float4 v, uint2 &p0, uint2 &p1) {
 }
 __device__ __forceinline__ float4 scale4(float4 v, float s) { return make_float4(v.x * s, v.y * s, v.z * s, v.w * s); }
 
+// A raw sum times the powers of two of its row and its column (or a column's scale), the smaller first: a row of 1e35 against
+// a column of 1e-35 would pass infinity on the way to one.
+__device__ __forceinline__ float pair_descale(float v, float rs, float cs) { return rs < cs ? v * rs * cs : v * cs * rs; }
+__device__ __forceinline__ float4 pair_descale4(float4 v, float rs, float4 cs) {
+  return make_float4(pair_descale(v.x, rs, cs.x), pair_descale(v.y, rs, cs.y), pair_descale(v.z, rs, cs.z), pair_descale(v.w, rs, cs.w));
+}
+
 // Epilogue of the kernels that multiply pairs: four raw sums of row m, columns n..n+3, with the columns' constants and
 // the residual already in registers -> the finished values, and their store.
 __device__ __forceinline__ float4 pair_epi_value4(const Epilogue &e, float4 v, float4 cs, float4 bs, float4 res, int m) {
-  if (e.rowscale != nullptr) v = scale4(v, __ldcg(e.rowscale + m));
-  v = make_float4(v.x * cs.x + bs.x, v.y * cs.y + bs.y, v.z * cs.z + bs.z, v.w * cs.w + bs.w);
+  v = e.rowscale != nullptr ? add4(pair_descale4(v, __ldcg(e.rowscale + m), cs), bs)
+                            : make_float4(v.x * cs.x + bs.x, v.y * cs.y + bs.y, v.z * cs.z + bs.z, v.w * cs.w + bs.w);
   if (e.act == 1) v = make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
   return make_float4(v.x + res.x, v.y + res.y, v.z + res.z, v.w + res.w);
 }
@@ -83,10 +101,9 @@ __device__ __forceinline__ void pair_epi_block(const Epilogue &e, const float *p
       const float *src = pad + r * 33 + col4;
       float4 v = make_float4(src[0], src[1], src[2], src[3]);
       if (m >= M) continue;
-      if (e.rowscale != nullptr) v = scale4(v, __ldcg(e.rowscale + m));
-      *reinterpret_cast<float4 *>(epi_addr(e, m, n)) =
-          make_float4(v.x * cs.x + bs.x + res[it].x, v.y * cs.y + bs.y + res[it].y, v.z * cs.z + bs.z + res[it].z,
-                      v.w * cs.w + bs.w + res[it].w);
+      v = e.rowscale != nullptr ? add4(pair_descale4(v, __ldcg(e.rowscale + m), cs), bs)
+                                : make_float4(v.x * cs.x + bs.x, v.y * cs.y + bs.y, v.z * cs.z + bs.z, v.w * cs.w + bs.w);
+      *reinterpret_cast<float4 *>(epi_addr(e, m, n)) = add4(v, res[it]);
     }
   } else {
 #pragma unroll 1
