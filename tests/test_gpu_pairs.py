@@ -120,6 +120,46 @@ def test_attention_operator_on_pairs(dev, oracle, T, E, H):
     assert rel_err(o_d.read(np.float32, T * E).reshape(T, E), ref) < 2e-5
 
 
+def attention64(x, H, scale, wq, wk, wv, wo):
+    """Causal attention of one window in double precision, no biases."""
+    T, E = x.shape
+    q, k, v = ((x @ w).reshape(T, H, E // H).transpose(1, 0, 2) for w in (wq, wk, wv))
+    s = np.where(np.tri(T, dtype=bool), q @ k.transpose(0, 2, 1) * scale, -np.inf)
+    p = np.exp(s - s.max(-1, keepdims=True))
+    return ((p / p.sum(-1, keepdims=True)) @ v).transpose(1, 0, 2).reshape(T, E) @ wo
+
+
+@pytest.mark.parametrize("T,E,H", [(64, 64, 1), (130, 128, 2), (200, 192, 3), (450, 128, 2)])
+@pytest.mark.parametrize("rows,b", [("last", 24), ("first", 24), ("one in seven", 24), ("any", 14), ("last", 62)])
+def test_attention_operator_rows_of_any_size(dev, T, E, H, rows, b):
+    """Each row against its own magnitude, beside rows 2^b times its size: before it, behind it and between. The scale keeps
+    the largest scores near one, so that no row's softmax amplifies its operands' last bits. Bound as in
+    test_attention_operator_on_pairs; later rows leave no trace in earlier ones."""
+    from webgpt_b200 import _lib
+    rng = np.random.default_rng(T + E + b)
+    x = rng.standard_normal((T, E))
+    at = {"last": [T - 1], "first": [0], "one in seven": range(3, T, 7), "any": range(T)}[rows]
+    x[at] *= 2.0 ** (rng.integers(-b, b + 1, len(at)) if rows == "any" else np.full(len(at), b))[:, None]
+    x = x.astype(np.float32)
+    ws = [(rng.standard_normal((E, E)) * 0.15).astype(np.float32) for _ in range(4)]
+    scale = 2.0 ** -(2 * b + 1)
+    zero = dev.tensor(np.zeros(E, np.float32))
+    d = [dev.tensor(w) for w in ws]
+
+    def run(rows_in):
+        x_d, o_d = dev.tensor(rows_in), dev.buffer(T * E * 4)
+        _lib.call("wgpt_attention", dev.handle, T, E, scale, H, E // H, x_d.ptr, *[p for w in d for p in (w.ptr, zero.ptr)], o_d.ptr)
+        _lib.call("wgpt_device_check", dev.handle)
+        return o_d.read(np.float32, T * E).reshape(T, E)
+
+    got, ref = run(x), attention64(x.astype(np.float64), H, scale, *(w.astype(np.float64) for w in ws))
+    err = np.abs(got - ref).max(1) / np.abs(ref).max(1)
+    assert err.max() < 2e-5, (int(err.argmax()), float(err.max()))
+    other = x.copy()
+    other[T - 1] *= np.float32(0.5)
+    assert np.array_equal(run(other)[:T - 1], got[:T - 1])
+
+
 @pytest.fixture(scope="module")
 def model64(oracle):
     """Head size 64, two layers: every prefill and decode path of the model takes it."""

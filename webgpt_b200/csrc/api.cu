@@ -1206,25 +1206,32 @@ static bool attn_prefill_pair_ok(const wgpt_device *dev, int hs) {
   return attn_prefill_uses_mma(dev, hs, 64) && dev->precision == WGPT_PRECISION_TF32X3;
 }
 
-// Prefill attention of a pair model (attn_prefill_pair_ok): output planes [2][rows][ldo].
+// Prefill attention of a pair model (attn_prefill_pair_ok): output planes [2][rows][ldo]. own_out: FP32 rows instead, and
+// every row of the operands with a scale of its own.
 static int32_t launch_attn_prefill_pair(wgpt_device *dev, const float *q, int ldq, const float *kc, const float *vc,
                                         int ldkv, size_t kv_seq_stride, int n_tok, int n_seq, int H, const int *pos,
                                         float scale, float s_qk, float s_v, __half *planes, size_t plane, int ldo,
-                                        const AttnScaleSrc &src = AttnScaleSrc()) {
+                                        float *own_out = nullptr) {
   // Two groups of warps per 64 query rows, alternating key tiles, while all CTAs are resident at once, up to three per SM
   // (GPT-2 at 333 / 1024 tokens 0.85 / 1.64 ms per pass against 1.00 / 1.95 with one group; with the CTAs' order balanced over
   // the SMs 1024 tokens take 1.55, XL 12.15 against 12.5, and XL with one group 12.8); one group beyond that (64 x 128 tokens,
   // 1536 CTAs: 4.46 against 4.8 ms) and for a single tile.
   const long long ctas = (long long)((n_tok + 63) / 64) * H * n_seq;
-#define PAIR_ATTN(W, G)                                                                                                  \
+#define PAIR_ATTN(W, G, OWN)                                                                                               \
   do {                                                                                                                   \
-    CK(allow_smem(dev, attn_prefill64_pair_kernel<W, G>));                                                               \
-    LAUNCH_PDL(dev, (attn_prefill64_pair_kernel<W, G>), (n_tok + 16 * W - 1) / (16 * W) * H * n_seq, 32 * W * G,          \
-               attn_pair_smem_bytes(G), q, ldq, kc, vc, ldkv, kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes, plane, \
-               ldo, src, H, dev->sm_count);                                                                              \
+    CK(allow_smem(dev, attn_prefill64_pair_kernel<W, G, OWN>));                                                            \
+    LAUNCH_PDL(dev, (attn_prefill64_pair_kernel<W, G, OWN>), (n_tok + 16 * W - 1) / (16 * W) * H * n_seq, 32 * W * G,      \
+               attn_pair_smem_bytes(G, OWN), q, ldq, kc, vc, ldkv, kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes,    \
+               plane, own_out, ldo, H, dev->sm_count);                                                                   \
   } while (0)
-  if (n_tok > 64 && ctas <= 3 * dev->sm_count) PAIR_ATTN(4, 2);
-  else PAIR_ATTN(4, 1);
+  const bool two = n_tok > 64 && ctas <= 3 * dev->sm_count;
+  if (own_out != nullptr) {
+    if (two) PAIR_ATTN(4, 2, true);
+    else PAIR_ATTN(4, 1, true);
+  } else {
+    if (two) PAIR_ATTN(4, 2, false);
+    else PAIR_ATTN(4, 1, false);
+  }
 #undef PAIR_ATTN
   return WGPT_OK;
 }
@@ -1442,18 +1449,15 @@ WGPT_EXPORT int32_t wgpt_deembed(wgpt_device *dev, int32_t n_embd, int32_t vocab
                         plain_epi(logits, vocab_size, nullptr));
 }
 
-// wgpt_attention on half-precision pairs, four kernels: all four weights and the rows to pairs; q | k | v as one product;
-// attention (scales from the norms the first pass left, |q| <= |x| |w| + |b|), its output as a pair; output projection.
-// The passes it replaces were thirteen kernels (a transposition, a split-K product and its second stage per weight).
+// wgpt_attention on half-precision pairs, five kernels: all four weights and the rows to pairs; q | k | v as one product;
+// attention; its output to pairs, row by row; output projection. The passes it replaces were thirteen kernels (a
+// transposition, a split-K product and its second stage per weight).
 static int32_t attention_pair(wgpt_device *dev, int T, int E, float scale, int H, int hs, const float *in, const float *qW,
                               const float *qB, const float *kW, const float *kB, const float *vW, const float *vB,
                               const float *linW, const float *linB, float *out) {
   const size_t te = (size_t)T * E;
-  const int nblk = (E + 31) / 32;
   __half *xp = nullptr, *op = nullptr, *wp = nullptr, *wo = nullptr;
-  float *qkv = nullptr, *o = nullptr, *xd = nullptr, *od = nullptr, *wd = nullptr, *wod = nullptr, *bias = nullptr,
-        *xn = nullptr, *wn = nullptr;
-  const bool mma = attn_prefill_pair_ok(dev, hs);
+  float *qkv = nullptr, *o = nullptr, *xd = nullptr, *od = nullptr, *wd = nullptr, *wod = nullptr, *bias = nullptr;
   for (int pass = 0; pass < 2; pass++) {
     Carve c{pass ? static_cast<char *>(dev->scratch) : nullptr};
     xp = c.take<__half>(2 * te);
@@ -1461,14 +1465,14 @@ static int32_t attention_pair(wgpt_device *dev, int T, int E, float scale, int H
     wp = c.take<__half>((size_t)2 * 3 * E * E);
     wo = c.take<__half>((size_t)2 * E * E);
     qkv = c.take<float>(3 * te);
-    if (!mma) o = c.take<float>(te);
+    o = c.take<float>(te);
     xd = c.take<float>(T); od = c.take<float>(T); wd = c.take<float>((size_t)3 * E); wod = c.take<float>(E);
-    bias = c.take<float>((size_t)3 * E); xn = c.take<float>((size_t)T + 8); wn = c.take<float>((size_t)6 * nblk);
+    bias = c.take<float>((size_t)3 * E);
     if (!pass) TRY(scratch_reserve(dev, c.used));
   }
   PairOperands p;
   memset(&p, 0, sizeof p);
-  p.x = in; p.M = T; p.K = E; p.xp = xp; p.x_descale = xd; p.x_norm = xn;
+  p.x = in; p.M = T; p.K = E; p.xp = xp; p.x_descale = xd;
   p.n_w = 4; p.N = E;
   const float *w[4] = {qW, kW, vW, linW}, *b[3] = {qB, kB, vB};
   for (int i = 0; i < 4; i++) {
@@ -1479,7 +1483,6 @@ static int32_t attention_pair(wgpt_device *dev, int T, int E, float scale, int H
     if (i < 3) {
       p.bias[i] = b[i];
       p.bias_out[i] = bias + (size_t)i * E;
-      p.norm[i] = wn + (size_t)2 * i * nblk;
     }
   }
   TRY(launch_pair_operands(dev, p));
@@ -1487,14 +1490,14 @@ static int32_t attention_pair(wgpt_device *dev, int T, int E, float scale, int H
   e.colscale = wd;
   e.rowscale = xd;
   TRY(launch_pair_product(dev, xp, wp, T, E, 3 * E, e, true));
-  if (mma) {
-    AttnScaleSrc src{xn, wn, p.x_ctas, nblk, od};
-    TRY(launch_attn_prefill_pair(dev, qkv, 3 * E, qkv + E, qkv + 2 * E, 3 * E, 0, T, 1, H, nullptr, scale, 1.f, 1.f, op, te, E,
-                                 src));
-  } else {
+  if (attn_prefill_pair_ok(dev, hs))
+    TRY(launch_attn_prefill_pair(dev, qkv, 3 * E, qkv + E, qkv + 2 * E, 3 * E, 0, T, 1, H, nullptr, scale, 1.f, 1.f, nullptr, 0,
+                                 E, o));
+  else
     TRY(launch_attn_prefill(dev, hs, qkv, 3 * E, qkv + E, qkv + 2 * E, 3 * E, 0, o, E, T, 1, H, nullptr, scale));
-    LAUNCH_PDL(dev, pair_rows_kernel, (T + 7) / 8, 256, 0, (const float *)o, (size_t)E, T, E, op, od, (float *)nullptr);
-  }
+  memset(&p, 0, sizeof p);
+  p.x = o; p.M = T; p.K = E; p.xp = op; p.x_descale = od;
+  TRY(launch_pair_operands(dev, p));
   e = plain_epi(out, E, linB);
   e.colscale = wod;
   e.rowscale = od;

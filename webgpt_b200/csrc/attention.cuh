@@ -624,6 +624,12 @@ attn_prefill64_mma_kernel(const float *__restrict__ q, int ldq, const float *__r
 // probabilities need no shuffles. 16 WARPS query rows per CTA share a staged 64-key tile. KG > 1: KG groups of WARPS warps
 // take the same rows and alternate key tiles (staged together), their results merged at the end - for grids that leave SMs
 // idle, where the serial chain of a row's key tiles is what the kernel takes. Output as a pair.
+//
+// OWN: nothing is known of the operands (the per-operator attention, whose rows may be of any size). Every query, key and
+// value row of the head gets its own power of two, found while it is staged; a key's returns with its scores and a value's
+// goes into the probabilities, which are scaled by the largest weighted value a query has met so far (rescaled with the
+// running maximum), so that a row is as accurate beside one 2^24 times its size as alone, and later rows leave no trace in
+// earlier ones. Output as FP32 rows: their own exponents span all heads.
 constexpr int kAttnPairLd = 72;  // halves per staged row: 144 bytes, so that the eight rows of an ldmatrix hit all banks
 
 __device__ __forceinline__ void mma_f16_16x8x16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -649,17 +655,24 @@ __device__ __forceinline__ uint32_t pair_word(float x, float y, uint32_t &lo) {
   return *reinterpret_cast<const uint32_t *>(&a);
 }
 
-constexpr size_t attn_pair_smem_bytes(int kg) { return (size_t)4 * kg * 64 * kAttnPairLd * 2; }
+constexpr size_t attn_pair_smem_bytes(int kg, bool own) { return (size_t)4 * kg * 64 * kAttnPairLd * 2 + (own ? (size_t)2 * kg * 64 * 4 : 0); }
 
-template <int WARPS, int KG>
+// Largest of the four lanes that share a row of an accumulator fragment.
+__device__ __forceinline__ float quad_max(float v) {
+  v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+  return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+}
+
+template <int WARPS, int KG, bool OWN>
 __global__ void __launch_bounds__(32 * WARPS * KG)
 attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__restrict__ kc,
                            const float *__restrict__ vc, int ldkv, size_t kv_seq_stride, int n_tok,
                            const int *__restrict__ pos, float scale, float s_qk, float s_v,
-                           __half *__restrict__ planes, size_t plane, int ldo, AttnScaleSrc src, int H, int wave) {
+                           __half *__restrict__ planes, size_t plane, float *__restrict__ out, int ldo, int H, int wave) {
   constexpr int HS = 64, TQ = 16 * WARPS, T = 64, LD = kAttnPairLd, NT = 32 * WARPS * KG;
   extern __shared__ __align__(16) __half attn_pair_smem[];
   __half *Ks = attn_pair_smem, *Vs = attn_pair_smem + 2 * KG * T * LD;  // [plane][KG tiles of T keys][LD]
+  float *kd = reinterpret_cast<float *>(Vs + 2 * KG * T * LD), *vd = kd + KG * T;  // OWN: 1 / scale of every staged row
   // The query tiles with the most keys first. While all CTAs are resident at once an SM gets one of every `wave` (the SM
   // count): every other wave goes through its tiles backwards, so that an SM with a long CTA gets a short one next.
   const int w_at = (int)blockIdx.x / wave * wave, w_r = (int)blockIdx.x - w_at;
@@ -673,12 +686,6 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
   pdl_wait();
   const int pos0 = pos ? __ldcg(pos) : 0;
   const int nq = min(TQ, n_tok - t0);
-  if (src.x_norm != nullptr) {  // no bounds known at load: the per-operator attention
-    const float2 sc = attn_pair_scales(src);
-    s_qk = sc.x;
-    s_v = sc.y;
-    if (h == 0 && tid < nq) src.o_descale[t0 + tid] = 1.f / s_v;
-  }
   const int last_key = pos0 + t0 + nq - 1;  // newest key any query of this tile may see
   const int r0 = 16 * warp + g, r1 = r0 + 8;
   const int p0 = pos0 + t0 + min(r0, nq - 1), p1 = pos0 + t0 + min(r1, nq - 1);  // rows past the end shadow the last
@@ -687,24 +694,39 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
 
   // ---- Q fragments: element (row, dim) pairs straight from global memory, once
   uint32_t qh[4][4], ql[4][4];
+  float s_q0 = s_qk, s_q1 = s_qk;
   {
     const float *q0 = q + ((size_t)seq * n_tok + t0 + min(r0, nq - 1)) * ldq + h * HS + 2 * t;
     const float *q1 = q + ((size_t)seq * n_tok + t0 + min(r1, nq - 1)) * ldq + h * HS + 2 * t;
+    float2 a[4], b[4], c[4], d[4];
+    float top0 = 0.f, top1 = 0.f;
 #pragma unroll
     for (int ks = 0; ks < 4; ks++) {
-      const float2 a = __ldcg(reinterpret_cast<const float2 *>(q0 + 16 * ks)), b = __ldcg(reinterpret_cast<const float2 *>(q1 + 16 * ks));
-      const float2 c = __ldcg(reinterpret_cast<const float2 *>(q0 + 16 * ks + 8)), d = __ldcg(reinterpret_cast<const float2 *>(q1 + 16 * ks + 8));
-      qh[ks][0] = pair_word(a.x * s_qk, a.y * s_qk, ql[ks][0]);
-      qh[ks][1] = pair_word(b.x * s_qk, b.y * s_qk, ql[ks][1]);
-      qh[ks][2] = pair_word(c.x * s_qk, c.y * s_qk, ql[ks][2]);
-      qh[ks][3] = pair_word(d.x * s_qk, d.y * s_qk, ql[ks][3]);
+      a[ks] = __ldcg(reinterpret_cast<const float2 *>(q0 + 16 * ks));
+      b[ks] = __ldcg(reinterpret_cast<const float2 *>(q1 + 16 * ks));
+      c[ks] = __ldcg(reinterpret_cast<const float2 *>(q0 + 16 * ks + 8));
+      d[ks] = __ldcg(reinterpret_cast<const float2 *>(q1 + 16 * ks + 8));
+      top0 = fmaxf(top0, fmaxf(fmaxf(fabsf(a[ks].x), fabsf(a[ks].y)), fmaxf(fabsf(c[ks].x), fabsf(c[ks].y))));
+      top1 = fmaxf(top1, fmaxf(fmaxf(fabsf(b[ks].x), fabsf(b[ks].y)), fmaxf(fabsf(d[ks].x), fabsf(d[ks].y))));
+    }
+    if (OWN) {
+      s_q0 = pair_scale_for(quad_max(top0));
+      s_q1 = pair_scale_for(quad_max(top1));
+    }
+#pragma unroll
+    for (int ks = 0; ks < 4; ks++) {
+      qh[ks][0] = pair_word(a[ks].x * s_q0, a[ks].y * s_q0, ql[ks][0]);
+      qh[ks][1] = pair_word(b[ks].x * s_q1, b[ks].y * s_q1, ql[ks][1]);
+      qh[ks][2] = pair_word(c[ks].x * s_q0, c[ks].y * s_q0, ql[ks][2]);
+      qh[ks][3] = pair_word(d[ks].x * s_q1, d[ks].y * s_q1, ql[ks][3]);
     }
   }
   const float *kb = kc + (size_t)seq * kv_seq_stride * ldkv + h * HS;
   const float *vb = vc + (size_t)seq * kv_seq_stride * ldkv + h * HS;
-  const float score_scale = scale / (s_qk * s_qk);
+  const float f0 = OWN ? scale / s_q0 : scale / (s_qk * s_qk), f1 = OWN ? scale / s_q1 : f0;  // OWN: times the key's
 
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+  float wt0 = 0.f, wt1 = 0.f, od0 = 1.f, od1 = 1.f;  // OWN: largest weighted value so far, 1 / scale of o
   float o[8][4];
 #pragma unroll
   for (int j = 0; j < 8; j++)
@@ -715,28 +737,43 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
   const uint32_t k_row = smem_addr(Ks) + 2u * (uint32_t)((kg * T + (lane & 7) + 8 * (lane >> 4)) * LD + 8 * ((lane >> 3) & 1));
   const uint32_t v_row = smem_addr(Vs) + 2u * (uint32_t)((kg * T + (lane & 15)) * LD + 8 * (lane >> 4));
   constexpr uint32_t kPlane = 2u * KG * T * LD;
+  static_assert(KG * T * (HS / 4) == 8 * NT, "eight float4 of K and of V per thread");
 
   for (int jb = 0; jb <= last_key; jb += KG * T) {
     const int j0 = jb + kg * T;
     __syncthreads();  // the previous tile is no longer read
     {
-      constexpr int PER = KG * T * (HS / 4) / NT;  // float4 of K (and of V) per thread
+      constexpr int PER = KG * T * (HS / 4) / NT;  // float4 of K (and of V) per thread: 8
+      // sixteen lanes to a row; OWN: four, each with a quarter of it, so that a row's maximum is two exchanges away
+      auto row_of = [&](int i) { return OWN ? (tid >> 2) + (NT / 4) * (i >> 2) : (tid + NT * i) >> 4; };
+      auto col_of = [&](int i) { return OWN ? ((tid & 3) + 4 * (i & 3)) * 4 : ((tid + NT * i) & 15) * 4; };
       float4 kv[PER], vv[PER];
 #pragma unroll
       for (int i = 0; i < PER; i++) {
-        const int idx = tid + NT * i, r = idx >> 4, c4 = (idx & 15) * 4;
-        const size_t at = (size_t)min(jb + r, last_key) * ldkv + c4;
+        const size_t at = (size_t)min(jb + row_of(i), last_key) * ldkv + col_of(i);
         kv[i] = __ldcg(reinterpret_cast<const float4 *>(kb + at));
         vv[i] = __ldcg(reinterpret_cast<const float4 *>(vb + at));
       }
+      float sk = s_qk, sv = s_v;
 #pragma unroll
       for (int i = 0; i < PER; i++) {
-        const int idx = tid + NT * i, r = idx >> 4, c4 = (idx & 15) * 4;
+        const int r = row_of(i), c4 = col_of(i);
+        if (OWN && (i & 3) == 0) {
+          float mk = 0.f, mv = 0.f;
+#pragma unroll
+          for (int u = i; u < i + 4; u++) {
+            mk = fmaxf(mk, fmaxf(fmaxf(fabsf(kv[u].x), fabsf(kv[u].y)), fmaxf(fabsf(kv[u].z), fabsf(kv[u].w))));
+            mv = fmaxf(mv, fmaxf(fmaxf(fabsf(vv[u].x), fabsf(vv[u].y)), fmaxf(fabsf(vv[u].z), fabsf(vv[u].w))));
+          }
+          sk = pair_scale_for(quad_max(mk));
+          sv = pair_scale_for(quad_max(mv));
+          if ((tid & 3) == 0) { kd[r] = 1.f / sk; vd[r] = 1.f / sv; }
+        }
         uint2 a, b;
-        pair_split4(scale4(kv[i], s_qk), a, b);
+        pair_split4(scale4(kv[i], sk), a, b);
         *reinterpret_cast<uint2 *>(Ks + r * LD + c4) = a;
         *reinterpret_cast<uint2 *>(Ks + (KG * T + r) * LD + c4) = b;
-        pair_split4(scale4(vv[i], s_v), a, b);
+        pair_split4(scale4(vv[i], sv), a, b);
         *reinterpret_cast<uint2 *>(Vs + r * LD + c4) = a;
         *reinterpret_cast<uint2 *>(Vs + (KG * T + r) * LD + c4) = b;
       }
@@ -770,9 +807,11 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
     const bool masked = j0 + T - 1 > pos0 + t0 + 16 * warp;  // same for the whole warp: some key is beyond some row
 #pragma unroll
     for (int j = 0; j < 8; j++) {
+      const float2 kf = OWN ? *reinterpret_cast<const float2 *>(kd + kg * T + 8 * j + 2 * t) : make_float2(1.f, 1.f);
 #pragma unroll
       for (int e = 0; e < 4; e++) {
-        s[j][e] *= score_scale;
+        const float f = e < 2 ? f0 : f1;
+        s[j][e] *= OWN ? f * (e & 1 ? kf.y : kf.x) : f;
         if (masked) {
           const int key = j0 + 8 * j + 2 * t + (e & 1);
           if (key > (e < 2 ? p0 : p1)) s[j][e] = -INFINITY;
@@ -781,13 +820,13 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
       mx0 = fmaxf(mx0, fmaxf(s[j][0], s[j][1]));
       mx1 = fmaxf(mx1, fmaxf(s[j][2], s[j][3]));
     }
-    mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1)); mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
-    mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
+    mx0 = quad_max(mx0);
+    mx1 = quad_max(mx1);
     float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);  // finite with KG == 1: every row sees key 0 of its first tile
     m0 = KG > 1 && mn0 == -INFINITY ? 0.f : m0;        // a row that has seen no key yet: everything below gives zero
     m1 = KG > 1 && mn1 == -INFINITY ? 0.f : m1;
     const float b0 = KG > 1 && mn0 == -INFINITY ? 0.f : mn0, b1 = KG > 1 && mn1 == -INFINITY ? 0.f : mn1;
-    const float c0 = expf(m0 - b0), c1 = expf(m1 - b1);
+    float c0 = expf(m0 - b0), c1 = expf(m1 - b1);
     float ps0 = 0.f, ps1 = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; j++) {
@@ -800,6 +839,25 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
     }
     l0 = l0 * c0 + ps0; m0 = mn0;  // l holds this lane's share of the row sum
     l1 = l1 * c1 + ps1; m1 = mn1;
+    float sp0 = kPairTop, sp1 = kPairTop;  // scale of the probabilities
+    if (OWN) {
+      float w0 = 0.f, w1 = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const float2 vf = *reinterpret_cast<const float2 *>(vd + kg * T + 8 * j + 2 * t);
+        s[j][0] *= vf.x; s[j][1] *= vf.y; s[j][2] *= vf.x; s[j][3] *= vf.y;
+        w0 = fmaxf(w0, fmaxf(s[j][0], s[j][1]));
+        w1 = fmaxf(w1, fmaxf(s[j][2], s[j][3]));
+      }
+      wt0 = fmaxf(wt0 * c0, quad_max(w0));
+      wt1 = fmaxf(wt1 * c1, quad_max(w1));
+      sp0 = pair_scale_for(wt0);
+      sp1 = pair_scale_for(wt1);
+      c0 = c0 * sp0 * od0;  // wt0 never falls below its share of the old one: c0 sp0 od0 is at most 2
+      c1 = c1 * sp1 * od1;
+      od0 = 1.f / sp0;
+      od1 = 1.f / sp1;
+    }
 #pragma unroll
     for (int j = 0; j < 8; j++) {
       o[j][0] *= c0; o[j][1] *= c0; o[j][2] *= c1; o[j][3] *= c1;
@@ -808,10 +866,10 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
 #pragma unroll
     for (int ks = 0; ks < 4; ks++) {
       uint32_t ph[4], pl[4];
-      ph[0] = pair_word(s[2 * ks][0] * kPairTop, s[2 * ks][1] * kPairTop, pl[0]);
-      ph[1] = pair_word(s[2 * ks][2] * kPairTop, s[2 * ks][3] * kPairTop, pl[1]);
-      ph[2] = pair_word(s[2 * ks + 1][0] * kPairTop, s[2 * ks + 1][1] * kPairTop, pl[2]);
-      ph[3] = pair_word(s[2 * ks + 1][2] * kPairTop, s[2 * ks + 1][3] * kPairTop, pl[3]);
+      ph[0] = pair_word(s[2 * ks][0] * sp0, s[2 * ks][1] * sp0, pl[0]);
+      ph[1] = pair_word(s[2 * ks][2] * sp1, s[2 * ks][3] * sp1, pl[1]);
+      ph[2] = pair_word(s[2 * ks + 1][0] * sp0, s[2 * ks + 1][1] * sp0, pl[2]);
+      ph[3] = pair_word(s[2 * ks + 1][2] * sp1, s[2 * ks + 1][3] * sp1, pl[3]);
 #pragma unroll
       for (int jp = 0; jp < 4; jp++) {
         uint32_t vh[4], vl[4];
@@ -827,7 +885,7 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
     }
   }
   if (KG > 1) {  // merge the groups' results, in group order
-    constexpr int REC = 36;
+    constexpr int REC = OWN ? 38 : 36;
     float *mg = reinterpret_cast<float *>(attn_pair_smem);  // [KG - 1][WARPS][REC][32]
     __syncthreads();
     if (kg > 0) {
@@ -837,6 +895,7 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
 #pragma unroll
         for (int e = 0; e < 4; e++) r[(4 * j + e) * 32] = o[j][e];
       r[32 * 32] = m0; r[33 * 32] = m1; r[34 * 32] = l0; r[35 * 32] = l1;
+      if (OWN) { r[36 * 32] = od0; r[37 * 32] = od1; }
     }
     __syncthreads();
     if (kg > 0) return;
@@ -845,10 +904,15 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
       const float *r = mg + (size_t)(k * WARPS + warp) * REC * 32 + lane;
       const float n0 = r[32 * 32], n1 = r[33 * 32];
       const float x0 = fmaxf(m0, n0), x1 = fmaxf(m1, n1);  // finite: group 0 has seen key 0
-      const float a0 = expf(m0 - x0), a1 = expf(m1 - x1), d0 = expf(n0 - x0), d1 = expf(n1 - x1);
+      float a0 = expf(m0 - x0), a1 = expf(m1 - x1), d0 = expf(n0 - x0), d1 = expf(n1 - x1);
       l0 = l0 * a0 + r[34 * 32] * d0;
       l1 = l1 * a1 + r[35 * 32] * d1;
       m0 = x0; m1 = x1;
+      if (OWN) {  // both in units of the larger one
+        const float g0 = r[36 * 32], g1 = r[37 * 32], u0 = fmaxf(od0, g0), u1 = fmaxf(od1, g1);
+        a0 *= od0 / u0; d0 *= g0 / u0; od0 = u0;
+        a1 *= od1 / u1; d1 *= g1 / u1; od1 = u1;
+      }
 #pragma unroll
       for (int j = 0; j < 8; j++) {
         o[j][0] = o[j][0] * a0 + r[(4 * j) * 32] * d0; o[j][1] = o[j][1] * a0 + r[(4 * j + 1) * 32] * d0;
@@ -859,6 +923,16 @@ attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__
   if (!warp_live) return;
   l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
   l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
+  if (OWN) {
+    const float i0 = 1.f / l0, i1 = 1.f / l1;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      float *at = out + ((size_t)seq * n_tok + t0 + r0) * ldo + h * HS + 8 * j + 2 * t;
+      if (r0 < nq) *reinterpret_cast<float2 *>(at) = make_float2(o[j][0] * i0 * od0, o[j][1] * i0 * od0);
+      if (r1 < nq) *reinterpret_cast<float2 *>(at + (size_t)8 * ldo) = make_float2(o[j][2] * i1 * od1, o[j][3] * i1 * od1);
+    }
+    return;
+  }
   // the values' own scale is also the output pair's
   const float i0 = 1.f / (l0 * kPairTop), i1 = 1.f / (l1 * kPairTop);
 #pragma unroll

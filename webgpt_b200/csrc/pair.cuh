@@ -187,7 +187,6 @@ struct PairOperands {
   int M, K;
   __half *xp;         // [2][M][K]
   float *x_descale;   // [M]
-  float *x_norm;      // [x_ctas] largest row norm of each CTA's rows, or nullptr
   int x_ctas;         // a multiple of the cluster size
   int block_rows;     // 1: a CTA per row (K <= 8192), 0: a warp per row
   // weights [K,N]
@@ -197,37 +196,29 @@ struct PairOperands {
   size_t plane[4];
   float *descale[4];  // [N]
   float *bias_out[4]; // [N] copy of bias (zero where there is none), or nullptr
-  float *norm[4];     // [ceil(N / 32)][2]: largest column norm, largest |bias| of 32 columns, or nullptr
 };
 
 __device__ __forceinline__ void pair_operand_rows(const PairOperands &p) {
-  __shared__ float red[2][8];
+  __shared__ float red[8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, K4 = p.K >> 2;
-  float top = 0.f;
   if (p.block_rows) {
     constexpr int V = 8;
     for (int row = blockIdx.x; row < p.M; row += p.x_ctas) {
       const float4 *x = reinterpret_cast<const float4 *>(p.x + (size_t)row * p.K);
       float4 v[V];
-      float m = 0.f, q = 0.f;
+      float m = 0.f;
 #pragma unroll
       for (int j = 0; j < V; j++) v[j] = tid + 256 * j < K4 ? __ldcg(x + tid + 256 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int j = 0; j < V; j++) {
-        m = fmaxf(m, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
-        q += dot4(v[j], v[j]);
-      }
+      for (int j = 0; j < V; j++) m = fmaxf(m, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
       m = warp_max(m);
-      q = warp_sum(q);
-      if (lane == 0) { red[0][warp] = m; red[1][warp] = q; }
+      if (lane == 0) red[warp] = m;
       __syncthreads();
-      m = 0.f; q = 0.f;
 #pragma unroll
-      for (int w = 0; w < 8; w++) { m = fmaxf(m, red[0][w]); q += red[1][w]; }
+      for (int w = 0; w < 8; w++) m = fmaxf(m, red[w]);
       __syncthreads();
       const float s = pair_scale_for(m);
       if (tid == 0) p.x_descale[row] = 1.f / s;
-      top = fmaxf(top, sqrtf(q));
       uint2 *o0 = reinterpret_cast<uint2 *>(p.xp + (size_t)row * p.K);
       uint2 *o1 = reinterpret_cast<uint2 *>(p.xp + ((size_t)p.M + row) * p.K);
 #pragma unroll
@@ -242,15 +233,13 @@ __device__ __forceinline__ void pair_operand_rows(const PairOperands &p) {
   } else {
     for (int row = blockIdx.x * 8 + warp; row < p.M; row += p.x_ctas * 8) {
       const float4 *x = reinterpret_cast<const float4 *>(p.x + (size_t)row * p.K);
-      float m = 0.f, q = 0.f;
+      float m = 0.f;
 #pragma unroll 8
       for (int i = lane; i < K4; i += 32) {
         const float4 v = __ldcg(x + i);
         m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-        q += dot4(v, v);
       }
       m = warp_max(m);
-      top = fmaxf(top, sqrtf(warp_sum(q)));
       const float s = pair_scale_for(m);
       if (lane == 0) p.x_descale[row] = 1.f / s;
       uint2 *o0 = reinterpret_cast<uint2 *>(p.xp + (size_t)row * p.K);
@@ -263,19 +252,14 @@ __device__ __forceinline__ void pair_operand_rows(const PairOperands &p) {
         o1[i] = b;
       }
     }
-    if (lane == 0) red[0][warp] = top;
-    __syncthreads();
-#pragma unroll
-    for (int w = 0; w < 8; w++) top = fmaxf(top, red[0][w]);
   }
-  if (p.x_norm != nullptr && tid == 0) p.x_norm[blockIdx.x] = top;
 }
 
 // grid = x_ctas + n_w ceil(N / 32) S, cluster (S,1,1), 256 threads; dynamic shared memory klen x 33 floats.
 __global__ void __launch_bounds__(256)
 pair_operands_kernel(const __grid_constant__ PairOperands p) {
   extern __shared__ __align__(16) float po_tile[];  // [klen][33]
-  __shared__ float own[2][32], stat[8][2][32], scl[32];
+  __shared__ float own[32], stat[8][32], scl[32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   pdl_launch_dependents();
   if ((int)blockIdx.x < p.x_ctas) {  // whole clusters
@@ -312,29 +296,22 @@ pair_operands_kernel(const __grid_constant__ PairOperands p) {
 #pragma unroll
   for (int i = 0; i < 4; i++) {
     const int c = 4 * warp + i;
-    float m = 0.f, q = 0.f;
+    float m = 0.f;
 #pragma unroll 4
-    for (int r = lane; r < kn; r += 32) {
-      const float v = po_tile[r * 33 + c];
-      m = fmaxf(m, fabsf(v));
-      q += v * v;
-    }
+    for (int r = lane; r < kn; r += 32) m = fmaxf(m, fabsf(po_tile[r * 33 + c]));
     m = warp_max(m);
-    q = warp_sum(q);
-    if (lane == 0) { own[0][c] = m; own[1][c] = q; }
+    if (lane == 0) own[c] = m;
   }
   __syncthreads();
   cluster_wait();  // every CTA of the cluster is running
-  if (tid < 64) {
-    const int c = tid & 31, h = tid >> 5;
-    for (int r = 0; r < (int)S; r++) dsmem_st(dsmem_addr(&stat[rank][h][c], (uint32_t)r), own[h][c]);
-  }
+  if (tid < 32)
+    for (int r = 0; r < (int)S; r++) dsmem_st(dsmem_addr(&stat[rank][tid], (uint32_t)r), own[tid]);
   cluster_arrive();
   cluster_wait();
   pdl_wait();  // what this kernel writes may still be read by earlier ones
   if (tid < 32) {
-    float m = 0.f, q = 0.f;
-    for (int r = 0; r < (int)S; r++) { m = fmaxf(m, stat[r][0][tid]); q += stat[r][1][tid]; }
+    float m = 0.f;
+    for (int r = 0; r < (int)S; r++) m = fmaxf(m, stat[r][tid]);
     const float s = pair_scale_for(m);
     scl[tid] = s;
     if (rank == 0) {
@@ -343,10 +320,6 @@ pair_operands_kernel(const __grid_constant__ PairOperands p) {
       if (n < p.N) {
         p.descale[wi][n] = 1.f / s;
         if (p.bias_out[wi] != nullptr) p.bias_out[wi][n] = b;
-      }
-      if (p.norm[wi] != nullptr) {
-        const float qm = warp_max(sqrtf(q)), bm = warp_max(fabsf(b));
-        if (tid == 0) { p.norm[wi][2 * blk] = qm; p.norm[wi][2 * blk + 1] = bm; }
       }
     }
   }
@@ -367,38 +340,6 @@ pair_operands_kernel(const __grid_constant__ PairOperands p) {
       o1[k2] = __floats2half2_rn(x - f.x, y - f.y);
     }
   }
-}
-
-// Bounds of an attention's queries / keys and values from what pair_operands_kernel left (|w x + b| <= |w| |x| + |b|), as
-// the powers of two they are scaled by. Every thread of the CTA gets them.
-struct AttnScaleSrc {
-  const float *x_norm;   // [x_ctas]
-  const float *w_norm;   // [3 blocks][2]: q | k | v blocks of 32 columns
-  int x_ctas, blocks;    // blocks: per matrix
-  float *o_descale;      // [rows]: 1 / (the values' scale), for the product that reads the attention's output
-};
-__device__ __forceinline__ float2 attn_pair_scales(const AttnScaleSrc &a) {
-  __shared__ float red[32][3];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
-  float x = 0.f, qk = 0.f, v = 0.f, bqk = 0.f, bv = 0.f;
-  for (int i = tid; i < a.x_ctas; i += blockDim.x) x = fmaxf(x, __ldcg(a.x_norm + i));
-  for (int i = tid; i < 3 * a.blocks; i += blockDim.x) {
-    const float2 w = __ldcg(reinterpret_cast<const float2 *>(a.w_norm) + i);
-    if (i < 2 * a.blocks) { qk = fmaxf(qk, w.x); bqk = fmaxf(bqk, w.y); }
-    else { v = fmaxf(v, w.x); bv = fmaxf(bv, w.y); }
-  }
-  x = warp_max(x);
-  if (lane == 0) red[warp][0] = x;
-  __syncthreads();
-  x = 0.f;
-  for (int w = 0; w < nw; w++) x = fmaxf(x, red[w][0]);
-  qk = warp_max(qk) * x + warp_max(bqk);  // >= every thread's own bound
-  v = warp_max(v) * x + warp_max(bv);
-  if (lane == 0) { red[warp][1] = qk; red[warp][2] = v; }
-  __syncthreads();
-  qk = 0.f; v = 0.f;
-  for (int w = 0; w < nw; w++) { qk = fmaxf(qk, red[w][1]); v = fmaxf(v, red[w][2]); }
-  return make_float2(pair_scale_for(1.01f * qk), pair_scale_for(1.01f * v));
 }
 
 }  // namespace wgpt
