@@ -210,9 +210,21 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 }
 
 // Cluster barrier (hardware; threads that have exited count as arrived). release/acquire order the
-// st.shared::cluster stores before it against the reads after it.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// st.shared::cluster stores before it against the reads after it. The .aligned forms want the warp's lanes together, which
+// a branch that some of them took just before does not promise.
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Arrival that publishes nothing.
+__device__ __forceinline__ void cluster_arrive_relaxed() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
 // Address of this CTA's shared-memory location p in CTA `cta` of the cluster.
 __device__ __forceinline__ uint32_t dsmem_addr(const void *p, uint32_t cta) {
   uint32_t r;

@@ -341,8 +341,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     }
   }
   if (S > 1) {  // no CTA leaves while another may still read its partial tile (nothing is published by this barrier)
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    cluster_arrive_relaxed();
     cluster_wait();
   } else {
     __syncthreads();

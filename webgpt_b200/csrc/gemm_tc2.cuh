@@ -25,6 +25,7 @@ constexpr uint32_t TC2_IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(
                                ((uint32_t)(256 >> 4) << 24);
 
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();  // see cluster_arrive
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

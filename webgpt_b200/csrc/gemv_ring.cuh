@@ -264,8 +264,7 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     }
   }
   if (S > 1) {  // no CTA leaves while another may still read its sums
-    __syncwarp();
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    cluster_arrive_relaxed();
     cluster_wait();
   }
 }
