@@ -202,6 +202,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32
   return done != 0;
 }
 
+// What a kernel does once a bounded wait of its has run out: one more bounded wait for the newest copy into each stage of a
+// ring, so that shared memory is not given up under a copy. `issued` copies went round `stages` stages, copy i arming
+// full[i % stages] for its phase i / stages; an earlier phase of a stage was over before the next copy into it was requested.
+// False: some copy had still not landed.
+__device__ __noinline__ bool ring_drain(uint64_t *full, int stages, int issued, uint32_t max_polls) {
+  bool landed = true;
+  for (int i = issued > stages ? issued - stages : 0; i < issued; i++)
+    landed = mbar_wait(&full[i % stages], (uint32_t)(i / stages) & 1u, max_polls) && landed;
+  return landed;
+}
+
 // Rank of this CTA inside its thread-block cluster.
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;

@@ -328,7 +328,7 @@ __global__ void wait_expiry_probe_kernel(const float *__restrict__ src16, int *e
   const bool first = mbar_wait(&bar, 0, polls);
   if (!first) atomicExch(err, 2);
   bulk_g2s(buf + 4, src16, 16, &bar);                 // the rest of the bytes the barrier was armed for
-  const bool second = mbar_wait(&bar, 0, 1u << 22);   // drain: bounded as well
+  const bool second = ring_drain(&bar, 1, 1, 1u << 22);  // as a ring of one stage: bounded as well
   observed[0] = first ? 1 : 0;
   observed[1] = second ? 1 : 0;
 }

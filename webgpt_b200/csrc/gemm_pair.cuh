@@ -132,6 +132,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   pdl_launch_dependents();
   pdl_wait();  // A (activations) comes from the previous kernel
 
+  int issued = 0;  // stages that thread 0 has requested
   if (warp == 0) {
     if (lane == 0) {
       const uint32_t stage_tx = 2u * (uint32_t)stage_bytes;  // both CTAs
@@ -146,6 +147,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           if (leader) mbar_expect_tx(&full[s], stage_tx);
           tma_load_3d_pair(st, &map_a, kb * GP_BK, m0, lead_full);
           tma_load_3d_pair(st + GP_A_BYTES, &map_b, kb * GP_BK, nb0, lead_full);
+          issued++;
           if (++s == S) { s = 0; phase ^= 1; }
         }
       }
@@ -231,7 +233,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   }
 
   __syncthreads();
-  if (threadIdx.x == 0 && *abort_flag) atomicExch(err, 3);
+  if (threadIdx.x == 0 && *abort_flag) {
+    atomicExch(err, 3);
+    pair_drain(full, S, issued, leader);
+  }
   cluster_sync_all();  // neither CTA leaves (or frees tensor memory) while the other may still signal it
   if (warp == 1) {
     tc_fence_after();

@@ -22,7 +22,8 @@
 // columns: the main products and the first correction side by side) and a second one adds the other correction to the
 // latter: two instructions per 16 of K instead of three, and the large and the small sums have accumulators of their own.
 // The slices of K are added in FP32, rounding to nearest.
-// Every wait is bounded; on expiry the CTA sets *err = 3 and carries on through its cluster barriers (the result is void).
+// Every wait is bounded; on expiry the CTA sets *err = 3, gives its copies in flight another bounded wait and carries on
+// through its cluster barriers (the result is void).
 #pragma once
 #include "gemm_pair.cuh"
 #include "split_plan.h"
@@ -127,6 +128,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   float2 *tile_st = reinterpret_cast<float2 *>(bet + nkb * (GP_BK / 4));  // [rows][x_tiles], as their producers left them
   const uint32_t tmem_cols = rn <= 16 ? 32u : (rn <= 32 ? 64u : (rn <= 64 ? 128u : 256u));
 
+  int issued_w = min(stages, nkb), issued_x = 0;  // thread 0's counts of requested stages
   if (threadIdx.x == 0) {
     for (int i = 0; i < stages; i++) {
       mbar_init(&full_w[i], 1);
@@ -137,7 +139,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     abort_word = 0;
     fence_async_smem();
     if (p.dyn) pdl_wait();
-    const int pre = min(stages, nkb);
+    const int pre = issued_w;
     for (int j = 0; j < pre; j++) {  // weights: ahead of the dependency wait
       mbar_expect_tx(&full_w[j], (uint32_t)w_bytes);
       tma_load_3d(tiles + (size_t)j * stage_bytes, &map_w, (kb0 + j) * GP_BK, f0, &full_w[j]);
@@ -189,10 +191,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
           if (*abort_flag || !mbar_wait(&empty[s], (use & 1) ^ 1, TC_POLLS)) { *abort_flag = 1; break; }
           mbar_expect_tx(&full_w[s], (uint32_t)w_bytes);
           tma_load_3d(st, &map_w, (kb0 + j) * GP_BK, f0, &full_w[s]);
+          issued_w = j + 1;
         }
         if (RN == 0) {
           mbar_expect_tx(&full_x[s], (uint32_t)rn * (GP_BK * 4));
           tma_load_3d(st + w_bytes, &map_x, (kb0 + j) * GP_BK, row0, &full_x[s]);
+          issued_x = j + 1;
         }
       }
     }
@@ -298,7 +302,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   } else {
     __syncthreads();
   }
-  if (threadIdx.x == 0 && *abort_flag) atomicExch(p.err, 3);
+  if (threadIdx.x == 0 && *abort_flag) {
+    atomicExch(p.err, 3);
+    ring_drain(full_w, stages, issued_w, TC_POLLS);
+    if (RN == 0) ring_drain(full_x, stages, issued_x, TC_POLLS);
+  }
 
   const int cnt = min(128, p.N - f0);
   const uint32_t pbase = smem_addr(part) + (uint32_t)lane * 16u;

@@ -225,10 +225,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   pdl_wait();  // A (activations) comes from the previous kernel
   if (warp == 0) TC_TRACE(2);
 
+  int kc = 0;  // TMA producer: k-blocks requested so far by this CTA: stage = kc % S, use = kc / S
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
-      int kc = 0;  // k-blocks issued so far by this CTA: stage = kc % S, use = kc / S
       for (int w = blockIdx.x; w < n_work && !*abort_flag; w += gridDim.x) {
         const TcWork t = tc_work(w, m_tiles, n_tiles, kb_per_split, total_kb);
         for (int kb = 0; kb < t.num_kb; kb++, kc++) {
@@ -432,7 +432,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
   __syncthreads();
   if (warp == 0) TC_TRACE(8);
-  if (threadIdx.x == 0 && *abort_flag) atomicExch(err, 3);
+  if (threadIdx.x == 0 && *abort_flag) {
+    atomicExch(err, 3);
+    ring_drain(full, S, kc > pre ? kc : pre, TC_POLLS);
+  }
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 2 * TC_BN);

@@ -71,6 +71,13 @@ __device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *m
       : "memory");
 }
 
+// ring_drain for copies of both CTAs that are counted on the leader's barriers. The other CTA cannot wait on those: it waits
+// out the limit on a barrier of its own that nobody arrives at, and neither leaves before both have done so.
+__device__ __forceinline__ void pair_drain(uint64_t *full, int stages, int issued, bool leader) {
+  if (leader) ring_drain(full, stages, issued, TC_POLLS);
+  else mbar_wait(&full[0], 0, TC_POLLS);
+}
+
 // gridDim.x = 2 x pairs, cluster (2,1,1). Pair p walks the 256 x 256 tiles p, p + pairs, ... (row tile fastest).
 template <bool X3>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(TcPlan<X3>::kThreads, 1)
@@ -121,17 +128,18 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   pdl_launch_dependents();
   pdl_wait();  // A (activations) comes from the previous kernel
 
+  int issued = 0;  // stages that thread 0 has requested
   if (warp == 0) {
     // ---------------- TMA producer: this CTA's 128 rows of A and 128 of the tile's 256 rows of Wt ----------------
     if (lane == 0) {
-      int kc = 0;
       for (int w = pair; w < n_work && !*abort_flag; w += pairs) {
         const int nt = w / m_tiles, mt = w - nt * m_tiles;
         const int m0 = mt * 256 + (int)rank * 128, nb0 = nt * TC2_BN + (int)rank * 128;
-        for (int kb = 0; kb < total_kb; kb++, kc++) {
-          const int s = kc % S, it = kc / S;
+        for (int kb = 0; kb < total_kb; kb++) {
+          const int s = issued % S, it = issued / S;
           uint8_t *st = tiles + (size_t)s * Plan::kStageBytes;
           if (*abort_flag || !mbar_wait(&empty[s], (it & 1) ^ 1, TC_POLLS)) { *abort_flag = 1; break; }
+          issued++;
           if (!X3) {
             // plain TF32: nothing in this CTA looks at the staged tiles, so both CTAs' loads are counted on the
             // leader's barrier (which expects the bytes of both) and no relay is needed
@@ -291,7 +299,11 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
   }
 
   __syncthreads();
-  if (threadIdx.x == 0 && *abort_flag) atomicExch(err, 3);
+  if (threadIdx.x == 0 && *abort_flag) {
+    atomicExch(err, 3);
+    if (X3) ring_drain(full, S, issued, TC_POLLS);  // each CTA counts its own
+    else pair_drain(full, S, issued, leader);
+  }
   cluster_sync_all();  // neither CTA leaves (or frees tensor memory) while the other may still signal it
   if (warp == 1) {
     tc_fence_after();

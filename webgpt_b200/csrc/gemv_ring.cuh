@@ -15,7 +15,7 @@
 //      otherwise as it is. Rows of this CTA's slice of K live in shared memory.
 //   S > 1 (long K with many rows, where every CTA staging all of x would cost more than the weights): the CTAs of a
 //      cluster take slices of K and their sums are added in rank order through distributed shared memory.
-// Every wait is bounded; on expiry *err = 2 and the result is void.
+// Every wait is bounded; on expiry *err = 2, the copies in flight get another bounded wait, and the result is void.
 #pragma once
 #include "gemm_tc.cuh"
 
@@ -129,8 +129,9 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   }
   __syncthreads();
   const uint32_t tx = (uint32_t)stage_floats * 4u;
+  int issued = min(p.stages, nch);  // the producer thread's count
   if (warp == GR_WARPS && lane == 0) {
-    const int pre = min(p.stages, nch);
+    const int pre = issued;
     for (int i = 0; i < pre; i++) {  // weights: ahead of the dependency wait
       mbar_expect_tx(&full[i], tx);
       tma_load_2d(ring + (size_t)i * stage_floats, &map_w, (ch0 + i) * GR_KT, col0, &full[i]);
@@ -164,6 +165,7 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         if (*abort_flag || !mbar_wait(&empty[s], ph, GR_POLLS)) { *abort_flag = 1; break; }
         mbar_expect_tx(&full[s], tx);
         tma_load_2d(ring + (size_t)s * stage_floats, &map_w, (ch0 + i) * GR_KT, col0, &full[s]);
+        issued = i + 1;
         if (++s == p.stages) { s = 0; ph ^= 1; }
       }
     }
@@ -240,7 +242,10 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   } else {
     __syncthreads();
   }
-  if (tid == 0 && *abort_flag) atomicExch(p.err, 2);
+  if (tid == 32 * GR_WARPS && *abort_flag) {
+    atomicExch(p.err, 2);
+    ring_drain(full, p.stages, issued, GR_POLLS);
+  }
   // outputs: column fastest, so that a warp stores runs of a row; a cluster's CTAs share them
   for (int o = o_first; o < p.ft * p.rows; o += (int)S * GR_THREADS) {
     const int m = o / p.ft, c = o - m * p.ft;
