@@ -197,6 +197,28 @@ def test_decode_rows(model64, n_seq):
         assert rel_err(lg[i], m.run(np.concatenate([prompts[i], got[i, :1]]))) < 2e-5
 
 
+def test_int8_handle_memory(dev):
+    """Two bytes per code until a call of more than 16 rows wants the codes in half precision, then four; a handle of decode
+    rows stays at two, and all of it comes back."""
+    from webgpt_b200 import _lib
+    K, N = 4096, 16384
+    p_d, s_d = dev.tensor(np.zeros((K, N // 4), np.uint32)), dev.tensor(np.ones(N, np.float32))
+    a_d, o_d = dev.buffer(17 * K * 4), dev.buffer(17 * N * 4)
+    h = C.c_void_p()
+    for rows in (1, 16, 17):  # workspaces and code are in place from here on
+        _lib.call("wgpt_int8_weight_create", dev.handle, K, N, p_d.ptr, s_d.ptr, C.byref(h))
+        _lib.call("wgpt_int8_matmul_w", dev.handle, rows, h, a_d.ptr, o_d.ptr)
+        _lib.call("wgpt_int8_weight_destroy", h)
+    free = dev.mem_info()[0]
+    _lib.call("wgpt_int8_weight_create", dev.handle, K, N, p_d.ptr, s_d.ptr, C.byref(h))
+    slack = 4 << 20
+    for rows, per_code in ((1, 2), (16, 2), (17, 4)):
+        _lib.call("wgpt_int8_matmul_w", dev.handle, rows, h, a_d.ptr, o_d.ptr)
+        assert abs(free - dev.mem_info()[0] - per_code * K * N) < slack, rows
+    _lib.call("wgpt_int8_weight_destroy", h)
+    assert abs(free - dev.mem_info()[0]) < slack
+
+
 @pytest.fixture(scope="module")
 def model8(oracle):
     """Head size 8: a head's output is a quarter of a warp."""
