@@ -101,6 +101,29 @@ def test_products_of_integers_are_exact(dev, M, K, N):
     assert np.array_equal(matmul(dev, A, W, b).astype(np.float64), A.astype(np.float64) @ W + b)
 
 
+@pytest.mark.parametrize("M,K,N", [(33, 3072, 136), (64, 6400, 136), (128, 6400, 264), (257, 3080, 72), (600, 1600, 520)])
+def test_products_of_long_integers_are_exact(dev, M, K, N):
+    """Thirteen-bit integers take both planes and their sums against -1, 0 and 1 stay exact in FP32: a correction product
+    that goes missing in any stage of the ring, k-block or slice of a long K shows, from either side."""
+    rng = np.random.default_rng(M + K)
+    big = lambda *s: (rng.integers(4097, 4103, s) * rng.choice((-1, 1), s)).astype(np.float32)  # noqa: E731
+    unit = lambda *s: rng.integers(-1, 2, s).astype(np.float32)  # noqa: E731
+    for A, W in ((big(M, K), unit(K, N)), (unit(M, K), big(K, N))):
+        assert np.array_equal(matmul(dev, A, W).astype(np.float64), A.astype(np.float64) @ W)
+    # the same rows against codes of one plane
+    from webgpt_b200 import _lib
+    A, q = big(M, K), unit(K, N).astype(np.int8)
+    if K % 16 == 0:
+        h = C.c_void_p()
+        p_d, s_d = dev.tensor(q.view(np.uint32)), dev.tensor(np.ones(N, np.float32))
+        a_d, o_d = dev.tensor(A), dev.buffer(M * N * 4)
+        _lib.call("wgpt_int8_weight_create", dev.handle, K, N, p_d.ptr, s_d.ptr, C.byref(h))
+        _lib.call("wgpt_int8_matmul_w", dev.handle, M, h, a_d.ptr, o_d.ptr)
+        got = o_d.read(np.float32, M * N).reshape(M, N)
+        _lib.call("wgpt_int8_weight_destroy", h)
+        assert np.array_equal(got.astype(np.float64), A.astype(np.float64) @ q)
+
+
 @pytest.mark.parametrize("T,E,H", [(32, 128, 2), (63, 64, 1), (65, 128, 2), (128, 192, 3), (129, 128, 2), (200, 128, 4),
                                    (321, 64, 1)])
 def test_attention_operator_on_pairs(dev, oracle, T, E, H):
