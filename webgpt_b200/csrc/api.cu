@@ -311,8 +311,8 @@ WGPT_EXPORT int32_t wgpt_device_create(int32_t ordinal, wgpt_device **out) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     dev->max_clusters[S] = 0;
-    if (allow_smem(dev, gemm_split_kernel<0>) == cudaSuccess)
-      cudaOccupancyMaxActiveClusters(&dev->max_clusters[S], gemm_split_kernel<0>, &cfg);
+    if (allow_smem(dev, gemm_split_kernel<0, false>) == cudaSuccess)
+      cudaOccupancyMaxActiveClusters(&dev->max_clusters[S], gemm_split_kernel<0, false>, &cfg);
   }
   *out = dev;
   return WGPT_OK;
@@ -1079,16 +1079,17 @@ static int32_t launch_gemm_split(wgpt_device *dev, const SplitShape &sh, const _
   mx = mw;
   if (X != nullptr) TRY(make_pair_map(&mx, X, (uint64_t)M, (uint64_t)K, sh.rn));
   const dim3 grid(sh.row_tiles * a.f_tiles * sh.S);
-#define SPLIT_CASE(RNV)                                                                                              \
+#define SPLIT_CASE(...)                                                                                              \
   do {                                                                                                               \
-    CK(allow_smem(dev, gemm_split_kernel<RNV>));                                                                       \
-    CK(launch_ex_x(dev->pdl, sh.S, dev->stream, gemm_split_kernel<RNV>, grid, dim3(GS_THREADS), sh.smem, mw, mx, a)); \
+    CK(allow_smem(dev, gemm_split_kernel<__VA_ARGS__>));                                                                       \
+    CK(launch_ex_x(dev->pdl, sh.S, dev->stream, (gemm_split_kernel<__VA_ARGS__>), grid, dim3(GS_THREADS), sh.smem, mw, mx, a)); \
   } while (0)
-  if (X != nullptr) SPLIT_CASE(0);
-  else if (sh.rn == 16) SPLIT_CASE(16);
-  else if (sh.rn == 32) SPLIT_CASE(32);
-  else if (sh.rn == 48) SPLIT_CASE(48);
-  else if (sh.rn == 64) SPLIT_CASE(64);
+  if (X != nullptr && (a.dyn || epi.rowscale != nullptr)) SPLIT_CASE(0, true);
+  else if (X != nullptr) SPLIT_CASE(0, false);
+  else if (sh.rn == 16) SPLIT_CASE(16, false);
+  else if (sh.rn == 32) SPLIT_CASE(32, false);
+  else if (sh.rn == 48) SPLIT_CASE(48, false);
+  else if (sh.rn == 64) SPLIT_CASE(64, false);
   else return fail(WGPT_ERR_SHAPE, "no normalising product for row tiles of %d", sh.rn);
 #undef SPLIT_CASE
   dev->launches++;

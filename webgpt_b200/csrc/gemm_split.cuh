@@ -99,8 +99,9 @@ __device__ __forceinline__ float2 merge_row_stats(const float2 *st, int tiles, i
 }
 
 // grid.x = row tiles x feature tiles x S, cluster (S, 1, 1). map_w: box of 128 rows; map_x (RN == 0): box of rn rows.
-// RN == 0: activations as planes by TMA, rn at run time. RN > 0: normalised on the way in, rn == RN.
-template <int RN>
+// RN == 0: activations as planes by TMA, rn at run time. RN > 0: normalised on the way in, rn == RN. OP: a per-operator
+// product, with row factors and, where p.dyn says so, a weight that the previous kernel wrote.
+template <int RN, bool OP>
 __global__ void __launch_bounds__(GS_THREADS, 2)
 gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                   const __grid_constant__ SplitArgs p) {
@@ -108,7 +109,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   uint8_t *tiles = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(gs_smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ uint64_t full_w[GS_MAX_STAGES], full_x[GS_MAX_STAGES], empty[GS_MAX_STAGES], acc_full;
   __shared__ uint32_t tmem_slot;
-  __shared__ int abort_word;
+  __shared__ int abort_word, requested;  // requested: k-blocks, as the producer leaves it
   __shared__ float2 row_norm[RN > 0 ? RN : 1];
   volatile int *abort_flag = &abort_word;
   float *part = reinterpret_cast<float *>(tiles);  // [rn][128], over the ring once its last tile has been read
@@ -128,7 +129,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   float2 *tile_st = reinterpret_cast<float2 *>(bet + nkb * (GP_BK / 4));  // [rows][x_tiles], as their producers left them
   const uint32_t tmem_cols = rn <= 16 ? 32u : (rn <= 32 ? 64u : (rn <= 64 ? 128u : 256u));
 
-  int issued_w = min(stages, nkb), issued_x = 0;  // thread 0's counts of requested stages
   if (threadIdx.x == 0) {
     for (int i = 0; i < stages; i++) {
       mbar_init(&full_w[i], 1);
@@ -138,8 +138,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
     mbar_init(&acc_full, 1);
     abort_word = 0;
     fence_async_smem();
-    if (p.dyn) pdl_wait();
-    const int pre = issued_w;
+    if (OP && p.dyn) pdl_wait();
+    const int pre = min(stages, nkb);
+    requested = nkb;
     for (int j = 0; j < pre; j++) {  // weights: ahead of the dependency wait
       mbar_expect_tx(&full_w[j], (uint32_t)w_bytes);
       tma_load_3d(tiles + (size_t)j * stage_bytes, &map_w, (kb0 + j) * GP_BK, f0, &full_w[j]);
@@ -164,7 +165,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   const bool n_live = n < p.N;
   float4 cs = make_float4(1.f, 1.f, 1.f, 1.f), bs = make_float4(0.f, 0.f, 0.f, 0.f);
   pdl_launch_dependents();
-  if (p.dyn) pdl_wait();
+  if (OP && p.dyn) pdl_wait();
   if (n_live && e.colscale != nullptr) cs = __ldcg(reinterpret_cast<const float4 *>(e.colscale + n));
   if (n_live && e.bias != nullptr) bs = __ldcg(reinterpret_cast<const float4 *>(e.bias + n));
   pdl_wait();  // the activations come from the previous kernel
@@ -188,15 +189,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const int s = j % stages, use = j / stages;
         uint8_t *st = tiles + (size_t)s * stage_bytes;
         if (j >= stages) {
-          if (*abort_flag || !mbar_wait(&empty[s], (use & 1) ^ 1, TC_POLLS)) { *abort_flag = 1; break; }
+          if (*abort_flag || !mbar_wait(&empty[s], (use & 1) ^ 1, TC_POLLS)) { *abort_flag = 1; requested = j; break; }
           mbar_expect_tx(&full_w[s], (uint32_t)w_bytes);
           tma_load_3d(st, &map_w, (kb0 + j) * GP_BK, f0, &full_w[s]);
-          issued_w = j + 1;
         }
         if (RN == 0) {
           mbar_expect_tx(&full_x[s], (uint32_t)rn * (GP_BK * 4));
           tma_load_3d(st + w_bytes, &map_x, (kb0 + j) * GP_BK, row0, &full_x[s]);
-          issued_x = j + 1;
         }
       }
     }
@@ -302,11 +301,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   } else {
     __syncthreads();
   }
-  if (threadIdx.x == 0 && *abort_flag) {
-    atomicExch(p.err, 3);
-    ring_drain(full_w, stages, issued_w, TC_POLLS);
-    if (RN == 0) ring_drain(full_x, stages, issued_x, TC_POLLS);
-  }
+  if (threadIdx.x == 0 && *abort_flag) atomicExch(p.err, 3);
 
   const int cnt = min(128, p.N - f0);
   const uint32_t pbase = smem_addr(part) + (uint32_t)lane * 16u;
@@ -339,7 +334,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
       for (int s = 1; s < 8; s++)
         if (s < (int)S) v = add4(v, q[u][s]);
       if (n_live) {
-        v = pair_epi_value4(e, v, cs, bs, res[u], m);
+        v = pair_epi_value4(e, v, cs, bs, res[u], m, OP);
         pair_epi_store4(e, v, m, n);
       }
       if (p.stats != nullptr) {
@@ -357,6 +352,11 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_acc, tmem_cols);
+  }
+  // here, where nothing else is in registers (ahead of the epilogue: prompts of 21 tokens 431 -> 446 us, XL 64 3.06 -> 3.18 ms)
+  if (threadIdx.x == 0 && *abort_flag) {
+    ring_drain(full_w, stages, requested, TC_POLLS);
+    if (RN == 0) ring_drain(full_x, stages, requested, TC_POLLS);
   }
 }
 

@@ -59,10 +59,13 @@ __device__ __forceinline__ float4 pair_descale4(float4 v, float rs, float4 cs) {
 }
 
 // Epilogue of the kernels that multiply pairs: four raw sums of row m, columns n..n+3, with the columns' constants and
-// the residual already in registers -> the finished values, and their store.
-__device__ __forceinline__ float4 pair_epi_value4(const Epilogue &e, float4 v, float4 cs, float4 bs, float4 res, int m) {
-  v = e.rowscale != nullptr ? add4(pair_descale4(v, __ldcg(e.rowscale + m), cs), bs)
-                            : make_float4(v.x * cs.x + bs.x, v.y * cs.y + bs.y, v.z * cs.z + bs.z, v.w * cs.w + bs.w);
+// the residual already in registers -> the finished values, and their store. `rows`: the product may have row factors (a
+// model's have none, and kernels made for them leave the branch out).
+__device__ __forceinline__ float4 pair_epi_value4(const Epilogue &e, float4 v, float4 cs, float4 bs, float4 res, int m, bool rows) {
+  if (rows && e.rowscale != nullptr)
+    v = add4(pair_descale4(v, __ldcg(e.rowscale + m), cs), bs);
+  else
+    v = make_float4(v.x * cs.x + bs.x, v.y * cs.y + bs.y, v.z * cs.z + bs.z, v.w * cs.w + bs.w);
   if (e.act == 1) v = make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
   return make_float4(v.x + res.x, v.y + res.y, v.z + res.z, v.w + res.w);
 }
@@ -79,7 +82,8 @@ __device__ __forceinline__ void pair_epi_store4(const Epilogue &e, float4 v, int
 }
 // The same for 32 rows of a 32-column block held in `pad` (row stride 33): this lane finishes columns n..n+3 (block
 // columns col4..col4+3) of rows row0 + 4 it + sub_r. Without an activation the residuals of all its rows are requested
-// together (one row at a time, the epilogue is a chain of L2 round trips longer than the MMAs it has to hide behind);
+// together (one row at a time, the epilogue is a chain of L2 round trips longer than the MMAs it has to hide behind), or the
+// row factors of a per-operator product, which has no residual (one loop for both took a model's products 0.5 to 1 %);
 // with one, the loop stays rolled: 32 inlined GELUs per block made the kernel miss in the instruction cache at every
 // step (36 000 cycles per tile instead of 18 000).
 __device__ __forceinline__ void pair_epi_block(const Epilogue &e, const float *pad, int row0, int sub_r, int col4, int n,
@@ -87,7 +91,7 @@ __device__ __forceinline__ void pair_epi_block(const Epilogue &e, const float *p
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
   const float4 cs = e.colscale != nullptr ? __ldcg(reinterpret_cast<const float4 *>(e.colscale + n)) : make_float4(1.f, 1.f, 1.f, 1.f);
   const float4 bs = e.bias != nullptr ? __ldg(reinterpret_cast<const float4 *>(e.bias + n)) : zero4;
-  if (e.act == 0 && e.pair == nullptr) {
+  if (e.act == 0 && e.pair == nullptr && e.rowscale == nullptr) {
     float4 res[8];
 #pragma unroll
     for (int it = 0; it < 8; it++) {
@@ -101,9 +105,21 @@ __device__ __forceinline__ void pair_epi_block(const Epilogue &e, const float *p
       const float *src = pad + r * 33 + col4;
       float4 v = make_float4(src[0], src[1], src[2], src[3]);
       if (m >= M) continue;
-      v = e.rowscale != nullptr ? add4(pair_descale4(v, __ldcg(e.rowscale + m), cs), bs)
-                                : make_float4(v.x * cs.x + bs.x, v.y * cs.y + bs.y, v.z * cs.z + bs.z, v.w * cs.w + bs.w);
-      *reinterpret_cast<float4 *>(epi_addr(e, m, n)) = add4(v, res[it]);
+      *reinterpret_cast<float4 *>(epi_addr(e, m, n)) =
+          make_float4(v.x * cs.x + bs.x + res[it].x, v.y * cs.y + bs.y + res[it].y, v.z * cs.z + bs.z + res[it].z,
+                      v.w * cs.w + bs.w + res[it].w);
+    }
+  } else if (e.act == 0 && e.pair == nullptr && e.residual == nullptr) {
+    float rs[8];
+#pragma unroll
+    for (int it = 0; it < 8; it++) rs[it] = row0 + it * 4 + sub_r < M ? __ldcg(e.rowscale + row0 + it * 4 + sub_r) : 0.f;
+#pragma unroll
+    for (int it = 0; it < 8; it++) {
+      const int r = it * 4 + sub_r, m = row0 + r;
+      const float *src = pad + r * 33 + col4;
+      if (m >= M) continue;
+      *reinterpret_cast<float4 *>(epi_addr(e, m, n)) =
+          add4(pair_descale4(make_float4(src[0], src[1], src[2], src[3]), rs[it], cs), bs);
     }
   } else {
 #pragma unroll 1
@@ -112,7 +128,7 @@ __device__ __forceinline__ void pair_epi_block(const Epilogue &e, const float *p
       if (m >= M) break;
       const float *src = pad + r * 33 + col4;
       const float4 res = e.residual != nullptr ? __ldcg(reinterpret_cast<const float4 *>(e.residual + (size_t)m * e.ld + n)) : zero4;
-      pair_epi_store4(e, pair_epi_value4(e, make_float4(src[0], src[1], src[2], src[3]), cs, bs, res, m), m, n);
+      pair_epi_store4(e, pair_epi_value4(e, make_float4(src[0], src[1], src[2], src[3]), cs, bs, res, m, true), m, n);
     }
   }
 }
