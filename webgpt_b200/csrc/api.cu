@@ -1213,17 +1213,18 @@ static int32_t launch_attn_prefill_pair(wgpt_device *dev, const float *q, int ld
                                         int ldkv, size_t kv_seq_stride, int n_tok, int n_seq, int H, const int *pos,
                                         float scale, float s_qk, float s_v, __half *planes, size_t plane, int ldo,
                                         float *own_out = nullptr) {
-  // Two groups of warps per 64 query rows, alternating key tiles, while all CTAs are resident at once, up to three per SM
-  // (GPT-2 at 333 / 1024 tokens 0.85 / 1.64 ms per pass against 1.00 / 1.95 with one group; with the CTAs' order balanced over
-  // the SMs 1024 tokens take 1.55, XL 12.15 against 12.5, and XL with one group 12.8); one group beyond that (64 x 128 tokens,
-  // 1536 CTAs: 4.46 against 4.8 ms) and for a single tile.
+  // Two groups of warps per 64 query rows, alternating key tiles, halve the chain of key tiles that a row's softmax is, and
+  // cost an SM warps: one CTA of eight (186 registers a thread) against three CTAs of four (168). ms per pass with one / two
+  // groups: GPT-2 333 tokens (72 CTAs) 0.96 / 0.80, 1024 (192) 1.93 / 1.42, XL 512 (200) 7.70 / 6.84, 1024 (400) 12.66 / 11.33;
+  // 16 x 96 tokens of XL (800) 13.0 / 14.2, 64 x 128 of GPT-2 (1536) 4.5 / 4.95. The line of three CTAs per SM lies between.
+  // A single tile has one key tile.
   const long long ctas = (long long)((n_tok + 63) / 64) * H * n_seq;
 #define PAIR_ATTN(W, G, OWN)                                                                                               \
   do {                                                                                                                   \
     CK(allow_smem(dev, attn_prefill64_pair_kernel<W, G, OWN>));                                                            \
     LAUNCH_PDL(dev, (attn_prefill64_pair_kernel<W, G, OWN>), (n_tok + 16 * W - 1) / (16 * W) * H * n_seq, 32 * W * G,      \
                attn_pair_smem_bytes(G, OWN), q, ldq, kc, vc, ldkv, kv_seq_stride, n_tok, pos, scale, s_qk, s_v, planes,    \
-               plane, own_out, ldo, H, dev->sm_count);                                                                   \
+               plane, own_out, ldo, H);                                                                                  \
   } while (0)
   const bool two = n_tok > 64 && ctas <= 3 * dev->sm_count;
   if (own_out != nullptr) {

@@ -668,15 +668,13 @@ __global__ void __launch_bounds__(32 * WARPS * KG)
 attn_prefill64_pair_kernel(const float *__restrict__ q, int ldq, const float *__restrict__ kc,
                            const float *__restrict__ vc, int ldkv, size_t kv_seq_stride, int n_tok,
                            const int *__restrict__ pos, float scale, float s_qk, float s_v,
-                           __half *__restrict__ planes, size_t plane, float *__restrict__ out, int ldo, int H, int wave) {
+                           __half *__restrict__ planes, size_t plane, float *__restrict__ out, int ldo, int H) {
   constexpr int HS = 64, TQ = 16 * WARPS, T = 64, LD = kAttnPairLd, NT = 32 * WARPS * KG;
   extern __shared__ __align__(16) __half attn_pair_smem[];
   __half *Ks = attn_pair_smem, *Vs = attn_pair_smem + 2 * KG * T * LD;  // [plane][KG tiles of T keys][LD]
   float *kd = reinterpret_cast<float *>(Vs + 2 * KG * T * LD), *vd = kd + KG * T;  // OWN: 1 / scale of every staged row
-  // The query tiles with the most keys first. While all CTAs are resident at once an SM gets one of every `wave` (the SM
-  // count): every other wave goes through its tiles backwards, so that an SM with a long CTA gets a short one next.
-  const int w_at = (int)blockIdx.x / wave * wave, w_r = (int)blockIdx.x - w_at;
-  const int order = ((int)blockIdx.x / wave) & 1 ? w_at + min(wave, (int)gridDim.x - w_at) - 1 - w_r : (int)blockIdx.x;
+  // The query tiles with the most keys first: an SM takes its next CTA when one of its own ends, so the short ones fill up.
+  const int order = (int)blockIdx.x;
   const int n_tiles = (n_tok + TQ - 1) / TQ, heads = (int)gridDim.x / n_tiles, hq = order % heads;
   const int h = hq % H, seq = hq / H;
   const int t0 = (n_tiles - 1 - order / heads) * TQ;
