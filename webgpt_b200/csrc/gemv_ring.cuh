@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(GR_THREADS, 1)
 gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ RingArgs p) {
   extern __shared__ uint8_t gr_smem_raw[];
   __shared__ uint64_t full[GR_MAX_STAGES], empty[GR_MAX_STAGES];
-  __shared__ int abort_word, requested;  // requested: stages, as the producer leaves it
+  __shared__ int abort_word;
   __shared__ float ln_red[16];
   volatile int *abort_flag = &abort_word;
   float *ring = reinterpret_cast<float *>((reinterpret_cast<uintptr_t>(gr_smem_raw) + 127) & ~uintptr_t(127));
@@ -129,9 +129,9 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   }
   __syncthreads();
   const uint32_t tx = (uint32_t)stage_floats * 4u;
+  int issued = min(p.stages, nch);  // the producer thread's count
   if (warp == GR_WARPS && lane == 0) {
-    const int pre = min(p.stages, nch);
-    requested = nch;
+    const int pre = issued;
     for (int i = 0; i < pre; i++) {  // weights: ahead of the dependency wait
       mbar_expect_tx(&full[i], tx);
       tma_load_2d(ring + (size_t)i * stage_floats, &map_w, (ch0 + i) * GR_KT, col0, &full[i]);
@@ -162,9 +162,10 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   if (warp == GR_WARPS) {
     if (lane == 0) {
       for (int i = p.stages, s = 0, ph = 0; i < nch; i++) {
-        if (*abort_flag || !mbar_wait(&empty[s], ph, GR_POLLS)) { *abort_flag = 1; requested = i; break; }
+        if (*abort_flag || !mbar_wait(&empty[s], ph, GR_POLLS)) { *abort_flag = 1; break; }
         mbar_expect_tx(&full[s], tx);
         tma_load_2d(ring + (size_t)s * stage_floats, &map_w, (ch0 + i) * GR_KT, col0, &full[s]);
+        issued = i + 1;
         if (++s == p.stages) { s = 0; ph ^= 1; }
       }
     }
@@ -241,7 +242,10 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   } else {
     __syncthreads();
   }
-  if (tid == 0 && *abort_flag) atomicExch(p.err, 2);
+  if (tid == 32 * GR_WARPS && *abort_flag) {
+    atomicExch(p.err, 2);
+    ring_drain(full, p.stages, issued, GR_POLLS);
+  }
   // outputs: column fastest, so that a warp stores runs of a row; a cluster's CTAs share them
   for (int o = o_first; o < p.ft * p.rows; o += (int)S * GR_THREADS) {
     const int m = o / p.ft, c = o - m * p.ft;
@@ -268,7 +272,6 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     cluster_arrive_relaxed();
     cluster_wait();
   }
-  if (tid == 0 && *abort_flag) ring_drain(full, p.stages, requested, GR_POLLS);
 }
 
 }  // namespace wgpt
