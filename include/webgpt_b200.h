@@ -207,11 +207,11 @@ int32_t wgpt_int8_matmul(wgpt_device *dev, int32_t M, int32_t K, int32_t N, cons
 /* The prototype's load step for a weight that is used many times (it uploads the packed matrix once and then
  * dispatches against it, other/int8-gemm.js:101-113): the handle owns a copy of Bq [K, N/4] and scale [N] (both
  * device memory) and, when K % 16 == 0, a re-laid-out copy with each output column's codes contiguous, which the
- * kernels stream with 128-bit loads: two bytes per code. wgpt_int8_matmul_w computes what wgpt_int8_matmul computes,
- * out[M,N] = A[M,K] . (f32(q) * scale[n]): up to 16 rows by a weight-streaming kernel, 8 rows a launch, more than 16 rows on
- * the tensor cores (device precision mode), otherwise through wgpt_int8_matmul. The first call of more than 16 rows adds a
- * half-precision copy of the codes to the handle, two more bytes per code; make it before recording a pass list or calls
- * that must not allocate (while recording, and where the memory is not there, the call runs without that copy). */
+ * kernels stream with 128-bit loads, and a copy as half-precision values for the tensor cores: four bytes per code, or two
+ * without the latter (WGPT_INT8_HALVES=0 in the environment, or where the memory is not there), which makes calls of more
+ * than 16 rows slower. wgpt_int8_matmul_w computes what wgpt_int8_matmul computes, out[M,N] = A[M,K] . (f32(q) * scale[n]):
+ * up to 16 rows by a weight-streaming kernel, 8 rows a launch, more than 16 rows on the tensor cores (device precision mode),
+ * otherwise through wgpt_int8_matmul. */
 typedef struct wgpt_int8_weight wgpt_int8_weight;
 int32_t wgpt_int8_weight_create(wgpt_device *dev, int32_t K, int32_t N, const uint32_t *Bq, const float *scale,
                                 wgpt_int8_weight **out);

@@ -220,26 +220,35 @@ def test_decode_rows(model64, n_seq):
         assert rel_err(lg[i], m.run(np.concatenate([prompts[i], got[i, :1]]))) < 2e-5
 
 
-def test_int8_handle_memory(dev):
-    """Two bytes per code until a call of more than 16 rows wants the codes in half precision, then four; a handle of decode
-    rows stays at two, and all of it comes back."""
+@pytest.mark.parametrize("halves,per_code", [("1", 4), ("0", 2)])
+def test_int8_handle_memory(dev, monkeypatch, halves, per_code):
+    """Four bytes per code, or two without the half-precision copy, for any number of rows; all of it comes back, and both
+    forms agree with the codes (bounds as in test_int8_handle_rows, of the less precise of two splits)."""
     from webgpt_b200 import _lib
-    K, N = 4096, 16384
-    p_d, s_d = dev.tensor(np.zeros((K, N // 4), np.uint32)), dev.tensor(np.ones(N, np.float32))
-    a_d, o_d = dev.buffer(17 * K * 4), dev.buffer(17 * N * 4)
+    monkeypatch.setenv("WGPT_INT8_HALVES", halves)
+    K, N, M = 4096, 16384, 40
+    rng = np.random.default_rng(4)
+    q, scale = rng.integers(-127, 128, (K, N), dtype=np.int8), np.full(N, 0.5, np.float32)
+    A = rng.standard_normal((M, K), dtype=np.float32)
+    p_d, s_d, a_d, o_d = dev.tensor(q.view(np.uint32)), dev.tensor(scale), dev.tensor(A), dev.buffer(M * N * 4)
     h = C.c_void_p()
-    for rows in (1, 16, 17):  # workspaces and code are in place from here on
+    for rows in (1, M):  # workspaces and code are in place from here on
         _lib.call("wgpt_int8_weight_create", dev.handle, K, N, p_d.ptr, s_d.ptr, C.byref(h))
         _lib.call("wgpt_int8_matmul_w", dev.handle, rows, h, a_d.ptr, o_d.ptr)
         _lib.call("wgpt_int8_weight_destroy", h)
     free = dev.mem_info()[0]
     _lib.call("wgpt_int8_weight_create", dev.handle, K, N, p_d.ptr, s_d.ptr, C.byref(h))
     slack = 4 << 20
-    for rows, per_code in ((1, 2), (16, 2), (17, 4)):
+    for rows in (1, M):
         _lib.call("wgpt_int8_matmul_w", dev.handle, rows, h, a_d.ptr, o_d.ptr)
+        _lib.call("wgpt_device_check", dev.handle)
         assert abs(free - dev.mem_info()[0] - per_code * K * N) < slack, rows
+    got = o_d.read(np.float32, M * N).reshape(M, N)
     _lib.call("wgpt_int8_weight_destroy", h)
     assert abs(free - dev.mem_info()[0]) < slack
+    cols = slice(0, N, 37)
+    Wf = q[:, cols].astype(np.float64) * 0.5
+    assert (np.abs(got[:, cols] - A.astype(np.float64) @ Wf) <= (2.0 ** -20 + K / 4 * 2.0 ** -23) * (np.abs(A).astype(np.float64) @ np.abs(Wf))).all()
 
 
 @pytest.fixture(scope="module")

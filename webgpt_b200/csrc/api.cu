@@ -1631,9 +1631,9 @@ WGPT_EXPORT int32_t wgpt_int8_matmul(wgpt_device *dev, int32_t M, int32_t K, int
 struct wgpt_int8_weight {
   wgpt_device *dev;
   int K, N;
-  uint32_t *words;   // [K, N/4], the prototype's packing (copy); owns the allocation of words, scale and bytes
+  uint32_t *words;   // [K, N/4], the prototype's packing (copy); owns the allocation of all four
   uint8_t *bytes;    // [N, K], K contiguous; nullptr when K % 16 != 0
-  mutable __half *halves;  // [N, K]: the codes as half-precision values (exact), made by the first call of more than 16 rows
+  __half *halves;    // [N, K]: the codes as half-precision values (exact), for the tensor cores; nullptr as bytes, or for want of memory
   float *scale;      // [N]
 };
 
@@ -1650,11 +1650,23 @@ WGPT_EXPORT int32_t wgpt_int8_weight_create(wgpt_device *dev, int32_t K, int32_t
   const size_t nbytes = (size_t)K * N;
   const size_t a256 = (nbytes + 255) & ~size_t(255), s256 = ((size_t)N * 4 + 255) & ~size_t(255);
   const bool relaid = K % 16 == 0;
-  char *base = nullptr;  // one allocation: words | scale | bytes
-  cudaError_t e = cudaMalloc(&base, a256 + s256 + (relaid ? a256 : 0));
+  // One allocation: words | scale | bytes | halves. Where the memory for the halves, two more bytes a code, is not there, or
+  // the caller does not want to spend it (WGPT_INT8_HALVES=0), the handle does without and calls of more than 16 rows expand
+  // the codes into the workspace: 256 x 3072 x 768 24.6 against 12.0 us. (Codes converted beside the rows on every call, in the
+  // same launch: 12.1 us there, but 15.2 against 10.4 at 17 x 1600 x 6400 and 34 against 21.5 at 256 x 6400 x 1600.)
+  const char *ev = getenv("WGPT_INT8_HALVES");
+  bool halves = relaid && !(ev && ev[0] == '0');
+  char *base = nullptr;
+  cudaError_t e = cudaMalloc(&base, a256 + s256 + (relaid ? (halves ? 3 : 1) * a256 : 0));
+  if (e == cudaErrorMemoryAllocation && halves) {
+    cudaGetLastError();
+    halves = false;
+    e = cudaMalloc(&base, a256 + s256 + a256);
+  }
   w->words = reinterpret_cast<uint32_t *>(base);
   w->scale = reinterpret_cast<float *>(base + a256);
   if (relaid) w->bytes = reinterpret_cast<uint8_t *>(base + a256 + s256);
+  if (halves) w->halves = reinterpret_cast<__half *>(base + 2 * a256 + s256);
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->words, Bq, nbytes, cudaMemcpyDeviceToDevice, dev->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(w->scale, scale, (size_t)N * 4, cudaMemcpyDeviceToDevice, dev->stream);
   if (e != cudaSuccess) {
@@ -1665,6 +1677,9 @@ WGPT_EXPORT int32_t wgpt_int8_weight_create(wgpt_device *dev, int32_t K, int32_t
   if (w->bytes) {
     dim3 grid((N / 4 + 31) / 32, (K + 31) / 32);
     LAUNCH(dev, int8_relayout_nk_kernel, grid, 256, 0, (const uint32_t *)w->words, K, N, w->bytes);
+    const size_t n16 = (size_t)N * K / 16;
+    if (w->halves)
+      LAUNCH(dev, int8_half_kernel, grid_for(n16, 256, dev->sm_count), 256, 0, (const uint8_t *)w->bytes, n16, w->halves);
   }
   CK(cudaStreamSynchronize(dev->stream));
   *out = w;
@@ -1677,24 +1692,7 @@ WGPT_EXPORT int32_t wgpt_int8_weight_destroy(wgpt_int8_weight *w) {
   NOT_RECORDING(w->dev, "wgpt_int8_weight_destroy");
   CK(cudaStreamSynchronize(w->dev->stream));
   cudaFree(w->words);
-  cudaFree(w->halves);
   delete w;
-  return WGPT_OK;
-}
-
-// The codes as half-precision values, two more bytes each, kept from the first call that multiplies them on the tensor cores:
-// a handle that only ever sees decode rows stays at two bytes a code. Without the memory, or while a pass list is being
-// recorded, there are none and the call takes the path without them.
-static int32_t int8_halves(wgpt_device *dev, const wgpt_int8_weight *w) {
-  if (w->halves != nullptr || dev->capturing) return WGPT_OK;
-  __half *p = nullptr;
-  const size_t n = (size_t)w->N * w->K;
-  if (cudaMalloc(&p, n * sizeof(__half)) != cudaSuccess) {
-    cudaGetLastError();
-    return WGPT_OK;
-  }
-  w->halves = p;
-  LAUNCH(dev, int8_half_kernel, grid_for(n / 16, 256, dev->sm_count), 256, 0, (const uint8_t *)w->bytes, n / 16, p);
   return WGPT_OK;
 }
 
@@ -1784,7 +1782,6 @@ WGPT_EXPORT int32_t wgpt_int8_matmul_w(wgpt_device *dev, int32_t M, const wgpt_i
       return WGPT_OK;
     }
   }
-  if (w->bytes != nullptr && M > 16 && dev->precision != WGPT_PRECISION_FP32) TRY(int8_halves(dev, w));
   if (w->halves != nullptr && M > 16 && dev->precision != WGPT_PRECISION_FP32) {
     // Many rows: the codes are exact in half precision, the rows become pairs (pair.cuh), the scales are in the epilogue of
     // a two-MMA product. 256 x 3072 x 768: 24.6 us when the codes were expanded to an FP32 weight on every call and the

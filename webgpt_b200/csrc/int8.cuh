@@ -269,7 +269,7 @@ int8_relayout_nk_kernel(const uint32_t *__restrict__ Bq, int K, int N, uint8_t *
   }
 }
 
-// Bytes [N, K] -> half-precision [N, K] (exact), for the tensor-core product of many rows. Once per handle.
+// Bytes [N, K] -> half-precision [N, K] (exact), for the tensor-core product of many rows. Load time.
 __global__ void int8_half_kernel(const uint8_t *__restrict__ q, size_t n16, __half *__restrict__ out) {
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n16; i += (size_t)gridDim.x * blockDim.x) {
     const uint4 w = ldg_stream4u(reinterpret_cast<const uint4 *>(q) + i);
