@@ -1018,7 +1018,9 @@ static int32_t launch_gemv_kn_t(wgpt_device *dev, const float *x, const KnWeight
 
 // Rows of a reference-layout product below the tensor cores' 32, and how many of them a CTA takes: all of up to eight, above
 // that 12 or 16 in one or two groups (16 float4 sums are what a thread's registers hold). 9 to 31 rows used to run on the
-// 64 x 64 tiles of gemm_simt_kernel, 12 CTAs for 768 columns: the operators of a GPT-2 pass took 6.4 ms, now 1.1 to 1.2.
+// 64 x 64 tiles of gemm_simt_kernel, 12 CTAs for 768 columns: the operators of a GPT-2 pass took 6.4 ms, now 1.1 to 1.2. The
+// tensor cores would be faster already there (32 tokens 0.90 ms): the line is the entry points' promise of FP32 sums below 32
+// rows (4e-7 of a result against 1e-6 and more), not the time.
 constexpr int kKnMaxRows = 31;
 static int kn_rows(int M) {
   if (M <= 8) return M;
@@ -1758,7 +1760,8 @@ WGPT_EXPORT int32_t wgpt_int8_matmul_w(wgpt_device *dev, int32_t M, const wgpt_i
     // Rows in equal groups of at most eight, or of what fits shared memory beside the weight (five at K = 6400); the groups
     // after the first find the weight in L2. Against the kernel on the packed words, 9 / 12 / 16 rows: 768 x 3072 6.8 / 8.1 /
     // 9.1 us (9.9 / 11.6 / 12.9), 1600 x 6400 13.3 / 15.9 / 19.2 (17.5 / 20.4 / 24.2), 6400 x 1600 in two and three groups
-    // 16.9 / 20.3 (20.3 / 23.2); four groups there are no faster (16 rows 27.8 / 27.5), which sets the limit.
+    // 16.9 / 20.3 (20.3 / 23.2); four groups there are no faster (16 rows 27.8 / 27.5), which sets the limit of groups. The limit
+    // of 16 rows keeps FP32 sums for them; on the tensor cores 17 rows of 1600 x 6400 take 10.4 us.
     int most = M < 8 ? M : 8;
     while (most > 0 && int8_block_plan(dev, K, N, most).smem == 0) most--;
     if (most > 0 && (M + most - 1) / most <= kInt8BlockGroups) {
@@ -2517,6 +2520,8 @@ static SplitBlockShapes split_block_shapes(const wgpt_device *dev, int M, int E)
   return b;
 }
 
+// Fewest sequences of a decode pass on pairs. Five stay in FP32 (4e-7 of the logits against 2.9e-6) although they take longer
+// than eight on pairs: GPT-2 390 against 358 us a pass, XL 2.55 against 2.2 ms.
 constexpr int kSplitMinRows = 6;
 // The transformer blocks of a pass of up to 64 rows (a decode step, a short prompt) as five kernels per block
 // (gemm_split.cuh): both LayerNorms ride on the products that consume them, the attention finishes its own output, and
@@ -2646,7 +2651,8 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
   // From six sequences on, where the de-embedding leaves the FP32 kernels too (logits of a decode step against double
   // precision, 2-norm: GPT-2 2.9e-6, XL 6.0e-6; five sequences in FP32 4e-7, and eight with FP32 blocks and the 3xTF32
   // de-embedding 6.3e-6 and 1.45e-5). Decode pass of eight sequences 0.369 ms (FP32 blocks 0.489), XL 2.21 (5.08).
-  // Prompts: from nine rows on; up to eight stay in FP32 where the products fit the block form, as they always have.
+  // Prompts: from nine rows on; up to eight stay in FP32 where the products fit the block form, as they always have; six to
+  // eight of larger models left it before (XL 6.9e-6 in three TF32 products, 1.6e-6 here).
   const bool split = pair_mode && M <= 64 &&
                      (n_tok == 1 ? M >= kSplitMinRows : M > 8 || (M >= kSplitMinRows && !layers_fit_block_form(dev, M, E))) &&
                      split_block_shapes(dev, M, E).ok;

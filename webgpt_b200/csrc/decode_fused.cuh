@@ -119,7 +119,7 @@ __device__ __forceinline__ void bulk_g2s_block(void *dst, const void *src, uint3
 constexpr int kAttnBlockThreads = 256;
 constexpr int kMlpBlockThreads = 512;
 // Cache positions per lane group that attn_block_kernel holds in registers ahead of the attention phase. GPT-2 step at
-// 64 / 200 / 500 / 900 positions with 2: 217.1 / 217.9 / 230.6 / 240.3 us, 3: 217.3 / 217.9 / 225.1 / 236.7 (76 registers),
+// 64 / 200 / 500 / 900 positions with 2: 217.1 / 217.9 / 230.6 / 240.3 us, 3: 217.3 / 217.9 / 225.1 / 236.7 (73 registers),
 // 4: 218.8 / 219.3 / 228.2 / 233.0; none requested ahead and two in flight in the loop: 217.0 / 221.1 / 238.7 / 258.9.
 constexpr int kAttnKvPre = 3;
 constexpr uint32_t kFusedPolls = 1u << 20;

@@ -2,7 +2,7 @@
 // step whose weights do not fit the SMs' shared memory (gemv_block_kernel) and are a stream from HBM.
 //
 // A CTA owns FT output columns (N / FT CTAs fill the SMs once) and pulls its rows of Wt through a ring of shared-memory
-// stages by TMA ({128 or 256 of K, FT rows} per box, one producer warp). Eight warps share the columns (warp w: w, w + 8,
+// stages by TMA ({256 of K, FT rows} per box, one producer warp). Eight warps share the columns (warp w: w, w + 8,
 // ..), lanes share K: a step reads one float4 per column and one per row of x, which all of the warp's columns use. Sums
 // stay in registers over the whole of K, so warps meet only at the ring's barriers.
 //
