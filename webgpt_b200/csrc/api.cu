@@ -1455,7 +1455,9 @@ WGPT_EXPORT int32_t wgpt_deembed(wgpt_device *dev, int32_t n_embd, int32_t vocab
 
 // wgpt_attention on half-precision pairs, five kernels: all four weights and the rows to pairs; q | k | v as one product;
 // attention; its output to pairs, row by row; output projection. The passes it replaces were thirteen kernels (a
-// transposition, a split-K product and its second stage per weight).
+// transposition, a split-K product and its second stage per weight). One exponent for all queries and keys and one for all
+// values and outputs, from the largest norms, saved the fourth kernel (128 / 1024 tokens x 768: 29.8 / 73.9 us against 31.0 /
+// 84.7) and cost a row beside a larger one its low bits.
 static int32_t attention_pair(wgpt_device *dev, int T, int E, float scale, int H, int hs, const float *in, const float *qW,
                               const float *qB, const float *kW, const float *kB, const float *vW, const float *vB,
                               const float *linW, const float *linB, float *out) {
