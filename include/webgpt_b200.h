@@ -46,10 +46,11 @@ enum {
 
 /* Arithmetic used by matrix products with more than 8 rows (prefill, batched decode, wgpt_matmul_nk; wgpt_matmul and
  * wgpt_attention on reference-layout weights from 32 rows on), by a model's decode passes of more than 5 sequences and by
- * prompts of 6 to 8 rows of models whose layer products do not fit shared memory (GPT-2 XL). The other products of up to 8 rows always run in FP32 on the CUDA cores. A new device starts in
- * WGPT_PRECISION_TF32X3, in which every tensor-core product is three products of operands split in two: models, wgpt_matmul,
- * wgpt_attention and the int8 weight handles split an operand into two half-precision values and a power of two per row
- * (22 significant bits), the others into two TF32 values (21 bits). */
+ * prompts of 6 to 8 rows of models whose layer products do not fit shared memory (GPT-2 XL). The other products of up to
+ * 8 rows always run in FP32 on the CUDA cores. A new device starts in WGPT_PRECISION_TF32X3, in which every tensor-core
+ * product is three products of operands split in two: models, wgpt_matmul, wgpt_attention and the int8 weight handles split
+ * an operand into two half-precision values and a power of two per row (22 significant bits of a row's larger values), the
+ * others into two TF32 values (21 bits). */
 enum {
   WGPT_PRECISION_FP32 = 0,   /* FP32 FMA on the CUDA cores */
   WGPT_PRECISION_TF32X3 = 1, /* tensor cores, three products per FP32 product (error 1e-6..2e-5, growing with K) */
