@@ -288,6 +288,28 @@ def test_decode_attention_slices(request, monkeypatch, fixture, slices, n_seq):
         s.destroy()
 
 
+@pytest.mark.parametrize("n_seq", [2, 150])
+def test_decode_attention_steps(model64, monkeypatch, n_seq):
+    """One slice of every head: the newest position as the first or last of a step of 32, in a step copied ahead of the wait
+    (two steps of many sequences, four of few) and in one copied later; all stages in use and used again."""
+    from webgpt_b200.model import Session
+    gpt, m, p = model64
+    monkeypatch.setenv("WGPT_ATTN_SPLIT", "1")
+    ids = np.stack([synth.make_tokens(p["vocab_size"], 300, seed=53, stream=i) for i in range(n_seq)])
+    s = Session(gpt, n_seq)
+    try:
+        at = 0
+        for t in (31, 32, 33, 63, 64, 127, 128, 129, 160, 192, 299):
+            if t > at:
+                s.forward(ids[:, at:t], want_logits=False)
+            lg = s.forward(ids[:, t:t + 1])
+            at = t + 1
+            for i in (0, n_seq - 1):
+                assert rel_err(lg[i], m.run(ids[i, :t + 1])) < 2e-5, t
+    finally:
+        s.destroy()
+
+
 def test_decode_slices_follow_the_context(model64, monkeypatch):
     """Sums over another number of slices differ in their last bits, so equal logits show which number ran: one-token
     forwards take it from the context they meet, and a captured completion changes it as it grows (at 64 and 192 positions

@@ -1277,11 +1277,22 @@ static int32_t launch_attn_decode(wgpt_device *dev, int hs, const float *q, int 
                                   const int *pos, float scale, const QkvPartials *qp = nullptr, __half *planes = nullptr,
                                   size_t plane = 0, float pair_scale = 1.f) {
   dim3 grid(H, n_seq, n_split);
-#define CASE(HSV, FROM)                                                                                               \
-  case HSV:                                                                                                           \
-    CK(launch_ex(dev->pdl, n_split, dev->stream, (attn_decode_kernel<HSV, FROM>), grid, dim3(256), 0, q, ldq, kc, vc, \
-                 ldkv, kv_seq_stride, out, ldo, pos, scale, qp ? *qp : QkvPartials(), planes, plane, pair_scale));    \
-    dev->launches++;                                                                                                  \
+  // Four steps of a slice ahead of the wait where an SM holds at most three CTAs, two (six CTAs an SM) where there are more. ms
+  // with two / four: GPT-2 3 sequences 64 + 64 tokens 21.47 / 20.12, 8 24.11 / 23.14, 64 x 128 + 64 44.0 / 44.9, 16 x 300 + 64
+  // 30.8 / 32.0; XL 1 x 200 + 32 57.8 / 54.8, 4 x 100 + 24 58.4 / 56.1, 16 x 96 + 24 63.4 / 65.9.
+  const bool deep = (long long)H * n_seq * n_split <= 3 * dev->sm_count;
+#define CASE_N(HSV, NST, FROM)                                                                                         \
+  do {                                                                                                                 \
+    CK(allow_smem(dev, attn_decode_kernel<HSV, NST, FROM>, true));                                                     \
+    CK(launch_ex(dev->pdl, n_split, dev->stream, (attn_decode_kernel<HSV, NST, FROM>), grid, dim3(256),                \
+                 attn_decode_smem_bytes(NST), q, ldq, kc, vc, ldkv, kv_seq_stride, out, ldo, pos, scale,               \
+                 qp ? *qp : QkvPartials(), planes, plane, pair_scale));                                                \
+  } while (0)
+#define CASE(HSV, FROM)                                                                                                \
+  case HSV:                                                                                                            \
+    if (deep) CASE_N(HSV, 4, FROM);                                                                                    \
+    else CASE_N(HSV, 2, FROM);                                                                                         \
+    dev->launches++;                                                                                                   \
     return WGPT_OK;
   if (qp != nullptr) {  // the attention CTAs are the QKV product's second stage (one position slice, 3*hs <= 256)
     switch (hs) {
@@ -1293,6 +1304,7 @@ static int32_t launch_attn_decode(wgpt_device *dev, int hs, const float *q, int 
     CASE(4, false) CASE(8, false) CASE(16, false) CASE(32, false) CASE(64, false) CASE(128, false)
   }
 #undef CASE
+#undef CASE_N
   return fail(WGPT_ERR_UNSUPPORTED, "head_size %d: supported sizes are 4, 8, 16, 32, 64, 128", hs);
 }
 

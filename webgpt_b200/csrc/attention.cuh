@@ -17,9 +17,13 @@ namespace wgpt {
 // over its slice; with n_split > 1 the slices' CTAs are a cluster and the first one merges their un-normalised results
 // (acc, max, sum) in slice order. Left to the consumer, the merge cost every CTA of the output projection the partial
 // results of every row (GPT-2 pass of 2 / 4 / 5 sequences 319 / 397 / 466 us, merged here 298 / 354 / 409).
-// HBM-bound: reads 2*HS*4 bytes per position per head. Before the dependency wait the CTA asks for its slice of
-// the cache in L2, computed from the position counter as it stands then (possibly one step old: the rows of
-// earlier positions never change, so a stale bound only misses the newest row).
+// HBM-bound for many sequences: reads 2*HS*4 bytes per position per head; for few, the chain q -> scores -> merge behind the
+// dependency wait. Cache rows of earlier steps do not depend on the previous kernel, only the newest one does: the first
+// NST steps of a CTA's slice are copied to shared memory ahead of the wait (cp.async, each thread the pieces that it will
+// use itself, so that no barrier is needed and no registers are held), the lines beyond them are asked for in L2. With eight
+// rows in registers per thread instead, requested behind the wait, 768 CTAs were five to an SM and a few of them a second
+// wave, and a CTA took 4 us from the wait. Whole completions in ms, before / now: GPT-2 8 x 64 + 64 tokens 23.6 / 23.1, 64 x 128
+// + 64 46.0 / 44.0, 16 x 300 + 64 32.9 / 30.8; XL 1 x 200 + 32 56.5 / 54.8, 16 x 96 + 24 66.2 / 63.4.
 // Split-K partial tiles of the QKV product that feeds a decode attention (batched decode on the tensor cores):
 // [slice][feature tile of 128][row = sequence][128], feature n of [0, 3E) = q | k | v. With FROM_QKV_PART the
 // attention CTA is that product's second stage for its own (sequence, head): it adds the slices in order, adds the
@@ -42,8 +46,11 @@ __device__ __forceinline__ void attn_put(float *out, __half *planes, size_t plan
   }
 }
 
-template <int HS, bool FROM_QKV_PART = false>
-__global__ void __launch_bounds__(256)
+constexpr int kAttnDecodeU = 2;  // positions per lane group and step
+constexpr size_t attn_decode_smem_bytes(int nst) { return (size_t)nst * kAttnDecodeU * 2 * 256 * 16; }
+
+template <int HS, int NST, bool FROM_QKV_PART = false>
+__global__ void __launch_bounds__(256, NST == 2 ? 6 : 3)
 attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict__ kc, const float *__restrict__ vc,
                    int ldkv, size_t kv_seq_stride, float *__restrict__ out, int ldo, const int *__restrict__ pos,
                    float scale, QkvPartials qp, __half *__restrict__ planes, size_t plane, float pair_scale) {
@@ -59,22 +66,59 @@ attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict
   trace(3, 0);
   if (n_split > 1) cluster_arrive();  // pairs with the wait ahead of the first remote store
   pdl_launch_dependents();
+  constexpr int U = kAttnDecodeU, STEP = NW * G * U;  // positions per step of the CTA
+  extern __shared__ __align__(16) float4 kv_stage[];      // [NST][U][K, V][256]
+  const uint32_t slot = smem_addr(kv_stage + tid);
+  const float *kbl = kb + lig * 4, *vbl = vb + lig * 4;
+  int beg = 0, end = 0;  // this CTA's slice of positions 0 .. p
+  auto slice = [&](int p) {
+    const int chunk = (p + n_split) / n_split;
+    beg = split * chunk;
+    end = min(p + 1, beg + chunk);
+  };
+  // Step i of the slice into stage i % NST: rows below `limit` only.
+  auto request = [&](int i, int limit) {
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int j = beg + i * STEP + (warp + u * NW) * G + g;
+      if (j < end && j < limit) {
+        const uint32_t at = slot + (uint32_t)(((i % NST) * U + u) * 2) * 4096u;
+        cp_async16(at, kbl + (size_t)j * ldkv);
+        cp_async16(at + 4096u, vbl + (size_t)j * ldkv);
+      }
+    }
+    cp_async_commit();
+  };
+  // Rows below *pos as it stands now (possibly one step old) were finished by the steps that advanced it there.
+  const int pos_s = __ldcg(pos);
+  slice(pos_s);
+#pragma unroll
+  for (int i = 0; i < NST; i++) request(i, pos_s);
   {
-    const int Ls = __ldcg(pos) + 1;
-    const int chunk_s = (Ls + n_split - 1) / n_split;
-    const int beg_s = split * chunk_s, end_s = min(Ls, beg_s + chunk_s);
     constexpr int LPR = HS * 4 >= 128 ? HS * 4 / 128 : 1;  // 128-byte lines per row slice
-    const int total = max(end_s - beg_s, 0) * 2 * LPR;
+    const int first = beg + NST * STEP, total = max(end - first, 0) * 2 * LPR;
     for (int i = tid; i < total; i += 256) {
-      const int r = beg_s + i / (2 * LPR), w = i % (2 * LPR);
+      const int r = first + i / (2 * LPR), w = i % (2 * LPR);
       prefetch_line_l2((w < LPR ? kb : vb) + (size_t)r * ldkv + (w % LPR) * 32);
     }
   }
   pdl_wait();  // q, the cache row of this step and *pos come from earlier kernels
   trace(3, 1);
+  // The newest row, where its step is among those requested already: together with q and *pos, one round trip for all three.
+  auto request_newest = [&] {
+#pragma unroll
+    for (int i = 0; i < NST; i++)
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (beg + i * STEP + (warp + u * NW) * G + g == pos_s && pos_s < end) {
+          const uint32_t at = slot + (uint32_t)((i * U + u) * 2) * 4096u;
+          cp_async16(at, kbl + (size_t)pos_s * ldkv);
+          cp_async16(at + 4096u, vbl + (size_t)pos_s * ldkv);
+        }
+    cp_async_commit();
+  };
+  if (!FROM_QKV_PART) request_newest();
   const int L = __ldcg(pos) + 1;
-  const int chunk = (L + n_split - 1) / n_split;
-  const int beg = split * chunk, end = min(L, beg + chunk);
   float4 q4;
   if (FROM_QKV_PART) {
     __shared__ __align__(16) float s_q[HS];
@@ -94,39 +138,34 @@ attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict
       else const_cast<float *>(vb)[(size_t)(L - 1) * ldkv + d] = a;
     }
     __syncthreads();
+    request_newest();
     q4 = *reinterpret_cast<const float4 *>(&s_q[lig * 4]);
   } else {
     q4 = __ldcg(reinterpret_cast<const float4 *>(q + (size_t)seq * ldq + h * HS + lig * 4));
   }
-  kb += lig * 4;
-  vb += lig * 4;
+  if (L - 1 != pos_s) {  // the position has moved since: another slice
+    slice(L - 1);
+    cp_async_wait<0>();
+#pragma unroll
+    for (int i = 0; i < NST; i++) request(i, L);
+  }
 
   float m = -INFINITY, l = 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  // Four positions per group and step: eight cache rows in flight per thread (a step is one round trip to HBM, so with two
-  // the loop was a chain of twice as many), one maximum and one rescale for the four. The trip count is the same for
-  // every lane of the warp (the shuffles below name all 32 lanes); a position past the end of the slice reads an
-  // in-bounds row and contributes nothing.
-  constexpr int U = 4;
-  for (int j0 = beg + warp * G; j0 < end; j0 += NW * G * U) {
-    float4 k4[U], v4[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int jj = min(j0 + u * NW * G + g, end - 1);
-      k4[u] = __ldcg(reinterpret_cast<const float4 *>(kb + (size_t)jj * ldkv));
-    }
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const int jj = min(j0 + u * NW * G + g, end - 1);
-      v4[u] = __ldcg(reinterpret_cast<const float4 *>(vb + (size_t)jj * ldkv));
-    }
+  // One maximum and one rescale for the U positions of a group's step. The trip count is the same for every lane of the warp
+  // (the shuffles below name all 32 lanes); a position past the end of the slice contributes nothing.
+  const int steps = (end - beg + STEP - 1) / STEP;
+  for (int i = 0; i < steps; i++) {
+    if (i + 1 < steps) cp_async_wait<NST - 1>();
+    else cp_async_wait<0>();  // the newest row's copies are the last ones
+    const float4 *st = kv_stage + (size_t)((i % NST) * U * 2) * 256 + tid;
     float s[U], mn = m;
 #pragma unroll
     for (int u = 0; u < U; u++) {
-      s[u] = dot4(q4, k4[u]);
+      s[u] = dot4(q4, st[u * 512]);  // past the end the stage holds anything
 #pragma unroll
       for (int o = LPP / 2; o > 0; o >>= 1) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
-      s[u] = j0 + u * NW * G + g < end ? s[u] * scale : -INFINITY;
+      s[u] = beg + i * STEP + (warp + u * NW) * G + g < end ? s[u] * scale : -INFINITY;
       mn = fmaxf(mn, s[u]);
     }
     if (mn != -INFINITY) {  // otherwise this group has seen no position yet
@@ -134,13 +173,16 @@ attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict
       l *= corr;
       acc.x *= corr; acc.y *= corr; acc.z *= corr; acc.w *= corr;
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        const float pr = expf(s[u] - mn);  // exactly 0 for a position past the end
-        l += pr;
-        acc.x += pr * v4[u].x; acc.y += pr * v4[u].y; acc.z += pr * v4[u].z; acc.w += pr * v4[u].w;
-      }
+      for (int u = 0; u < U; u++)
+        if (beg + i * STEP + (warp + u * NW) * G + g < end) {
+          const float pr = expf(s[u] - mn);
+          const float4 v = st[u * 512 + 256];
+          l += pr;
+          acc.x += pr * v.x; acc.y += pr * v.y; acc.z += pr * v.z; acc.w += pr * v.w;
+        }
       m = mn;
     }
+    request(i + NST, L);  // into the stage that has just been used
   }
   __syncwarp();
   // merge the G groups of the warp

@@ -169,8 +169,17 @@ __device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
 // large requests.
 __device__ __forceinline__ void prefetch_line_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
-// ---- bulk asynchronous copy (TMA, untiled form) global -> shared, completion counted on an mbarrier ----
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// Copies 16 bytes to shared memory without holding a register for them (through L2 only, as __ldcg).
+__device__ __forceinline__ void cp_async16(uint32_t saddr, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(saddr), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// ---- bulk asynchronous copy (TMA, untiled form) global -> shared, completion counted on an mbarrier ----
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t arrivals) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(arrivals) : "memory");
