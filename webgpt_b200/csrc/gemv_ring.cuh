@@ -9,7 +9,9 @@
 // What bounds it: HBM, and the hand-off between dependent products (wait, read of x, LayerNorm, exchange: 3-4 us of a
 // 10 us product). The ring is filled before the dependency wait, while the previous product finishes, so the stream stops
 // for less than that. GPT-2 XL, one sequence, four products of a block: 51 us in the register-streaming kernel (2.4
-// TB/s), 38 us here (3.2 TB/s); asking for the rest of the tile in L2 ahead of the wait gained nothing.
+// TB/s), 38 us here (3.2 TB/s); asking for the rest of the tile in L2 ahead of the wait gained nothing. Once its own last
+// stage is requested, a CTA asks for its share of the next product's first 10 MB in L2 (RingArgs::ahead), so that HBM has
+// something to do while the kernels change places: the next kernel's CTAs find no room before this one's leave.
 //
 //   x: gamma != nullptr: LayerNorm (instructions.js:451-550) of the rows by 8 / M warps each, the row in registers;
 //      otherwise as it is. Rows of this CTA's slice of K live in shared memory.
@@ -32,13 +34,15 @@ struct RingArgs {
   const float *gamma, *beta;  // LayerNorm of x, or nullptr (only then may S exceed 1)
   int rows, K, N, ft, stages;
   Epilogue epi;
+  const char *ahead;          // the first bytes of the next product's weights, or nullptr
+  unsigned int ahead_bytes;
   int *err;
 };
 
 // LayerNorm of the rows into shared memory by 8 / M warps each (M = 8, 4, 2, 1), a row of K <= 2048 values in registers
-// throughout; gamma and beta are in shared memory already. red: 2 x 8 floats. With one warp for a row of 1600, fetching
-// its scale and shift as it went, the stream waited 6 us.
-template <int M>
+// throughout; gamma and beta are in shared memory already, or (ASYNC) on their way there by cp.async of these threads. red: 2 x
+// 8 floats. With one warp for a row of 1600, fetching its scale and shift as it went, the stream waited 6 us.
+template <int M, bool ASYNC>
 __device__ __forceinline__ void ring_layernorm(const float *__restrict__ x, int rows, int K, const float4 *gam,
                                                const float4 *bet, float *xs, int xld, float *red, int warp, int lane) {
   constexpr int WPR = GR_WARPS / M, V = 16 / WPR > 1 ? 16 / WPR : 2;  // float4 per lane
@@ -51,6 +55,8 @@ __device__ __forceinline__ void ring_layernorm(const float *__restrict__ x, int 
     const int i = (j * WPR + part) * 32 + lane;
     v[j] = live && i < K4 ? __ldcg(src + i) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
+  static_assert(!ASYNC || WPR > 1, "the barrier behind the first sum shows gamma and beta to everybody");
+  if (ASYNC) cp_async_wait<0>();
   float s = 0.f;
 #pragma unroll
   for (int j = 0; j < V; j++) s += (v[j].x + v[j].y) + (v[j].z + v[j].w);
@@ -119,6 +125,17 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   float *sums = xs + (size_t)M * xld;
   float4 *gam = reinterpret_cast<float4 *>(sums + ((p.ft * M + 3) & ~3)), *bet = gam + (p.K >> 2);
 
+  // Scale and shift, up to two rows: asked for ahead of the weights and not waited for until the row is there. A CTA that
+  // starts late, on an SM that its predecessor has just left, otherwise waits for them behind 148 rings of requests (3 us).
+  // XL 1 x 200 + 32 / 2 x 300 + 24 tokens: 54.4 / 50.3 -> 53.3 / 49.0 ms; with four rows 54.9 -> 56.1.
+  constexpr bool kAsyncNorm = M <= 2;
+  if (kAsyncNorm && p.gamma != nullptr && warp < GR_WARPS) {
+    for (int i = tid; i < (p.K >> 2); i += 32 * GR_WARPS) {
+      cp_async16(smem_addr(gam + i), p.gamma + 4 * i);
+      cp_async16(smem_addr(bet + i), p.beta + 4 * i);
+    }
+    cp_async_commit();
+  }
   if (tid == 0) {
     for (int i = 0; i < p.stages; i++) {
       mbar_init(&full[i], 1);
@@ -144,7 +161,7 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
   const int m_first = o_first / p.ft, n_first = col0 + o_first % p.ft;
   float bias_v = 0.f, res_v = 0.f;
   if (has && e.bias != nullptr) bias_v = __ldg(e.bias + n_first);
-  if (p.gamma != nullptr) {
+  if (!kAsyncNorm && p.gamma != nullptr) {
     for (int i = tid; i < (p.K >> 2); i += GR_THREADS) {
       gam[i] = __ldg(reinterpret_cast<const float4 *>(p.gamma) + i);
       bet[i] = __ldg(reinterpret_cast<const float4 *>(p.beta) + i);
@@ -168,12 +185,18 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         issued = i + 1;
         if (++s == p.stages) { s = 0; ph ^= 1; }
       }
+      if (p.ahead != nullptr) {  // this CTA's share of what the next product is to find in L2
+        const unsigned int n16 = p.ahead_bytes >> 4;
+        const unsigned int beg = (unsigned int)((unsigned long long)n16 * blockIdx.x / gridDim.x);
+        const unsigned int end = (unsigned int)((unsigned long long)n16 * (blockIdx.x + 1) / gridDim.x);
+        for (unsigned int o = beg; o < end; o += 1024u) prefetch_l2(p.ahead + ((size_t)o << 4), min(end - o, 1024u) << 4);
+      }
     }
     __syncwarp();
   } else {
     const int k_lo = ch0 * GR_KT, k_len = min(nch * GR_KT, p.K - k_lo);
     if (p.gamma != nullptr) {
-      ring_layernorm<(M <= 2 ? M : (M <= 4 ? 4 : 8))>(p.x, p.rows, p.K, gam, bet, xs, xld, ln_red, warp, lane);
+      ring_layernorm<(M <= 2 ? M : (M <= 4 ? 4 : 8)), kAsyncNorm>(p.x, p.rows, p.K, gam, bet, xs, xld, ln_red, warp, lane);
     } else {
       // eight loads in flight per thread, whatever rows they fall into; every CTA reads the same rows at the same time,
       // so each starts at another place
