@@ -202,6 +202,24 @@ def test_prompt_lengths(model64, n):
     assert rel_err(gpt.run(ids), m.run(ids)) < 2e-5  # two layers of the products above
 
 
+@pytest.mark.parametrize("n", [65, 96, 128, 129, 193])
+def test_prompts_of_many_sequences(model64, n):
+    """More query tiles than SMs: one group of softmax warps per CTA, key tiles from the first to the diagonal, ragged last
+    tiles beside the next sequence's rows; a second chunk meets the cache that the first one left."""
+    from webgpt_b200.model import Session
+    gpt, m, p = model64
+    n_seq = 52
+    ids = np.stack([synth.make_tokens(p["vocab_size"], n + 70, seed=54, stream=i) for i in range(n_seq)])
+    s = Session(gpt, n_seq)
+    try:
+        for a, b in ((0, n), (n, n + 70)):
+            lg = s.forward(ids[:, a:b])
+            for i in (0, 1, n_seq - 1):
+                assert rel_err(lg[i], m.run(ids[i, :b])) < 2e-5, (i, b)
+    finally:
+        s.destroy()
+
+
 @pytest.mark.parametrize("n_seq", [2, 5, 6, 16, 17, 48, 49, 64, 65, 70])
 def test_decode_rows(model64, n_seq):
     """Row tiles of 16, 32, 48 and 64, the step to the planes of more rows, ragged last tiles; greedy ids of the first and

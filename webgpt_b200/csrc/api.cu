@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "attention.cuh"
+#include "attention_tc.cuh"
 #include "common.cuh"
 #include "decode_fused.cuh"
 #include "elementwise.cuh"
@@ -1217,8 +1218,9 @@ static bool attn_prefill_pair_ok(const wgpt_device *dev, int hs) {
   return attn_prefill_uses_mma(dev, hs, 64) && dev->precision == WGPT_PRECISION_TF32X3;
 }
 
-// Prefill attention of a pair model (attn_prefill_pair_ok): output planes [2][rows][ldo]. own_out: FP32 rows instead, and
-// every row of the operands with a scale of its own.
+// Prefill attention of a pair model (attn_prefill_pair_ok) over the FP32 cache: prompts of one tile and later chunks of a prompt
+// (from position 0 on, longer ones: launch_attn_prefill_tc). Output planes [2][rows][ldo]. own_out: the attention operator, FP32
+// rows instead, and every row of the operands with a scale of its own.
 static int32_t launch_attn_prefill_pair(wgpt_device *dev, const float *q, int ldq, const float *kc, const float *vc,
                                         int ldkv, size_t kv_seq_stride, int n_tok, int n_seq, int H, const int *pos,
                                         float scale, float s_qk, float s_v, __half *planes, size_t plane, int ldo,
@@ -1245,6 +1247,43 @@ static int32_t launch_attn_prefill_pair(wgpt_device *dev, const float *q, int ld
     else PAIR_ATTN(4, 1, false);
   }
 #undef PAIR_ATTN
+  return WGPT_OK;
+}
+
+// Tensor map of q | k | v as pairs, planes [2][n_seq][n_tok][3 E]: boxes of {64 halves, box_rows, 1, 2}, 128-byte swizzle, zero
+// fill beyond a sequence's tokens. E % 8 == 0.
+static int32_t make_qkv_map(CUtensorMap *map, const __half *planes, int n_seq, int n_tok, int E, int box_rows) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  REQUIRE(fn != nullptr, WGPT_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  const cuuint64_t row = (cuuint64_t)3 * E * 2;
+  cuuint64_t dims[4] = {(cuuint64_t)3 * E, (cuuint64_t)n_tok, (cuuint64_t)n_seq, 2};
+  cuuint64_t strides[3] = {row, row * n_tok, row * n_tok * n_seq};
+  cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 1, 2}, estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<__half *>(planes), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  REQUIRE(r == CUDA_SUCCESS, WGPT_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
+  return WGPT_OK;
+}
+
+// Prefill attention of a pair model over q | k | v as pairs (map_q, map_kv), a prompt from position 0: output planes
+// [2][rows][H * 64].
+static int32_t launch_attn_prefill_tc(wgpt_device *dev, const CUtensorMap &map_q, const CUtensorMap &map_kv, int n_tok,
+                                      int n_seq, int H, float scale, float s_qk, __half *planes, size_t plane) {
+  const float to_exp2 = (float)((double)scale / ((double)s_qk * s_qk) * 1.4426950408889634);
+  const int ctas = (n_tok + AT_Q - 1) / AT_Q * H * n_seq;
+#define ATTN_TC(KG)                                                                                                         \
+  do {                                                                                                                      \
+    CK(allow_smem(dev, attn_prefill64_tc_kernel<KG>));                                                                      \
+    LAUNCH_PDL(dev, attn_prefill64_tc_kernel<KG>, ctas, 128 * KG + 64, attn_tc_smem_bytes(), map_q, map_kv, n_tok, H,       \
+               to_exp2, planes, plane, H * 64, dev->d_err);                                                                 \
+  } while (0)
+  // Two groups of softmax warps where every CTA has an SM to itself. us per pass with one / two: GPT-2 333 tokens (36 CTAs)
+  // 828 / 791, 1024 (96) 1440 / 1334, 16 x 128 (192) 1886 / 1936, 64 x 128 (768) 5147 / 5298; XL 512 (100) 6826 / 6693, 1024
+  // (200) 10230 / 10390.
+  if (ctas <= dev->sm_count) ATTN_TC(2);
+  else ATTN_TC(1);
+#undef ATTN_TC
   return WGPT_OK;
 }
 
@@ -2486,6 +2525,15 @@ static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
   const size_t kv_layer = (size_t)s->n_seq * p.n_ctx * E, plane_e = (size_t)M * E, plane_f = (size_t)M * F;
   __half *h = reinterpret_cast<__half *>(s->h), *o = reinterpret_cast<__half *>(s->o), *f = reinterpret_cast<__half *>(s->f);
   const bool o_pair = n_tok == 1 || attn_prefill_pair_ok(dev, hs);
+  // A prompt from position 0 of more than one tile: q, k and v leave their product as pairs too, in the MLP's place (free then).
+  // us per pass, attn_prefill64_pair_kernel / this: GPT-2 65 / 333 / 1024 tokens 568 / 564, 846 / 790, 1525 / 1333, 64 x 128
+  // 5280 / 5090; XL 200 / 512 / 1024 4900 / 4800, 6900 / 6690, 12160 / 10400. One tile stays where it was.
+  const bool tc = n_tok > 64 && s->len == 0 && attn_prefill_pair_ok(dev, hs);
+  CUtensorMap map_q, map_kv;
+  if (tc) {
+    TRY(make_qkv_map(&map_q, f, s->n_seq, n_tok, E, AT_Q));
+    TRY(make_qkv_map(&map_kv, f, s->n_seq, n_tok, E, AT_K));
+  }
   for (int l = 0; l < p.n_layer; l++) {
     const LayerWeights &L = m->layers[l];
     float *kc = s->kc + (size_t)l * kv_layer, *vc = s->vc + (size_t)l * kv_layer;
@@ -2493,8 +2541,11 @@ static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
     Epilogue e = plain_epi(s->q, E, L.bqkv);
     e.colscale = L.wqkv_p.cs;
     e.kc = kc; e.vc = vc; e.E = E; e.n_tok = n_tok; e.n_ctx = p.n_ctx; e.pos = s->d_pos;
+    if (tc) { e.pair = f; e.pair_plane = 3 * plane_e; e.pair_scale = L.s_qk; e.pair_scale_v = L.s_o; e.ld = 3 * E; }
     TRY(launch_pair_product(dev, h, L.wqkv_p.p, M, E, 3 * E, e));
-    if (n_tok == 1) {
+    if (tc) {
+      TRY(launch_attn_prefill_tc(dev, map_q, map_kv, n_tok, s->n_seq, H, m->scale, L.s_qk, o, plane_e));
+    } else if (n_tok == 1) {
       TRY(launch_attn_decode(dev, hs, s->q, E, kc, vc, E, (size_t)p.n_ctx, nullptr, E, s->n_seq, H, s->n_split, s->d_pos,
                              m->scale, nullptr, o, plane_e, L.s_o));
     } else if (o_pair) {

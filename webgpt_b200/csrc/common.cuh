@@ -27,11 +27,12 @@ struct Epilogue {
   int pos_base;    // used when pos == nullptr
   // Operands stored as pairs of half-precision values (pair.cuh). rowscale: [M] or nullptr, multiplies the raw product
   // beside colscale. pair != nullptr: the finished value goes out as a pair (scaled by the power of two pair_scale)
-  // into the planes pair and pair + pair_plane, rows of ld values, instead of to out.
+  // into the planes pair and pair + pair_plane, rows of ld values, instead of to out. With a KV scatter the pairs are q | k | v
+  // (columns from 2E on scaled by pair_scale_v), and k and v go to the cache as FP32 besides.
   const float *rowscale;
   __half *pair;
   size_t pair_plane;
-  float pair_scale;
+  float pair_scale, pair_scale_v;
 };
 
 __device__ __forceinline__ float gelu_f(float x) {

@@ -72,13 +72,13 @@ __device__ __forceinline__ float4 pair_epi_value4(const Epilogue &e, float4 v, f
 __device__ __forceinline__ void pair_epi_store4(const Epilogue &e, float4 v, int m, int n) {
   if (e.pair != nullptr) {
     uint2 p0, p1;
-    pair_split4(scale4(v, e.pair_scale), p0, p1);
+    pair_split4(scale4(v, e.kc != nullptr && n >= 2 * e.E ? e.pair_scale_v : e.pair_scale), p0, p1);
     __half *o = e.pair + (size_t)m * e.ld + n;
     *reinterpret_cast<uint2 *>(o) = p0;
     *reinterpret_cast<uint2 *>(o + e.pair_plane) = p1;
-  } else {
-    *reinterpret_cast<float4 *>(epi_addr(e, m, n)) = v;
+    if (e.kc == nullptr || n < e.E) return;
   }
+  *reinterpret_cast<float4 *>(epi_addr(e, m, n)) = v;
 }
 // The same for 32 rows of a 32-column block held in `pad` (row stride 33): this lane finishes columns n..n+3 (block
 // columns col4..col4+3) of rows row0 + 4 it + sub_r. Without an activation the residuals of all its rows are requested
@@ -108,6 +108,14 @@ __device__ __forceinline__ void pair_epi_block(const Epilogue &e, const float *p
       *reinterpret_cast<float4 *>(epi_addr(e, m, n)) =
           make_float4(v.x * cs.x + bs.x + res[it].x, v.y * cs.y + bs.y + res[it].y, v.z * cs.z + bs.z + res[it].z,
                       v.w * cs.w + bs.w + res[it].w);
+    }
+  } else if (e.act == 0 && e.kc != nullptr && e.rowscale == nullptr) {  // q | k | v as pairs, and to the cache
+#pragma unroll
+    for (int it = 0; it < 8; it++) {
+      const int r = it * 4 + sub_r, m = row0 + r;
+      const float *src = pad + r * 33 + col4;
+      if (m >= M) continue;
+      pair_epi_store4(e, make_float4(src[0] * cs.x + bs.x, src[1] * cs.y + bs.y, src[2] * cs.z + bs.z, src[3] * cs.w + bs.w), m, n);
     }
   } else if (e.act == 0 && e.pair == nullptr && e.residual == nullptr) {
     float rs[8];
