@@ -58,6 +58,31 @@ def test_product_of_pairs_error_bound(dev, M, K, N):
     assert np.array_equal(scaled, (got * r[:, None] * c[None, :]).astype(np.float32))
 
 
+@pytest.mark.parametrize("M,K,N", [(700, 1608, 1608), (900, 1160, 1304)])
+def test_product_of_pairs_with_k_over_two_pairs(dev, M, K, N):
+    """Fewer tiles than CTA pairs: two pairs share a tile's K (even and odd numbers of k-blocks), ragged rows and columns."""
+    test_product_of_pairs_error_bound(dev, M, K, N)
+
+
+def test_deembedding_of_a_small_odd_vocabulary(oracle):
+    """Two pairs a tile again, rows that are no multiple of 16 bytes."""
+    from webgpt_b200 import GPT
+    from webgpt_b200.model import Session
+    p = dict(n_layer=1, n_head=12, n_embd=768, n_ctx=32, vocab_size=515)
+    w = synth.make_weights(p, seed=23, std=0.05, ln_random=True)
+    gpt, m = GPT(None, params=p, weights=w), oracle.Model(p, synth.weight_list(p, w))
+    gpt.initialize()
+    s = Session(gpt, 7)
+    try:
+        ids = np.stack([synth.make_tokens(p["vocab_size"], 9, seed=24, stream=i) for i in range(7)])
+        lg = s.forward(ids)
+        for i in range(7):
+            assert rel_err(lg[i], m.run(ids[i])) < 2e-5
+    finally:
+        s.destroy()
+        gpt.destroy()
+
+
 @pytest.mark.parametrize("M,N,a,w", [(40, 72, 128, -124), (40, 72, -124, 128), (600, 520, 128, -124), (40, 72, 114, 10),
                                      (40, 72, -60, -60)])
 def test_product_of_pairs_at_the_ends_of_the_exponent_range(dev, M, N, a, w):

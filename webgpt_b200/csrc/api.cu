@@ -965,13 +965,14 @@ static int32_t make_pair_map(CUtensorMap *map, const __half *planes, uint64_t ro
 // Tile width of gemm_pair_kernel: the multiple of 32 whose rounds over the pairs cost least, a tile costing
 // max(tensor pipe, shared memory) cycles per k-block (gemm_pair.cuh). *cycles: the estimate with 40 bytes per cycle from
 // L2 as a third bound and 12 000 cycles for the first copies and the last epilogue, to compare with gemm_split_kernel.
+static int pair_kb_cycles(int bn) { return 6 * bn > 640 + 5 * bn / 2 ? 6 * bn : 640 + 5 * bn / 2; }
 static int pair_tile_columns(const wgpt_device *dev, int M, int N, int K = 0, double *cycles = nullptr) {
   const int pairs = dev->sm_count / 2, m_tiles = (M + 255) / 256;
   int best = 256;
   long long best_cost = -1;
   for (int bn = 256; bn >= 64; bn -= 32) {
     const long long rounds = ((long long)m_tiles * ((N + bn - 1) / bn) + pairs - 1) / pairs;
-    const long long cost = rounds * (6 * bn > 640 + 5 * bn / 2 ? 6 * bn : 640 + 5 * bn / 2);
+    const long long cost = rounds * pair_kb_cycles(bn);
     if (best_cost < 0 || cost < best_cost) {
       best = bn;
       best_cost = cost;
@@ -981,21 +982,46 @@ static int pair_tile_columns(const wgpt_device *dev, int M, int N, int K = 0, do
   }
   return best;
 }
+// The same with K split over clusters of two pairs where that is shorter: a tile each, half the k-blocks, and for the exchange
+// 4000 cycles and 12 per column; the last epilogue, 70 cycles a column, is shared too. us per pass without / with: GPT-2 1024 tokens
+// 1390 / 1326, XL 512 / 700 / 1024 6840 / 6657, 9010 / 8480, 10960 / 10360. Four pairs gained less (6858 at 512, 8612 at 700), and
+// against gemm_split_kernel the form without the split decides: with this estimate plus 10 000 cycles XL 200 tokens took 4949 ->
+// 4730, but 333 6085 -> 6514 and GPT-2 512 969 -> 1004.
+struct PairShape {
+  int bn, KS;
+};
+static PairShape pair_shape(const wgpt_device *dev, int M, int N, int K) {
+  const int kb = (K + GP_BK - 1) / GP_BK, m_tiles = (M + 255) / 256, bn1 = pair_tile_columns(dev, M, N);
+  const int pairs = dev->sm_count / 2;
+  PairShape best = {bn1, 1};
+  double least = (double)((m_tiles * ((N + bn1 - 1) / bn1) + pairs - 1) / pairs) * pair_kb_cycles(bn1) * kb + 70.0 * bn1;
+  for (int bn = 256; kb >= 2 && bn >= 64; bn -= 32) {
+    if (m_tiles * ((N + bn - 1) / bn) > dev->max_clusters[4]) continue;
+    const double c = (double)((kb + 1) / 2) * pair_kb_cycles(bn) + 4000 + 12.0 * bn + 70.0 * ((bn / 32 + 1) / 2 * 32);
+    if (c < least) {
+      least = c;
+      best = {bn, 2};
+    }
+  }
+  return best;
+}
 
 // C = A . Wt^T from pair planes A [2][M][K] and W [2][N][K]; the exponents are in epi.colscale / epi.rowscale.
 static int32_t launch_gemm_pair(wgpt_device *dev, const __half *A, const __half *W, int M, int K, int N,
                                 const Epilogue &epi, bool b_exact = false) {
   REQUIRE(aligned16(A) && aligned16(W) && K % 8 == 0, WGPT_ERR_ALIGN, "pair operands need 16-byte aligned rows");
-  const int bn = pair_tile_columns(dev, M, N);
+  const PairShape ps = pair_shape(dev, M, N, K);
+  const int bn = ps.bn;
   CUtensorMap ma, mb;
   TRY(make_pair_map(&ma, A, (uint64_t)M, (uint64_t)K, GP_BM));
   TRY(make_pair_map(&mb, W, (uint64_t)N, (uint64_t)K, bn / 2, b_exact ? 1 : 2));
   const int work = ((M + 255) / 256) * ((N + bn - 1) / bn);
-  int pairs = dev->sm_count / 2;
-  if (pairs > work) pairs = work;
+  int clusters = dev->sm_count / 2;
+  if (clusters > work || ps.KS > 1) clusters = work;
   CK(allow_smem(dev, gemm_pair_kernel));
-  LAUNCH_PDL(dev, gemm_pair_kernel, 2 * pairs, GP_THREADS, GP_SMEM_BYTES, ma, mb, M, K, N, bn, b_exact ? 1 : 0, epi,
-             dev->d_err);
+  CK(launch_ex_x(dev->pdl, 2 * ps.KS, dev->stream, gemm_pair_kernel, dim3(2 * ps.KS * clusters), dim3(GP_THREADS), GP_SMEM_BYTES,
+                 ma, mb, M, K, N, bn, b_exact ? 1 : 0, epi, dev->d_err));
+  dev->launches++;
   return WGPT_OK;
 }
 

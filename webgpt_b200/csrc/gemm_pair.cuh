@@ -22,6 +22,10 @@
 // of K into registers instead leaves the MMAs no room to run ahead: pieces of 128 / 256 / 384 took 109 / 91 / 79 us for
 // 8192 x 2304 x 768 (3xTF32: 135 us).
 //
+// K split (clusters of 2 KS CTAs): where a product has fewer tiles than pairs, KS pairs share a tile, each with a slice of K, as
+// their own accumulators; every CTA leaves its FP32 tile in its ring, the cluster synchronises once, and each pair finishes
+// every KS-th 32-column block of the tile, adding the KS partial sums in slice order. One tile per cluster.
+//
 // Roles: warp 0 TMA producer, warp 1 MMA issuer (leader CTA only), warps 2-9 epilogue, two per quarter of the
 // accumulator lanes. Every wait is bounded; on expiry the CTA sets *err = 3, drains and exits.
 #pragma once
@@ -37,6 +41,8 @@ constexpr int GP_RING_BYTES = 3 * 2 * GP_A_BYTES;  // stages of A, then Wt: thre
 constexpr int GP_EPI_WARPS = 8;
 constexpr int GP_THREADS = 32 * (2 + GP_EPI_WARPS);
 constexpr int GP_PAD = 32 * 33;
+constexpr int GP_PART_LD = 36;                     // floats per row of a 32-column block of a partial tile: 16-byte rows, all banks
+static_assert(8 * GP_BM * GP_PART_LD * 4 <= GP_RING_BYTES, "a 256-column partial tile lies over the ring");
 constexpr size_t GP_SMEM_BYTES = 1024 + (size_t)GP_RING_BYTES + 256;
 
 // One box of both planes of a pair matrix: {64 halves, box rows, 2 planes}.
@@ -83,10 +89,11 @@ __host__ __device__ constexpr uint32_t f16_idesc(int m, int n) {
   return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 
-// gridDim.x = 2 x pairs, cluster (2,1,1). Pair p walks the 256 x bn tiles p, p + pairs, ... (row tile fastest).
+// gridDim.x = 2 KS x clusters, cluster (2 KS,1,1). Cluster p walks the 256 x bn tiles p, p + clusters, ... (row tile fastest);
+// with KS > 1 there are as many clusters as tiles.
 // map_a: box of 128 rows; map_b: box of bn/2 rows. bn % 32 == 0, bn <= 256.
 // b_exact: the weight is exact in one plane (integers of at most 11 bits) and has no second one (map_b: one plane).
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
+__global__ void __launch_bounds__(GP_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int K,
                  int N, int bn, int b_exact, Epilogue epi, int *err) {
   // narrower tiles leave room for a fourth stage (a copy takes about 3000 cycles to arrive under load)
@@ -102,12 +109,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   __shared__ float epi_pad[GP_EPI_WARPS * GP_PAD];
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();
+  uint32_t cluster_size;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(cluster_size));
+  const uint32_t crank = cluster_ctarank(), rank = crank & 1, lead = crank & ~1u;  // place in the pair, the pair's leader
   const bool leader = rank == 0;
-  const int total_kb = (K + GP_BK - 1) / GP_BK;
+  const int KS = (int)cluster_size >> 1, slice = (int)crank >> 1;
+  const int all_kb = (K + GP_BK - 1) / GP_BK, kb0 = all_kb * slice / KS, total_kb = all_kb * (slice + 1) / KS - kb0;
   const int m_tiles = (M + 255) / 256, n_tiles = (N + bn - 1) / bn;
   const int n_work = m_tiles * n_tiles;
-  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const int pair = (int)(blockIdx.x / cluster_size), pairs = (int)(gridDim.x / cluster_size);
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < S; i++) {
@@ -143,10 +153,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         for (int kb = 0; kb < total_kb; kb++) {
           uint8_t *st = tiles + (size_t)s * stage_bytes;
           if (*abort_flag || !mbar_wait(&empty[s], phase ^ 1, TC_POLLS)) { *abort_flag = 1; break; }
-          const uint32_t lead_full = peer_smem_addr(&full[s], 0);
+          const uint32_t lead_full = peer_smem_addr(&full[s], lead);
           if (leader) mbar_expect_tx(&full[s], stage_tx);
-          tma_load_3d_pair(st, &map_a, kb * GP_BK, m0, lead_full);
-          tma_load_3d_pair(st + GP_A_BYTES, &map_b, kb * GP_BK, nb0, lead_full);
+          tma_load_3d_pair(st, &map_a, (kb0 + kb) * GP_BK, m0, lead_full);
+          tma_load_3d_pair(st + GP_A_BYTES, &map_b, (kb0 + kb) * GP_BK, nb0, lead_full);
           issued++;
           if (++s == S) { s = 0; phase ^= 1; }
         }
@@ -176,11 +186,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             umma2_f16(tmem_acc, a1 + 2 * k, b0 + 2 * k, idesc, 1u);
           }
           umma2_commit_elect(smem_addr(&empty[s]));  // both CTAs may refill the stage once these MMAs have read it
-          umma2_commit_elect(peer_smem_addr(&empty[s], 1));
+          umma2_commit_elect(peer_smem_addr(&empty[s], lead + 1));
           if (++s == S) { s = 0; phase ^= 1; }
         }
         umma2_commit_elect(smem_addr(&acc_full[buf]));  // (also reached after an abort)
-        umma2_commit_elect(peer_smem_addr(&acc_full[buf], 1));
+        umma2_commit_elect(peer_smem_addr(&acc_full[buf], lead + 1));
       }
     }
   } else {
@@ -194,8 +204,67 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
     const int chunks = bn >> 5;
     const bool vec_ok = ((N | e.ld) & 3) == 0;
+    // a finished 32 x 32 block in `pad`: rows row0 .., columns nb ..
+    auto out_block = [&](int row0, int nb) {
+      const int n = nb + col4;
+      if (vec_ok) {
+        if (n < N) pair_epi_block(e, pad, row0, sub_r, col4, n, M);
+      } else {
+#pragma unroll 1
+        for (int it = 0; it < 8; it++) {
+          const int r = it * 4 + sub_r, m = row0 + r;
+          if (m >= M) break;
+#pragma unroll 1
+          for (int k = 0; k < 4; k++)
+            if (n + k < N) pair_epi1(e, pad[r * 33 + col4 + k], m, n + k);
+        }
+      }
+    };
     int i = 0;
-    for (int w = pair; w < n_work; w += pairs, i++) {
+    if (KS > 1) {
+      float *part = reinterpret_cast<float *>(tiles);
+      if (!mbar_wait(&acc_full[0], 0, TC_POLLS << 4) || *abort_flag) *abort_flag = 1;
+      tc_fence_after();
+#pragma unroll 1
+      for (int c = half; c < chunks; c += 2) {
+        float v[32];
+        tmem_ld_32x32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32), v);
+        float4 *dst = reinterpret_cast<float4 *>(part + (size_t)(c * GP_BM + quad * 32 + lane) * GP_PART_LD);
+#pragma unroll
+        for (int j = 0; j < 8; j++) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+      }
+      tc_fence_before();
+      cluster_arrive();
+      cluster_wait();
+      const int nt = pair / m_tiles, mt = pair - nt * m_tiles;
+      const int row0 = mt * 256 + (int)rank * GP_BM + quad * 32;
+#pragma unroll 1
+      for (int c = slice + half * KS; c < chunks; c += 2 * KS) {
+        const int nb = nt * bn + c * 32;
+        if (row0 >= M || nb >= N) break;  // same for the whole warp
+        const uint32_t at = smem_addr(part + (size_t)(c * GP_BM + quad * 32 + sub_r) * GP_PART_LD + col4);
+        float4 t[8];
+#pragma unroll 1
+        for (int k = 0; k < KS; k++) {
+          uint32_t ra;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(at), "r"(2 * k + (int)rank));
+          float4 q[8];
+#pragma unroll
+          for (int it = 0; it < 8; it++) q[it] = dsmem_ld4(ra + (uint32_t)(it * 4 * GP_PART_LD * 4));
+#pragma unroll
+          for (int it = 0; it < 8; it++) t[it] = k == 0 ? q[it] : add4(t[it], q[it]);
+        }
+#pragma unroll
+        for (int it = 0; it < 8; it++) {
+          float *d = pad + (it * 4 + sub_r) * 33 + col4;
+          d[0] = t[it].x; d[1] = t[it].y; d[2] = t[it].z; d[3] = t[it].w;
+        }
+        __syncwarp();
+        out_block(row0, nb);
+        __syncwarp();
+      }
+    }
+    for (int w = KS > 1 ? n_work : pair; w < n_work; w += pairs, i++) {
       const int nt = w / m_tiles, mt = w - nt * m_tiles;
       const int row0 = mt * 256 + (int)rank * GP_BM + quad * 32, n0 = nt * bn;
       const int buf = i & 1, use = i >> 1;
@@ -204,34 +273,27 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       const uint32_t tmem_acc = tmem_base + (uint32_t)(buf * 256) + ((uint32_t)(quad * 32) << 16);
 #pragma unroll 1
       for (int c = half; c < chunks; c += 2) {
-        const int nb = n0 + c * 32, n = nb + col4;
+        const int nb = n0 + c * 32;
         if (row0 >= M || nb >= N) break;  // same for the whole warp; nothing to read from here on
         float v[32];
         tmem_ld_32x32(tmem_acc + (uint32_t)(c * 32), v);
 #pragma unroll
         for (int j = 0; j < 32; j++) pad[lane * 33 + j] = v[j];
         __syncwarp();
-        if (vec_ok) {
-          if (n < N) pair_epi_block(e, pad, row0, sub_r, col4, n, M);
-        } else {
-#pragma unroll 1
-          for (int it = 0; it < 8; it++) {
-            const int r = it * 4 + sub_r, m = row0 + r;
-            if (m >= M) break;
-#pragma unroll 1
-            for (int k = 0; k < 4; k++)
-              if (n + k < N) pair_epi1(e, pad[r * 33 + col4 + k], m, n + k);
-          }
-        }
+        out_block(row0, nb);
         __syncwarp();
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(peer_smem_addr(&acc_empty[buf], 0));
+      if (lane == 0) mbar_arrive_cluster(peer_smem_addr(&acc_empty[buf], lead));
     }
     tc_fence_before();
   }
 
+  if (KS > 1 && warp < 2) {  // the epilogue warps' barrier between partial tiles and sums
+    cluster_arrive();
+    cluster_wait();
+  }
   __syncthreads();
   if (threadIdx.x == 0 && *abort_flag) {
     atomicExch(err, 3);
