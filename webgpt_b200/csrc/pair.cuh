@@ -226,12 +226,12 @@ struct PairOperands {
   float *bias_out[4]; // [N] copy of bias (zero where there is none), or nullptr
 };
 
-__device__ __forceinline__ void pair_operand_rows(const PairOperands &p) {
+__device__ __forceinline__ void pair_operand_rows(const PairOperands &p, int cta) {  // cta: of p.x_ctas
   __shared__ float red[8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, K4 = p.K >> 2;
   if (p.block_rows) {
     constexpr int V = 8;
-    for (int row = blockIdx.x; row < p.M; row += p.x_ctas) {
+    for (int row = cta; row < p.M; row += p.x_ctas) {
       const float4 *x = reinterpret_cast<const float4 *>(p.x + (size_t)row * p.K);
       float4 v[V];
       float m = 0.f;
@@ -259,7 +259,7 @@ __device__ __forceinline__ void pair_operand_rows(const PairOperands &p) {
         }
     }
   } else {
-    for (int row = blockIdx.x * 8 + warp; row < p.M; row += p.x_ctas * 8) {
+    for (int row = cta * 8 + warp; row < p.M; row += p.x_ctas * 8) {
       const float4 *x = reinterpret_cast<const float4 *>(p.x + (size_t)row * p.K);
       float m = 0.f;
 #pragma unroll 8
@@ -283,21 +283,26 @@ __device__ __forceinline__ void pair_operand_rows(const PairOperands &p) {
   }
 }
 
-// grid = x_ctas + n_w ceil(N / 32) S, cluster (S,1,1), 256 threads; dynamic shared memory klen x 33 floats.
+// grid = n_w ceil(N / 32) S + x_ctas, cluster (S,1,1), 256 threads; dynamic shared memory klen x 33 floats. The weights' CTAs come
+// first: they have work ahead of the dependency wait, and behind the rows' CTAs, which only wait, they found room 1.5 to 2.5 us
+// later. U: rows a thread has in flight, for 32 U of a strip; with twelve an SM holds three CTAs, with six four, so twelve only
+// where a strip's slice is longer than 192 rows (3072 x 768 took 5 us to read in two rounds).
+template <int U>
 __global__ void __launch_bounds__(256)
 pair_operands_kernel(const __grid_constant__ PairOperands p) {
   extern __shared__ __align__(16) float po_tile[];  // [klen][33]
   __shared__ float own[32], stat[8][32], scl[32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   pdl_launch_dependents();
-  if ((int)blockIdx.x < p.x_ctas) {  // whole clusters
+  const int w_ctas = (int)gridDim.x - p.x_ctas;
+  if ((int)blockIdx.x >= w_ctas) {  // whole clusters
     pdl_wait();
-    pair_operand_rows(p);
+    pair_operand_rows(p, (int)blockIdx.x - w_ctas);
     return;
   }
   uint32_t S;
   asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(S));
-  const int rank = (int)cluster_ctarank(), cl = (int)((blockIdx.x - p.x_ctas) / S);
+  const int rank = (int)cluster_ctarank(), cl = (int)(blockIdx.x / S);
   const int nblk = (p.N + 31) >> 5, wi = cl / nblk, blk = cl - wi * nblk, n0 = blk * 32;
   const int kb = min(p.K, rank * p.klen), kn = min(p.K, kb + p.klen) - kb;
   cluster_arrive();
@@ -305,7 +310,6 @@ pair_operands_kernel(const __grid_constant__ PairOperands p) {
     const int c4 = (tid & 7) * 4, r0 = tid >> 3;
     const bool in = n0 + c4 < p.N;  // N % 4 == 0
     const float *src = p.w[wi] + (size_t)kb * p.N + n0 + c4;
-    constexpr int U = 6;
     for (int r = r0; r < kn; r += 32 * U) {
       float4 v[U];
 #pragma unroll
