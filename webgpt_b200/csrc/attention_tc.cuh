@@ -14,7 +14,7 @@
 //              accumulated across tiles in tensor memory.
 // S and O have two buffers each, so that the scores of the next tile are there when a tile is done. 256 columns of tensor memory
 // and 97 KB of shared memory. KG == 1: one group of four softmax warps, two CTAs an SM. KG == 2: two groups take alternate
-// tiles and meet at the end, one CTA an SM (168 registers): for grids where the chain of a row's tiles is what the kernel takes.
+// tiles and meet at the end, one CTA an SM (167 registers): for grids where the chain of a row's tiles is what the kernel takes.
 // What bounds it: a softmax warp's own path, 0.75 us per tile of 64 keys (64 exponentials at eight cycles, six instructions each
 // around them, two trips to tensor memory) and 0.7 us until the tile's O is added; the tensor pipe needs 0.5. A GPT-2 layer of
 // 333 tokens 14.5 -> 8.5 us, an XL layer of 1024 66 -> 20 us. Against float64 the logits of one block are nearer than before
@@ -147,8 +147,7 @@ attn_prefill64_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     const float c = to_exp2;  // raw score -> exponent of two; positive
     // Running maximum of this thread's row as a power of two, rounded up, and sum of the probabilities. With a whole number the
     // shift and every rescale are exact, and an exponent has the rounding of one multiply-add. A probability is held times
-    // 2^AT_P_EXP: enough that its pair resolves 2^-28 of the row's largest, and little enough that the exponents of the ones that
-    // count keep their bits (with 2^15 the logits of XL at 1024 tokens were 2 % further from float64 than the kernel before).
+    // 2^AT_P_EXP: its pair resolves 2^-28 of the row's largest, and the exponents of the ones that count are small numbers.
     float m = -INFINITY, l = 0.f;
     float o[64];
 #pragma unroll
