@@ -245,6 +245,46 @@ def test_prompts_of_many_sequences(model64, n):
         s.destroy()
 
 
+@pytest.mark.parametrize("n,n_seq", [(65, 1), (130, 1), (256, 1), (129, 52)])
+def test_prefill_attention_keeps_small_probabilities(oracle, n, n_seq):
+    """The first key takes a row's probability and its values are zero, so the output is what the other keys add with
+    probabilities of about 2^-24.5; everything behind the attention is linear or a normalisation.
+
+    Bound, relative: a probability is off by 2^-40 of the largest at most, n of them in one direction against a sum of n random
+    ones are sqrt(n) 2^-15.5 (3.4e-4 at 256 keys); the output's own pair, 2^-40 of a bound that is 34 times the values' size at
+    most, adds 9e-5 at 64 keys."""
+    from webgpt_b200 import GPT
+    from webgpt_b200.model import Session
+    E, rng = 128, np.random.default_rng(31)
+    p = dict(n_layer=1, n_head=2, n_embd=E, n_ctx=256, vocab_size=520)
+    w = {k: np.zeros(synth.tensor_shape(p, k), np.float32) for k in synth.tensor_names(p)}
+    for k in ("ln_f", "h.0.ln_1", "h.0.ln_2"):
+        w[f"transformer.{k}.weight"][:] = 1
+    wte, wpe = w["transformer.wte.weight"], w["transformer.wpe.weight"]
+    wte[1:, 1:] = rng.standard_normal((519, E - 1))
+    wpe[0, 0] = 100  # token 0 at position 0: normalised to 11.3 in dimension 0, equal values in all others
+    qkv, bias = w["transformer.h.0.attn.c_attn.weight"], w["transformer.h.0.attn.c_attn.bias"]
+    qkv[1:, :2 * E] = rng.standard_normal((E - 1, 2 * E)) * 0.05
+    for h in (0, 64):
+        qkv[1:, h] = 0
+        bias[h], qkv[0, E + h] = 4, 3.02  # 4 x 3.02 x 11.27 / 8 = 17.0, e^-17.0 = 2^-24.5
+    for d in range(E):  # differences of two dimensions: exactly zero at position 0
+        m, v = 1 + d % 63, rng.uniform(0.5, 1.5)
+        qkv[2 * m, 2 * E + d], qkv[2 * m + 1, 2 * E + d] = v, -v
+    w["transformer.h.0.attn.c_proj.weight"][:] = rng.standard_normal((E, E)) * 2.0 ** 26 / np.sqrt(E)
+    ids = np.concatenate([np.zeros((n_seq, 1)), rng.integers(1, 520, (n_seq, n - 1))], 1).astype(np.uint32)
+    gpt, m = GPT(None, params=p, weights=w), oracle.Model(p, synth.weight_list(p, w))
+    gpt.initialize()
+    s = Session(gpt, n_seq)
+    try:
+        lg = s.forward(ids)
+        for i in {0, n_seq - 1}:
+            assert rel_err(np.asarray(lg).reshape(n_seq, -1)[i], m.run(ids[i])) < 1e-3
+    finally:
+        s.destroy()
+        gpt.destroy()
+
+
 @pytest.mark.parametrize("n_seq", [2, 5, 6, 16, 17, 48, 49, 64, 65, 70])
 def test_decode_rows(model64, n_seq):
     """Row tiles of 16, 32, 48 and 64, the step to the planes of more rows, ragged last tiles; greedy ids of the first and
