@@ -93,6 +93,26 @@ def test_gelu_clamps_and_softmax_odd(dev, ops, oracle):
         assert np.max(np.abs(got - oracle.softmax(x))) < 1e-6
 
 
+def test_gelu_error_bound(dev):
+    """Elementwise, against float64 with the shader's constants, in units of 2^-24. From rounding alone: u is off by 2 + 3 f of
+    itself (f: the cubic term's share; three roundings there, the sum's and the product's), which moves tanh u by u (1 - tanh^2 u)
+    times that; tanhf adds one unit in the last place, 1 + tanh u one rounding, the product with x another."""
+    from webgpt_b200 import _lib
+    n = 1 << 20
+    x = np.linspace(-10, 10, n).astype(np.float32)
+    x_d, o_d = dev.tensor(x), dev.buffer(4 * n)
+    _lib.call("wgpt_gelu", dev.handle, n // 1024, 1024, x_d.ptr, o_d.ptr)
+    got, x = o_d.read(np.float32, n).astype(np.float64), x.astype(np.float64)
+    cubic = float(np.float32(0.044715)) * x * x
+    u = float(np.float32(0.7978845608)) * x * (1 + cubic)
+    t = np.tanh(u)
+    moved = np.abs(u) * (1 - t * t) * (2 + 3 * cubic / (1 + cubic)) + np.spacing(np.abs(t).astype(np.float32)) * 2.0 ** 24
+    # halves of 1 + t are multiplied with x: what t is off by counts against x, not against the result
+    bound = 2.0 ** -24 * (np.abs(x) * (moved + 1 + t) / 2 + np.abs(x * (1 + t) / 2)) + 2.0 ** -149
+    err = np.abs(got - x / (1 + np.exp(-2 * u)))
+    assert (err <= bound).all(), (float(x[(err / bound).argmax()]), float((err / bound).max()))
+
+
 def test_embed_deembed(dev, ops, oracle):
     rng = np.random.default_rng(5)
     V, E, T = 211, 128, 33

@@ -61,16 +61,12 @@ __device__ __forceinline__ float4 pair_descale4(float4 v, float rs, float4 cs) {
 // Epilogue of the kernels that multiply pairs: four raw sums of row m, columns n..n+3, with the columns' constants and
 // the residual already in registers -> the finished values, and their store. `rows`: the product may have row factors (a
 // model's have none, and kernels made for them leave the branch out).
-// ROLLED: from pair_epi_block's rolled loop, where the tanh form is the faster one (XL at 200 tokens 4742 us a pass, 4808).
-template <bool ROLLED = false>
 __device__ __forceinline__ float4 pair_epi_value4(const Epilogue &e, float4 v, float4 cs, float4 bs, float4 res, int m, bool rows) {
   if (rows && e.rowscale != nullptr)
     v = add4(pair_descale4(v, __ldcg(e.rowscale + m), cs), bs);
   else
     v = make_float4(v.x * cs.x + bs.x, v.y * cs.y + bs.y, v.z * cs.z + bs.z, v.w * cs.w + bs.w);
-  if (e.act == 1)
-    v = ROLLED ? make_float4(gelu_tanh_f(v.x), gelu_tanh_f(v.y), gelu_tanh_f(v.z), gelu_tanh_f(v.w))
-               : make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
+  if (e.act == 1) v = make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
   return make_float4(v.x + res.x, v.y + res.y, v.z + res.z, v.w + res.w);
 }
 __device__ __forceinline__ void pair_epi_store4(const Epilogue &e, float4 v, int m, int n) {
@@ -140,7 +136,7 @@ __device__ __forceinline__ void pair_epi_block(const Epilogue &e, const float *p
       if (m >= M) break;
       const float *src = pad + r * 33 + col4;
       const float4 res = e.residual != nullptr ? __ldcg(reinterpret_cast<const float4 *>(e.residual + (size_t)m * e.ld + n)) : zero4;
-      pair_epi_store4(e, pair_epi_value4<true>(e, make_float4(src[0], src[1], src[2], src[3]), cs, bs, res, m, true), m, n);
+      pair_epi_store4(e, pair_epi_value4(e, make_float4(src[0], src[1], src[2], src[3]), cs, bs, res, m, true), m, n);
     }
   }
 }
