@@ -1146,9 +1146,9 @@ static int32_t launch_pair_operands(wgpt_device *dev, PairOperands &p) {
   p.x_ctas = (p.x_ctas + S - 1) / S * S;
   const size_t smem = p.n_w == 0 ? 0 : (size_t)p.klen * 33 * 4;
   REQUIRE(smem <= (size_t(200) << 10), WGPT_ERR_SHAPE, "shared dimension %d too long", p.K);
-  auto kern = p.n_w == 0 || p.klen <= 192 ? pair_operands_kernel<6> : pair_operands_kernel<12>;
-  CK(allow_smem(dev, kern));
-  CK(launch_ex_x(dev->pdl, S, dev->stream, kern, dim3(p.x_ctas + p.n_w * ((p.N + 31) / 32) * S), dim3(256), smem, p));
+  CK(allow_smem(dev, pair_operands_kernel));
+  CK(launch_ex_x(dev->pdl, S, dev->stream, pair_operands_kernel, dim3(p.x_ctas + p.n_w * ((p.N + 31) / 32) * S), dim3(256),
+                 smem, p));
   dev->launches++;
   return WGPT_OK;
 }

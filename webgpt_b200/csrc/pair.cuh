@@ -281,9 +281,8 @@ __device__ __forceinline__ void pair_operand_rows(const PairOperands &p, int cta
 
 // grid = n_w ceil(N / 32) S + x_ctas, cluster (S,1,1), 256 threads; dynamic shared memory klen x 33 floats. The weights' CTAs come
 // first: they have work ahead of the dependency wait, and behind the rows' CTAs, which only wait, they found room 1.5 to 2.5 us
-// later. U: rows a thread has in flight, for 32 U of a strip; with twelve an SM holds three CTAs, with six four, so twelve only
-// where a strip's slice is longer than 192 rows (3072 x 768 took 5 us to read in two rounds).
-template <int U>
+// later (pass list of GPT-2, us, rows first / weights first: 64 tokens 940 / 940, 128 1115 / 1056, 250 1329 / 1258). A thread has
+// six rows in flight; with twelve, for slices of more than 192 rows, the kernel spills and the lists take 1.2 to 2 % longer.
 __global__ void __launch_bounds__(256)
 pair_operands_kernel(const __grid_constant__ PairOperands p) {
   extern __shared__ __align__(16) float po_tile[];  // [klen][33]
@@ -306,6 +305,7 @@ pair_operands_kernel(const __grid_constant__ PairOperands p) {
     const int c4 = (tid & 7) * 4, r0 = tid >> 3;
     const bool in = n0 + c4 < p.N;  // N % 4 == 0
     const float *src = p.w[wi] + (size_t)kb * p.N + n0 + c4;
+    constexpr int U = 6;
     for (int r = r0; r < kn; r += 32 * U) {
       float4 v[U];
 #pragma unroll
