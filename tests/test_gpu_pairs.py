@@ -58,10 +58,36 @@ def test_product_of_pairs_error_bound(dev, M, K, N):
     assert np.array_equal(scaled, (got * r[:, None] * c[None, :]).astype(np.float32))
 
 
-@pytest.mark.parametrize("M,K,N", [(700, 1608, 1608), (900, 1160, 1304)])
+K_OVER_TWO_PAIRS = [(700, 1608, 1608), (900, 1160, 1304), (250, 1160, 3080), (700, 1544, 1608), (512, 3080, 2312)]
+WIDTH_OVER_TWO_PAIRS = (1216, (238, 250, 256))  # n_embd and tokens: q | k | v and the up projection
+
+
+@pytest.mark.parametrize("M,K,N", K_OVER_TWO_PAIRS)
 def test_product_of_pairs_with_k_over_two_pairs(dev, M, K, N):
-    """Fewer tiles than CTA pairs: two pairs share a tile's K (even and odd numbers of k-blocks), ragged rows and columns."""
+    """Fewer tiles than CTA pairs: two pairs share a tile's K (26 k-blocks, 19, 25 and 49), ragged rows and columns, one row tile
+    and several. test_pair_plan.py follows the rule; (900, 1160, 1304) takes this form on 36 clusters of four or more only."""
     test_product_of_pairs_error_bound(dev, M, K, N)
+
+
+@pytest.mark.parametrize("n", WIDTH_OVER_TWO_PAIRS[1])
+def test_model_products_with_k_over_two_pairs(oracle, n):
+    """K over two pairs with what a model's products do at their end: q, k and v as pairs and into the cache, GELU and pairs. The
+    logits behind the prompt, and of two more tokens over the cache it left; bound as in test_prompt_lengths."""
+    from webgpt_b200 import GPT
+    from webgpt_b200.model import Session
+    E = WIDTH_OVER_TWO_PAIRS[0]
+    p = dict(n_layer=1, n_head=E // 64, n_embd=E, n_ctx=260, vocab_size=512)
+    w = synth.make_weights(p, seed=61, std=0.04, ln_random=True)
+    gpt, m = GPT(None, params=p, weights=w), oracle.Model(p, synth.weight_list(p, w))
+    gpt.initialize()
+    s = Session(gpt, 1)
+    try:
+        ids = synth.make_tokens(512, n + 2, seed=62)
+        for a, b in ((0, n), (n, n + 1), (n + 1, n + 2)):
+            assert rel_err(s.forward(ids[a:b])[0], m.run(ids[:b])) < 2e-5, b
+    finally:
+        s.destroy()
+        gpt.destroy()
 
 
 def test_deembedding_of_a_small_odd_vocabulary(oracle):

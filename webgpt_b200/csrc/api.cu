@@ -31,6 +31,7 @@
 #include "int8.cuh"
 #include "sampling.cuh"
 #include "matmul.cuh"
+#include "pair_plan.h"
 
 using namespace wgpt;
 
@@ -962,55 +963,13 @@ static int32_t make_pair_map(CUtensorMap *map, const __half *planes, uint64_t ro
   return WGPT_OK;
 }
 
-// Tile width of gemm_pair_kernel: the multiple of 32 whose rounds over the pairs cost least, a tile costing
-// max(tensor pipe, shared memory) cycles per k-block (gemm_pair.cuh). *cycles: the estimate with 40 bytes per cycle from
-// L2 as a third bound and 12 000 cycles for the first copies and the last epilogue, to compare with gemm_split_kernel.
-static int pair_kb_cycles(int bn) { return 6 * bn > 640 + 5 * bn / 2 ? 6 * bn : 640 + 5 * bn / 2; }
-static int pair_tile_columns(const wgpt_device *dev, int M, int N, int K = 0, double *cycles = nullptr) {
-  const int pairs = dev->sm_count / 2, m_tiles = (M + 255) / 256;
-  int best = 256;
-  long long best_cost = -1;
-  for (int bn = 256; bn >= 64; bn -= 32) {
-    const long long rounds = ((long long)m_tiles * ((N + bn - 1) / bn) + pairs - 1) / pairs;
-    const long long cost = rounds * pair_kb_cycles(bn);
-    if (best_cost < 0 || cost < best_cost) {
-      best = bn;
-      best_cost = cost;
-      const double per_kb = fmax((double)cost / rounds, 820 + 3.2 * bn);
-      if (cycles) *cycles = rounds * per_kb * ((K + GP_BK - 1) / GP_BK) + 12000;
-    }
-  }
-  return best;
-}
-// The same with K split over clusters of two pairs where that is shorter: a tile each, half the k-blocks, and for the exchange
-// 4000 cycles and 12 per column; the last epilogue, 70 cycles a column, is shared too. us per pass without / with: GPT-2 1024 tokens
-// 1390 / 1326, XL 512 / 700 / 1024 6840 / 6657, 9010 / 8480, 10960 / 10360. Four pairs gained less (6858 at 512, 8612 at 700), and
-// against gemm_split_kernel the form without the split decides: with this estimate plus 10 000 cycles XL 200 tokens took 4949 ->
-// 4730, but 333 6085 -> 6514 and GPT-2 512 969 -> 1004.
-struct PairShape {
-  int bn, KS;
-};
-static PairShape pair_shape(const wgpt_device *dev, int M, int N, int K) {
-  const int kb = (K + GP_BK - 1) / GP_BK, m_tiles = (M + 255) / 256, bn1 = pair_tile_columns(dev, M, N);
-  const int pairs = dev->sm_count / 2;
-  PairShape best = {bn1, 1};
-  double least = (double)((m_tiles * ((N + bn1 - 1) / bn1) + pairs - 1) / pairs) * pair_kb_cycles(bn1) * kb + 70.0 * bn1;
-  for (int bn = 256; kb >= 2 && bn >= 64; bn -= 32) {
-    if (m_tiles * ((N + bn - 1) / bn) > dev->max_clusters[4]) continue;
-    const double c = (double)((kb + 1) / 2) * pair_kb_cycles(bn) + 4000 + 12.0 * bn + 70.0 * ((bn / 32 + 1) / 2 * 32);
-    if (c < least) {
-      least = c;
-      best = {bn, 2};
-    }
-  }
-  return best;
-}
+static SplitLimits split_limits(const wgpt_device *dev) { return SplitLimits{dev->max_clusters, dev->smem_optin - 2048}; }
 
 // C = A . Wt^T from pair planes A [2][M][K] and W [2][N][K]; the exponents are in epi.colscale / epi.rowscale.
 static int32_t launch_gemm_pair(wgpt_device *dev, const __half *A, const __half *W, int M, int K, int N,
                                 const Epilogue &epi, bool b_exact = false) {
   REQUIRE(aligned16(A) && aligned16(W) && K % 8 == 0, WGPT_ERR_ALIGN, "pair operands need 16-byte aligned rows");
-  const PairShape ps = pair_shape(dev, M, N, K);
+  const PairShape ps = pair_shape(split_limits(dev), dev->sm_count / 2, M, N, K);
   const int bn = ps.bn;
   CUtensorMap ma, mb;
   TRY(make_pair_map(&ma, A, (uint64_t)M, (uint64_t)K, GP_BM));
@@ -1098,8 +1057,6 @@ static int32_t gemm_kn_via_transpose(wgpt_device *dev, const float *A, size_t ld
   return launch_gemm_tc(dev, dev->precision == WGPT_PRECISION_TF32X3, A, lda, wt, M, K, N, epi, nullptr, false);
 }
 
-static SplitLimits split_limits(const wgpt_device *dev) { return SplitLimits{dev->max_clusters, dev->smem_optin - 2048}; }
-
 // X: pair planes [2][M][K], or nullptr with the LayerNorm input described in a (kNorm, M <= 64).
 static int32_t launch_gemm_split(wgpt_device *dev, const SplitShape &sh, const __half *X, const __half *W, int M, int K,
                                  int N, const Epilogue &epi, SplitArgs a) {
@@ -1159,10 +1116,9 @@ static bool pair_operands_fit(int K) { return K % 8 == 0 && K <= 8 * 1536; }
 // over a cluster where the former would leave most pairs without a tile (GPT-2 at 333 rows: 0.98 against 1.24 ms per pass).
 static int32_t launch_pair_product(wgpt_device *dev, const __half *X, const __half *W, int M, int K, int N,
                                    const Epilogue &epi, bool dyn = false, bool b_exact = false) {
-  double big = 0, split = 0;
-  pair_tile_columns(dev, M, N, K, &big);
-  const SplitShape sh = split_shape_rows(split_limits(dev), M, K, N, b_exact ? 1 : 2, &split);
-  if (sh.smem > 0 && split < big && N % 4 == 0 && (epi.ld & 3) == 0) {
+  SplitShape sh;
+  if (pair_product_splits(split_limits(dev), dev->sm_count / 2, M, K, N, b_exact ? 1 : 2, &sh) && N % 4 == 0 &&
+      (epi.ld & 3) == 0) {
     SplitArgs a;
     memset(&a, 0, sizeof a);
     a.dyn = dyn ? 1 : 0;

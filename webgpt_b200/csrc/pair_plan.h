@@ -1,0 +1,70 @@
+// Launch shapes of the products of pairs: gemm_pair_kernel's tile width and CTA pairs per tile (gemm_pair.cuh), and which
+// products gemm_split_kernel takes (gemm_split.cuh). Plain C++, so that the routes can be followed on the host.
+#pragma once
+#include <cmath>
+
+#include "split_plan.h"
+
+namespace wgpt {
+
+struct PairShape {
+  int bn, KS;  // tile columns, CTA pairs that share a tile's K
+};
+
+// A tile's cycles per k-block of GS_BK: max(tensor pipe, shared memory).
+inline int pair_kb_cycles(int bn) { return 6 * bn > 640 + 5 * bn / 2 ? 6 * bn : 640 + 5 * bn / 2; }
+
+// Tile width of gemm_pair_kernel without a split: the multiple of 32 whose rounds over the pairs cost least. *cycles: the
+// estimate with 40 bytes per cycle from L2 as a third bound and 12 000 cycles for the first copies and the last epilogue.
+inline int pair_tile_columns(int pairs, int M, int N, int K = 0, double *cycles = nullptr) {
+  const int m_tiles = (M + 255) / 256;
+  int best = 256;
+  long long best_cost = -1;
+  for (int bn = 256; bn >= 64; bn -= 32) {
+    const long long rounds = ((long long)m_tiles * ((N + bn - 1) / bn) + pairs - 1) / pairs;
+    const long long cost = rounds * pair_kb_cycles(bn);
+    if (best_cost < 0 || cost < best_cost) {
+      best = bn;
+      best_cost = cost;
+      const double per_kb = std::fmax((double)cost / rounds, 820 + 3.2 * bn);
+      if (cycles) *cycles = rounds * per_kb * ((K + GS_BK - 1) / GS_BK) + 12000;
+    }
+  }
+  return best;
+}
+
+// The same with K split over clusters of two pairs where that is shorter: a tile each, half the k-blocks, and for the exchange
+// 4000 cycles and 12 per column; the last epilogue, 70 cycles a column, is shared too. Of GPT-2's and XL's products it is q | k | v
+// of XL at 145 to 256 rows, XL's down projection from 641 on and its output projection to 768 (33 clusters of four). us per pass
+// without / with: XL 145 / 175 / 200 tokens 4818 / 4658, 4985 / 4822, 4961 / 4918, but 210 / 235 / 255 4860 / 4927, 4920 / 5026,
+// 4858 / 4983; 645 / 700 / 765 9194 / 8816, 9398 / 9017, 9699 / 9307; 800 to 1024 the same. Sums of half as many steps: logits of
+// three XL layers at 200 / 700 / 1024 tokens 7.4e-6 / 1.59e-5 / 1.64e-5 from float64, 1.20e-5 / 2.13e-5 / 2.18e-5 without. Six
+// layers of other widths: n_embd 1216 and 1408 at 180 to 256 rows 1 to 2.5 % faster, 1344 to 1856 at 600 to 768 1 to 3, 2432 at 400
+// and 512 4 to 6, 1792 and 1856 at 200 to 256 1 to 2 % slower. So the estimate is off for one row tile of many columns; 35 cycles
+// a column in place of 12 put XL at 205 to 256 right, and cost XL 0.9 % at 641 to 768 and n_embd 1216 to 1408 what they had gained.
+inline PairShape pair_shape(const SplitLimits &lim, int pairs, int M, int N, int K) {
+  const int kb = (K + GS_BK - 1) / GS_BK, m_tiles = (M + 255) / 256, bn1 = pair_tile_columns(pairs, M, N);
+  PairShape best = {bn1, 1};
+  double least = (double)(((long long)m_tiles * ((N + bn1 - 1) / bn1) + pairs - 1) / pairs) * pair_kb_cycles(bn1) * kb + 70.0 * bn1;
+  for (int bn = 256; kb >= 2 && bn >= 64; bn -= 32) {
+    if ((long long)m_tiles * ((N + bn - 1) / bn) > lim.max_clusters[4]) continue;
+    const double c = (double)((kb + 1) / 2) * pair_kb_cycles(bn) + 4000 + 12.0 * bn + 70.0 * ((bn / 32 + 1) / 2 * 32);
+    if (c < least) {
+      least = c;
+      best = {bn, 2};
+    }
+  }
+  return best;
+}
+
+// Whether gemm_split_kernel should be the faster one, by the estimates of both; *sh: its shape. The form without the K split
+// stands for gemm_pair_kernel here: with the better estimate plus 10 000 cycles XL at 200 tokens took 4949 -> 4730 us, but 333
+// 6085 -> 6514 and GPT-2 512 969 -> 1004.
+inline bool pair_product_splits(const SplitLimits &lim, int pairs, int M, int K, int N, int w_planes, SplitShape *sh) {
+  double big = 0, split = 0;
+  pair_tile_columns(pairs, M, N, K, &big);
+  *sh = split_shape_rows(lim, M, K, N, w_planes, &split);
+  return sh->smem > 0 && split < big;
+}
+
+}  // namespace wgpt

@@ -66,7 +66,7 @@ inline SplitShape split_shape_decode(const SplitLimits &lim, int M, int K, int N
 }
 
 // Any number of rows, activations as planes: row tiles of up to 128 and K slices by the same kind of estimate
-// (pair_tile_columns): a k-block costs max(6 RN tensor-core cycles, 32 KB + 256 RN bytes from L2 at 40 a cycle), a round
+// (pair_plan.h): a k-block costs max(6 RN tensor-core cycles, 32 KB + 256 RN bytes from L2 at 40 a cycle), a round
 // 9000 cycles of start, exchange and store and 60 more per row of the tile.
 inline SplitShape split_shape_rows(const SplitLimits &lim, int M, int K, int N, int w_planes, double *cycles) {
   SplitShape best = {};
