@@ -419,6 +419,32 @@ def test_decode_attention_steps(model64, monkeypatch, n_seq):
         s.destroy()
 
 
+@pytest.mark.parametrize("slices", ["1", "4"])
+@pytest.mark.parametrize("n_seq", [6, 16, 64])
+def test_decode_steps_behind_one_another(model64, monkeypatch, n_seq, slices):
+    """Steps launched one behind the other without a graph: the first layer's attention starts while the step before has yet to
+    advance the position, so it has asked for rows of another slice (seen in nearly every CTA of that layer at 6 and 16
+    sequences, in most at 64). Captured steps follow one another whole. Same ids, and the same caches bit for bit."""
+    from webgpt_b200 import GPT
+    from webgpt_b200.model import Session
+    gpt, m, p = model64
+    monkeypatch.setenv("WGPT_ATTN_SPLIT", slices)
+    monkeypatch.setenv("WGPT_GRAPH", "0")
+    eager = GPT(None, params=p, weights=synth.make_weights(p, seed=17, std=0.08, ln_random=True))
+    eager.initialize()
+    prompts = np.stack([synth.make_tokens(p["vocab_size"], 29, seed=57, stream=i) for i in range(n_seq)])
+    s, t = Session(gpt, n_seq), Session(eager, n_seq)
+    try:
+        a, b = s.generate_greedy(prompts, 110), t.generate_greedy(prompts, 110)
+        assert np.array_equal(a, b)
+        assert np.array_equal(a[0], m.kv_generate_greedy(prompts[0], 110))
+        assert np.array_equal(s.forward(a[:, 109:]), t.forward(b[:, 109:]))
+    finally:
+        s.destroy()
+        t.destroy()
+        eager.destroy()
+
+
 def test_decode_slices_follow_the_context(model64, monkeypatch):
     """Sums over another number of slices differ in their last bits, so equal logits show which number ran: one-token
     forwards take it from the context they meet, and a captured completion changes it as it grows (at 64 and 192 positions

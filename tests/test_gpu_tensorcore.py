@@ -118,10 +118,9 @@ def test_model_in_tf32x3_matches_oracle(oracle):
 
 
 def test_batched_decode_gpt2_width(oracle):
-    """GPT-2 width (d = 768, 12 heads of 64) cut to two layers, 16 and 64 sequences decoded together: the layer
-    products run split-K with exchanged operands, the attention adds the QKV slices itself, the residual products'
-    second stage applies the next LayerNorm, and the de-embedding runs without split. Tokens must equal the
-    oracle's for every checked sequence, logits within 5e-5."""
+    """GPT-2 width (d = 768, 12 heads of 64) cut to two layers, 16 and 64 sequences decoded together on pairs: the layer
+    products split K over clusters and normalise their own input rows. Tokens must equal the oracle's for every checked
+    sequence, logits within 5e-5."""
     from webgpt_b200 import GPT
     params = dict(n_layer=2, n_head=12, n_embd=768, n_ctx=48, vocab_size=1000)
     w = synth.make_weights(params, seed=31, std=0.05, ln_random=True)
@@ -143,6 +142,52 @@ def test_batched_decode_gpt2_width(oracle):
                 ref = m.run(np.concatenate([prompts[i], batch[i, :1]]))
                 assert rel_err(lg[i], ref) < 5e-5
     finally:
+        gpt.destroy()
+
+
+@pytest.mark.parametrize("H,hs,mode,n_seq,contexts", [
+    (37, 4, "tf32x3", 12, (30, 511, 512, 1023, 1024, 2047, 2048)),
+    (37, 4, "tf32x3", 13, (30, 511, 512, 1023, 1024, 1030)),
+    (7, 64, "tf32", 63, (31, 32, 63, 64, 127, 128, 129)),
+    (7, 64, "tf32", 64, (31, 32, 63, 64, 65, 96))])
+def test_decode_attention_adds_the_qkv_slices(oracle, monkeypatch, H, hs, mode, n_seq, contexts):
+    """Models that do not decode on pairs (n_embd no multiple of 8, or plain TF32): the attention CTAs of one slice are the q | k | v
+    product's second stage, which saves its launch; with two slices it runs. Up to 444 heads and sequences four steps are copied
+    ahead of the wait, beyond that two; contexts around a step (2048 / head size positions) and around all that are copied ahead.
+
+    Both routes add the same FP32 partial sums. 3xTF32: 1e-5 between them, 2e-5 to the oracle as for other decode paths. TF32: an
+    FP32 rounding can carry an operand over a TF32 step, and what that moves carries over more in the next product, until both
+    routes truncate as if independently: 2^-10 / sqrt(6) of a sum of random terms per product, 1.2e-3 after nine. A missing
+    position is 1/130 or more."""
+    from webgpt_b200 import GPT, _lib
+    from webgpt_b200.model import Session
+    p = dict(n_layer=2, n_head=H, n_embd=H * hs, n_ctx=max(contexts) + 2, vocab_size=304)
+    w = synth.make_weights(p, seed=37, std=0.08, ln_random=True)
+    gpt, m = GPT(None, params=p, weights=w), oracle.Model(p, synth.weight_list(p, w))
+    gpt.initialize()
+    gpt.device.set_precision(_lib.PRECISION_TF32X3 if mode == "tf32x3" else _lib.PRECISION_TF32)
+    ids = np.stack([synth.make_tokens(304, max(contexts) + 1, seed=58, stream=i) for i in range(n_seq)])
+    sessions = []
+    for slices in ("1", "2"):
+        monkeypatch.setenv("WGPT_ATTN_SPLIT", slices)
+        sessions.append(Session(gpt, n_seq))
+    try:
+        at = 0
+        for t in contexts:
+            out = []
+            for s in sessions:
+                if t > at:
+                    s.forward(ids[:, at:t], want_logits=False)
+                before = gpt.device.launch_count()
+                out.append((s.forward(ids[:, t:t + 1]), gpt.device.launch_count() - before))
+            at = t + 1
+            assert out[0][1] == out[1][1] - p["n_layer"]
+            assert rel_err(out[0][0], out[1][0]) < (1e-5 if mode == "tf32x3" else 2e-3), t
+            if mode == "tf32x3" and t <= 512:
+                assert rel_err(out[0][0][n_seq - 1], m.run(ids[n_seq - 1, :t + 1])) < 2e-5, t
+    finally:
+        for s in sessions:
+            s.destroy()
         gpt.destroy()
 
 

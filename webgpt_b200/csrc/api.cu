@@ -2308,7 +2308,7 @@ struct wgpt_session {
   float *pick_val;  // [n_seq][vocab] per-CTA arg-max candidates of the fused greedy pick
   int *pick_idx;
   unsigned long long *pick_keys;  // [8] (value, index) keys of gemv_loop_kernel's greedy pick, zero between launches
-  int *d_pos, *d_step;
+  int *d_pos, *d_step;  // advanced by kernels, taken back by stream memsets alone (the decode attention reads ahead on that)
   std::vector<uint32_t> prompts;  // host copy, [n_seq][n_prompt]
   int n_prompt, n_generated;
   bool ids_dirty;  // s->ids no longer holds the prompt window

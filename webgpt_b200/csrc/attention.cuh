@@ -89,7 +89,8 @@ attn_decode_kernel(const float *__restrict__ q, int ldq, const float *__restrict
     }
     cp_async_commit();
   };
-  // Rows below *pos as it stands now (possibly one step old) were finished by the steps that advanced it there.
+  // Rows below *pos as it stands now were finished by the steps that advanced it there (common.cuh). It is one step old, or zero
+  // ahead of a prompt's end, in most CTAs of a first layer whose step follows another without a graph launch in between.
   const int pos_s = __ldcg(pos);
   slice(pos_s);
 #pragma unroll

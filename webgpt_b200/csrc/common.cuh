@@ -154,8 +154,11 @@ __device__ __forceinline__ void trace_at(unsigned int base, int kid, int phase) 
 //
 // Programmatic dependent launch. A kernel launched with the programmatic-serialisation attribute may start
 // while its predecessor in the stream is still running; everything it does before pdl_wait() must therefore
-// touch only data no earlier kernel writes (here: weights). pdl_wait() returns once every earlier kernel has
-// completed and its writes are visible; without the attribute both calls are no-ops.
+// touch only data no earlier kernel still writes: weights, and in the decode attention the cache rows below *pos.
+// Those are final whenever *pos is read: a kernel advances it behind its own pdl_wait(), so behind every kernel that
+// wrote them, and only a memset in the stream, which neither starts nor ends inside a kernel, takes it back.
+// pdl_wait() returns once every earlier kernel has completed and its writes are visible; without the attribute both
+// calls are no-ops.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
