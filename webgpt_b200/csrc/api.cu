@@ -685,9 +685,10 @@ static int32_t launch_gemv_ring(wgpt_device *dev, const RingPlan &pl, int M, con
                                 const float *beta, const float *Wt, int K, int N, const Epilogue &epi,
                                 const float *next_w, size_t next_floats) {
   RingArgs a;
-  // 10 MB: 200 + 32 tokens of XL take 54.9 ms without, 53.9 / 53.2 / 53.6 / 54.2 ms with 4 / 10 / 20 / 50 MB of every next
-  // product (a bulk request waits in line with the next CTA's copies; line by line 54.1 / 53.9 / 54.7 / 57.2 at 5 / 10 / 20 / 50);
-  // requested ahead of the dependency wait by the output projection, which has the time: 53.9. 4 x 100 + 24 tokens 56.5 -> 56.2.
+  // 10 MB, swept with one row: 200 + 32 tokens of XL take 54.9 ms without, 53.9 / 53.2 / 53.6 / 54.2 ms with 4 / 10 / 20 / 50 MB of
+  // every next product (a bulk request waits in line with the next CTA's copies; line by line 54.1 / 53.9 / 54.7 / 57.2 at 5 / 10 /
+  // 20 / 50); requested ahead of the dependency wait by the output projection, which has the time: 53.9. Without / with at more
+  // rows: 2 x 300 + 24 tokens 49.5 / 49.1 ms, 4 x 100 + 24 56.7 / 56.2, 5 x 100 + 24 64.0 / 63.6, a prompt of 5 tokens 2.81 / 2.73.
   constexpr size_t kAheadBytes = size_t(10) << 20;
   a.ahead = reinterpret_cast<const char *>(next_w);
   a.ahead_bytes = (unsigned int)(std::min(next_floats * 4, kAheadBytes) & ~size_t(15));
@@ -2348,11 +2349,13 @@ static int32_t session_reserve(wgpt_session *s, int n_tok) {
 }
 
 // Position slices per (sequence, head) of the decode attention: 1, 2, 4 or 8 CTAs of a cluster share a head's cache rows.
-// Doubled while the grid stays within about 5.5 CTAs per SM (what is resident at once) and a slice keeps the positions that
-// a CTA has in flight in one step (4096 / head size), for the context at hand plus the 64 positions it may grow by before
-// the next look. Per pass with 1 / 2 / 4 / 8 slices, GPT-2 2 sequences at 100 positions 359 / 346 / 342 / 349, at 300
-// 418 / 379 / 360 / 357, at 900 643 / 488 / 413 / 377 us, 16 at 192 486 / 472 / 489 / 546, at 900 737 / 709 / 638 / 639; GPT-2
-// XL 1 sequence at 900 2710 / 2175 / 1943 / 1984, 4 at 448 3248 / 2847 / 2638 / 2658.
+// Doubled while the grid stays within 5.5 CTAs per SM and a slice keeps 4096 / head size positions, which are two steps of a CTA
+// (kAttnDecodeU), for the context at hand plus the 64 positions it may grow by before the next look. Six CTAs of the form with
+// two steps ahead are resident at once, three of the one with four. us per pass with 1 / 2 / 4 / 8 slices, GPT-2 2 sequences at
+// 100 positions 298 / 295 / 290 / 295, at 300 348 / 320 / 306 / 303, at 900 527 / 404 / 350 / 328, 16 at 192 408 / 407 / 422 / 466, at
+// 900 635 / 572 / 581 / 591, 64 at 160 629 / 652 / 737 / 914; GPT-2 XL 1 sequence at 900 2435 / 1965 / 1747 / 1689, 4 at 448
+// 2616 / 2466 / 2393 / 2455, 16 at 110 2219 / 2246 / 2447 / 2878. (The line was drawn for a kernel with four positions a step; the
+// worst of these is 3 % above its best.)
 constexpr int kMaxAttnSplit = 8;
 static int attn_split_for(const wgpt_device *dev, int n_head, int n_seq, int head_size, int context_len) {
   const int step = 4096 / head_size;
@@ -2508,8 +2511,8 @@ static int32_t forward_blocks_pair(wgpt_session *s, int n_tok) {
   __half *h = reinterpret_cast<__half *>(s->h), *o = reinterpret_cast<__half *>(s->o), *f = reinterpret_cast<__half *>(s->f);
   const bool o_pair = n_tok == 1 || attn_prefill_pair_ok(dev, hs);
   // A prompt from position 0 of more than one tile: q, k and v leave their product as pairs too, in the MLP's place (free then).
-  // us per pass, attn_prefill64_pair_kernel / this: GPT-2 65 / 333 / 1024 tokens 568 / 564, 846 / 790, 1525 / 1333, 64 x 128
-  // 5280 / 5090; XL 200 / 512 / 1024 4900 / 4800, 6900 / 6690, 12160 / 10400. One tile stays where it was.
+  // us per pass, back to back, attn_prefill64_pair_kernel / this: GPT-2 65 / 333 / 1024 tokens 572 / 572, 855 / 803, 1557 / 1385,
+  // 64 x 128 5630 / 5490; XL 200 / 510 / 1024 4977 / 4877, 7270 / 7066, 12460 / 11300. One tile stays where it was.
   const bool tc = n_tok > 64 && s->len == 0 && attn_prefill_pair_ok(dev, hs);
   CUtensorMap map_q, map_kv;
   if (tc) {

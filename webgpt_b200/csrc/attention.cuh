@@ -22,8 +22,9 @@ namespace wgpt {
 // NST steps of a CTA's slice are copied to shared memory ahead of the wait (cp.async, each thread the pieces that it will
 // use itself, so that no barrier is needed and no registers are held), the lines beyond them are asked for in L2. With eight
 // rows in registers per thread instead, requested behind the wait, 768 CTAs were five to an SM and a few of them a second
-// wave, and a CTA took 4 us from the wait. Whole completions in ms, before / now: GPT-2 8 x 64 + 64 tokens 23.6 / 23.1, 64 x 128
-// + 64 46.0 / 44.0, 16 x 300 + 64 32.9 / 30.8; XL 1 x 200 + 32 56.5 / 54.8, 16 x 96 + 24 66.2 / 63.4.
+// wave, and a CTA took 4 us from the wait. Whole completions in ms, that kernel / this one in one library: GPT-2 3 x 64 + 64
+// tokens 20.4 / 20.2, 8 x 64 + 64 23.8 / 23.3, 64 x 128 + 64 46.2 / 44.6, 16 x 300 + 64 33.1 / 31.1; XL 1 x 200 + 32 56.3 / 53.6,
+// 4 x 100 + 24 57.5 / 56.8, 16 x 96 + 24 67.5 / 64.7.
 // Split-K partial tiles of the QKV product that feeds a decode attention (batched decode on the tensor cores):
 // [slice][feature tile of 128][row = sequence][128], feature n of [0, 3E) = q | k | v. With FROM_QKV_PART the
 // attention CTA is that product's second stage for its own (sequence, head): it adds the slices in order, adds the

@@ -14,11 +14,11 @@
 //              accumulated across tiles in tensor memory.
 // S and O have two buffers each, so that the scores of the next tile are there when a tile is done. 256 columns of tensor memory
 // and 97 KB of shared memory. KG == 1: one group of four softmax warps, two CTAs an SM. KG == 2: two groups take alternate
-// tiles and meet at the end, one CTA an SM (167 registers): for grids where the chain of a row's tiles is what the kernel takes.
-// What bounds it: a softmax warp's own path, 0.75 us per tile of 64 keys (64 exponentials at eight cycles, six instructions each
-// around them, two trips to tensor memory) and 0.7 us until the tile's O is added; the tensor pipe needs 0.5. A GPT-2 layer of
-// 333 tokens 14.5 -> 8.5 us, an XL layer of 1024 66 -> 20 us. Against float64 the logits of one block are nearer than before
-// (GPT-2 at 1000 tokens 6.31e-6, was 6.61e-6; XL at 1024 2.00e-5, was 2.04e-5: most of it from the products).
+// tiles and meet at the end, one CTA an SM (168 registers): for grids where the chain of a row's tiles is what the kernel takes.
+// What bounds it: a softmax warp's own path, 0.75 us per tile of 64 keys (64 exponentials at eight cycles, seven instructions each
+// around them, two trips to tensor memory) and 0.7 us until the tile's O is added; the tensor pipe needs 0.5. Alone and
+// cold, that kernel / this one: a layer of GPT-2 at 333 / 1024 tokens 17.2 / 12.4 and 39.3 / 22.5 us, of XL at 1024 64 / 27 us.
+// Against float64 the logits are nearer than with that kernel (exp2_approx).
 // Every wait is bounded; on expiry *err = 3 and the result is void.
 #pragma once
 #include "attention.cuh"

@@ -127,7 +127,7 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
 
   // Scale and shift, up to two rows: asked for ahead of the weights and not waited for until the row is there. A CTA that
   // starts late, on an SM that its predecessor has just left, otherwise waits for them behind 148 rings of requests (3 us).
-  // XL 1 x 200 + 32 / 2 x 300 + 24 tokens: 54.4 / 50.3 -> 53.3 / 49.0 ms; with four rows 54.9 -> 56.1.
+  // XL 1 x 200 + 32 / 2 x 300 + 24 tokens: 54.15 / 49.9 -> 53.75 / 49.1 ms; with four rows 54.9 -> 56.1.
   constexpr bool kAsyncNorm = M <= 2;
   if (kAsyncNorm && p.gamma != nullptr && warp < GR_WARPS) {
     for (int i = tid; i < (p.K >> 2); i += 32 * GR_WARPS) {
