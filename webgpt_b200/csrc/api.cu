@@ -27,6 +27,7 @@
 #include "gemm_tc2.cuh"
 #include "gemm_pair.cuh"
 #include "gemm_split.cuh"
+#include "gemm_stream.cuh"
 #include "gemv_ring.cuh"
 #include "int8.cuh"
 #include "sampling.cuh"
@@ -982,6 +983,37 @@ static int32_t launch_gemm_pair(wgpt_device *dev, const __half *A, const __half 
   CK(launch_ex_x(dev->pdl, 2 * ps.KS, dev->stream, gemm_pair_kernel, dim3(2 * ps.KS * clusters), dim3(GP_THREADS), GP_SMEM_BYTES,
                  ma, mb, M, K, N, bn, b_exact ? 1 : 0, epi, dev->d_err));
   dev->launches++;
+  return WGPT_OK;
+}
+
+// Where gemm_stream_kernel is faster than gemm_pair_kernel, whose 256-row tile is mostly padding here: from two pieces of features
+// for every SM on, or where K is so short that the pair kernel's start and its epilogue are most of it. us per decode pass of one
+// block, pair / stream: n_embd 768, vocabulary 50257, 6 / 16 / 64 / 128 rows 92 / 67, 111 / 70, 172 / 98, 196 / 124; 9472, 6 / 64 / 128
+// rows 50.6 / 45.3, 75.8 / 73.5, 100 / 97; 4104, 6 / 128 rows 46.2 / 42.5, 94.6 / 94.3; 1000, 64 rows 64.8 / 67.0. n_embd 1600, 9472, 6 / 64 /
+// 128 rows 85.7 / 76.5, 118 / 115, 152 / 150; 4104, 64 rows 107 / 111. n_embd 384, 6 / 64 / 96 / 128 rows, vocabulary 65 37.6 / 35.0, 62.4 /
+// 54.6, 65.3 / 59.1, 74.8 / 69.5; 300 39.1 / 35.1, 58.1 / 54.9, 62.3 / 59.7, 70.5 / 71.2. n_embd 512 and 640, vocabulary 1000, 64 rows 61.7 /
+// 59.4, 65.6 / 63.4, 96 rows 65.4 / 64.8, 69.5 / 69.7.
+static bool stream_fits(const wgpt_device *dev, int M, int K, int N) {
+  return M <= GT_MAX_ROWS && (N >= 2 * GT_PIECE * dev->sm_count || (K <= 512 && M <= 96));
+}
+
+// out[M, N] = X . Wt^T from pair planes X [2][M][K] and W [2][N][K], the exponents in colscale [N].
+static int32_t launch_gemm_stream(wgpt_device *dev, const __half *X, const __half *W, int M, int K, int N, const float *colscale,
+                                  float *out) {
+  REQUIRE(aligned16(X) && aligned16(W) && K % 8 == 0, WGPT_ERR_ALIGN, "pair operands need 16-byte aligned rows");
+  StreamArgs a;
+  a.M = M; a.K = K; a.N = N;
+  a.rn = (M + 15) & ~15;
+  a.stages = (int)std::min<size_t>((dev->smem_optin - 2048) / stream_stage_bytes(a.rn), GT_MAX_STAGES);
+  a.colscale = colscale; a.out = out; a.ld = N;
+  a.err = dev->d_err;
+  CUtensorMap mw, mp, mx;
+  TRY(make_pair_map(&mw, W, 2 * (uint64_t)N, (uint64_t)K, 128, 1));
+  TRY(make_pair_map(&mp, W, 2 * (uint64_t)N, (uint64_t)K, GT_PIECE, 1));
+  TRY(make_pair_map(&mx, X, (uint64_t)M, (uint64_t)K, a.rn));
+  CK(allow_smem(dev, gemm_stream_kernel));
+  const int grid = std::min(dev->sm_count, (N + GT_PIECE - 1) / GT_PIECE);
+  LAUNCH_PDL(dev, gemm_stream_kernel, grid, GT_THREADS, 1024 + a.stages * stream_stage_bytes(a.rn), mw, mp, mx, a);
   return WGPT_OK;
 }
 
@@ -2830,13 +2862,14 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
     return WGPT_OK;
   }
   if (pair_mode) {
-    // pairs: the 256-row tile of the two-CTA kernel is mostly padding here, but 256 weight rows per 1536 tensor-core
-    // cycles and pair are what HBM delivers anyway
     __half *h = reinterpret_cast<__half *>(s->h);
     const size_t plane = (size_t)s->n_seq * E;
     TRY(launch_layernorm(dev, x_last, ld_last, m->lnf_g, m->lnf_b, nullptr, (size_t)E, s->n_seq, E, h, plane, m->s_hf));
     e.colscale = m->wte_p.cs;
-    TRY(launch_gemm_pair(dev, h, m->wte_p.p, s->n_seq, E, p.vocab_size, e));
+    if (stream_fits(dev, s->n_seq, E, p.vocab_size))
+      TRY(launch_gemm_stream(dev, h, m->wte_p.p, s->n_seq, E, p.vocab_size, m->wte_p.cs, s->logits));
+    else
+      TRY(launch_gemm_pair(dev, h, m->wte_p.p, s->n_seq, E, p.vocab_size, e));
     if (pick) TRY(pick_and_advance(s, n_tok));
     return WGPT_OK;
   }
