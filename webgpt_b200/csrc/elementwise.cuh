@@ -31,20 +31,22 @@ __global__ void gelu_kernel(const float4 *__restrict__ in, float4 *__restrict__ 
   }
 }
 
-// LayerNorm, one warp per row (normStats + norm, instructions.js:451-550):
+// LayerNorm (normStats + norm, instructions.js:451-550):
 // mean = sum/N, var = sum((x-mean)^2)/N, y = gamma*((x-mean)/sqrt(var+1e-5))+beta.
 // Row r of the input starts at in + r*ld_in (lets the caller normalise only the last row of each sequence).
-// V > 0: the row stays in registers, V float4 per lane (N <= 128 V), so it is read once and all its loads are in
-// flight together; V = 0 reads it three times (any N). planes != nullptr: the result goes out as a pair of
-// half-precision planes scaled by the power of two `scale` (pair.cuh), contiguous rows, plane stride `plane`.
-template <int V>
+// W warps share a row (1, 2 or 4; a CTA has four warps). V > 0: the row stays in registers, V float4 per lane (N <= 128 V W), so
+// it is read once and all its loads are in flight together; V = 0 (W = 1) reads it three times (any N). planes != nullptr: the
+// result goes out as a pair of half-precision planes scaled by the power of two `scale` (pair.cuh), contiguous rows, plane
+// stride `plane`.
+template <int V, int W>
 __global__ void __launch_bounds__(128)
 layernorm_kernel(const float *__restrict__ in, size_t ld_in, const float *__restrict__ gamma,
                  const float *__restrict__ beta, float *__restrict__ out, size_t ld_out, int rows, int N,
                  __half *__restrict__ planes, size_t plane, float scale) {
-  int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  int lane = threadIdx.x & 31;
-  const int n4 = N >> 2;
+  __shared__ float red[2][4];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = warp % W;
+  const int row = blockIdx.x * (4 / W) + warp / W;
+  const int n4 = N >> 2, i0 = part * 32 + lane;
   constexpr int R = V > 0 ? V : 1;
   pdl_launch_dependents();
   const float4 *g4 = reinterpret_cast<const float4 *>(gamma);
@@ -53,19 +55,31 @@ layernorm_kernel(const float *__restrict__ in, size_t ld_in, const float *__rest
   if (V > 0) {  // scale and shift are weights: ahead of the dependency wait
 #pragma unroll
     for (int j = 0; j < R; j++) {
-      const int i = lane + 32 * j;
+      const int i = i0 + 32 * W * j;
       gv[j] = i < n4 ? __ldg(g4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
       bv[j] = i < n4 ? __ldg(b4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
   pdl_wait();  // the rows come from the previous kernel (read through L2, see common.cuh)
-  if (row >= rows) return;
-  const float4 *x = reinterpret_cast<const float4 *>(in + (size_t)row * ld_in);
+  const bool live = row < rows;
+  if (W == 1 && !live) return;
+  const float4 *x = reinterpret_cast<const float4 *>(in + (size_t)(live ? row : 0) * ld_in);
+  // the row's sum out of its warps' sums, in warp order
+  auto row_sum = [&](float s, int k) {
+    s = warp_sum(s);
+    if (W == 1) return s;
+    if (lane == 0) red[k][warp] = s;
+    __syncthreads();
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < W; w++) t += red[k][warp - part + w];
+    return t;
+  };
   float4 v[R];
   float s = 0.f;
   if (V > 0) {
 #pragma unroll
-    for (int j = 0; j < R; j++) v[j] = lane + 32 * j < n4 ? __ldcg(x + lane + 32 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < R; j++) v[j] = i0 + 32 * W * j < n4 ? __ldcg(x + i0 + 32 * W * j) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int j = 0; j < R; j++) s += (v[j].x + v[j].y) + (v[j].z + v[j].w);
   } else {
@@ -74,12 +88,12 @@ layernorm_kernel(const float *__restrict__ in, size_t ld_in, const float *__rest
       s += (t.x + t.y) + (t.z + t.w);
     }
   }
-  const float mean = warp_sum(s) / (float)N;
+  const float mean = row_sum(s, 0) / (float)N;
   float q = 0.f;
   if (V > 0) {
 #pragma unroll
     for (int j = 0; j < R; j++)
-      if (lane + 32 * j < n4) {
+      if (i0 + 32 * W * j < n4) {
         const float a = v[j].x - mean, b = v[j].y - mean, c = v[j].z - mean, d = v[j].w - mean;
         q += (a * a + b * b) + (c * c + d * d);
       }
@@ -90,7 +104,8 @@ layernorm_kernel(const float *__restrict__ in, size_t ld_in, const float *__rest
       q += (a * a + b * b) + (c * c + d * d);
     }
   }
-  const float sd = sqrtf(warp_sum(q) / (float)N + 1e-5f);
+  const float sd = sqrtf(row_sum(q, 1) / (float)N + 1e-5f);
+  if (W > 1 && !live) return;
   auto put = [&](int i, float4 t, float4 g, float4 b) {
     const float4 y = make_float4(g.x * ((t.x - mean) / sd) + b.x, g.y * ((t.y - mean) / sd) + b.y,
                                  g.z * ((t.z - mean) / sd) + b.z, g.w * ((t.w - mean) / sd) + b.w);
@@ -106,7 +121,7 @@ layernorm_kernel(const float *__restrict__ in, size_t ld_in, const float *__rest
   if (V > 0) {
 #pragma unroll
     for (int j = 0; j < R; j++)
-      if (lane + 32 * j < n4) put(lane + 32 * j, v[j], gv[j], bv[j]);
+      if (i0 + 32 * W * j < n4) put(i0 + 32 * W * j, v[j], gv[j], bv[j]);
   } else {
     for (int i = lane; i < n4; i += 32) put(i, __ldcg(x + i), __ldg(g4 + i), __ldg(b4 + i));
   }
