@@ -1,0 +1,74 @@
+"""CPU checks of the rule that gives a prompt's products their kernel and shape (csrc/pair_plan.h, product_shape): every shape
+that it can return can be launched, and the prompts that the GPU test names take every form."""
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+from test_gpu_product_forms import PROMPTS
+from test_split_plan import SMEM
+
+DRIVER = r"""
+#include "pair_plan.h"
+using namespace wgpt;
+extern "C" void shape(const int *clusters, long long smem, int M, int K, int N, long long *out) {
+  const ProductShape s = product_shape(SplitLimits{clusters, (size_t)smem}, 74, M, N, K);
+  const long long v[] = {s.split, s.pair.bn, s.pair.KS, s.sh.row_tiles, s.sh.rn, s.sh.S, s.sh.stages, (long long)s.sh.smem};
+  for (int i = 0; i < 8; i++) out[i] = v[i];
+}
+"""
+B200 = (0, 148, 74, 45, 33, 26, 22, 15, 15)
+
+
+@pytest.fixture(scope="module")
+def shape(tmp_path_factory):
+    d = tmp_path_factory.mktemp("product_plan")
+    src, lib = d / "plan.cpp", d / "plan.so"
+    src.write_text(DRIVER)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-I", os.path.join(ROOT, "webgpt_b200", "csrc"),
+                    str(src), "-o", str(lib)], check=True)
+    so = C.CDLL(str(lib))
+
+    def call(M, K, N, clusters=B200):
+        out = (C.c_longlong * 8)()
+        so.shape((C.c_int * 9)(*clusters), C.c_longlong(SMEM), M, K, N, out)
+        return dict(zip(("split", "bn", "KS", "row_tiles", "rn", "S", "stages", "smem"), out))
+
+    return call
+
+
+@pytest.mark.parametrize("clusters", [B200, (0, 148, 74, 48, 36, 28, 23, 20, 16), (0, 140, 66, 40, 28, 0, 0, 0, 0)])
+@pytest.mark.parametrize("E", [8, 64, 200, 384, 768, 1160, 1600, 3072])
+def test_shapes_can_be_launched(shape, E, clusters):
+    for K, N in ((E, 3 * E), (E, E), (E, 4 * E), (4 * E, E)):
+        for M in (9, 16, 17, 63, 64, 65, 100, 128, 129, 255, 256, 257, 300, 333, 384, 385, 511, 512, 513, 700, 768, 769, 1000, 1024):
+            s = shape(M, K, N, clusters)
+            if s["split"]:
+                assert s["rn"] % 16 == 0 and 16 <= s["rn"] <= 128 and s["row_tiles"] * s["rn"] >= M, (M, K, N, s)
+                assert 1 <= s["S"] <= min(8, (K + 63) // 64) and clusters[s["S"]] > 0 and s["stages"] >= 1, (M, K, N, s)
+                ring = max(s["stages"] * (32768 + s["rn"] * 256), s["rn"] * 512)
+                assert 1024 + ring <= s["smem"] <= SMEM, (M, K, N, s)
+            else:
+                assert s["bn"] % 32 == 0 and 64 <= s["bn"] <= 256 and s["KS"] in (1, 2), (M, K, N, s)
+                if s["KS"] == 2:
+                    assert K > 64 and ((M + 255) // 256) * -(-N // s["bn"]) <= clusters[4], (M, K, N, s)
+
+
+def form(s):
+    return ("split", min(s["S"], 2)) if s["split"] else ("pair", s["KS"])
+
+
+def test_prompts_of_the_gpu_test_take_every_form(shape):
+    """Each epilogue (q | k | v, output, GELU, down) with each form that the rule gives it at any width up to XL's."""
+    seen = set()
+    for E, M in PROMPTS:
+        for name, K, N in (("qkv", E, 3 * E), ("o", E, E), ("up", E, 4 * E), ("down", 4 * E, E)):
+            seen.add((name, form(shape(M, K, N))))
+    want = set()
+    for E in (384, 768, 1024, 1216, 1280, 1600):
+        for M in range(65, min(1024, 1200000 // E) + 1, 9):  # where the rule applies
+            for name, K, N in (("qkv", E, 3 * E), ("o", E, E), ("up", E, 4 * E), ("down", 4 * E, E)):
+                want.add((name, form(shape(M, K, N))))
+    assert want - seen == set()

@@ -980,9 +980,9 @@ static SplitLimits split_limits(const wgpt_device *dev) { return SplitLimits{dev
 
 // C = A . Wt^T from pair planes A [2][M][K] and W [2][N][K]; the exponents are in epi.colscale / epi.rowscale.
 static int32_t launch_gemm_pair(wgpt_device *dev, const __half *A, const __half *W, int M, int K, int N,
-                                const Epilogue &epi, bool b_exact = false) {
+                                const Epilogue &epi, bool b_exact = false, const PairShape *shape = nullptr) {
   REQUIRE(aligned16(A) && aligned16(W) && K % 8 == 0, WGPT_ERR_ALIGN, "pair operands need 16-byte aligned rows");
-  const PairShape ps = pair_shape(split_limits(dev), dev->sm_count / 2, M, N, K);
+  const PairShape ps = shape != nullptr ? *shape : pair_shape(split_limits(dev), dev->sm_count / 2, M, N, K);
   const int bn = ps.bn;
   CUtensorMap ma, mb;
   TRY(make_pair_map(&ma, A, (uint64_t)M, (uint64_t)K, GP_BM));
@@ -1157,9 +1157,18 @@ static int32_t launch_pair_operands(wgpt_device *dev, PairOperands &p) {
 static bool pair_operands_fit(int K) { return K % 8 == 0 && K <= 8 * 1536; }
 
 // A product of pairs with whichever kernel should be faster: CTA pairs on 256-row tiles, or 128-feature tiles with K split
-// over a cluster where the former would leave most pairs without a tile (GPT-2 at 333 rows: 0.98 against 1.24 ms per pass).
+// over a cluster where the former would leave most pairs without a tile (GPT-2 at 333 rows: 0.98 against 1.24 ms per pass). A
+// model's prompts go by product_shape, operators and exact codes, which it was not fitted to, by pair_product_splits.
 static int32_t launch_pair_product(wgpt_device *dev, const __half *X, const __half *W, int M, int K, int N,
                                    const Epilogue &epi, bool dyn = false, bool b_exact = false) {
+  if (!dyn && !b_exact && epi.rowscale == nullptr && product_shape_fitted(M, N, K) && (epi.ld & 3) == 0) {
+    const ProductShape ps = product_shape(split_limits(dev), dev->sm_count / 2, M, N, K);
+    if (!ps.split) return launch_gemm_pair(dev, X, W, M, K, N, epi, false, &ps.pair);
+    SplitArgs a;
+    memset(&a, 0, sizeof a);
+    a.w_planes = 2;
+    return launch_gemm_split(dev, ps.sh, X, W, M, K, N, epi, a);
+  }
   SplitShape sh;
   if (pair_product_splits(split_limits(dev), dev->sm_count / 2, M, K, N, b_exact ? 1 : 2, &sh) && N % 4 == 0 &&
       (epi.ld & 3) == 0) {

@@ -67,4 +67,60 @@ inline bool pair_product_splits(const SplitLimits &lim, int pairs, int M, int K,
   return sh->smem > 0 && split < big;
 }
 
+// The kernel and shape of a prompt's product in a model (weights known ahead, both planes, no row factors): the cheapest of all
+// shapes of both kernels by one estimate, in cycles, fitted to 55 prompts of 70 to 1024 rows at n_embd 768, 1024, 1280 and 1600 of
+// which every shape of each of the four products was timed inside whole passes. What the estimates above had wrong: an MMA
+// step of the split form waits less for L2 than 40 bytes a cycle, its start and exchange are 2400 cycles and not 9000, and one
+// CTA without a cluster pays more, not less, for it stores its rows alone; the pair form's epilogue grows with its columns.
+// us per pass, those estimates / this rule: GPT-2 240 / 333 / 370 / 540 / 700 / 1024 tokens 681 / 665, 766 / 766, 841 / 782, 999 / 931, 1100 /
+// 1064, 1356 / 1307, 8 / 12 sequences of 64 / 128 959 / 909, 1455 / 1383; XL 200 / 290 / 333 / 512 / 700 / 1024 4604 / 4604, 5749 / 5339, 5889 /
+// 5453, 6903 / 6692, 8898 / 8677, 4 sequences of 96 6039 / 5671. Not beyond 1024 rows, which were not fitted (GPT-2 16 / 32 / 64 sequences of
+// 128 1753 / 1722, 2989 / 2904, 5412 / 5641, XL 12 / 16 of 96 11873 / 12045, 14336 / 14528), nor where a wide model's prompt runs into the
+// power cap and the shapes come out alike (XL 850 / 930 / 1024 10514 / 10529, 10763 / 10832, 11111 / 11077).
+constexpr int kFittedRows = 1024;
+inline bool product_shape_fitted(int M, int N, int K) { return M <= kFittedRows && (long long)M * (K < N ? K : N) <= 1200000; }
+struct ProductShape {
+  bool split;
+  SplitShape sh;   // split
+  PairShape pair;  // otherwise
+};
+inline ProductShape product_shape(const SplitLimits &lim, int pairs, int M, int N, int K) {
+  const int kb = (K + GS_BK - 1) / GS_BK, ft = (N + 127) / 128, rt0 = (M + 127) / 128, m_tiles = (M + 255) / 256;
+  ProductShape best = {false, {}, {256, 1}};
+  double least = 1e30;
+  for (int bn = 256; bn >= 64; bn -= 32) {
+    const int tiles = m_tiles * ((N + bn - 1) / bn);
+    const double per_kb = std::fmax(4.6 * bn, 408 + 1.5 * bn);
+    const double one = (double)((tiles + pairs - 1) / pairs) * kb * per_kb + 8050 + 86.0 * bn;
+    if (one < least) {
+      least = one;
+      best.pair = {bn, 1};
+    }
+    const double two = (double)((kb + 1) / 2) * per_kb + 8050 + 51.0 * bn;
+    if (kb >= 2 && tiles <= lim.max_clusters[4] && two < least) {
+      least = two;
+      best.pair = {bn, 2};
+    }
+  }
+  if (N % 4 != 0) return best;
+  for (int rt = rt0; rt <= rt0 + 2; rt++) {
+    SplitShape t = {};
+    t.rn = (((M + rt - 1) / rt) + 15) & ~15;
+    t.row_tiles = (M + t.rn - 1) / t.rn;
+    for (t.S = 1; t.S <= 8 && t.S <= kb; t.S++) {
+      if (lim.max_clusters[t.S] < 1) continue;
+      const int rounds = (ft * t.row_tiles + lim.max_clusters[t.S] - 1) / lim.max_clusters[t.S];
+      const double c = rounds * (((kb + t.S - 1) / t.S) * std::fmax(6.0 * t.rn, 620 + 1.35 * t.rn) + (t.S == 1 ? 5000 : 2400) + 68.0 * t.rn);
+      if (c >= least) continue;
+      SplitShape placed = t;
+      split_place(placed, lim, K, 2, false);
+      if (placed.smem == 0) continue;
+      least = c;
+      best.split = true;
+      best.sh = placed;
+    }
+  }
+  return best;
+}
+
 }  // namespace wgpt
