@@ -14,8 +14,8 @@
 //   store       : a lane is a feature, so a warp stores 32 neighbouring values of a row (128 bytes; a row of 50257 floats is
 //                 aligned to four bytes only).
 //
-// What bounds it: HBM. A decode pass of GPT-2 with 8 / 64 sequences 362 -> 335 / 636 -> 561 us against gemm_pair_kernel (107 us cold at 64
-// rows: 256 rows of the pair's tile are multiplied and read back whatever the batch is), XL with 16 sequences 2.56 -> 2.52 ms. See
+// What bounds it: HBM. A decode pass of GPT-2 with 8 / 64 sequences 362 -> 335 / 636 -> 561 us against gemm_pair_kernel (cold 54 and
+// 107 us there, 33 and 35 here: 256 rows of the pair's tile are multiplied and read back whatever the batch is), XL with 16 sequences 2.56 -> 2.52 ms. See
 // stream_fits in api.cu for where it takes over.
 // Every wait is bounded; on expiry *err = 3, the copies in flight get another bounded wait, and the result is void.
 #pragma once
