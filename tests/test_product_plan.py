@@ -7,7 +7,7 @@ import subprocess
 import pytest
 
 from conftest import ROOT
-from test_gpu_product_forms import PROMPTS
+from test_gpu_product_forms import PROMPTS, TRUNCATIONS
 from test_split_plan import SMEM
 
 DRIVER = r"""
@@ -17,6 +17,13 @@ extern "C" void shape(const int *clusters, long long smem, int M, int K, int N, 
   const ProductShape s = product_shape(SplitLimits{clusters, (size_t)smem}, 74, M, N, K);
   const long long v[] = {s.split, s.pair.bn, s.pair.KS, s.sh.row_tiles, s.sh.rn, s.sh.S, s.sh.stages, (long long)s.sh.smem};
   for (int i = 0; i < 8; i++) out[i] = v[i];
+}
+extern "C" void general(const int *clusters, long long smem, int M, int K, int N, int *out) {  // the route of other callers
+  const SplitLimits lim{clusters, (size_t)smem};
+  SplitShape sh;
+  out[0] = pair_product_splits(lim, 74, M, K, N, 2, &sh);
+  out[1] = sh.S;
+  out[2] = pair_shape(lim, 74, M, N, K).KS;
 }
 """
 B200 = (0, 148, 74, 45, 33, 26, 22, 15, 15)
@@ -36,7 +43,33 @@ def shape(tmp_path_factory):
         so.shape((C.c_int * 9)(*clusters), C.c_longlong(SMEM), M, K, N, out)
         return dict(zip(("split", "bn", "KS", "row_tiles", "rn", "S", "stages", "smem"), out))
 
+    def general(M, K, N, clusters=B200):
+        out = (C.c_int * 3)()
+        so.general((C.c_int * 9)(*clusters), C.c_longlong(SMEM), M, K, N, out)
+        return dict(zip(("split", "S", "KS"), out))
+
+    call.general = general
     return call
+
+
+def truncations(s, K):
+    """Truncating additions to the large sum: four per k-block and slice in the split form, twelve in the pair form."""
+    kb = (K + 63) // 64
+    return 4 * -(-kb // s["S"]) if s["split"] else 12 * -(-kb // s["KS"])
+
+
+@pytest.mark.parametrize("E", [64, 256, 384, 768, 1024, 1280, 1600, 2048, 3072])
+def test_no_prompt_truncates_more_often(shape, E):
+    """Against the shape that the same product takes outside a prompt, whose sums are what a prompt's have to be at least."""
+    for K, N in ((E, 3 * E), (E, E), (E, 4 * E), (4 * E, E)):
+        for M in range(9, 1025):
+            s, g = shape(M, K, N), shape.general(M, K, N)
+            assert truncations(s, K) <= truncations(g, K), (M, K, N, s, g)
+
+
+@pytest.mark.parametrize("E,n,up,down", TRUNCATIONS)
+def test_truncations_of_the_gpu_test(shape, E, n, up, down):
+    assert truncations(shape.general(n, E, 4 * E), E) == up and truncations(shape.general(n, 4 * E, E), 4 * E) == down
 
 
 @pytest.mark.parametrize("clusters", [B200, (0, 148, 74, 48, 36, 28, 23, 20, 16), (0, 140, 66, 40, 28, 0, 0, 0, 0)])

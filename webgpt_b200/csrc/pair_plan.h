@@ -84,40 +84,54 @@ struct ProductShape {
   SplitShape sh;   // split
   PairShape pair;  // otherwise
 };
+// Additions to the large sum of one output over K, each of which the tensor core truncates (gemm_pair.cuh): the pair form adds
+// all three products of a 16-deep step to it, the split form the large one alone; slices of K are sums of their own.
+inline int product_truncations(const ProductShape &s, int K) {
+  const int kb = (K + GS_BK - 1) / GS_BK;
+  return s.split ? 4 * ((kb + s.sh.S - 1) / s.sh.S) : 12 * ((kb + s.pair.KS - 1) / s.pair.KS);
+}
+// No shape that truncates more often than the one of the estimates above. Without that limit the down projection went to two pairs a
+// tile at n_embd 768 from 897 rows on, 1024 from 641, 1280 from 561, 1600 from 401 to 512; 2-norm from float64 of the rows behind one
+// block whose down projection prevails, estimates above / without / with the limit: 768 x 1000 rows 7.92e-6 / 8.42e-6 / 5.15e-6, 1024 x
+// 700 9.13e-6 / 1.06e-5 / 6.39e-6, 1280 x 600 1.10e-5 / 1.53e-5 / 1.10e-5, 1600 x 512 1.37e-5 / 1.91e-5 / 1.37e-5, 2048 x 300 1.76e-5 / 2.10e-5 /
+// 1.24e-5. What it costs: GPT-2 1024 tokens 1263 -> 1289 us, XL 416 / 512 6197 -> 6324, 6468 -> 6725.
 inline ProductShape product_shape(const SplitLimits &lim, int pairs, int M, int N, int K) {
   const int kb = (K + GS_BK - 1) / GS_BK, ft = (N + 127) / 128, rt0 = (M + 127) / 128, m_tiles = (M + 255) / 256;
-  ProductShape best = {false, {}, {256, 1}};
+  ProductShape best = {}, t = {};
+  best.split = pair_product_splits(lim, pairs, M, K, N, 2, &best.sh) && N % 4 == 0;
+  if (!best.split) best.pair = pair_shape(lim, pairs, M, N, K);
+  const int most = product_truncations(best, K);
   double least = 1e30;
-  for (int bn = 256; bn >= 64; bn -= 32) {
-    const int tiles = m_tiles * ((N + bn - 1) / bn);
+  for (t.pair.bn = 256; t.pair.bn >= 64; t.pair.bn -= 32) {
+    const int bn = t.pair.bn, tiles = m_tiles * ((N + bn - 1) / bn);
     const double per_kb = std::fmax(4.6 * bn, 408 + 1.5 * bn);
-    const double one = (double)((tiles + pairs - 1) / pairs) * kb * per_kb + 8050 + 86.0 * bn;
-    if (one < least) {
-      least = one;
-      best.pair = {bn, 1};
-    }
-    const double two = (double)((kb + 1) / 2) * per_kb + 8050 + 51.0 * bn;
-    if (kb >= 2 && tiles <= lim.max_clusters[4] && two < least) {
-      least = two;
-      best.pair = {bn, 2};
+    for (t.pair.KS = 1; t.pair.KS <= 2; t.pair.KS++) {
+      if ((t.pair.KS == 2 && (kb < 2 || tiles > lim.max_clusters[4])) || product_truncations(t, K) > most) continue;
+      const double c = t.pair.KS == 1 ? (double)((tiles + pairs - 1) / pairs) * kb * per_kb + 8050 + 86.0 * bn
+                                      : (double)((kb + 1) / 2) * per_kb + 8050 + 51.0 * bn;
+      if (c < least) {
+        least = c;
+        best = t;
+      }
     }
   }
   if (N % 4 != 0) return best;
+  t.split = true;
   for (int rt = rt0; rt <= rt0 + 2; rt++) {
-    SplitShape t = {};
-    t.rn = (((M + rt - 1) / rt) + 15) & ~15;
-    t.row_tiles = (M + t.rn - 1) / t.rn;
-    for (t.S = 1; t.S <= 8 && t.S <= kb; t.S++) {
-      if (lim.max_clusters[t.S] < 1) continue;
-      const int rounds = (ft * t.row_tiles + lim.max_clusters[t.S] - 1) / lim.max_clusters[t.S];
-      const double c = rounds * (((kb + t.S - 1) / t.S) * std::fmax(6.0 * t.rn, 620 + 1.35 * t.rn) + (t.S == 1 ? 5000 : 2400) + 68.0 * t.rn);
+    t.sh = {};
+    t.sh.rn = (((M + rt - 1) / rt) + 15) & ~15;
+    t.sh.row_tiles = (M + t.sh.rn - 1) / t.sh.rn;
+    for (t.sh.S = 1; t.sh.S <= 8 && t.sh.S <= kb; t.sh.S++) {
+      const int rn = t.sh.rn, S = t.sh.S;
+      if (lim.max_clusters[S] < 1 || product_truncations(t, K) > most) continue;
+      const int rounds = (ft * t.sh.row_tiles + lim.max_clusters[S] - 1) / lim.max_clusters[S];
+      const double c = rounds * (((kb + S - 1) / S) * std::fmax(6.0 * rn, 620 + 1.35 * rn) + (S == 1 ? 5000 : 2400) + 68.0 * rn);
       if (c >= least) continue;
-      SplitShape placed = t;
-      split_place(placed, lim, K, 2, false);
-      if (placed.smem == 0) continue;
+      ProductShape placed = t;
+      split_place(placed.sh, lim, K, 2, false);
+      if (placed.sh.smem == 0) continue;
       least = c;
-      best.split = true;
-      best.sh = placed;
+      best = placed;
     }
   }
   return best;
