@@ -8,7 +8,7 @@ from webgpt_b200 import synth
 
 pytestmark = pytest.mark.gpu
 
-PROMPTS = [(384, 70), (384, 700), (768, 420), (768, 1023), (1216, 250), (1600, 70), (1600, 200), (1600, 333), (1600, 700)]
+PROMPTS = [(384, 70), (384, 700), (768, 420), (768, 1023), (1216, 250), (1600, 70), (1600, 200), (1600, 333), (1600, 700), (1600, 800)]
 
 
 @pytest.mark.parametrize("E,n", PROMPTS)

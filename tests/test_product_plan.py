@@ -67,6 +67,13 @@ def test_no_prompt_truncates_more_often(shape, E):
             assert truncations(s, K) <= truncations(g, K), (M, K, N, s, g)
 
 
+@pytest.mark.parametrize("rows", range(129, 161))
+def test_shapes_within_the_estimates_error_stay(shape, rows):
+    """XL's up projection at 144 to 160 rows: the shape that the estimate has 5 % ahead makes a pass up to 3 % longer."""
+    s, g = shape(rows, 1600, 6400), shape.general(rows, 1600, 6400)
+    assert s["split"] == g["split"] == 0 and s["KS"] == g["KS"]
+
+
 @pytest.mark.parametrize("E,n,up,down", TRUNCATIONS)
 def test_truncations_of_the_gpu_test(shape, E, n, up, down):
     assert truncations(shape.general(n, E, 4 * E), E) == up and truncations(shape.general(n, 4 * E, E), 4 * E) == down
@@ -101,7 +108,7 @@ def test_prompts_of_the_gpu_test_take_every_form(shape):
             seen.add((name, form(shape(M, K, N))))
     want = set()
     for E in (384, 768, 1024, 1216, 1280, 1600):
-        for M in range(65, min(1024, 1200000 // E) + 1, 9):  # where the rule applies
+        for M in range(65, 1025, 9):  # where the rule applies
             for name, K, N in (("qkv", E, 3 * E), ("o", E, E), ("up", E, 4 * E), ("down", 4 * E, E)):
                 want.add((name, form(shape(M, K, N))))
     assert want - seen == set()

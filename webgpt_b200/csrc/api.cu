@@ -1161,7 +1161,7 @@ static bool pair_operands_fit(int K) { return K % 8 == 0 && K <= 8 * 1536; }
 // model's prompts go by product_shape, operators and exact codes, which it was not fitted to, by pair_product_splits.
 static int32_t launch_pair_product(wgpt_device *dev, const __half *X, const __half *W, int M, int K, int N,
                                    const Epilogue &epi, bool dyn = false, bool b_exact = false) {
-  if (!dyn && !b_exact && epi.rowscale == nullptr && product_shape_fitted(M, N, K) && (epi.ld & 3) == 0) {
+  if (!dyn && !b_exact && epi.rowscale == nullptr && M <= kFittedRows && (epi.ld & 3) == 0) {
     const ProductShape ps = product_shape(split_limits(dev), dev->sm_count / 2, M, N, K);
     if (!ps.split) return launch_gemm_pair(dev, X, W, M, K, N, epi, false, &ps.pair);
     SplitArgs a;

@@ -67,18 +67,6 @@ inline bool pair_product_splits(const SplitLimits &lim, int pairs, int M, int K,
   return sh->smem > 0 && split < big;
 }
 
-// The kernel and shape of a prompt's product in a model (weights known ahead, both planes, no row factors): the cheapest of all
-// shapes of both kernels by one estimate, in cycles, fitted to 55 prompts of 70 to 1024 rows at n_embd 768, 1024, 1280 and 1600 of
-// which every shape of each of the four products was timed inside whole passes. What the estimates above had wrong: an MMA
-// step of the split form waits less for L2 than 40 bytes a cycle, its start and exchange are 2400 cycles and not 9000, and one
-// CTA without a cluster pays more, not less, for it stores its rows alone; the pair form's epilogue grows with its columns.
-// us per pass, those estimates / this rule: GPT-2 240 / 333 / 370 / 540 / 700 / 1024 tokens 681 / 665, 766 / 766, 841 / 782, 999 / 931, 1100 /
-// 1064, 1356 / 1307, 8 / 12 sequences of 64 / 128 959 / 909, 1455 / 1383; XL 200 / 290 / 333 / 512 / 700 / 1024 4604 / 4604, 5749 / 5339, 5889 /
-// 5453, 6903 / 6692, 8898 / 8677, 4 sequences of 96 6039 / 5671. Not beyond 1024 rows, which were not fitted (GPT-2 16 / 32 / 64 sequences of
-// 128 1753 / 1722, 2989 / 2904, 5412 / 5641, XL 12 / 16 of 96 11873 / 12045, 14336 / 14528), nor where a wide model's prompt runs into the
-// power cap and the shapes come out alike (XL 850 / 930 / 1024 10514 / 10529, 10763 / 10832, 11111 / 11077).
-constexpr int kFittedRows = 1024;
-inline bool product_shape_fitted(int M, int N, int K) { return M <= kFittedRows && (long long)M * (K < N ? K : N) <= 1200000; }
 struct ProductShape {
   bool split;
   SplitShape sh;   // split
@@ -90,25 +78,60 @@ inline int product_truncations(const ProductShape &s, int K) {
   const int kb = (K + GS_BK - 1) / GS_BK;
   return s.split ? 4 * ((kb + s.sh.S - 1) / s.sh.S) : 12 * ((kb + s.pair.KS - 1) / s.pair.KS);
 }
-// No shape that truncates more often than the one of the estimates above. Without that limit the down projection went to two pairs a
-// tile at n_embd 768 from 897 rows on, 1024 from 641, 1280 from 561, 1600 from 401 to 512; 2-norm from float64 of the rows behind one
-// block whose down projection prevails, estimates above / without / with the limit: 768 x 1000 rows 7.92e-6 / 8.42e-6 / 5.15e-6, 1024 x
-// 700 9.13e-6 / 1.06e-5 / 6.39e-6, 1280 x 600 1.10e-5 / 1.53e-5 / 1.10e-5, 1600 x 512 1.37e-5 / 1.91e-5 / 1.37e-5, 2048 x 300 1.76e-5 / 2.10e-5 /
-// 1.24e-5. What it costs: GPT-2 1024 tokens 1263 -> 1289 us, XL 416 / 512 6197 -> 6324, 6468 -> 6725.
+
+// Cycles of a product in a prompt (weights known ahead, both planes, no row factors), fitted to 55 prompts of 70 to 1024 rows at
+// n_embd 768, 1024, 1280 and 1600 of which every shape of each of the four products was timed inside whole passes. Against the
+// estimates above: an MMA step of the split form waits less for L2 than 40 bytes a cycle, its start and exchange are 2400 cycles
+// and not 9000, and one CTA without a cluster pays more, not less, for it stores its rows alone; the pair form's epilogue grows
+// with its columns. Good to about a tenth.
+inline double product_cycles(const SplitLimits &lim, int pairs, int M, int N, int K, const ProductShape &s) {
+  const int kb = (K + GS_BK - 1) / GS_BK;
+  if (s.split) {
+    const int rn = s.sh.rn, S = s.sh.S, rounds = ((N + 127) / 128 * s.sh.row_tiles + lim.max_clusters[S] - 1) / lim.max_clusters[S];
+    return rounds * (((kb + S - 1) / S) * std::fmax(6.0 * rn, 620 + 1.35 * rn) + (S == 1 ? 5000 : 2400) + 68.0 * rn);
+  }
+  const int bn = s.pair.bn, tiles = (M + 255) / 256 * ((N + bn - 1) / bn);
+  const double per_kb = std::fmax(4.6 * bn, 408 + 1.5 * bn);
+  return s.pair.KS == 1 ? (double)((tiles + pairs - 1) / pairs) * kb * per_kb + 8050 + 86.0 * bn
+                        : (double)((kb + 1) / 2) * per_kb + 8050 + 51.0 * bn;
+}
+
+// The kernel and shape of a prompt's product in a model: the cheapest of all shapes of both kernels by product_cycles, if it is
+// cheaper by 6 % at least than the shape of the estimates above and truncates no more often.
+//
+// The 6 %: less than that the estimate does not tell apart. Without them XL at 144 to 160 rows takes its up projection in CTAs without a
+// cluster, 4173 -> 4224 and 4235 -> 4366 us a pass; 8 % and more give up what XL gains at 513 to 1024 rows.
+//
+// The truncations: without that limit the down projection went to two pairs a tile at n_embd 768 from 897 rows on, 1024 from 641, 1280
+// from 561, 1600 at 401 to 512; 2-norm from float64 of the rows behind one block whose down projection prevails, estimates above / without /
+// with the limit: 768 x 1000 rows 7.92e-6 / 8.42e-6 / 5.15e-6, 1024 x 700 9.13e-6 / 1.06e-5 / 6.39e-6, 1280 x 600 1.10e-5 / 1.53e-5 / 1.10e-5,
+// 1600 x 512 1.37e-5 / 1.91e-5 / 1.37e-5, 2048 x 300 1.76e-5 / 2.10e-5 / 1.24e-5. Without it GPT-2's 1024 tokens would take 1268 us in place of 1295,
+// XL's 416 / 512 6.20 / 6.47 ms in place of 6.37 / 6.77.
+//
+// us per pass, the estimates above / this rule:
+//   n_embd 256, 12 layers: 70 / 200 / 333 / 512 / 1024 tokens 384 / 384, 501 / 501, 621 / 583, 672 / 619, 832 / 796
+//   384, 6: 130 / 240 / 416 / 512 / 700 / 1024 261 / 258, 298 / 299, 341 / 343, 420 / 385, 462 / 436, 530 / 516
+//   768, 12: 130 / 224 / 333 / 352 / 450 / 544 / 768 / 1024 547 / 548, 625 / 626, 718 / 716, 787 / 730, 861 / 808, 958 / 886, 1064 / 1050, 1296 / 1282
+//   1024, 24: 240 / 320 / 480 / 700 / 1024 1472 / 1396, 1711 / 1583, 2065 / 1939, 2562 / 2507, 3180 / 2964
+//   1280, 24: 160 / 288 / 385 / 480 / 576 / 769 / 1024 1640 / 1639, 2276 / 1893, 2405 / 2411, 2575 / 2575, 3001 / 2890, 3477 / 3372, 4160 / 3990
+//   1600, 48: 160 / 333 / 480 / 576 / 700 / 850 / 1024 4324 / 4332, 5696 / 5374, 6572 / 6601, 8053 / 7715, 8807 / 8538, 10505 / 10369, 11022 / 10944
+//   2048, 12: 136 / 176 / 288 / 480 / 768 / 1024 1240 / 1159, 1331 / 1277, 2030 / 1854, 2302 / 2304, 3125 / 3025, 3887 / 3887
+//   3072, 4: 96 / 160 / 288 / 480 / 1024 723 / 661, 918 / 920, 1292 / 1207, 1525 / 1493, 2692 / 2677
+//   4096, 2: 100 / 200 / 300 / 512 / 1024 607 / 532, 749 / 750, 1127 / 1102, 1233 / 1237, 2216 / 2211
+// None of the 112 prompts of that run is slower by more than two runs of one side differ (0.5 %). Not beyond 1024 rows, which were not fitted.
+constexpr int kFittedRows = 1024;
 inline ProductShape product_shape(const SplitLimits &lim, int pairs, int M, int N, int K) {
-  const int kb = (K + GS_BK - 1) / GS_BK, ft = (N + 127) / 128, rt0 = (M + 127) / 128, m_tiles = (M + 255) / 256;
+  const int kb = (K + GS_BK - 1) / GS_BK, rt0 = (M + 127) / 128;
   ProductShape best = {}, t = {};
   best.split = pair_product_splits(lim, pairs, M, K, N, 2, &best.sh) && N % 4 == 0;
   if (!best.split) best.pair = pair_shape(lim, pairs, M, N, K);
   const int most = product_truncations(best, K);
-  double least = 1e30;
+  double least = 0.94 * product_cycles(lim, pairs, M, N, K, best);
   for (t.pair.bn = 256; t.pair.bn >= 64; t.pair.bn -= 32) {
-    const int bn = t.pair.bn, tiles = m_tiles * ((N + bn - 1) / bn);
-    const double per_kb = std::fmax(4.6 * bn, 408 + 1.5 * bn);
+    const int tiles = (M + 255) / 256 * ((N + t.pair.bn - 1) / t.pair.bn);
     for (t.pair.KS = 1; t.pair.KS <= 2; t.pair.KS++) {
       if ((t.pair.KS == 2 && (kb < 2 || tiles > lim.max_clusters[4])) || product_truncations(t, K) > most) continue;
-      const double c = t.pair.KS == 1 ? (double)((tiles + pairs - 1) / pairs) * kb * per_kb + 8050 + 86.0 * bn
-                                      : (double)((kb + 1) / 2) * per_kb + 8050 + 51.0 * bn;
+      const double c = product_cycles(lim, pairs, M, N, K, t);
       if (c < least) {
         least = c;
         best = t;
@@ -122,10 +145,8 @@ inline ProductShape product_shape(const SplitLimits &lim, int pairs, int M, int 
     t.sh.rn = (((M + rt - 1) / rt) + 15) & ~15;
     t.sh.row_tiles = (M + t.sh.rn - 1) / t.sh.rn;
     for (t.sh.S = 1; t.sh.S <= 8 && t.sh.S <= kb; t.sh.S++) {
-      const int rn = t.sh.rn, S = t.sh.S;
-      if (lim.max_clusters[S] < 1 || product_truncations(t, K) > most) continue;
-      const int rounds = (ft * t.sh.row_tiles + lim.max_clusters[S] - 1) / lim.max_clusters[S];
-      const double c = rounds * (((kb + S - 1) / S) * std::fmax(6.0 * rn, 620 + 1.35 * rn) + (S == 1 ? 5000 : 2400) + 68.0 * rn);
+      if (lim.max_clusters[t.sh.S] < 1 || product_truncations(t, K) > most) continue;
+      const double c = product_cycles(lim, pairs, M, N, K, t);
       if (c >= least) continue;
       ProductShape placed = t;
       split_place(placed.sh, lim, K, 2, false);
