@@ -96,29 +96,30 @@ inline double product_cycles(const SplitLimits &lim, int pairs, int M, int N, in
                         : (double)((kb + 1) / 2) * per_kb + 8050 + 51.0 * bn;
 }
 
-// The kernel and shape of a prompt's product in a model: the cheapest of all shapes of both kernels by product_cycles, if it is
-// cheaper by 6 % at least than the shape of the estimates above and truncates no more often.
+// The kernel and shape of a prompt's product in a model: the cheapest of all shapes of both kernels by product_cycles, if that has it
+// ahead of the shape of the estimates above by 3 % with the same kernel or by 6 % with the other, and if it truncates no more often.
 //
-// The 6 %: less than that the estimate does not tell apart. Without them XL at 144 to 160 rows takes its up projection in CTAs without a
-// cluster, 4173 -> 4224 and 4235 -> 4366 us a pass; 8 % and more give up what XL gains at 513 to 1024 rows.
+// The margins: within a kernel the estimate orders shapes well, between the two it errs by up to a tenth. With 3 % for both XL at 144 to 160
+// rows takes its up projection in CTAs without a cluster, 4173 -> 4221 and 4235 -> 4378 us a pass; with 6 % for both XL loses 2 % at 257 to 512.
 //
 // The truncations: without that limit the down projection went to two pairs a tile at n_embd 768 from 897 rows on, 1024 from 641, 1280
 // from 561, 1600 at 401 to 512; 2-norm from float64 of the rows behind one block whose down projection prevails, estimates above / without /
 // with the limit: 768 x 1000 rows 7.92e-6 / 8.42e-6 / 5.15e-6, 1024 x 700 9.13e-6 / 1.06e-5 / 6.39e-6, 1280 x 600 1.10e-5 / 1.53e-5 / 1.10e-5,
-// 1600 x 512 1.37e-5 / 1.91e-5 / 1.37e-5, 2048 x 300 1.76e-5 / 2.10e-5 / 1.24e-5. Without it GPT-2's 1024 tokens would take 1268 us in place of 1295,
-// XL's 416 / 512 6.20 / 6.47 ms in place of 6.37 / 6.77.
+// 1600 x 512 1.37e-5 / 1.91e-5 / 1.37e-5, 2048 x 300 1.76e-5 / 2.10e-5 / 1.24e-5. Without it GPT-2's 1024 tokens would take 1268 us in place of 1291,
+// XL's 416 / 512 6.24 / 6.53 ms in place of 6.38 / 6.73.
 //
-// us per pass, the estimates above / this rule:
-//   n_embd 256, 12 layers: 70 / 200 / 333 / 512 / 1024 tokens 384 / 384, 501 / 501, 621 / 583, 672 / 619, 832 / 796
-//   384, 6: 130 / 240 / 416 / 512 / 700 / 1024 261 / 258, 298 / 299, 341 / 343, 420 / 385, 462 / 436, 530 / 516
-//   768, 12: 130 / 224 / 333 / 352 / 450 / 544 / 768 / 1024 547 / 548, 625 / 626, 718 / 716, 787 / 730, 861 / 808, 958 / 886, 1064 / 1050, 1296 / 1282
-//   1024, 24: 240 / 320 / 480 / 700 / 1024 1472 / 1396, 1711 / 1583, 2065 / 1939, 2562 / 2507, 3180 / 2964
-//   1280, 24: 160 / 288 / 385 / 480 / 576 / 769 / 1024 1640 / 1639, 2276 / 1893, 2405 / 2411, 2575 / 2575, 3001 / 2890, 3477 / 3372, 4160 / 3990
-//   1600, 48: 160 / 333 / 480 / 576 / 700 / 850 / 1024 4324 / 4332, 5696 / 5374, 6572 / 6601, 8053 / 7715, 8807 / 8538, 10505 / 10369, 11022 / 10944
-//   2048, 12: 136 / 176 / 288 / 480 / 768 / 1024 1240 / 1159, 1331 / 1277, 2030 / 1854, 2302 / 2304, 3125 / 3025, 3887 / 3887
-//   3072, 4: 96 / 160 / 288 / 480 / 1024 723 / 661, 918 / 920, 1292 / 1207, 1525 / 1493, 2692 / 2677
-//   4096, 2: 100 / 200 / 300 / 512 / 1024 607 / 532, 749 / 750, 1127 / 1102, 1233 / 1237, 2216 / 2211
-// None of the 112 prompts of that run is slower by more than two runs of one side differ (0.5 %). Not beyond 1024 rows, which were not fitted.
+// us per pass, the estimates above / this rule (n_embd, layers):
+//   384, 6: 200 / 416 / 512 / 700 / 1024 tokens 291 / 292, 344 / 345, 423 / 386, 466 / 436, 532 / 515
+//   512, 8: 352 / 512 / 880 / 1000 tokens 481 / 451, 560 / 506, 690 / 668, 720 / 707
+//   768, 12: 352 / 450 / 544 / 700 / 900 / 1024 tokens 787 / 729, 861 / 810, 963 / 883, 1039 / 1014, 1231 / 1233, 1320 / 1291
+//   1024, 24: 240 / 320 / 500 / 700 / 1024 tokens 1481 / 1402, 1725 / 1582, 2074 / 1987, 2528 / 2490, 3168 / 2962
+//   1280, 24: 160 / 288 / 385 / 416 / 576 / 769 / 1024 tokens 1629 / 1630, 2255 / 1888, 2385 / 2414, 2468 / 2436, 2982 / 2871, 3580 / 3417, 4214 / 3976
+//   1600, 48: 160 / 333 / 416 / 512 / 576 / 700 / 850 / 1024 tokens 4218 / 4252, 5803 / 5328, 6503 / 6380, 6794 / 6734, 8109 / 7807, 8842 / 8593, 10520 / 10357, 11156 / 10991
+//   2048, 12: 136 / 176 / 288 / 450 / 576 / 768 / 1024 tokens 1243 / 1160, 1355 / 1304, 2048 / 1818, 2284 / 2239, 2938 / 2795, 3223 / 3055, 3937 / 3916
+//   3072, 4: 96 / 160 / 288 / 480 / 641 / 1024 tokens 720 / 657, 922 / 924, 1282 / 1204, 1509 / 1473, 1994 / 1966, 2656 / 2667
+//   4096, 2: 100 / 200 / 300 / 1024 tokens 601 / 528, 737 / 739, 1116 / 1118, 2227 / 2238
+// Of 108 prompts only 1280 x 385 is slower by more than two runs of one side differ (1.2 %, 416 rows 1.4 % faster). Not beyond 1024 rows,
+// which were not fitted.
 constexpr int kFittedRows = 1024;
 inline ProductShape product_shape(const SplitLimits &lim, int pairs, int M, int N, int K) {
   const int kb = (K + GS_BK - 1) / GS_BK, rt0 = (M + 127) / 128;
@@ -126,12 +127,13 @@ inline ProductShape product_shape(const SplitLimits &lim, int pairs, int M, int 
   best.split = pair_product_splits(lim, pairs, M, K, N, 2, &best.sh) && N % 4 == 0;
   if (!best.split) best.pair = pair_shape(lim, pairs, M, N, K);
   const int most = product_truncations(best, K);
-  double least = 0.94 * product_cycles(lim, pairs, M, N, K, best);
+  const bool general = best.split;
+  double least = product_cycles(lim, pairs, M, N, K, best);
   for (t.pair.bn = 256; t.pair.bn >= 64; t.pair.bn -= 32) {
     const int tiles = (M + 255) / 256 * ((N + t.pair.bn - 1) / t.pair.bn);
     for (t.pair.KS = 1; t.pair.KS <= 2; t.pair.KS++) {
       if ((t.pair.KS == 2 && (kb < 2 || tiles > lim.max_clusters[4])) || product_truncations(t, K) > most) continue;
-      const double c = product_cycles(lim, pairs, M, N, K, t);
+      const double c = (general ? 1.06 : 1.03) * product_cycles(lim, pairs, M, N, K, t);
       if (c < least) {
         least = c;
         best = t;
@@ -146,7 +148,7 @@ inline ProductShape product_shape(const SplitLimits &lim, int pairs, int M, int 
     t.sh.row_tiles = (M + t.sh.rn - 1) / t.sh.rn;
     for (t.sh.S = 1; t.sh.S <= 8 && t.sh.S <= kb; t.sh.S++) {
       if (lim.max_clusters[t.sh.S] < 1 || product_truncations(t, K) > most) continue;
-      const double c = product_cycles(lim, pairs, M, N, K, t);
+      const double c = (general ? 1.03 : 1.06) * product_cycles(lim, pairs, M, N, K, t);
       if (c >= least) continue;
       ProductShape placed = t;
       split_place(placed.sh, lim, K, 2, false);
