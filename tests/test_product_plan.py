@@ -18,6 +18,7 @@ extern "C" void shape(const int *clusters, long long smem, int M, int K, int N, 
   const long long v[] = {s.split, s.pair.bn, s.pair.KS, s.sh.row_tiles, s.sh.rn, s.sh.S, s.sh.stages, (long long)s.sh.smem};
   for (int i = 0; i < 8; i++) out[i] = v[i];
 }
+extern "C" int ln_warps(int rows, int N) { return layernorm_warps(rows, N); }
 extern "C" void general(const int *clusters, long long smem, int M, int K, int N, int *out) {  // the route of other callers
   const SplitLimits lim{clusters, (size_t)smem};
   SplitShape sh;
@@ -49,6 +50,7 @@ def shape(tmp_path_factory):
         return dict(zip(("split", "S", "KS"), out))
 
     call.general = general
+    call.ln_warps = so.ln_warps
     return call
 
 
@@ -72,6 +74,14 @@ def test_shapes_within_the_estimates_error_stay(shape, rows):
     """XL's up projection at 144 to 160 rows: the shape that the estimate has 5 % ahead makes a pass up to 3 % longer."""
     s, g = shape(rows, 1600, 6400), shape.general(rows, 1600, 6400)
     assert s["split"] == g["split"] == 0 and s["KS"] == g["KS"]
+
+
+def test_warps_of_a_narrow_row(shape):
+    """Rows that one warp holds in a float4 a lane: past 1024 of them more warps make a pass up to 4 % longer."""
+    for N in (32, 64, 128):
+        assert [shape.ln_warps(rows, N) for rows in (1, 1024, 1025, 4096)] == [4, 4, 1, 1]
+    for N in (132, 384, 768, 1600, 2048):
+        assert [shape.ln_warps(rows, N) for rows in (1, 1536, 1537, 4096, 4097)] == [4, 4, 2, 2, 1]
 
 
 @pytest.mark.parametrize("E,n,up,down", TRUNCATIONS)

@@ -902,16 +902,13 @@ static int32_t launch_gemm_nk(wgpt_device *dev, const float *A, size_t lda, cons
   return launch_gemm_tc(dev, dev->precision == WGPT_PRECISION_TF32X3, A, lda, Wt, M, K, N, epi, ln, true, handoff);
 }
 
-// Rows of up to 2048 values stay in registers (V float4 per lane, W warps a row, see layernorm_kernel). One warp a row is a long chain
-// on few warps: up to 1536 rows four share one, up to 4096 two; beyond that every SM has warps enough and the barriers cost more.
-// us per pass with 1 / 2 / 4 warps a row: GPT-2 70 / 333 / 1024 tokens 559 / 544 / 538, 789 / 772 / 763, 1374 / 1354 / 1347, 16 / 32 / 64
-// sequences of 128 1749 / 1728 / 1736, 2912 / 2869 / 2897, 5269 / 5281 / 5306; XL 70 / 200 / 512 / 1024 tokens 3173 / 3034 / 2896, 4855 /
-// 4714 / 4570, 6866 / 6768 / 6712, 10989 / 10932 / 10877; 384-wide, 70 tokens 233 / 233 / 228. FP32 rows out keep one warp a row: what
-// follows the operator converts weights beside it, on the SMs that it leaves (pass list of 128 tokens 1048 / - / 1068).
+// Rows of up to 2048 values stay in registers (V float4 per lane, W warps a row, see layernorm_kernel). FP32 rows out keep one warp a
+// row: what follows the operator converts weights beside it, on the SMs that it leaves (pass list of 128 tokens 1048 us, with four
+// warps 1068).
 static int32_t launch_layernorm(wgpt_device *dev, const float *in, size_t ld_in, const float *gamma, const float *beta,
                                 float *out, size_t ld_out, int rows, int N, __half *planes = nullptr, size_t plane = 0,
                                 float scale = 1.f) {
-  const int w = planes == nullptr ? 1 : rows <= 1536 ? 4 : rows <= 4096 ? 2 : 1;
+  const int w = planes == nullptr ? 1 : layernorm_warps(rows, N);
 #define LN_CASE(V, W)                                                                                                       \
   LAUNCH_PDL(dev, (layernorm_kernel<V, W>), (rows * W + 3) / 4, 128, 0, in, ld_in, gamma, beta, out, ld_out, rows, N, planes, plane, scale)
   if (w == 4 && N <= 512) LN_CASE(1, 4);

@@ -1,11 +1,26 @@
 // Launch shapes of the products of pairs: gemm_pair_kernel's tile width and CTA pairs per tile (gemm_pair.cuh), and which
-// products gemm_split_kernel takes (gemm_split.cuh). Plain C++, so that the routes can be followed on the host.
+// products gemm_split_kernel takes (gemm_split.cuh); and of the LayerNorm ahead of them. Plain C++, so that the routes can be
+// followed on the host.
 #pragma once
 #include <cmath>
 
 #include "split_plan.h"
 
 namespace wgpt {
+
+// Warps that share a row of a LayerNorm whose result leaves as pairs (layernorm_kernel). One warp a row is a long chain on few warps:
+// up to 1536 rows four share one, up to 4096 two; beyond that every SM has warps enough and the barriers cost more. Rows of up to 128
+// values are one float4 a lane of one warp: the other three have nothing to do, and that a CTA holds one row in place of four, so that
+// few rows spread over more SMs, stops paying at 1024 rows.
+// us per pass, 1 / 2 / 4 warps: GPT-2 70 / 333 tokens 559 / 544 / 538, 789 / 772 / 763, 16 / 32 / 64 sequences of 128 1749 / 1728 / 1736, 2912 / 2869 /
+// 2897, 5269 / 5281 / 5306. One warp / this rule: n_embd 1600, 48 layers, 129 / 200 / 333 / 513 / 1024 tokens 4460 / 4089, 4774 / 4502, 5919 / 5696,
+// 7869 / 7706, 11271 / 11022 (power cap: runs of one side differ by 1.4 %); 384, 6 layers, 100 / 576 / 1536 / 4096 rows 244 / 240, 427 / 425, 452 / 438,
+// 690 / 688; 256, 12 layers, 100 / 1600 / 4096 412 / 407, 768 / 740, 975 / 981; 128, 12 layers, 150 / 512 / 1024 414 / 407, 573 / 555, 623 / 612, and were
+// 3200 / 4096 rows 696 / 707, 728 / 739 with two warps; 64, 1200 / 2048 / 4096 rows 563 / 569, 576 / 587, 612 / 623 with four, two and two.
+inline int layernorm_warps(int rows, int N) {
+  if (N <= 128) return rows <= 1024 ? 4 : 1;
+  return rows <= 1536 ? 4 : rows <= 4096 ? 2 : 1;
+}
 
 struct PairShape {
   int bn, KS;  // tile columns, CTA pairs that share a tile's K
