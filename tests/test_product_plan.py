@@ -19,6 +19,7 @@ extern "C" void shape(const int *clusters, long long smem, int M, int K, int N, 
   for (int i = 0; i < 8; i++) out[i] = v[i];
 }
 extern "C" int ln_warps(int rows, int N) { return layernorm_warps(rows, N); }
+extern "C" int streams(int M, int K, int N) { return stream_fits(148, M, K, N); }
 extern "C" void general(const int *clusters, long long smem, int M, int K, int N, int *out) {  // the route of other callers
   const SplitLimits lim{clusters, (size_t)smem};
   SplitShape sh;
@@ -50,7 +51,7 @@ def shape(tmp_path_factory):
         return dict(zip(("split", "S", "KS"), out))
 
     call.general = general
-    call.ln_warps = so.ln_warps
+    call.ln_warps, call.streams = so.ln_warps, so.streams
     return call
 
 
@@ -74,6 +75,14 @@ def test_shapes_within_the_estimates_error_stay(shape, rows):
     """XL's up projection at 144 to 160 rows: the shape that the estimate has 5 % ahead makes a pass up to 3 % longer."""
     s, g = shape(rows, 1600, 6400), shape.general(rows, 1600, 6400)
     assert s["split"] == g["split"] == 0 and s["KS"] == g["KS"]
+
+
+def test_deembeddings_that_stream(shape):
+    """Two pieces of 32 features an SM: at exactly that, one full round of the pair kernel, a long K stays with it (1 to 2 %)."""
+    for M in (6, 128):
+        for K in (768, 2048, 3072, 4096):
+            assert [shape.streams(M, K, N) for N in (9471, 9472, 9473, 50257)] == [0, K <= 2048, 1, 1]
+    assert [shape.streams(M, 512, 65) for M in (6, 96, 97)] == [1, 1, 0] and not shape.streams(129, 64, 50257)
 
 
 def test_warps_of_a_narrow_row(shape):

@@ -994,17 +994,6 @@ static int32_t launch_gemm_pair(wgpt_device *dev, const __half *A, const __half 
   return WGPT_OK;
 }
 
-// Where gemm_stream_kernel is faster than gemm_pair_kernel, whose 256-row tile is mostly padding here: from two pieces of features
-// for every SM on, or where K is so short that the pair kernel's start and its epilogue are most of it. us per decode pass of one
-// block, pair / stream: n_embd 768, vocabulary 50257, 6 / 16 / 64 / 128 rows 92 / 67, 111 / 70, 172 / 98, 196 / 124; 9472, 6 / 64 / 128
-// rows 50.6 / 45.3, 75.8 / 73.5, 100 / 97; 4104, 6 / 128 rows 46.2 / 42.5, 94.6 / 94.3; 1000, 64 rows 64.8 / 67.0. n_embd 1600, 9472, 6 / 64 /
-// 128 rows 85.7 / 76.5, 118 / 115, 152 / 150; 4104, 64 rows 107 / 111. n_embd 384, 6 / 64 / 96 / 128 rows, vocabulary 65 37.6 / 35.0, 62.4 /
-// 54.6, 65.3 / 59.1, 74.8 / 69.5; 300 39.1 / 35.1, 58.1 / 54.9, 62.3 / 59.7, 70.5 / 71.2. n_embd 512 and 640, vocabulary 1000, 64 rows 61.7 /
-// 59.4, 65.6 / 63.4, 96 rows 65.4 / 64.8, 69.5 / 69.7.
-static bool stream_fits(const wgpt_device *dev, int M, int K, int N) {
-  return M <= GT_MAX_ROWS && (N >= 2 * GT_PIECE * dev->sm_count || (K <= 512 && M <= 96));
-}
-
 // out[M, N] = X . Wt^T from pair planes X [2][M][K] and W [2][N][K], the exponents in colscale [N].
 static int32_t launch_gemm_stream(wgpt_device *dev, const __half *X, const __half *W, int M, int K, int N, const float *colscale,
                                   float *out) {
@@ -2883,7 +2872,7 @@ static int32_t forward(wgpt_session *s, const uint32_t *ids, int n_tok, bool pic
     const size_t plane = (size_t)s->n_seq * E;
     TRY(launch_layernorm(dev, x_last, ld_last, m->lnf_g, m->lnf_b, nullptr, (size_t)E, s->n_seq, E, h, plane, m->s_hf));
     e.colscale = m->wte_p.cs;
-    if (stream_fits(dev, s->n_seq, E, p.vocab_size))
+    if (stream_fits(dev->sm_count, s->n_seq, E, p.vocab_size))
       TRY(launch_gemm_stream(dev, h, m->wte_p.p, s->n_seq, E, p.vocab_size, m->wte_p.cs, s->logits));
     else
       TRY(launch_gemm_pair(dev, h, m->wte_p.p, s->n_seq, E, p.vocab_size, e));

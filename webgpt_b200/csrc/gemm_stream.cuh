@@ -16,17 +16,16 @@
 //
 // What bounds it: HBM. A decode pass of GPT-2 with 8 / 64 sequences 362 -> 335 / 636 -> 561 us against gemm_pair_kernel (cold 54 and
 // 107 us there, 33 and 35 here: 256 rows of the pair's tile are multiplied and read back whatever the batch is), XL with 16 sequences 2.56 -> 2.52 ms. See
-// stream_fits in api.cu for where it takes over.
+// stream_fits in pair_plan.h for where it takes over.
 // Every wait is bounded; on expiry *err = 3, the copies in flight get another bounded wait, and the result is void.
 #pragma once
 #include "gemm_split.cuh"
+#include "pair_plan.h"
 
 namespace wgpt {
 
 constexpr int GT_THREADS = 192;      // warp 0 TMA, warp 1 MMA, warps 2-5 accumulator read-back and store
 constexpr int GT_MAX_STAGES = 6;
-constexpr int GT_MAX_ROWS = 128;
-constexpr int GT_PIECE = 32;         // features per copy of a run's last tile, and the granularity of the runs
 
 struct StreamArgs {
   int M, K, N, rn, stages;

@@ -22,6 +22,22 @@ inline int layernorm_warps(int rows, int N) {
   return rows <= 1536 ? 4 : rows <= 4096 ? 2 : 1;
 }
 
+// Where gemm_stream_kernel (gemm_stream.cuh) takes a product of few rows from gemm_pair_kernel, whose 256-row tile is mostly padding
+// there: from two pieces of features for every SM on, or where K is so short that the pair kernel's start and its epilogue are most of it.
+// At exactly two pieces (9472 on 148 SMs) the pair kernel's tiles are one full round, which a long K makes the better one. us per decode
+// pass of one block, pair / stream: n_embd 768, vocabulary 50257, 6 / 16 / 64 / 128 rows 92 / 67, 111 / 70, 172 / 98, 196 / 124; 4104, 6 / 128 rows 46.2 /
+// 42.5, 94.6 / 94.3; 1000, 64 rows 64.8 / 67.0. n_embd 1600, 4104, 64 rows 107 / 111. Vocabulary 9472, 6 / 64 / 128 rows, n_embd 1024 57.1 / 52.1, 95.6 /
+// 91.4, 133 / 129; 2048 97.1 / 90.0, 147 / 145, 184 / 184; 3072 164 / 157, 228 / 229, 291 / 294; 4096 240 / 229, 325 / 330, 393 / 400, 33 rows 275 / 281; one
+// feature more, 3072 168 / 159, 250 / 231, 314 / 296; 4096 247 / 231, 349 / 332, 416 / 400. n_embd 384, 64 / 96 rows, vocabulary 65 82.4 / 73.8, 95.8 / 88.0; 2000 69.4 /
+// 66.1, 79.0 / 76.8; 9400 75.6 / 70.9, 87.4 / 83.8. n_embd 512, 64 / 80 / 96 rows, 1000 70.8 / 67.9, 73.9 / 73.7, 80.1 / 79.9; 4104 74.9 / 72.2, 80.1 / 79.1, 87.3 /
+// 86.2; 4700 75.0 / 72.3, 79.8 / 79.3, 87.8 / 88.2; 9400 78.2 / 73.8, 82.9 / 80.1, 90.2 / 88.4. 640, 1000, 64 / 96 rows 65.6 / 63.4, 69.5 / 69.7.
+constexpr int GT_MAX_ROWS = 128;
+constexpr int GT_PIECE = 32;  // features per copy of a run's last tile, and the granularity of the runs
+inline bool stream_fits(int sms, int M, int K, int N) {
+  const int two = 2 * GT_PIECE * sms;
+  return M <= GT_MAX_ROWS && (N > two || (N == two && K <= 2048) || (K <= 512 && M <= 96));
+}
+
 struct PairShape {
   int bn, KS;  // tile columns, CTA pairs that share a tile's K
 };
