@@ -59,7 +59,7 @@ def test_product_of_pairs_error_bound(dev, M, K, N):
 
 
 K_OVER_TWO_PAIRS = [(700, 1608, 1608), (900, 1160, 1304), (250, 1160, 3080), (700, 1544, 1608), (512, 3080, 2312)]
-WIDTH_OVER_TWO_PAIRS = (1216, (238, 250, 256))  # n_embd and tokens: q | k | v and the up projection
+WIDTH_OVER_TWO_PAIRS = [("up", 1216, (238, 250, 256)), ("qkv", 1600, (238, 250, 256))]  # the product, n_embd and tokens
 
 
 @pytest.mark.parametrize("M,K,N", K_OVER_TWO_PAIRS)
@@ -69,13 +69,12 @@ def test_product_of_pairs_with_k_over_two_pairs(dev, M, K, N):
     test_product_of_pairs_error_bound(dev, M, K, N)
 
 
-@pytest.mark.parametrize("n", WIDTH_OVER_TWO_PAIRS[1])
-def test_model_products_with_k_over_two_pairs(oracle, n):
+@pytest.mark.parametrize("E,n", [(E, n) for _, E, tokens in WIDTH_OVER_TWO_PAIRS for n in tokens])
+def test_model_products_with_k_over_two_pairs(oracle, E, n):
     """K over two pairs with what a model's products do at their end: q, k and v as pairs and into the cache, GELU and pairs. The
     logits behind the prompt, and of two more tokens over the cache it left; bound as in test_prompt_lengths."""
     from webgpt_b200 import GPT
     from webgpt_b200.model import Session
-    E = WIDTH_OVER_TWO_PAIRS[0]
     p = dict(n_layer=1, n_head=E // 64, n_embd=E, n_ctx=260, vocab_size=512)
     w = synth.make_weights(p, seed=61, std=0.04, ln_random=True)
     gpt, m = GPT(None, params=p, weights=w), oracle.Model(p, synth.weight_list(p, w))

@@ -14,18 +14,15 @@ DRIVER = r"""
 #include "pair_plan.h"
 using namespace wgpt;
 extern "C" void shape(const int *clusters, long long smem, int M, int K, int N, long long *out) {
-  const ProductShape s = product_shape(SplitLimits{clusters, (size_t)smem}, 74, M, N, K);
+  const ProductShape s = product_shape(SplitLimits{clusters, (size_t)smem}, 74, M, N, K, N % 4 == 0, 2, true);
   const long long v[] = {s.split, s.pair.bn, s.pair.KS, s.sh.row_tiles, s.sh.rn, s.sh.S, s.sh.stages, (long long)s.sh.smem};
   for (int i = 0; i < 8; i++) out[i] = v[i];
 }
 extern "C" int ln_warps(int rows, int N) { return layernorm_warps(rows, N); }
 extern "C" int streams(int M, int K, int N) { return stream_fits(148, M, K, N); }
 extern "C" void general(const int *clusters, long long smem, int M, int K, int N, int *out) {  // the route of other callers
-  const SplitLimits lim{clusters, (size_t)smem};
-  SplitShape sh;
-  out[0] = pair_product_splits(lim, 74, M, K, N, 2, &sh);
-  out[1] = sh.S;
-  out[2] = pair_shape(lim, 74, M, N, K).KS;
+  const ProductShape s = product_shape(SplitLimits{clusters, (size_t)smem}, 74, M, N, K, N % 4 == 0, 2, false);
+  out[0] = s.split, out[1] = s.sh.S, out[2] = s.pair.KS;
 }
 """
 B200 = (0, 148, 74, 45, 33, 26, 22, 15, 15)

@@ -1142,29 +1142,19 @@ static int32_t launch_pair_operands(wgpt_device *dev, PairOperands &p) {
 // Reference-layout products that can go this way: TMA strides, and a column strip that fits shared memory.
 static bool pair_operands_fit(int K) { return K % 8 == 0 && K <= 8 * 1536; }
 
-// A product of pairs with whichever kernel should be faster: CTA pairs on 256-row tiles, or 128-feature tiles with K split
-// over a cluster where the former would leave most pairs without a tile (GPT-2 at 333 rows: 0.98 against 1.24 ms per pass). A
-// model's prompts go by product_shape, operators and exact codes, which it was not fitted to, by pair_product_splits.
+// A product of pairs with whichever kernel and shape should be faster (product_shape): CTA pairs on 256-row tiles, or 128-feature
+// tiles with K split over a cluster where the former would leave most pairs without a tile. dyn: an operator, whose weights come from
+// the kernel before; b_exact: weights that are exact in one plane.
 static int32_t launch_pair_product(wgpt_device *dev, const __half *X, const __half *W, int M, int K, int N,
                                    const Epilogue &epi, bool dyn = false, bool b_exact = false) {
-  if (!dyn && !b_exact && epi.rowscale == nullptr && M <= kFittedRows && (epi.ld & 3) == 0) {
-    const ProductShape ps = product_shape(split_limits(dev), dev->sm_count / 2, M, N, K);
-    if (!ps.split) return launch_gemm_pair(dev, X, W, M, K, N, epi, false, &ps.pair);
-    SplitArgs a;
-    memset(&a, 0, sizeof a);
-    a.w_planes = 2;
-    return launch_gemm_split(dev, ps.sh, X, W, M, K, N, epi, a);
-  }
-  SplitShape sh;
-  if (pair_product_splits(split_limits(dev), dev->sm_count / 2, M, K, N, b_exact ? 1 : 2, &sh) && N % 4 == 0 &&
-      (epi.ld & 3) == 0) {
-    SplitArgs a;
-    memset(&a, 0, sizeof a);
-    a.dyn = dyn ? 1 : 0;
-    a.w_planes = b_exact ? 1 : 2;
-    return launch_gemm_split(dev, sh, X, W, M, K, N, epi, a);
-  }
-  return launch_gemm_pair(dev, X, W, M, K, N, epi, b_exact);
+  SplitArgs a;
+  memset(&a, 0, sizeof a);
+  a.dyn = dyn ? 1 : 0;
+  a.w_planes = b_exact ? 1 : 2;
+  const ProductShape ps = product_shape(split_limits(dev), dev->sm_count / 2, M, N, K, N % 4 == 0 && (epi.ld & 3) == 0, a.w_planes,
+                                        !dyn && epi.rowscale == nullptr);
+  if (ps.split) return launch_gemm_split(dev, ps.sh, X, W, M, K, N, epi, a);
+  return launch_gemm_pair(dev, X, W, M, K, N, epi, b_exact, &ps.pair);
 }
 
 // Pieces of the workspace, each 256-byte aligned; first pass (base == nullptr) counts.

@@ -66,8 +66,8 @@ inline int pair_tile_columns(int pairs, int M, int N, int K = 0, double *cycles 
 
 // The same with K split over clusters of two pairs where that is shorter: a tile each, half the k-blocks, and for the exchange
 // 4000 cycles and 12 per column; the last epilogue, 70 cycles a column, is shared too. Of GPT-2's and XL's products it is q | k | v
-// of XL at 145 to 256 rows, XL's down projection from 641 on and its output projection to 768 (33 clusters of four). us per pass
-// without / with: XL 145 / 175 / 200 tokens 4818 / 4658, 4985 / 4822, 4961 / 4918, but 210 / 235 / 255 4860 / 4927, 4920 / 5026,
+// of XL at 145 to 256 rows, XL's down projection from 641 on and its output projection to 768 (33 clusters of four); product_shape
+// leaves those as they are in prompts. us per pass without / with, when this alone chose: XL 145 / 175 / 200 tokens 4818 / 4658, 4985 / 4822, 4961 / 4918, but 210 / 235 / 255 4860 / 4927, 4920 / 5026,
 // 4858 / 4983; 645 / 700 / 765 9194 / 8816, 9398 / 9017, 9699 / 9307; 800 to 1024 the same. Sums of half as many steps: logits of
 // three XL layers at 200 / 700 / 1024 tokens 7.4e-6 / 1.59e-5 / 1.64e-5 from float64, 1.20e-5 / 2.13e-5 / 2.18e-5 without. Six
 // layers of other widths: n_embd 1216 and 1408 at 180 to 256 rows 1 to 2.5 % faster, 1344 to 1856 at 600 to 768 1 to 3, 2432 at 400
@@ -90,7 +90,7 @@ inline PairShape pair_shape(const SplitLimits &lim, int pairs, int M, int N, int
 
 // Whether gemm_split_kernel should be the faster one, by the estimates of both; *sh: its shape. The form without the K split
 // stands for gemm_pair_kernel here: with the better estimate plus 10 000 cycles XL at 200 tokens took 4949 -> 4730 us, but 333
-// 6085 -> 6514 and GPT-2 512 969 -> 1004.
+// 6085 -> 6514 and GPT-2 512 969 -> 1004 (prompts that went by this alone then).
 inline bool pair_product_splits(const SplitLimits &lim, int pairs, int M, int K, int N, int w_planes, SplitShape *sh) {
   double big = 0, split = 0;
   pair_tile_columns(pairs, M, N, K, &big);
@@ -127,8 +127,10 @@ inline double product_cycles(const SplitLimits &lim, int pairs, int M, int N, in
                         : (double)((kb + 1) / 2) * per_kb + 8050 + 51.0 * bn;
 }
 
-// The kernel and shape of a prompt's product in a model: the cheapest of all shapes of both kernels by product_cycles, if that has it
-// ahead of the shape of the estimates above by 3 % with the same kernel or by 6 % with the other, and if it truncates no more often.
+// The kernel and shape of a product of pairs. split_ok: rows that gemm_split_kernel can store (N and the row stride multiples of four
+// floats). Operators, exact codes (w_planes 1) and more than kFittedRows rows, to none of which product_cycles was fitted: by the
+// estimates above. A prompt's product in a model: the cheapest of all shapes of both kernels by product_cycles, if that has it ahead of
+// the former by 3 % with the same kernel or by 6 % with the other, and if it truncates no more often.
 //
 // The margins: within a kernel the estimate orders shapes well, between the two it errs by up to a tenth. With 3 % for both XL at 144 to 160
 // rows takes its up projection in CTAs without a cluster, 4173 -> 4221 and 4235 -> 4378 us a pass; with 6 % for both XL loses 2 % at 257 to 512.
@@ -152,11 +154,12 @@ inline double product_cycles(const SplitLimits &lim, int pairs, int M, int N, in
 // Of 108 prompts only 1280 x 385 is slower by more than two runs of one side differ (1.2 %, 416 rows 1.4 % faster). Not beyond 1024 rows,
 // which were not fitted.
 constexpr int kFittedRows = 1024;
-inline ProductShape product_shape(const SplitLimits &lim, int pairs, int M, int N, int K) {
+inline ProductShape product_shape(const SplitLimits &lim, int pairs, int M, int N, int K, bool split_ok, int w_planes, bool prompt) {
   const int kb = (K + GS_BK - 1) / GS_BK, rt0 = (M + 127) / 128;
   ProductShape best = {}, t = {};
-  best.split = pair_product_splits(lim, pairs, M, K, N, 2, &best.sh) && N % 4 == 0;
+  best.split = pair_product_splits(lim, pairs, M, K, N, w_planes, &best.sh) && split_ok;
   if (!best.split) best.pair = pair_shape(lim, pairs, M, N, K);
+  if (!prompt || w_planes != 2 || M > kFittedRows) return best;
   const int most = product_truncations(best, K);
   const bool general = best.split;
   double least = product_cycles(lim, pairs, M, N, K, best);
@@ -171,7 +174,7 @@ inline ProductShape product_shape(const SplitLimits &lim, int pairs, int M, int 
       }
     }
   }
-  if (N % 4 != 0) return best;
+  if (!split_ok) return best;
   t.split = true;
   for (int rt = rt0; rt <= rt0 + 2; rt++) {
     t.sh = {};
