@@ -8,8 +8,9 @@
 //
 // What bounds it: the tensor pipe, 6 BN cycles per k-block and pair; shared memory (operand reads of the MMAs, 4 KB + 16
 // BN bytes each, plus the copies coming in) needs 640 + 2.5 BN cycles at 128 bytes a cycle, so a tile of fewer than
-// about 180 columns is bound by shared memory instead. BN is a run-time multiple of 32 chosen by the host so that
-// rounds x max(6 BN, 640 + 2.5 BN) is smallest (pair_plan.h): products of a few tiles per pair would
+// about 180 columns is bound by shared memory instead. BN is a run-time multiple of 32 chosen by the host (pair_plan.h) so that
+// rounds x max(6 BN, 640 + 2.5 BN) is smallest, in a model's prompts of up to 1024 rows by product_cycles, which knows the epilogue
+// too: products of a few tiles per pair would
 // otherwise leave a nearly empty last round (8192 x 768: 96 tiles of 256 columns on 74 pairs take two rounds, 128 of
 // 192 columns take two shorter ones). 8192 x 8192 x 8192 runs at 470 TFLOP/s = 1410 issued, the rate a plain
 // half-precision product sustains under the power cap.

@@ -6,17 +6,21 @@
 // a time), the rows the instruction's N, and two accumulators alternate, so that a tile is stored while the next one is
 // multiplied. Rows cost what they are (RN = M rounded up to 16), in tensor-core time and in stored bytes alike.
 //
-//   weights     : tiles of {64 of K, 128 features} per plane; a run's last tile in pieces of 32 features, so that nothing is
-//                 read that no feature of the run needs; the ring's first tiles ahead of the dependency wait;
+//   weights     : tiles of {64 of K, 128 features} per plane; a run's last tile in pieces of 32 features, so that at most 31
+//                 rows are read that no feature of the run needs (past N: the second plane's first, or zeros; lanes that are never
+//                 stored); the ring's first tiles ahead of the dependency wait;
 //   activations : {64 of K, RN rows, 2 planes} by TMA with every weight tile, out of L2;
 //   products    : as in gemm_split_kernel: the weights' first plane with both planes of the rows (2 RN columns), the second
 //                 with the first, so that the large and the small sums have accumulators of their own;
 //   store       : a lane is a feature, so a warp stores 32 neighbouring values of a row (128 bytes; a row of 50257 floats is
 //                 aligned to four bytes only).
 //
-// What bounds it: HBM. A decode pass of GPT-2 with 8 / 64 sequences 362 -> 335 / 636 -> 561 us against gemm_pair_kernel (cold 54 and
-// 107 us there, 33 and 35 here: 256 rows of the pair's tile are multiplied and read back whatever the batch is), XL with 16 sequences 2.56 -> 2.52 ms. See
-// stream_fits in pair_plan.h for where it takes over.
+// What bounds it: HBM in a decode step, where the first tiles arrive beside the kernel before: one more launch of it costs GPT-2's step of
+// 8 / 16 / 64 / 128 sequences 27.6 / 27.6 / 28.5 / 35.7 us for 154 MB, 0.85 of the copy rate up to 64 (some of it perhaps out of L2, behind a launch
+// that has just read the same). Cold and alone 33 us at 8 rows and 35 at 64, 0.7 of it, the rest start and the ring's latency; the
+// tensor pipe is busy for 6 and 22 % of that. A step with 8 / 64 sequences 362 -> 335 / 636 -> 561 us against gemm_pair_kernel (cold 54 and 107 us:
+// 256 rows of the pair's tile are multiplied and read back whatever the batch is), XL with 16 2.56 -> 2.52 ms. See stream_fits in
+// pair_plan.h for where it takes over.
 // Every wait is bounded; on expiry *err = 3, the copies in flight get another bounded wait, and the result is void.
 #pragma once
 #include "gemm_split.cuh"

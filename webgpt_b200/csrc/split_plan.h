@@ -67,7 +67,8 @@ inline SplitShape split_shape_decode(const SplitLimits &lim, int M, int K, int N
 
 // Any number of rows, activations as planes: row tiles of up to 128 and K slices by the same kind of estimate
 // (pair_plan.h): a k-block costs max(6 RN tensor-core cycles, 32 KB + 256 RN bytes from L2 at 40 a cycle), a round
-// 9000 cycles of start, exchange and store and 60 more per row of the tile.
+// 9000 cycles of start, exchange and store and 60 more per row of the tile. A model's prompts of up to 1024 rows depart from it where
+// product_shape has another shape well ahead.
 inline SplitShape split_shape_rows(const SplitLimits &lim, int M, int K, int N, int w_planes, double *cycles) {
   SplitShape best = {};
   const int ft = (N + 127) / 128, kb = (K + GS_BK - 1) / GS_BK, rt0 = (M + 127) / 128;
